@@ -81,14 +81,67 @@ __device__ __forceinline__ void load_pos(const Problem& p, int64_t n, float (&po
     for (int i = 0; i < D; ++i) pos[i] = __ldg(src + i * p.pos_stride_d);
 }
 
-// unsigned modulo by the capacity (EncodingGPU.cuh:34-36); a mask when it is a power of two
+// Hash modulo the capacity (EncodingGPU.cuh:34-36): a mask when it is a power of two, else an exact
+// remainder by multiplication with the host-computed 2^64 / capacity (Lemire, Kaser, Kurz 2019).
+__device__ __forceinline__ uint32_t to_slot(const Problem& p, uint32_t h) {
+    if (p.cap_is_pow2) return h & (p.capacity - 1u);
+    return (uint32_t)__umul64hi(p.cap_magic * h, (uint64_t)p.capacity);
+}
 __device__ __forceinline__ void to_slots(const Problem& p, const Simplex<D>& s, uint32_t (&slot)[D + 1]) {
-    if (p.cap_is_pow2) {
+    uint32_t h[D + 1];
+    vertex_hashes<D>(s, h);
 #pragma unroll
-        for (int r = 0; r <= D; ++r) slot[r] = s.hash[r] & (p.capacity - 1u);
-    } else {
+    for (int q = 0; q <= D; ++q) slot[q] = to_slot(p, h[q]);
+}
+
+// Vertices of the walk (q = 0..D) renumbered by the reference's remainder r = q - s modulo D+1, under
+// which a lattice point keeps its number in every simplex it belongs to.
+template <class T>
+__device__ __forceinline__ void to_remainders(int s, T (&v)[D + 1]) {
+    constexpr bool kPow2 = ((D + 1) & D) == 0;
+    const int by = kPow2 ? (s & D) : (s < 0 ? s + D + 1 : s);
 #pragma unroll
-        for (int r = 0; r <= D; ++r) slot[r] = s.hash[r] % p.capacity;
+    for (int bit = 1; bit <= D; bit <<= 1) {
+        T t[D + 1];
+#pragma unroll
+        for (int r = 0; r <= D; ++r) t[r] = (by & bit) ? v[(r + bit) % (D + 1)] : v[r];
+#pragma unroll
+        for (int r = 0; r <= D; ++r) v[r] = t[r];
+    }
+}
+
+// ---- level constants in shared memory ---------------------------------------------------------
+// A level's weight, shift and scale are 2D+1 floats that every thread of a block reads: staged once
+// per block they cost a point one or two 16-byte shared loads per level instead of 2D+1 global ones
+// (7 of the 11 load instructions of a level at pos_dim 3).
+constexpr int kRecord = (2 * D + 1 + 3) / 4 * 4;
+constexpr int kStage = 32;  // levels staged at a time
+
+__device__ __forceinline__ void stage_levels(const Problem& p, int begin, int end, float* table) {
+    for (int i = threadIdx.x; i < (end - begin) * kRecord; i += blockDim.x) {
+        const int l = begin + i / kRecord, c = i % kRecord;
+        float v = 0.f;
+        if (c == 0) v = __ldg(p.anneal + l);
+        else if (c <= D) v = __ldg(p.shift + l * D + c - 1);
+        else if (c <= 2 * D) v = __ldg(p.scale + l * D + c - 1 - D);
+        table[i] = v;
+    }
+}
+__device__ __forceinline__ void load_level(const float* table, int i, LevelConst<D>& lc) {
+    float v[kRecord];
+#pragma unroll
+    for (int j = 0; j < kRecord / 4; ++j) {
+        const float4 t = reinterpret_cast<const float4*>(table + i * kRecord)[j];
+        v[4 * j] = t.x;
+        v[4 * j + 1] = t.y;
+        v[4 * j + 2] = t.z;
+        v[4 * j + 3] = t.w;
+    }
+    lc.weight = v[0];
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+        lc.shift[j] = v[1 + j];
+        lc.scale[j] = v[1 + D + j];
     }
 }
 
@@ -241,7 +294,7 @@ __device__ __forceinline__ void store_row_segment(const Problem& p, float* rows,
 // One step of a point's feature row: LPS levels of F features (8 floats) starting at level l0;
 // levels at or beyond `end` give zeros (EncodingGPU.cuh:130-254 for one level).
 template <int F, int LPS, bool HALF>
-__device__ __forceinline__ void encode_step(const Problem& p, const float (&pos)[D], int l0, int end,
+__device__ __forceinline__ void encode_step(const Problem& p, const float* levels, const float (&pos)[D], int l0, int end,
                                             float (&out)[F * LPS]) {
 #pragma unroll
     for (int k = 0; k < LPS; ++k) {
@@ -250,20 +303,22 @@ __device__ __forceinline__ void encode_step(const Problem& p, const float (&pos)
 #pragma unroll
         for (int f = 0; f < F; ++f) acc[f] = 0.f;
         if (l < end) {  // uniform over the block
-            const float w_lvl = __ldg(p.anneal + l);
-            if (w_lvl != 0.0f) {  // a closed coarse-to-fine window contributes exact zeros
+            LevelConst<D> lc;
+            load_level(levels, k, lc);
+            if (lc.weight != 0.0f) {  // a closed coarse-to-fine window contributes exact zeros
                 Simplex<D> s;
-                locate_simplex<D>(pos, p.shift + l * D, p.scale + l * D, s);
+                locate_simplex<D>(pos, lc, s);
                 uint32_t slot[D + 1];
                 to_slots(p, s, slot);
                 float v[D + 1][F];
 #pragma unroll
-                for (int r = 0; r <= D; ++r) gather<F, HALF>(p.table, l, p.capacity, slot[r], v[r]);
+                for (int q = 0; q <= D; ++q) gather<F, HALF>(p.table, l, p.capacity, slot[q], v[q]);
+                float w[D + 1];
+                vertex_weights<D>(s, lc.weight * (1.0f / (D + 1)), w);  // EncodingGPU.cuh:234
 #pragma unroll
-                for (int r = 0; r <= D; ++r) {
-                    const float w = s.bary[r] * w_lvl;  // EncodingGPU.cuh:234
+                for (int q = 0; q <= D; ++q) {
 #pragma unroll
-                    for (int f = 0; f < F; ++f) acc[f] = fmaf(v[r][f], w, acc[f]);
+                    for (int f = 0; f < F; ++f) acc[f] = fmaf(v[q][f], w[q], acc[f]);
                 }
             }
         }
@@ -275,8 +330,10 @@ __device__ __forceinline__ void encode_step(const Problem& p, const float (&pos)
 template <int F, int LPS, bool HALF>
 __global__ void __launch_bounds__(kThreads, (F == 2 ? PERMUTO_MIN_BLOCKS_FORWARD : min_blocks(F, false))) forward_kernel(const ForwardArgs a) {
     const Problem& p = a.p;
-    const int64_t n = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (n >= p.n_points) return;
+    __shared__ __align__(16) float levels[kStage * kRecord];
+    const int64_t n_raw = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const bool active = n_raw < p.n_points;
+    const int64_t n = active ? n_raw : p.n_points - 1;  // idle threads shadow the last point
     const int pass_begin = p.level_begin + (int)blockIdx.y * p.levels_per_pass;
     const int pass_end = min(pass_begin + p.levels_per_pass, p.level_end);
 
@@ -284,14 +341,21 @@ __global__ void __launch_bounds__(kThreads, (F == 2 ? PERMUTO_MIN_BLOCKS_FORWARD
     load_pos(p, n, pos);
 
 #pragma unroll 1
-    for (int l0 = pass_begin; l0 < pass_end; l0 += LPS) {
-        float out[F * LPS];
-        encode_step<F, LPS, HALF>(p, pos, l0, pass_end, out);
-        store_row_segment<F, LPS>(p, a.features, n, l0, out);
+    for (int begin = pass_begin; begin < pass_end; begin += kStage) {
+        const int end = min(begin + kStage, pass_end);
+        if (begin != pass_begin) __syncthreads();
+        stage_levels(p, begin, end, levels);
+        __syncthreads();
+#pragma unroll 1
+        for (int l0 = begin; l0 < end; l0 += LPS) {
+            float out[F * LPS];
+            encode_step<F, LPS, HALF>(p, levels + (l0 - begin) * kRecord, pos, l0, end, out);
+            if (active) store_row_segment<F, LPS>(p, a.features, n, l0, out);
+        }
     }
 
     // raw points appended after the lattice levels (EncodingGPU.cuh:105-121)
-    if (p.extra_levels > 0 && blockIdx.y == 0 && p.level_begin == 0) {
+    if (active && p.extra_levels > 0 && blockIdx.y == 0 && p.level_begin == 0) {
         float* dst = a.features + n * p.width + F * p.nr_levels;
         for (int c = 0; c < F * p.extra_levels; ++c) {
             float v = 0.f;
@@ -520,6 +584,8 @@ forward_mlp_kernel(const ForwardLinearArgs a) {
     // shared memory: the slice ring, then the weight of every layer that runs on the tensor core
     unsigned char* tile_w = smem_raw + kRing * kSliceBytes;
     const int chunks0 = a.k_pad / 4;
+    float* levels = reinterpret_cast<float*>(smem_raw + a.levels_offset);  // behind the weights
+    stage_levels(p, 0, p.nr_levels, levels);
     stage_weight(tile_w, a.layer[0].weight, H0, p.width, chunks0);
     if (HMAX > 0) {
         unsigned char* next = tile_w + (size_t)H0 * a.k_pad * 4;
@@ -569,7 +635,7 @@ forward_mlp_kernel(const ForwardLinearArgs a) {
             float out[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) out[i] = 0.f;
-            if (s < nsteps) encode_step<F, LPS, HALF>(p, pos, s * LPS, p.nr_levels, out);
+            if (s < nsteps) encode_step<F, LPS, HALF>(p, levels + s * LPS * kRecord, pos, s * LPS, p.nr_levels, out);
             if (8 * s + 8 > lattice_cols) {  // block-uniform: only the last step(s) reach past the lattice levels
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -786,14 +852,23 @@ __device__ __forceinline__ void merge_from(const Scatter& sc, float* level_base,
     }
 }
 
+// adds w[q] * g[f] to entry slot[q] of the level for every vertex q; `s` renumbers the vertices by remainder
 template <int F>
-__device__ __forceinline__ void scatter_level(Scatter& sc, float* level_base, const uint32_t (&slot)[D + 1],
-                                              float (&add)[D + 1][F]) {
+__device__ __forceinline__ void scatter_level(Scatter& sc, float* level_base, int s, uint32_t (&slot)[D + 1],
+                                              float (&w)[D + 1], const float (&g)[F]) {
+    float add[D + 1][F];
     if (sc.probe) {
+        to_remainders(s, slot);
         const unsigned lane = sc.lane;
         const unsigned group0 = __match_any_sync(kFullMask, sc.active ? slot[0] : 0xffffffffu - lane);
         const int distinct = __popc(__ballot_sync(kFullMask, (group0 & ((1u << lane) - 1u)) == 0u));
+        to_remainders(s, w);
         if (distinct <= kMergeBelow) {
+#pragma unroll
+            for (int r = 0; r <= D; ++r) {
+#pragma unroll
+                for (int f = 0; f < F; ++f) add[r][f] = w[r] * g[f];
+            }
             merge_from<F, 0>(sc, level_base, slot, add, group0);
             return;
         }
@@ -801,7 +876,11 @@ __device__ __forceinline__ void scatter_level(Scatter& sc, float* level_base, co
     }
     if (sc.active) {
 #pragma unroll
-        for (int r = 0; r <= D; ++r) red_add<F>(level_base, slot[r], add[r]);
+        for (int r = 0; r <= D; ++r) {
+#pragma unroll
+            for (int f = 0; f < F; ++f) add[r][f] = w[r] * g[f];
+            red_add<F>(level_base, slot[r], add[r]);
+        }
     }
 }
 
@@ -812,6 +891,7 @@ template <int F, int LPS, bool TABLE, bool POS, bool HALF>
 __global__ void __launch_bounds__(kThreads, min_blocks(F, !TABLE))
 backward_kernel(const BackwardArgs a) {
     const Problem& p = a.p;
+    __shared__ __align__(16) float levels[kStage * kRecord];
     const int64_t n_raw = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const bool active = n_raw < p.n_points;
     const int64_t n = active ? n_raw : p.n_points - 1;  // idle lanes shadow the last point
@@ -828,81 +908,75 @@ backward_kernel(const BackwardArgs a) {
     for (int i = 0; i < D; ++i) dpos[i] = 0.f;
     Scatter sc{lane, active, a.aggregate != 0};
 
-    // steps of the pass are walked cyclically from a block-dependent start (see PERMUTO_STAGGER)
-    const int nsteps = (pass_end - pass_begin + LPS - 1) / LPS;
-    int step = (TABLE && kStagger) ? (int)(blockIdx.x % (unsigned)nsteps) : 0;
-
-    // the next step's 32 bytes of the gradient row are requested before this step is worked on
-    float g_next[F * LPS];
-    load_row_segment<F, LPS>(p, a.grad_features, n, pass_begin + step * LPS, g_next);
 #pragma unroll 1
-    for (int it = 0; it < nsteps; ++it) {
-        const int l0 = pass_begin + step * LPS;
-        step = (step + 1 == nsteps) ? 0 : step + 1;
-        if (TABLE && l0 == pass_begin) sc.probe = a.aggregate != 0;
-        float g[F * LPS];
+    for (int begin = pass_begin; begin < pass_end; begin += kStage) {
+        const int end = min(begin + kStage, pass_end);
+        // steps are walked cyclically from a block-dependent start (see PERMUTO_STAGGER)
+        const int nsteps = (end - begin + LPS - 1) / LPS;
+        int step = (TABLE && kStagger) ? (int)(blockIdx.x % (unsigned)nsteps) : 0;
+        // the next step's 32 bytes of the gradient row are requested before this step is worked on
+        float g_next[F * LPS];
+        load_row_segment<F, LPS>(p, a.grad_features, n, begin + step * LPS, g_next);
+        if (begin != pass_begin) __syncthreads();
+        stage_levels(p, begin, end, levels);
+        __syncthreads();
+#pragma unroll 1
+        for (int it = 0; it < nsteps; ++it) {
+            const int l0 = begin + step * LPS;
+            step = (step + 1 == nsteps) ? 0 : step + 1;
+            if (TABLE && l0 == begin) sc.probe = a.aggregate != 0;
+            float g[F * LPS];
 #pragma unroll
-        for (int i = 0; i < F * LPS; ++i) g[i] = g_next[i];
-        if (it + 1 < nsteps) load_row_segment<F, LPS>(p, a.grad_features, n, pass_begin + step * LPS, g_next);
+            for (int i = 0; i < F * LPS; ++i) g[i] = g_next[i];
+            if (it + 1 < nsteps) load_row_segment<F, LPS>(p, a.grad_features, n, begin + step * LPS, g_next);
 #pragma unroll
-        for (int k = 0; k < LPS; ++k) {
-            const int l = l0 + k;
-            if (l >= pass_end) continue;  // uniform
-            const float w_lvl = __ldg(p.anneal + l);
-            if (w_lvl == 0.0f) continue;  // every addend of this level is an exact zero
-            Simplex<D> s;
-            locate_simplex<D>(pos, p.shift + l * D, p.scale + l * D, s);
-            uint32_t slot[D + 1];
-            to_slots(p, s, slot);
+            for (int k = 0; k < LPS; ++k) {
+                const int l = l0 + k;
+                if (l >= end) continue;  // uniform
+                LevelConst<D> lc;
+                load_level(levels, l - begin, lc);
+                if (lc.weight == 0.0f) continue;  // every addend of this level is an exact zero
+                Simplex<D> s;
+                locate_simplex<D>(pos, lc, s);
+                uint32_t slot[D + 1];
+                to_slots(p, s, slot);
 
-            if (POS) {
-                // EncodingGPU.cuh:671-749
-                float gs[F];  // upstream gradient with the level weight and 1/(d+1) folded in
+                if (POS) {
+                    // EncodingGPU.cuh:671-749
+                    float gs[F];  // upstream gradient with the level weight and 1/(d+1) folded in
 #pragma unroll
-                for (int f = 0; f < F; ++f) gs[f] = g[F * k + f] * w_lvl * kInv;
-                float dBs[D + 2];
+                    for (int f = 0; f < F; ++f) gs[f] = g[F * k + f] * lc.weight * kInv;
+                    float dBs[D + 2];
 #pragma unroll
-                for (int r = 0; r <= D; ++r) {
-                    float v[F];
-                    gather<F, HALF>(p.table, l, p.capacity, slot[r], v);
-                    float t = v[0] * gs[0];
+                    for (int q = 0; q <= D; ++q) {
+                        float v[F];
+                        gather<F, HALF>(p.table, l, p.capacity, slot[q], v);
+                        float t = v[0] * gs[0];
 #pragma unroll
-                    for (int f = 1; f < F; ++f) t = fmaf(v[f], gs[f], t);
-                    dBs[r] = t;
+                        for (int f = 1; f < F; ++f) t = fmaf(v[f], gs[f], t);
+                        dBs[q] = t;
+                    }
+                    dBs[D + 1] = dBs[0];
+                    float dE[D + 1];  // of the coordinate whose rank is k, then by coordinate
+#pragma unroll
+                    for (int kk = 0; kk <= D; ++kk) dE[kk] = dBs[D - kk] - dBs[D + 1 - kk];
+                    to_coordinates(s, dE);
+                    float run = 0.f;
+#pragma unroll
+                    for (int i = 0; i < D; ++i) {
+                        run += dE[i];
+                        dpos[i] += lc.scale[i] * (run - (float)(i + 1) * dE[i + 1]);
+                    }
                 }
-                dBs[D + 1] = dBs[0];
-                float T[D + 1];  // dE of the coordinate whose rank is k
-#pragma unroll
-                for (int kk = 0; kk <= D; ++kk) T[kk] = dBs[D - kk] - dBs[D + 1 - kk];
-                float dE[D + 1];
-#pragma unroll
-                for (int i = 0; i <= D; ++i) {
-                    float v = 0.f;
-#pragma unroll
-                    for (int kk = 0; kk <= D; ++kk) v = (s.rank[i] == kk) ? T[kk] : v;
-                    dE[i] = v;
-                }
-                float run = 0.f;
-#pragma unroll
-                for (int i = 0; i < D; ++i) {
-                    run += dE[i];
-                    const float sc = __ldg(p.scale + l * D + i);
-                    dpos[i] += sc * (run - (float)(i + 1) * dE[i + 1]);
-                }
-            }
 
-            if (TABLE) {
-                float* gbase = a.lattice_grad + (size_t)l * p.capacity * F;
-                float gw[F];  // EncodingGPU.cuh:405-410
+                if (TABLE) {
+                    float* gbase = a.lattice_grad + (size_t)l * p.capacity * F;
+                    float gk[F], w[D + 1];
 #pragma unroll
-                for (int f = 0; f < F; ++f) gw[f] = g[F * k + f] * w_lvl;
-                float add[D + 1][F];
-#pragma unroll
-                for (int r = 0; r <= D; ++r) {
-#pragma unroll
-                    for (int f = 0; f < F; ++f) add[r][f] = s.bary[r] * gw[f];
+                    for (int f = 0; f < F; ++f) gk[f] = g[F * k + f];
+                    vertex_weights<D>(s, lc.weight * kInv, w);  // EncodingGPU.cuh:405-410
+                    scatter_level<F>(sc, gbase, s.s, slot, w, gk);
                 }
-                scatter_level<F>(sc, gbase, slot, add);
             }
         }
     }
@@ -927,6 +1001,7 @@ backward_kernel(const BackwardArgs a) {
 template <int F, int LPS, bool TABLE, bool GGF, bool HALF>
 __global__ void __launch_bounds__(kThreads, min_blocks(F, false)) double_backward_kernel(const DoubleBackwardArgs a) {
     const Problem& p = a.p;
+    __shared__ __align__(16) float levels[kStage * kRecord];
     const int64_t n_raw = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const bool active = n_raw < p.n_points;
     const int64_t n = active ? n_raw : p.n_points - 1;
@@ -940,89 +1015,89 @@ __global__ void __launch_bounds__(kThreads, min_blocks(F, false)) double_backwar
 #pragma unroll
     for (int i = 0; i < D; ++i) dpg[i] = __ldg(a.double_positions_grad + n * D + i);
     Scatter sc{lane, active, a.aggregate != 0};  // as in backward_kernel
-    const int nsteps = (pass_end - pass_begin + LPS - 1) / LPS;
-    int step = (TABLE && kStagger) ? (int)(blockIdx.x % (unsigned)nsteps) : 0;
 
-    float g_next[F * LPS];  // as in backward_kernel: the next step's gradient segment is requested early
-    if (TABLE) load_row_segment<F, LPS>(p, a.grad_features, n, pass_begin + step * LPS, g_next);
 #pragma unroll 1
-    for (int it = 0; it < nsteps; ++it) {
-        const int l0 = pass_begin + step * LPS;
-        step = (step + 1 == nsteps) ? 0 : step + 1;
-        if (TABLE && l0 == pass_begin) sc.probe = a.aggregate != 0;
-        float g[F * LPS];
-        if (TABLE) {
+    for (int begin = pass_begin; begin < pass_end; begin += kStage) {
+        const int end = min(begin + kStage, pass_end);
+        const int nsteps = (end - begin + LPS - 1) / LPS;
+        int step = (TABLE && kStagger) ? (int)(blockIdx.x % (unsigned)nsteps) : 0;
+        float g_next[F * LPS];  // as in backward_kernel: the next step's gradient segment is requested early
+        if (TABLE) load_row_segment<F, LPS>(p, a.grad_features, n, begin + step * LPS, g_next);
+        if (begin != pass_begin) __syncthreads();
+        stage_levels(p, begin, end, levels);
+        __syncthreads();
+#pragma unroll 1
+        for (int it = 0; it < nsteps; ++it) {
+            const int l0 = begin + step * LPS;
+            step = (step + 1 == nsteps) ? 0 : step + 1;
+            if (TABLE && l0 == begin) sc.probe = a.aggregate != 0;
+            float g[F * LPS];
+            if (TABLE) {
 #pragma unroll
-            for (int i = 0; i < F * LPS; ++i) g[i] = g_next[i];
-            if (it + 1 < nsteps) load_row_segment<F, LPS>(p, a.grad_features, n, pass_begin + step * LPS, g_next);
-        }
-        float out[F * LPS];
+                for (int i = 0; i < F * LPS; ++i) g[i] = g_next[i];
+                if (it + 1 < nsteps) load_row_segment<F, LPS>(p, a.grad_features, n, begin + step * LPS, g_next);
+            }
+            float out[F * LPS];
 #pragma unroll
-        for (int k = 0; k < LPS; ++k) {
-            const int l = l0 + k;
-            float o[F];
+            for (int k = 0; k < LPS; ++k) {
+                const int l = l0 + k;
+                float o[F];
 #pragma unroll
-            for (int f = 0; f < F; ++f) o[f] = 0.f;
-            if (l < pass_end) {
-                const float w_lvl = __ldg(p.anneal + l);
-                if (w_lvl != 0.0f) {
-                    Simplex<D> s;
-                    locate_simplex<D>(pos, p.shift + l * D, p.scale + l * D, s);
-                    uint32_t slot[D + 1];
-                    to_slots(p, s, slot);
+                for (int f = 0; f < F; ++f) o[f] = 0.f;
+                if (l < end) {
+                    LevelConst<D> lc;
+                    load_level(levels, l - begin, lc);
+                    if (lc.weight != 0.0f) {
+                        Simplex<D> s;
+                        locate_simplex<D>(pos, lc, s);
+                        uint32_t slot[D + 1];
+                        to_slots(p, s, slot);
 
-                    // d loss / d elevated (EncodingGPU.cuh:1187-1199)
-                    float gsd[D], dE[D + 1];
+                        // d loss / d elevated (EncodingGPU.cuh:1187-1199)
+                        float gsd[D], dE[D + 1];
 #pragma unroll
-                    for (int i = 0; i < D; ++i) gsd[i] = dpg[i] * __ldg(p.scale + l * D + i);
+                        for (int i = 0; i < D; ++i) gsd[i] = dpg[i] * lc.scale[i];
 #pragma unroll
-                    for (int j = 0; j <= D; ++j) dE[j] = 0.f;
+                        for (int j = 0; j <= D; ++j) dE[j] = 0.f;
 #pragma unroll
-                    for (int i = 0; i < D; ++i) {
+                        for (int i = 0; i < D; ++i) {
 #pragma unroll
-                        for (int j = 0; j <= i; ++j) dE[j] += gsd[i];
-                    }
+                            for (int j = 0; j <= i; ++j) dE[j] += gsd[i];
+                        }
 #pragma unroll
-                    for (int i = 0; i < D; ++i) dE[i + 1] -= gsd[i] * (float)(i + 1);
-                    // d loss / d barycentric (EncodingGPU.cuh:1213-1218), via the rank-sorted vector
-                    float sdE[D + 1];
+                        for (int i = 0; i < D; ++i) dE[i + 1] -= gsd[i] * (float)(i + 1);
+                        // d loss / d barycentric (EncodingGPU.cuh:1213-1218): the gaps of dE in rank order
 #pragma unroll
-                    for (int kk = 0; kk <= D; ++kk) {
-                        float v = 0.f;
+                        for (int i = 0; i <= D; ++i) dE[i] *= kInv;
+                        to_ranks(s, dE);
+                        float dBw[D + 1];  // dB * level weight
 #pragma unroll
-                        for (int i = 0; i <= D; ++i) v = (s.rank[i] == kk) ? dE[i] * kInv : v;
-                        sdE[kk] = v;
-                    }
-                    float dBw[D + 1];  // dB * level weight
-#pragma unroll
-                    for (int m = 1; m <= D; ++m) dBw[m] = (sdE[D - m] - sdE[D + 1 - m]) * w_lvl;
-                    dBw[0] = (sdE[D] - sdE[0]) * w_lvl;
+                        for (int m = 1; m <= D; ++m) dBw[m] = (dE[D - m] - dE[D + 1 - m]) * lc.weight;
+                        dBw[0] = (dE[D] - dE[0]) * lc.weight;
 
-                    if (GGF) {
+                        if (GGF) {
 #pragma unroll
-                        for (int r = 0; r <= D; ++r) {
-                            float v[F];
-                            gather<F, HALF>(p.table, l, p.capacity, slot[r], v);  // EncodingGPU.cuh:1484-1485
+                            for (int q = 0; q <= D; ++q) {
+                                float v[F];
+                                gather<F, HALF>(p.table, l, p.capacity, slot[q], v);  // EncodingGPU.cuh:1484-1485
 #pragma unroll
-                            for (int f = 0; f < F; ++f) o[f] = fmaf(dBw[r], v[f], o[f]);
+                                for (int f = 0; f < F; ++f) o[f] = fmaf(dBw[q], v[f], o[f]);
+                            }
                         }
-                    }
-                    if (TABLE) {
-                        float* gbase = a.lattice_grad + (size_t)l * p.capacity * F;
-                        float add[D + 1][F];
+                        if (TABLE) {  // EncodingGPU.cuh:1244-1245
+                            float* gbase = a.lattice_grad + (size_t)l * p.capacity * F;
+                            float gk[F];
 #pragma unroll
-                        for (int r = 0; r <= D; ++r) {
-#pragma unroll
-                            for (int f = 0; f < F; ++f) add[r][f] = dBw[r] * g[F * k + f];  // EncodingGPU.cuh:1244-1245
+                            for (int f = 0; f < F; ++f) gk[f] = g[F * k + f];
+                            scatter_level<F>(sc, gbase, s.s, slot, dBw, gk);
                         }
-                        scatter_level<F>(sc, gbase, slot, add);
                     }
                 }
-            }
 #pragma unroll
-            for (int f = 0; f < F; ++f) out[F * k + f] = o[f];
+                for (int f = 0; f < F; ++f) out[F * k + f] = o[f];
+            }
+            if (GGF && active) store_row_segment<F, LPS>(p, a.grad_grad_features, n, l0, out);
         }
-        if (GGF && active) store_row_segment<F, LPS>(p, a.grad_grad_features, n, l0, out);
     }
     if (GGF && active && p.extra_levels > 0 && blockIdx.y == 0 && p.level_begin == 0) {  // EncodingGPU.cuh:1290-1295
         float* dst = a.grad_grad_features + n * p.width + F * p.nr_levels;
@@ -1040,22 +1115,40 @@ __global__ void __launch_bounds__(kThreads) debug_kernel(const DebugArgs a) {
     const int l = blockIdx.y;
     float pos[D];
     load_pos(p, n, pos);
+    LevelConst<D> lc;
+    lc.weight = 1.0f;
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+        lc.shift[i] = __ldg(p.shift + l * D + i);
+        lc.scale[i] = __ldg(p.scale + l * D + i);
+    }
     Simplex<D> s;
-    locate_simplex<D>(pos, p.shift + l * D, p.scale + l * D, s);
+    locate_simplex<D>(pos, lc, s);
     uint32_t slot[D + 1];
     to_slots(p, s, slot);
+    float w[D + 1];
+    vertex_weights<D>(s, 1.0f / (D + 1), w);
+    to_remainders(s.s, slot);
+    to_remainders(s.s, w);
+    int k[D + 1];  // rank of every coordinate before the wrap
+#pragma unroll
+    for (int i = 0; i <= D; ++i) k[i] = i;
+    to_coordinates(s, k);
     const int64_t base = (n * p.nr_levels + l) * (D + 1);
+    int q = s.s < 0 ? s.s + D + 1 : s.s;  // vertex of remainder 0
 #pragma unroll
     for (int r = 0; r <= D; ++r) {
         if (a.keys) {
-            int key[D];
-            vertex_key<D>(s, r, key);
 #pragma unroll
-            for (int i = 0; i < D; ++i) a.keys[(base + r) * D + i] = key[i];
+            for (int i = 0; i < D; ++i) a.keys[(base + r) * D + i] = s.lift[i] + q - (k[i] > D - q ? D + 1 : 0);
         }
         if (a.slots) a.slots[base + r] = (int32_t)slot[r];
-        if (a.bary) a.bary[base + r] = s.bary[r];
-        if (a.rank) a.rank[base + r] = s.rank[r];
+        if (a.bary) a.bary[base + r] = w[r];
+        if (a.rank) {
+            const int wrapped = k[r] + s.s;
+            a.rank[base + r] = wrapped < 0 ? wrapped + D + 1 : (wrapped > D ? wrapped - (D + 1) : wrapped);
+        }
+        q = q == D ? 0 : q + 1;
     }
 }
 
@@ -1145,13 +1238,16 @@ cudaError_t launch_forward(const ForwardArgs& a, cudaStream_t st) {
 }
 
 template <int F, int LPS>
-cudaError_t launch_forward_linear(const ForwardLinearArgs& a, cudaStream_t st) {
+cudaError_t launch_forward_linear(const ForwardLinearArgs& in, cudaStream_t st) {
+    ForwardLinearArgs a = in;
     size_t smem = (size_t)kRing * kSliceBytes + (size_t)a.layer[0].out_features * a.k_pad * sizeof(float);
     int hmax = 0;  // widest hidden layer
     for (int i = 1; i < a.nr_layers; ++i) {
         if (a.layer[i].in_features > hmax) hmax = a.layer[i].in_features;
         if (a.layer[i].out_features % 16 == 0) smem += (size_t)a.layer[i].out_features * a.layer[i].in_features * sizeof(float);
     }
+    a.levels_offset = (int32_t)smem;
+    smem += (size_t)a.p.nr_levels * kRecord * sizeof(float);
     const dim3 g((unsigned)((a.p.n_points + kTileRows - 1) / kTileRows));
     auto launch = [&](auto kernel) -> cudaError_t {
         if (smem + 1024 > 48 * 1024) {  // the kernel's few static shared words count against the default limit

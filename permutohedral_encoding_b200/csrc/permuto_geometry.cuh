@@ -4,11 +4,7 @@
 // Behaviour follows kernels/permutohedral_encoding/EncodingGPU.cuh:130-223 and :22-45 of the
 // reference (paths relative to its project root): the integer results (remainder-0 point,
 // ranks, keys, slots) are bit-identical to it; the barycentric weights agree to fp32 rounding
-// (about 1e-7 absolute) but not bit for bit, because nvcc contracts the reference's
-// `b[..] += (e - rem0) * inv` into fused multiply-adds in its own way.  The code is
-// organised differently: ranks are turned into a "sorted residual" vector with selects so
-// that nothing is indexed dynamically (no local memory), and the d+1 hashes are derived from
-// one base hash because the hash is linear over Z/2^32.
+// (about 1e-7 absolute) but not bit for bit.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -24,54 +20,128 @@ __host__ __device__ constexpr uint32_t hash_pow(int e) {
     return r;
 }
 
+// sum of the hash powers of the d key coordinates: what adding 1 to every coordinate adds to the hash
 template <int D>
-struct Simplex {
-    int rem0[D + 1];    // remainder-0 lattice point after the rank wrap (multiples of D+1)
-    int rank[D + 1];    // permutation of 0..D
-    float bary[D + 1];  // barycentric weight of the vertex with remainder r
-    uint32_t hash[D + 1];  // hash of the vertex with remainder r, before the modulo
-};
-
-// -1 if a < b else 0, in one instruction
-__device__ __forceinline__ int minus_one_if_less(float a, float b) {
-    int d;
-    asm("set.lt.s32.f32 %0, %1, %2;" : "=r"(d) : "f"(a), "f"(b));
-    return d;
+__host__ __device__ constexpr uint32_t hash_all() {
+    uint32_t r = 0u;
+    for (int i = 0; i < D; ++i) r += hash_pow(D - i);
+    return r;
 }
 
-// pos: D floats.  shift, scale: this level's rows.  Rounding of every operation of the elevate
-// step is explicit, because simplex selection at fine levels hinges on single ulps of the
-// elevated coordinates (they reach 1e5..1e6).  The sequence below is what nvcc's default
-// -fmad=true makes of the reference source (.cuh:130-138), established by comparing against the
-// reference's own outputs for every pos_dim (cf_i = t_i*scale_i, t_i = pos_i + shift_i):
+// Hash step of coordinate i: walking from vertex q-1 to vertex q of the simplex adds 1 to every
+// coordinate and takes D+1 off one of them, and the hash is linear over Z/2^32.
+template <int D>
+__host__ __device__ constexpr uint32_t hash_step(int i) {
+    return hash_all<D>() - (i < D ? (uint32_t)(D + 1) * hash_pow(D - i) : 0u);
+}
+
+// One level's constants.  Kernels keep the records of the levels of a sweep in shared memory
+// (kRecord floats each, moved as 16-byte vectors): weight, then shift and scale of coordinate 0, 1, ...
+template <int D>
+struct LevelConst {
+    float weight;
+    float shift[D];
+    float scale[D];
+};
+
+// The simplex around a point, its vertices numbered q = 0..D along the walk that leaves the
+// *unwrapped* nearest remainder-0 point:
+//     key_q[i] = R_i - s + q - (D+1) * [k_i > D - q],   s = sum(R) / (D+1)
+// with k_i the descending rank of coordinate i's residual.  The reference first shifts the ranks by
+// s, wraps them back into 0..D and corrects R accordingly (.cuh:177-186); that only renumbers the
+// same D+1 vertices cyclically (its remainder r is q - s modulo D+1), so nothing that sums over the
+// vertices needs the wrap, and the weight of vertex q is the gap between neighbouring residuals
+// whichever way they are numbered.
+template <int D>
+struct Simplex {
+    float x[D + 1];     // residuals e - R in descending order (units of the elevated space)
+    uint32_t step[D + 1];  // hash steps in the same order
+    uint32_t hash0;     // hash of vertex 0, before the modulo
+    int s;              // sum(R) / (D+1); only computed where it is used
+    int lift[D + 1];    // R_i - s (debug view)
+    bool swapped[(D + 1) * D / 2];  // outcome of every comparator of the sorting network
+};
+
+// Adjacent comparators of an odd-even transposition network (D+1 stages, (D+1)D/2 comparators).
+// Only neighbours are exchanged and only on strict inequality, so equal residuals keep their order:
+// a tie raises the later index's rank, as .cuh:166-173 has it.
+template <int D, class F>
+__device__ __forceinline__ void for_each_comparator(F&& f) {
+    int c = 0;
+#pragma unroll
+    for (int stage = 0; stage <= D; ++stage) {
+#pragma unroll
+        for (int i = stage & 1; i < D; i += 2) f(c++, i);
+    }
+}
+template <int D, class F>
+__device__ __forceinline__ void for_each_comparator_reversed(F&& f) {
+    int c = (D + 1) * D / 2;
+#pragma unroll
+    for (int stage = D; stage >= 0; --stage) {
+#pragma unroll
+        for (int i = D - 1; i >= 0; --i)
+            if ((i & 1) == (stage & 1)) f(--c, i);
+    }
+}
+
+// order by rank -> order by coordinate (runs the network backwards)
+template <int D, class T>
+__device__ __forceinline__ void to_coordinates(const Simplex<D>& s, T (&v)[D + 1]) {
+    for_each_comparator_reversed<D>([&](int c, int i) {
+        const T a = v[i], b = v[i + 1];
+        v[i] = s.swapped[c] ? b : a;
+        v[i + 1] = s.swapped[c] ? a : b;
+    });
+}
+// order by coordinate -> order by rank
+template <int D, class T>
+__device__ __forceinline__ void to_ranks(const Simplex<D>& s, T (&v)[D + 1]) {
+    for_each_comparator<D>([&](int c, int i) {
+        const T a = v[i], b = v[i + 1];
+        v[i] = s.swapped[c] ? b : a;
+        v[i + 1] = s.swapped[c] ? a : b;
+    });
+}
+
+// Rounding of every operation of the elevate step is explicit, because simplex selection at fine
+// levels hinges on single ulps of the elevated coordinates (they reach 1e5..1e6).  The sequence
+// below is what nvcc's default -fmad=true makes of the reference source (.cuh:130-138), established
+// by comparing against the reference's own outputs for every pos_dim (cf_i = t_i*scale_i,
+// t_i = pos_i + shift_i):
 //   i = D      : e[D] = -(D*cf_D), sm = cf_D
 //   2 <= i < D : e[i] = fma(-i, cf_i, sm), sm = sm + cf_i       (cf_i rounded, it feeds i*cf_i)
 //   i = 1      : e[1] = fma(-t_1, scale_1, sm), e[0] = fma(t_1, scale_1, sm)
 //
-// Everything after the elevate step produces the reference's integers (.cuh:146-223) with far
-// fewer instructions than a transcription would:
-//  * ceil(v)*(D+1) is floor(v)*(D+1) + (D+1) unless v is an integer, in which case the
-//    reference's choice is the lower multiple whatever the comparison says; both products are
-//    exact while |e| < 2^22, and a rarely taken branch keeps the reference's own formula above;
-//  * ranks come from one set.lt per pair and three-input adds; the wrap of rank and rem0 is a
-//    mask when D+1 is a power of two;
-//  * barycentric weights and vertex hashes are read off the rank-sorted residuals / hash powers
-//    (selected with compares, never indexed dynamically): every b[m], m >= 1, receives exactly
-//    one +delta and one -delta in the reference (.cuh:193-199), so it equals one rounded
-//    difference whatever the visiting order, and the hash is linear over Z/2^32:
-//    h(r) = h(0) + r*S - (D+1) * sum_{i<D} [rank_i > D-r] M^(D-i)  (.cuh:24-31, :216-220).
+// Nearest remainder-0 point.  The reference takes the closer of floor(e/(D+1))*(D+1) and
+// ceil(e/(D+1))*(D+1), the lower one on a tie (.cuh:150-161): r = ceil((e - (D+1)/2) / (D+1)).
+// Below 2^22 this comes out of the float adder without a conversion instruction (conversions and
+// floor run at a quarter of the rate of an add or less): adding 1.5*2^23 leaves the integer in the
+// low mantissa bits, read as an integer for the hash and, after subtracting it again, as a float.
+//  * D+1 a power of two: both additions round upwards, so rounding never crosses a multiple of D+1
+//    from above (the multiple itself is representable) and the ceiling is exact.
+//  * otherwise the reciprocal is inexact: round to nearest, then move by one where the residual is
+//    outside (-(D+1)/2, (D+1)/2].
+// The residual e - (D+1)*r is exact in both cases (r*(D+1) <= 2|e| or r = 0), which is the
+// reference's -(up - e) or e - down.  From 2^22 on the reference's own expressions are used.
+//
+// Instructions per point and level, pos_dim 3: about 110 against 245 for a version with floor,
+// rank counting, rank wrap and select-by-rank.
 template <int D>
-__device__ __forceinline__ void locate_simplex(const float (&pos)[D], const float* __restrict__ shift,
-                                               const float* __restrict__ scale, Simplex<D>& s) {
+__device__ __forceinline__ void locate_simplex(const float (&pos)[D], const LevelConst<D>& lc, Simplex<D>& s) {
     constexpr float kInv = 1.0f / (D + 1);
     constexpr float kDp1 = (float)(D + 1);
+    constexpr float kHalf = 0.5f * (D + 1);
     constexpr bool kPow2 = ((D + 1) & D) == 0;
+    constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
+    constexpr int kMagicBits = 0x4B400000;
+
     float e[D + 1];
     float sm = 0.0f;
 #pragma unroll
     for (int i = D; i > 0; --i) {
-        const float t = __fadd_rn(pos[i - 1], __ldg(shift + i - 1));
-        const float sc = __ldg(scale + i - 1);
+        const float t = __fadd_rn(pos[i - 1], lc.shift[i - 1]);
+        const float sc = lc.scale[i - 1];
         if (i == 1) {
             e[1] = __fmaf_rn(-t, sc, sm);
             sm = __fmaf_rn(t, sc, sm);
@@ -88,98 +158,94 @@ __device__ __forceinline__ void locate_simplex(const float (&pos)[D], const floa
     }
     e[0] = sm;
 
-    // nearest remainder-0 point, ties towards the lower multiple (.cuh:150-161)
-    float v[D + 1], down[D + 1], up[D + 1];
     float biggest = 0.0f;
 #pragma unroll
-    for (int i = 0; i <= D; ++i) {
-        v[i] = __fmul_rn(e[i], kInv);
-        down[i] = floorf(v[i]) * kDp1;
-        up[i] = (v[i] != floorf(v[i])) ? down[i] + kDp1 : down[i];
-        biggest = fmaxf(biggest, fabsf(e[i]));
-    }
-    if (biggest >= 4194304.0f) {  // products no longer exact: the reference's own expression
-#pragma unroll
-        for (int i = 0; i <= D; ++i) up[i] = ceilf(v[i]) * kDp1;
-    }
-    float rem0f[D + 1], res[D + 1];
-    float sumf = 0.0f;
-#pragma unroll
-    for (int i = 0; i <= D; ++i) {
-        const float du = __fsub_rn(up[i], e[i]);
-        const float dd = __fsub_rn(e[i], down[i]);
-        const bool take_up = du < dd;
-        rem0f[i] = take_up ? up[i] : down[i];
-        res[i] = take_up ? -du : dd;  // == e - rem0 with one rounding, as .cuh:167-169
-        sumf += rem0f[i];
-    }
-    const int sum = __float2int_rn(sumf * kInv);  // exact: every rem0 is a multiple of D+1
+    for (int i = 0; i <= D; ++i) biggest = fmaxf(biggest, fabsf(e[i]));
 
-    // rank of each residual; a tie raises the later index (.cuh:166-173):
-    // rank_i = i + sum_{j<i} c_ji - sum_{j>i} c_ij with c_ab = -[res_a < res_b]
-    int rk[D + 1];
+    float res[D + 1];
+    int rint[D + 1];  // R_i / (D+1)
+    if (biggest < 4194304.0f) {
+        uint32_t h = 0u;
+        int sum = 0;
 #pragma unroll
-    for (int i = 0; i <= D; ++i) rk[i] = i + sum;
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-#pragma unroll
-        for (int j = i + 1; j <= D; ++j) {
-            const int c = minus_one_if_less(res[i], res[j]);
-            rk[i] -= c;
-            rk[j] += c;
+        for (int i = 0; i <= D; ++i) {
+            float w, r;
+            if (kPow2) {
+                w = __fmaf_ru(__fadd_ru(e[i], -kHalf), kInv, kMagic);
+                r = __fsub_rn(w, kMagic);
+                res[i] = __fmaf_rn(-kDp1, r, e[i]);
+            } else {
+                w = __fmaf_rn(e[i], kInv, kMagic);
+                r = __fsub_rn(w, kMagic);
+                res[i] = __fmaf_rn(-kDp1, r, e[i]);
+                const float fix = (res[i] > kHalf ? 1.0f : 0.0f) - (res[i] <= -kHalf ? 1.0f : 0.0f);
+                w = __fadd_rn(w, fix);
+                res[i] = __fmaf_rn(-kDp1, fix, res[i]);
+            }
+            const int bits = __float_as_int(w);
+            rint[i] = bits - kMagicBits;
+            sum += rint[i];
+            // hash of the vertex-0 key R_i - s over the D hashed coordinates, with R_i = (D+1)*rint_i
+            // and s = sum(rint); the D+1 steps add up to zero, so the bias of `bits` drops out
+            h -= (uint32_t)bits * hash_step<D>(i);
         }
+        s.hash0 = h;
+        s.s = sum;
+#pragma unroll
+        for (int i = 0; i <= D; ++i) s.lift[i] = (D + 1) * rint[i] - sum;
+    } else {
+        // coordinates beyond the exact range of the adder trick: the reference's expressions (.cuh:150-161, :176)
+        float rem0f[D + 1], sumf = 0.0f;
+#pragma unroll
+        for (int i = 0; i <= D; ++i) {
+            const float v = __fmul_rn(e[i], kInv);
+            const float down = __fmul_rn(floorf(v), kDp1), up = __fmul_rn(ceilf(v), kDp1);
+            const float du = __fsub_rn(up, e[i]), dd = __fsub_rn(e[i], down);
+            rem0f[i] = du < dd ? up : down;
+            res[i] = du < dd ? -du : dd;
+            sumf = __fadd_rn(sumf, rem0f[i]);
+        }
+        s.s = __float2int_rn(__fmul_rn(sumf, kInv));
+        uint32_t h = 0u;
+#pragma unroll
+        for (int i = 0; i <= D; ++i) {
+            s.lift[i] = (int)rem0f[i] - s.s;
+            if (i < D) h += (uint32_t)s.lift[i] * hash_pow(D - i);
+        }
+        s.hash0 = h;
     }
-    // bring the point back onto the plane (.cuh:177-186)
-    float delta[D + 1];
+
 #pragma unroll
     for (int i = 0; i <= D; ++i) {
-        const int r = rk[i];
-        const float off = (r < 0) ? kDp1 : ((r > D) ? -kDp1 : 0.0f);
-        rk[i] = kPow2 ? (r & D) : ((r < 0) ? r + D + 1 : ((r > D) ? r - (D + 1) : r));
-        rem0f[i] += off;
-        s.rank[i] = rk[i];
-        s.rem0[i] = (int)rem0f[i];
-        delta[i] = __fmul_rn(__fsub_rn(e[i], rem0f[i]), kInv);  // .cuh:194
+        s.x[i] = res[i];
+        s.step[i] = hash_step<D>(i);
     }
-    // sorted[k] = delta of the coordinate whose rank is k; pw[k] = its hash power (0 for i = D)
-    float sorted[D + 1];
-    uint32_t pw[D + 1];
-#pragma unroll
-    for (int k = 0; k <= D; ++k) {
-        float dv = delta[D];
-        uint32_t pv = 0u;
-#pragma unroll
-        for (int i = D - 1; i >= 0; --i) {
-            const bool is = rk[i] == k;
-            dv = is ? delta[i] : dv;
-            pv = is ? hash_pow(D - i) : pv;
-        }
-        sorted[k] = dv;
-        pw[k] = pv;
-    }
-#pragma unroll
-    for (int m = 1; m <= D; ++m) s.bary[m] = __fsub_rn(sorted[D - m], sorted[D + 1 - m]);
-    s.bary[0] = __fadd_rn(sorted[D], __fsub_rn(1.0f, sorted[0]));
-
-    uint32_t base = 0u, all = 0u;
-#pragma unroll
-    for (int i = 0; i < D; ++i) {
-        base += (uint32_t)s.rem0[i] * hash_pow(D - i);
-        all += hash_pow(D - i);
-    }
-    uint32_t lowered = 0u;  // hash powers of the coordinates already lowered by D+1
-    s.hash[0] = base;
-#pragma unroll
-    for (int r = 1; r <= D; ++r) {
-        lowered += pw[D + 1 - r];
-        s.hash[r] = base + (uint32_t)r * all - (uint32_t)(D + 1) * lowered;
-    }
+    for_each_comparator<D>([&](int c, int i) {
+        const float a = s.x[i], b = s.x[i + 1];
+        const bool sw = a < b;
+        s.x[i] = sw ? b : a;
+        s.x[i + 1] = sw ? a : b;
+        const uint32_t p = s.step[i], q = s.step[i + 1];
+        s.step[i] = sw ? q : p;
+        s.step[i + 1] = sw ? p : q;
+        s.swapped[c] = sw;
+    });
 }
 
+// hash of vertex q = 0..D, before the modulo
 template <int D>
-__device__ __forceinline__ void vertex_key(const Simplex<D>& s, int r, int (&key)[D]) {
+__device__ __forceinline__ void vertex_hashes(const Simplex<D>& s, uint32_t (&h)[D + 1]) {
+    h[0] = s.hash0;
 #pragma unroll
-    for (int i = 0; i < D; ++i) key[i] = s.rem0[i] + r - ((s.rank[i] > D - r) ? (D + 1) : 0);
+    for (int q = 1; q <= D; ++q) h[q] = h[q - 1] + s.step[D + 1 - q];
+}
+
+// barycentric weight of vertex q = 0..D times `factor` * (D+1)
+template <int D>
+__device__ __forceinline__ void vertex_weights(const Simplex<D>& s, float factor, float (&w)[D + 1]) {
+    w[0] = __fadd_rn(__fsub_rn(s.x[D], s.x[0]), (float)(D + 1)) * factor;
+#pragma unroll
+    for (int q = 1; q <= D; ++q) w[q] = __fsub_rn(s.x[D - q], s.x[D + 1 - q]) * factor;
 }
 
 __device__ __forceinline__ void red_add1(float* p, float x) {

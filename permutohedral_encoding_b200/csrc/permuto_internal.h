@@ -21,6 +21,7 @@ struct Problem {
     int32_t nr_levels;
     uint32_t capacity;
     int32_t cap_is_pow2;
+    uint64_t cap_magic;   // 2^64 / capacity rounded up (modulo 2^64), for the exact remainder by multiplication
     int32_t table_half;   // the value table is stored as fp16 (gathers only; gradients stay fp32)
     int32_t nr_feat;      // F: features per level, 2, 4 or 8
     int32_t width;        // F * (L + extra): row length of features / gradients
@@ -57,6 +58,7 @@ struct ForwardLinearArgs {
     int32_t tmem_cols;     // tensor-memory columns per block: a power of two >= 32
     int32_t tmem_half;     // column offset of the second accumulator range (hidden layers ping-pong)
     int32_t* status;       // device word set non-zero when a wait on the tensor core ran out
+    int32_t levels_offset; // shared-memory offset of the level constants (set by the launcher)
     int32_t out_vec8_ok;   // out rows can be written with 256-bit stores
 };
 
