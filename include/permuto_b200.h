@@ -177,6 +177,31 @@ int permuto_double_backward(const permuto_config *cfg, const permuto_inputs *in,
                             float *lattice_grad, float *grad_grad_features, uint32_t flags,
                             void *stream);
 
+/* Spatial order of a batch.  Sorting the points along a space-filling curve first puts neighbours
+ * into the same warp, which is what the gathers and reductions of a large batch of independent samples
+ * gain from (no counterpart in the reference; results do not depend on it, rows keep their place).
+ * permuto_order_points fills a caller-owned device buffer of permuto_order_bytes(pos_dim, N) bytes,
+ * 256-byte aligned, for in->positions; the *_ordered entry points below take it together with the SAME
+ * positions (NULL = no order, which is what the plain entry points pass).  One order serves the forward,
+ * backward and double backward of a batch; it holds a copy of the coordinates, so it is only valid
+ * while the positions are unchanged. */
+int permuto_order_pays(const permuto_config *cfg, int64_t nr_positions, int32_t with_gradients); /* 1: worth it */
+int64_t permuto_order_bytes(int32_t pos_dim, int64_t nr_positions);
+int permuto_order_points(const permuto_config *cfg, const permuto_inputs *in, void *order, int64_t order_bytes,
+                         void *stream);
+int permuto_forward_ordered(const permuto_config *cfg, const permuto_inputs *in, const void *order,
+                            float *features, void *stream);
+int permuto_forward_mlp_ordered(const permuto_config *cfg, const permuto_inputs *in, const void *order,
+                                const permuto_mlp_layer *layers, int32_t nr_layers, int32_t activation,
+                                float *out, int32_t *status, void *stream);
+int permuto_backward_ordered(const permuto_config *cfg, const permuto_inputs *in, const void *order,
+                             const float *grad_features, float *lattice_grad, float *positions_grad,
+                             int32_t level_begin, int32_t level_end, uint32_t flags, void *stream);
+int permuto_double_backward_ordered(const permuto_config *cfg, const permuto_inputs *in, const void *order,
+                                    const float *double_positions_grad, const float *grad_features,
+                                    float *lattice_grad, float *grad_grad_features, uint32_t flags,
+                                    void *stream);
+
 /* Debug view of the lattice geometry (the reference has no counterpart; it exists so that
  * keys and hash slots can be compared bit for bit).  Any output may be NULL.
  *   keys  int32 [N, L, pos_dim+1, pos_dim]   slots int32 [N, L, pos_dim+1]

@@ -51,7 +51,7 @@ int extra_levels(int pos_dim, int nr_feat, int concat) { return concat ? (pos_di
 
 // Checks shared by every entry point; the messages mirror the reference's CHECKs
 // (src/Encoding.cu:37-45, :63-66) and factory errors (Encoding.cuh:142,155).
-int build_problem(const permuto_config* cfg, const permuto_inputs* in, permuto::Problem& p) {
+int build_problem(const permuto_config* cfg, const permuto_inputs* in, const void* order, permuto::Problem& p) {
     if (!cfg || !in) return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "cfg and in must not be NULL");
     if (cfg->pos_dim < 2 || cfg->pos_dim > 7)
         return set_error(PERMUTO_ERR_UNSUPPORTED, "Encoding: pos_dim must be 2,3,4,5,6 or 7 (got %d)", cfg->pos_dim);
@@ -79,6 +79,7 @@ int build_problem(const permuto_config* cfg, const permuto_inputs* in, permuto::
     p.positions = in->positions;
     p.pos_stride_n = in->pos_stride_n;
     p.pos_stride_d = in->pos_stride_d;
+    p.order = order;
     p.table = in->lattice_values;
     p.scale = in->scale_factor;
     p.shift = in->random_shift;
@@ -156,9 +157,9 @@ int permuto_scale_factor(const double* sigmas, int32_t nr_levels, int32_t pos_di
     return PERMUTO_OK;
 }
 
-int permuto_forward(const permuto_config* cfg, const permuto_inputs* in, float* features, void* stream) {
+int permuto_forward_ordered(const permuto_config* cfg, const permuto_inputs* in, const void* order, float* features, void* stream) {
     permuto::ForwardArgs a;
-    if (int rc = build_problem(cfg, in, a.p)) return rc;
+    if (int rc = build_problem(cfg, in, order, a.p)) return rc;
     if (!features) return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "features must not be NULL");
     if (!aligned(features, row_align(a.p))) return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "features must be %d-byte aligned", (int)row_align(a.p));
     a.features = features;
@@ -170,10 +171,11 @@ int permuto_forward(const permuto_config* cfg, const permuto_inputs* in, float* 
     return PERMUTO_OK;
 }
 
-int permuto_forward_mlp(const permuto_config* cfg, const permuto_inputs* in, const permuto_mlp_layer* layers,
-                        int32_t nr_layers, int32_t activation, float* out, int32_t* status, void* stream) {
+int permuto_forward_mlp_ordered(const permuto_config* cfg, const permuto_inputs* in, const void* order,
+                                const permuto_mlp_layer* layers, int32_t nr_layers, int32_t activation, float* out,
+                                int32_t* status, void* stream) {
     permuto::ForwardLinearArgs a;
-    if (int rc = build_problem(cfg, in, a.p)) return rc;
+    if (int rc = build_problem(cfg, in, order, a.p)) return rc;
     if (!layers || !out) return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "layers and out must not be NULL");
     if (nr_layers < 1 || nr_layers > permuto::kMaxMlpLayers)
         return set_error(PERMUTO_ERR_UNSUPPORTED, "nr_layers must be in 1..%d (got %d)", permuto::kMaxMlpLayers, nr_layers);
@@ -243,11 +245,11 @@ int permuto_forward_linear(const permuto_config* cfg, const permuto_inputs* in, 
     return permuto_forward_mlp(cfg, in, &one, 1, PERMUTO_ACT_NONE, out, status, stream);
 }
 
-int permuto_backward(const permuto_config* cfg, const permuto_inputs* in, const float* grad_features,
+int permuto_backward_ordered(const permuto_config* cfg, const permuto_inputs* in, const void* order, const float* grad_features,
                      float* lattice_grad, float* positions_grad, int32_t level_begin, int32_t level_end,
                      uint32_t flags, void* stream) {
     permuto::BackwardArgs a;
-    if (int rc = build_problem(cfg, in, a.p)) return rc;
+    if (int rc = build_problem(cfg, in, order, a.p)) return rc;
     if (!grad_features) return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "grad_features must not be NULL");
     if (!aligned(grad_features, row_align(a.p)))
         return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "grad_features must be %d-byte aligned", (int)row_align(a.p));
@@ -281,11 +283,11 @@ int permuto_backward(const permuto_config* cfg, const permuto_inputs* in, const 
     return PERMUTO_OK;
 }
 
-int permuto_double_backward(const permuto_config* cfg, const permuto_inputs* in, const float* double_positions_grad,
-                            const float* grad_features, float* lattice_grad, float* grad_grad_features,
+int permuto_double_backward_ordered(const permuto_config* cfg, const permuto_inputs* in, const void* order,
+                            const float* double_positions_grad, const float* grad_features, float* lattice_grad, float* grad_grad_features,
                             uint32_t flags, void* stream) {
     permuto::DoubleBackwardArgs a;
-    if (int rc = build_problem(cfg, in, a.p)) return rc;
+    if (int rc = build_problem(cfg, in, order, a.p)) return rc;
     if (!double_positions_grad) return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "double_positions_grad must not be NULL");
     if (lattice_grad && !grad_features)
         return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "grad_features is needed for the lattice gradient");
@@ -313,10 +315,34 @@ int permuto_double_backward(const permuto_config* cfg, const permuto_inputs* in,
     return PERMUTO_OK;
 }
 
+// The entry points without an order: the points are taken in the sequence they come in.
+int permuto_forward(const permuto_config* cfg, const permuto_inputs* in, float* features, void* stream) {
+    return permuto_forward_ordered(cfg, in, nullptr, features, stream);
+}
+
+int permuto_forward_mlp(const permuto_config* cfg, const permuto_inputs* in, const permuto_mlp_layer* layers,
+                        int32_t nr_layers, int32_t activation, float* out, int32_t* status, void* stream) {
+    return permuto_forward_mlp_ordered(cfg, in, nullptr, layers, nr_layers, activation, out, status, stream);
+}
+
+int permuto_backward(const permuto_config* cfg, const permuto_inputs* in, const float* grad_features,
+                     float* lattice_grad, float* positions_grad, int32_t level_begin, int32_t level_end,
+                     uint32_t flags, void* stream) {
+    return permuto_backward_ordered(cfg, in, nullptr, grad_features, lattice_grad, positions_grad, level_begin, level_end,
+                                    flags, stream);
+}
+
+int permuto_double_backward(const permuto_config* cfg, const permuto_inputs* in, const float* double_positions_grad,
+                            const float* grad_features, float* lattice_grad, float* grad_grad_features,
+                            uint32_t flags, void* stream) {
+    return permuto_double_backward_ordered(cfg, in, nullptr, double_positions_grad, grad_features, lattice_grad,
+                                           grad_grad_features, flags, stream);
+}
+
 int permuto_debug_lattice(const permuto_config* cfg, const permuto_inputs* in, int32_t* keys, int32_t* slots,
                           float* bary, int32_t* rank, void* stream) {
     permuto::DebugArgs a;
-    if (int rc = build_problem(cfg, in, a.p)) return rc;
+    if (int rc = build_problem(cfg, in, nullptr, a.p)) return rc;
     a.keys = keys;
     a.slots = slots;
     a.bary = bary;

@@ -48,6 +48,9 @@ constexpr int D = PERMUTO_DIM;
 #ifndef PERMUTO_MIN_BLOCKS_FORWARD
 #define PERMUTO_MIN_BLOCKS_FORWARD (PERMUTO_DIM <= 3 ? 8 : (PERMUTO_DIM == 4 ? 6 : 4))
 #endif
+#ifndef PERMUTO_FWD_STAGGER
+#define PERMUTO_FWD_STAGGER 1
+#endif
 constexpr int kThreads = PERMUTO_THREADS;
 // wider table entries keep more addends live per vertex: leave them more registers
 constexpr int min_blocks(int feats, bool gather_only) {
@@ -184,6 +187,27 @@ __device__ __forceinline__ void store8(float* dst, const float (&v)[8]) {
     asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "f"(v[0]), "f"(v[1]),
                  "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
                  : "memory");
+}
+
+// Point number i of the sweep and the row it belongs to: i itself, or, when the batch has been put
+// into spatial order, the i-th record {coordinates, row} (16 bytes up to pos_dim 3, else 32).
+__device__ __forceinline__ int64_t load_point(const Problem& p, int64_t i, float (&pos)[D]) {
+    if (p.order == nullptr) {
+        load_pos(p, i, pos);
+        return i;
+    }
+    if (D <= 3) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p.order) + i);
+        pos[0] = t.x;
+        pos[1] = t.y;
+        if (D == 3) pos[D - 1] = t.z;
+        return (int64_t)__float_as_uint(t.w);
+    }
+    float r[8];
+    load8(reinterpret_cast<const float*>(p.order) + 8 * i, r);
+#pragma unroll
+    for (int j = 0; j < D; ++j) pos[j] = r[j];
+    return (int64_t)__float_as_uint(r[7]);
 }
 
 // Aligned gather of one table entry (all F features) through the read-only path.  HALF: the
@@ -331,14 +355,13 @@ template <int F, int LPS, bool HALF>
 __global__ void __launch_bounds__(kThreads, (F == 2 ? PERMUTO_MIN_BLOCKS_FORWARD : min_blocks(F, false))) forward_kernel(const ForwardArgs a) {
     const Problem& p = a.p;
     __shared__ __align__(16) float levels[kStage * kRecord];
-    const int64_t n_raw = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    const bool active = n_raw < p.n_points;
-    const int64_t n = active ? n_raw : p.n_points - 1;  // idle threads shadow the last point
+    const int64_t i_raw = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const bool active = i_raw < p.n_points;
     const int pass_begin = p.level_begin + (int)blockIdx.y * p.levels_per_pass;
     const int pass_end = min(pass_begin + p.levels_per_pass, p.level_end);
 
     float pos[D];
-    load_pos(p, n, pos);
+    const int64_t n = load_point(p, active ? i_raw : p.n_points - 1, pos);  // idle threads shadow the last point
 
 #pragma unroll 1
     for (int begin = pass_begin; begin < pass_end; begin += kStage) {
@@ -346,8 +369,12 @@ __global__ void __launch_bounds__(kThreads, (F == 2 ? PERMUTO_MIN_BLOCKS_FORWARD
         if (begin != pass_begin) __syncthreads();
         stage_levels(p, begin, end, levels);
         __syncthreads();
+        const int nsteps = (end - begin + LPS - 1) / LPS;
+        int step = (PERMUTO_FWD_STAGGER && p.order == nullptr) ? (int)(blockIdx.x % (unsigned)nsteps) : 0;
 #pragma unroll 1
-        for (int l0 = begin; l0 < end; l0 += LPS) {
+        for (int it = 0; it < nsteps; ++it) {
+            const int l0 = begin + step * LPS;
+            step = (step + 1 == nsteps) ? 0 : step + 1;
             float out[F * LPS];
             encode_step<F, LPS, HALF>(p, levels + (l0 - begin) * kRecord, pos, l0, end, out);
             if (active) store_row_segment<F, LPS>(p, a.features, n, l0, out);
@@ -611,12 +638,12 @@ forward_mlp_kernel(const ForwardLinearArgs a) {
     ring.ok = true;
 
     // ---- layer 0: this thread's point -> row t of every slice ----------------------------------
-    const int64_t n_raw = (int64_t)blockIdx.x * kTileRows + t;
-    const bool active = n_raw < p.n_points;
-    const int64_t n = active ? n_raw : p.n_points - 1;  // idle rows shadow the last point and are not stored
+    const int64_t i_raw = (int64_t)blockIdx.x * kTileRows + t;
+    const bool active = i_raw < p.n_points;
+    int64_t n;
     {
         float pos[D];
-        load_pos(p, n, pos);
+        n = load_point(p, active ? i_raw : p.n_points - 1, pos);  // idle rows shadow the last point and are not stored
         const int lattice_cols = F * p.nr_levels;
         // a column past the lattice levels: a concatenated raw coordinate (EncodingGPU.cuh:105-121) or padding
         auto tail_value = [&](int c) -> float {
@@ -694,7 +721,7 @@ forward_mlp_kernel(const ForwardLinearArgs a) {
 #pragma unroll
                         for (int k = 0; k < HM; ++k)
                             if (k < width) acc = fmaf(h[k], __ldg(w + k), acc);
-                        a.out[n_raw * ly.out_features + o] = acc;
+                        a.out[n * ly.out_features + o] = acc;
                     }
                 }
                 last = -1;  // everything is written
@@ -723,7 +750,7 @@ forward_mlp_kernel(const ForwardLinearArgs a) {
         const int H = a.layer[last].out_features;
         const float* bias = a.layer[last].bias;
         if (ok) {
-            float* dst = a.out + n_raw * H;
+            float* dst = a.out + n * H;
             for (int c = 0; c < H; c += 16) {
                 float v[16];
                 tmem_load16(lane_base + col + (uint32_t)c, v);
@@ -892,16 +919,15 @@ __global__ void __launch_bounds__(kThreads, min_blocks(F, !TABLE))
 backward_kernel(const BackwardArgs a) {
     const Problem& p = a.p;
     __shared__ __align__(16) float levels[kStage * kRecord];
-    const int64_t n_raw = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    const bool active = n_raw < p.n_points;
-    const int64_t n = active ? n_raw : p.n_points - 1;  // idle lanes shadow the last point
+    const int64_t i_raw = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const bool active = i_raw < p.n_points;
     const int pass_begin = p.level_begin + (int)blockIdx.y * p.levels_per_pass;
     const int pass_end = min(pass_begin + p.levels_per_pass, p.level_end);
     const unsigned lane = threadIdx.x & 31u;
     constexpr float kInv = 1.0f / (D + 1);
 
     float pos[D];
-    load_pos(p, n, pos);
+    const int64_t n = load_point(p, active ? i_raw : p.n_points - 1, pos);  // idle lanes shadow the last point
 
     float dpos[D];
 #pragma unroll
@@ -996,22 +1022,185 @@ backward_kernel(const BackwardArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------
+// table gradient of a coherent batch: P consecutive points per thread
+// ------------------------------------------------------------------------------------------
+#ifndef PERMUTO_RUN_POINTS
+#define PERMUTO_RUN_POINTS 2
+#endif
+#ifndef PERMUTO_RUN_BLOCKS
+#define PERMUTO_RUN_BLOCKS 8
+#endif
+#ifndef PERMUTO_RUN_THREADS
+#define PERMUTO_RUN_THREADS 128
+#endif
+constexpr int kRunPoints = PERMUTO_RUN_POINTS;
+constexpr int kRunThreads = PERMUTO_RUN_THREADS;
+constexpr int kPosVec = D <= 3 ? 1 : 2;  // float4s per point: coordinates, row index last
+struct RunStage {
+    float levels[kStage * kRecord];
+    float4 point[kRunPoints][kPosVec][kRunThreads];
+    float4 grad[kRunPoints][2][kRunThreads];  // gradient row segments: [point][4 floats of the step][thread]
+};
+template <int F>
+__global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_kernel(const BackwardArgs a) {
+    constexpr int P = kRunPoints;
+    constexpr int LPS = 8 / F;
+    const Problem& p = a.p;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    RunStage& sm = *reinterpret_cast<RunStage*>(smem_raw);
+    const int t = threadIdx.x;
+    const int pass_begin = p.level_begin + (int)blockIdx.y * p.levels_per_pass;
+    const int pass_end = min(pass_begin + p.levels_per_pass, p.level_end);
+    constexpr float kInv = 1.0f / (D + 1);
+
+    const int64_t first = ((int64_t)blockIdx.x * kRunThreads + t) * P;
+    const int count = (int)max((int64_t)0, min((int64_t)P, p.n_points - first));  // points this thread owns
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        float x[D];
+        const int64_t n = load_point(p, min(first + j, p.n_points - 1), x);
+        float r[4 * kPosVec];
+#pragma unroll
+        for (int i = 0; i < 4 * kPosVec; ++i) r[i] = i < D ? x[i < D ? i : 0] : 0.f;
+        r[4 * kPosVec - 1] = __uint_as_float((uint32_t)n);
+#pragma unroll
+        for (int i = 0; i < kPosVec; ++i) sm.point[j][i][t] = make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+    }
+    Scatter sc{threadIdx.x & 31u, true, a.aggregate != 0};
+
+#pragma unroll 1
+    for (int begin = pass_begin; begin < pass_end; begin += kStage) {
+        const int end = min(begin + kStage, pass_end);
+        const int nsteps = (end - begin + LPS - 1) / LPS;
+        int step = kStagger ? (int)(blockIdx.x % (unsigned)nsteps) : 0;
+        if (begin != pass_begin) __syncthreads();
+        stage_levels(p, begin, end, sm.levels);
+        __syncthreads();
+#pragma unroll 1
+        for (int it = 0; it < nsteps; ++it) {
+            const int l0 = begin + step * LPS;
+            step = (step + 1 == nsteps) ? 0 : step + 1;
+            if (l0 == begin) sc.probe = a.aggregate != 0;
+            {
+                float g[P][8];
+#pragma unroll
+                for (int j = 0; j < P; ++j)
+                    load_row_segment<F, LPS>(p, a.grad_features, __float_as_uint(sm.point[j][kPosVec - 1][t].w), l0, g[j]);
+#pragma unroll
+                for (int j = 0; j < P; ++j) {
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                        sm.grad[j][q][t] = j < count ? make_float4(g[j][4 * q], g[j][4 * q + 1], g[j][4 * q + 2], g[j][4 * q + 3])
+                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+#pragma unroll 1
+            for (int k = 0; k < LPS && l0 + k < end; ++k) {
+                const int l = l0 + k;
+                LevelConst<D> lc;
+                load_level(sm.levels, l - begin, lc);
+                if (lc.weight == 0.0f) continue;
+                float* gbase = a.lattice_grad + (size_t)l * p.capacity * F;
+                uint32_t cur[D + 1];
+                float acc[D + 1][F];
+                int kept = 0;
+                const bool runs = sc.probe;
+#pragma unroll
+                for (int r = 0; r <= D; ++r) {
+                    cur[r] = 0u;
+#pragma unroll
+                    for (int f = 0; f < F; ++f) acc[r][f] = 0.f;
+                }
+#pragma unroll 1
+                for (int j = 0; j < P; ++j) {
+                    float x[D], g[F];
+#pragma unroll
+                    for (int i = 0; i < kPosVec; ++i) {
+                        const float4 v = sm.point[j][i][t];
+                        x[4 * i] = v.x;
+                        x[4 * i + 1] = v.y;
+                        if (4 * i + 2 < D) x[(4 * i + 2) % D] = v.z;
+                        if (4 * i + 3 < D) x[(4 * i + 3) % D] = v.w;
+                    }
+                    {
+                        const float4* src = &sm.grad[j][F * k / 4][t];
+                        if (F == 2) {
+                            const float2 v = reinterpret_cast<const float2*>(src)[k & 1];
+                            g[0] = v.x;
+                            g[1] = v.y;
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < F / 4; ++q) {
+                                const float4 v = src[q * kRunThreads];
+                                g[(4 * q) % F] = v.x;
+                                g[(4 * q + 1) % F] = v.y;
+                                g[(4 * q + 2) % F] = v.z;
+                                g[(4 * q + 3) % F] = v.w;
+                            }
+                        }
+                    }
+                    Simplex<D> s;
+                    locate_simplex<D>(x, lc, s);
+                    uint32_t slot[D + 1];
+                    to_slots(p, s, slot);
+                    float w[D + 1];
+                    vertex_weights<D>(s, lc.weight * kInv, w);
+                    if (runs) {
+                        to_remainders(s.s, slot);
+                        to_remainders(s.s, w);
+#pragma unroll
+                        for (int r = 0; r <= D; ++r) {
+                            const bool same = slot[r] == cur[r];
+                            if (j > 0 && !same) red_add<F>(gbase, cur[r], acc[r]);
+                            cur[r] = slot[r];
+#pragma unroll
+                            for (int f = 0; f < F; ++f) acc[r][f] = fmaf(w[r], g[f], same ? acc[r][f] : 0.f);
+                            if (r == 0) kept += same ? 1 : 0;
+                        }
+                    } else if (j < count) {
+#pragma unroll
+                        for (int r = 0; r <= D; ++r) {
+                            float add[F];
+#pragma unroll
+                            for (int f = 0; f < F; ++f) add[f] = w[r] * g[f];
+                            red_add<F>(gbase, slot[r], add);
+                        }
+                    }
+                }
+                if (runs) {
+                    const unsigned lane = sc.lane;
+                    const unsigned group0 = __match_any_sync(kFullMask, cur[0]);
+                    const int distinct = __popc(__ballot_sync(kFullMask, (group0 & ((1u << lane) - 1u)) == 0u));
+                    if (distinct <= kMergeBelow) {
+                        merge_from<F, 0>(sc, gbase, cur, acc, group0);
+                    } else {
+#pragma unroll
+                        for (int r = 0; r <= D; ++r) red_add<F>(gbase, cur[r], acc[r]);
+                        kept = __reduce_add_sync(kFullMask, kept);
+                        if (kept + 32 - distinct < 8 * P) sc.probe = false;
+                    }
+                }
+            }
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------
 // double backward of the position gradient
 // ------------------------------------------------------------------------------------------
 template <int F, int LPS, bool TABLE, bool GGF, bool HALF>
 __global__ void __launch_bounds__(kThreads, min_blocks(F, false)) double_backward_kernel(const DoubleBackwardArgs a) {
     const Problem& p = a.p;
     __shared__ __align__(16) float levels[kStage * kRecord];
-    const int64_t n_raw = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    const bool active = n_raw < p.n_points;
-    const int64_t n = active ? n_raw : p.n_points - 1;
+    const int64_t i_raw = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const bool active = i_raw < p.n_points;
     const int pass_begin = p.level_begin + (int)blockIdx.y * p.levels_per_pass;
     const int pass_end = min(pass_begin + p.levels_per_pass, p.level_end);
     const unsigned lane = threadIdx.x & 31u;
     constexpr float kInv = 1.0f / (D + 1);
 
     float pos[D], dpg[D];
-    load_pos(p, n, pos);
+    const int64_t n = load_point(p, active ? i_raw : p.n_points - 1, pos);
 #pragma unroll
     for (int i = 0; i < D; ++i) dpg[i] = __ldg(a.double_positions_grad + n * D + i);
     Scatter sc{lane, active, a.aggregate != 0};  // as in backward_kernel
@@ -1167,7 +1356,9 @@ enum class Traffic { Gather, Scatter, Both };
 inline int pick_levels_per_pass(const Problem& p, int requested, Traffic t, int lps) {
     const int levels = p.level_end - p.level_begin;
     int lpp = requested;
-    if (lpp <= 0) {
+    if (lpp <= 0 && p.order != nullptr && t != Traffic::Both) {
+        lpp = levels;
+    } else if (lpp <= 0) {
         const double slice = (p.table_half ? 2.0 : 4.0) * p.nr_feat * p.capacity;
         const double mb = 1024.0 * 1024.0;
         if (t == Traffic::Scatter) {
@@ -1221,6 +1412,9 @@ inline bool use_single_level(const Problem& p) {
     return lps > 1 && blocks < 2 * (sms > 0 ? sms : 148);
 }
 
+// table gradient alone of a batch in spatial order
+inline bool use_runs(const BackwardArgs& a) { return a.p.order != nullptr && a.lattice_grad != nullptr && a.positions_grad == nullptr; }
+
 template <class Args>
 inline Args with_schedule(const Args& in, bool single, Traffic t) {
     Args a = in;
@@ -1272,6 +1466,11 @@ cudaError_t launch_backward(const BackwardArgs& a, cudaStream_t st) {
     if (a.lattice_grad && a.positions_grad) {
         if (h) backward_kernel<F, LPS, true, true, true><<<g, kThreads, 0, st>>>(a);
         else backward_kernel<F, LPS, true, true, false><<<g, kThreads, 0, st>>>(a);
+    } else if (use_runs(a)) {
+        const dim3 gr((unsigned)((a.p.n_points + kRunThreads * kRunPoints - 1) / (kRunThreads * kRunPoints)), g.y);
+        const cudaError_t e = cudaFuncSetAttribute(scatter_runs_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RunStage));
+        if (e != cudaSuccess) return e;
+        scatter_runs_kernel<F><<<gr, kRunThreads, sizeof(RunStage), st>>>(a);
     } else if (a.lattice_grad) {
         backward_kernel<F, LPS, true, false, false><<<g, kThreads, 0, st>>>(a);
     } else if (a.positions_grad) {
@@ -1327,7 +1526,8 @@ cudaError_t PERMUTO_CAT(launch_forward_linear_dim, PERMUTO_DIM)(const ForwardLin
 }
 
 cudaError_t PERMUTO_CAT(launch_backward_dim, PERMUTO_DIM)(const BackwardArgs& a0, cudaStream_t st) {
-    const bool single = use_single_level(a0.p);
+    // the runs kernel takes whole steps of 8 floats, so its sweeps have to start on a step
+    const bool single = use_single_level(a0.p) && !use_runs(a0);
     const Traffic t = (a0.lattice_grad && a0.positions_grad) ? Traffic::Both
                                                              : (a0.lattice_grad ? Traffic::Scatter : Traffic::Gather);
     const BackwardArgs a = with_schedule(a0, single, t);

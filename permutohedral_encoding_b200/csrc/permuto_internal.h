@@ -13,6 +13,7 @@ struct Problem {
     const float* positions;
     int64_t pos_stride_n;
     int64_t pos_stride_d;
+    const void* order;    // records {coordinates, row} of the points in spatial order (permuto_order.cu), or null
     const void* table;    // [L, C, F], fp32 or (table_half) fp16
     const float* scale;   // [L, D]
     const float* shift;   // [L, D]
