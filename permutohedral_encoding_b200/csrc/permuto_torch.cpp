@@ -1,0 +1,487 @@
+// PyTorch side of the encoding: checks, output allocation, launches and the autograd graph in C++.
+//
+// A README-sized batch runs for a few microseconds on the device, so what a call costs is host work:
+// with checks, ctypes marshalling and torch.autograd.Function in Python a forward of 1000 points took
+// 14 us and a training step on 4096 points 117 us, most of it in the interpreter.  Nothing here is
+// remembered between calls except the scale factors of the encoding on each device.
+//
+// The two nodes mirror the reference's chained autograd Functions (src/pytorch_modules/funcs.py:8-72).
+// Unlike a Python Function, a C++ node can ask the engine which of its inputs the running backward
+// needs: autograd.grad(y, positions) does not compute the lattice gradient, and a backward restricted
+// to the lattice values does not compute the position gradient.
+//
+// The C ABI is called through the pointers of the library the Python side has loaded.
+#include <torch/extension.h>
+
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <mutex>
+#include <optional>
+#include <string>
+#include <unordered_map>
+#include <vector>
+
+#include "permuto_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+struct Api {
+    decltype(&permuto_last_error) last_error;
+    decltype(&permuto_order_pays) order_pays;
+    decltype(&permuto_order_bytes) order_bytes;
+    decltype(&permuto_order_points) order_points;
+    decltype(&permuto_forward_ordered) forward;
+    decltype(&permuto_forward_mlp_ordered) forward_mlp;
+    decltype(&permuto_backward_ordered) backward;
+    decltype(&permuto_double_backward_ordered) double_backward;
+    decltype(&permuto_adam_step) adam_step;
+} api = {};
+
+template <class F>
+void take(F& slot, const std::unordered_map<std::string, uintptr_t>& table, const char* name) {
+    const auto it = table.find(name);
+    if (it == table.end()) throw std::runtime_error(std::string("missing C ABI symbol ") + name);
+    slot = reinterpret_cast<F>(it->second);
+}
+
+void bind_api(const std::unordered_map<std::string, uintptr_t>& t) {
+    take(api.last_error, t, "permuto_last_error");
+    take(api.order_pays, t, "permuto_order_pays");
+    take(api.order_bytes, t, "permuto_order_bytes");
+    take(api.order_points, t, "permuto_order_points");
+    take(api.forward, t, "permuto_forward_ordered");
+    take(api.forward_mlp, t, "permuto_forward_mlp_ordered");
+    take(api.backward, t, "permuto_backward_ordered");
+    take(api.double_backward, t, "permuto_double_backward_ordered");
+    take(api.adam_step, t, "permuto_adam_step");
+}
+
+void check(int status) {
+    if (status != PERMUTO_OK) throw std::runtime_error(api.last_error());
+}
+
+std::string sizes_of(const Tensor& t) {
+    std::string s = "(";
+    for (int64_t i = 0; i < t.dim(); ++i) s += (i ? ", " : "") + std::to_string(t.size(i));
+    return s + (t.dim() == 1 ? ",)" : ")");
+}
+
+[[noreturn]] void fail(const std::string& what) { throw std::runtime_error(what); }
+
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+// fp32, contiguous, on `device`, without a graph
+Tensor plain(const Tensor& t, const c10::Device& device) {
+    if (t.device() == device && t.scalar_type() == at::kFloat && t.is_contiguous()) return t;
+    return t.detach().to(t.options().device(device).dtype(at::kFloat).requires_grad(false)).contiguous();
+}
+
+const void* data(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+
+// Fixed description of an encoding and what it keeps on every device.
+struct Lattice : torch::CustomClassHolder {
+    permuto_config cfg = {};
+    int64_t width = 0;
+    bool aggregate = true;
+    bool concat_positions_grad = false;
+    // data-parallel hooks: callables kept by the Python wrapper, empty objects when not installed
+    py::object on_backward, on_double_backward;
+
+    Lattice(int pos_dim, int feat, int levels, int capacity, bool concat, double scaling, int64_t width_, Tensor scale_host)
+        : width(width_), scale_host_(std::move(scale_host)) {
+        cfg.pos_dim = pos_dim;
+        cfg.nr_feat_per_level = feat;
+        cfg.nr_levels = levels;
+        cfg.capacity = capacity;
+        cfg.concat_points = concat ? 1 : 0;
+        cfg.points_scaling = (float)scaling;
+    }
+    ~Lattice() override {
+        if ((on_backward || on_double_backward) && Py_IsInitialized()) {
+            py::gil_scoped_acquire gil;  // the last owner may be a graph released on the engine's thread
+            on_backward = py::object();
+            on_double_backward = py::object();
+        } else {
+            on_backward.release();
+            on_double_backward.release();
+        }
+    }
+
+    Tensor scale_on(const c10::Device& device) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        Tensor& t = scale_[device.index()];
+        if (!t.defined()) t = scale_host_.to(device);
+        return t;
+    }
+
+  private:
+    Tensor scale_host_;
+    std::mutex mutex_;
+    std::unordered_map<int, Tensor> scale_;
+};
+
+// One call's inputs, checked; holds what the pointers of `in` refer to.
+struct Call : torch::CustomClassHolder {
+    c10::intrusive_ptr<Lattice> lattice;
+    Tensor values, positions, window, shift, half, order;
+    int levels_per_pass = 0;
+    bool need_values = false, need_positions = false;
+};
+
+// Same checks and messages as the reference (src/Encoding.cu:37-45, :63-66, :119-125).
+void check_inputs(const Call& c) {
+    const permuto_config& cfg = c.lattice->cfg;
+    const Tensor& pos = c.positions;
+    if (!pos.is_cuda()) fail("positions should be in GPU memory. Please call .cuda() on the tensor");
+    if (pos.scalar_type() != at::kFloat) fail("positions should be of type float");
+    if (pos.dim() != 2) fail("positions should have dim 2 correspondin to HW. However it has sizes " + sizes_of(pos));
+    if (pos.size(0) == 0) fail("Why do we have 0 points");
+    if (pos.size(1) != cfg.pos_dim)
+        fail("Pos dim for the lattice doesn't correspond with the position of the points. Lattice was initialized with " +
+             std::to_string(cfg.pos_dim) + " and points have pos dim " + std::to_string(pos.size(1)));
+    const Tensor& lv = c.values;
+    if (lv.dim() != 3 || lv.size(0) != cfg.nr_levels || lv.size(1) != cfg.capacity || lv.size(2) != cfg.nr_feat_per_level)
+        fail("lattice_values should be nr_levels x capacity x " + std::to_string(cfg.nr_feat_per_level) + ", got " + sizes_of(lv));
+    if (!lv.is_contiguous())
+        fail("We assume that the lattice_values_monolithic are contiguous because in the cuda code we make a load of 2 float "
+             "values at a time");
+    if ((lv.scalar_type() != at::kFloat && lv.scalar_type() != at::kHalf) || lv.device() != pos.device())
+        fail("lattice_values should be float32 (or float16 storage) on the device of the positions");
+    if (c.half.defined() && (c.half.scalar_type() != at::kHalf || c.half.sizes() != lv.sizes() || c.half.device() != lv.device() ||
+                             !c.half.is_contiguous()))
+        fail("lattice_values_half should be a contiguous float16 tensor of the shape and device of lattice_values");
+    if (c.shift.dim() != 2 || c.shift.size(0) != cfg.nr_levels || c.shift.size(1) != cfg.pos_dim)
+        fail("Random shift should be nr of resolutions x pos dim");
+    if (c.window.dim() != 1 || c.window.size(0) != cfg.nr_levels)
+        fail("anneal_window should have the first dimension the same as the nr of resolutions");
+}
+
+// The C ABI's view of a checked call.
+struct Bound {
+    permuto_config cfg;
+    permuto_inputs in;
+    c10::cuda::OptionalCUDAGuard guard;
+    Tensor scale, shift, window;
+
+    explicit Bound(const Call& c) : cfg(c.lattice->cfg) {
+        const c10::Device device = c.positions.device();
+        if (device.index() != c10::cuda::current_device()) guard.set_device(device);
+        scale = c.lattice->scale_on(device);
+        shift = plain(c.shift, device);
+        window = plain(c.window, device);
+        const Tensor& table = c.half.defined() ? c.half : c.values;
+        cfg.table_dtype = table.scalar_type() == at::kHalf ? PERMUTO_TABLE_F16 : PERMUTO_TABLE_F32;
+        cfg.levels_per_pass = c.levels_per_pass;
+        in.nr_positions = c.positions.size(0);
+        in.positions = c.positions.data_ptr<float>();
+        in.pos_stride_n = c.positions.stride(0);
+        in.pos_stride_d = c.positions.stride(1);
+        in.lattice_values = table.data_ptr();
+        in.scale_factor = scale.data_ptr<float>();
+        in.random_shift = shift.data_ptr<float>();
+        in.anneal_window = window.data_ptr<float>();
+    }
+};
+
+Tensor make_order(const Call& c, Bound& b) {
+    const int64_t bytes = api.order_bytes(b.cfg.pos_dim, b.in.nr_positions);
+    Tensor order = at::empty({bytes}, c.positions.options().dtype(at::kByte));
+    check(api.order_points(&b.cfg, &b.in, order.data_ptr(), bytes, stream_of(c.positions)));
+    return order;
+}
+
+// features [N, W]; where the batch is large enough to be worth it the points are put into spatial order
+// first, and the order stays with the call for its backward passes
+Tensor run_forward(Call& c, bool may_order) {
+    check_inputs(c);
+    Bound b(c);
+    if (may_order && !c.order.defined() && api.order_pays(&b.cfg, b.in.nr_positions, c.need_values || c.need_positions ? 1 : 0))
+        c.order = make_order(c, b);
+    Tensor out = at::empty({b.in.nr_positions, c.lattice->width}, c.positions.options());
+    check(api.forward(&b.cfg, &b.in, data(c.order), out.data_ptr<float>(), stream_of(c.positions)));
+    return out;
+}
+
+struct Gradients {
+    Tensor values, positions;
+};
+
+Gradients run_backward(const Call& c, const Tensor& grad, bool need_values, bool need_positions, const Tensor& values_out,
+                       int level_begin, int level_end, bool zero, const Tensor& positions_out) {
+    check_inputs(c);
+    const int64_t n = c.positions.size(0);
+    if (grad.dim() != 2 || grad.size(0) != n || grad.size(1) != c.lattice->width)
+        fail("The nr of positions should match between the input positions and the sliced values: expected (" +
+             std::to_string(n) + ", " + std::to_string(c.lattice->width) + "), got " + sizes_of(grad));
+    if (!grad.is_contiguous()) fail("Grad sliced values needs to be contiguous. Please call .contiguous() on it");
+    Bound b(c);
+    uint32_t flags = zero ? PERMUTO_ZERO_OUTPUTS : 0;
+    if (!c.lattice->aggregate) flags |= PERMUTO_NO_AGGREGATE;
+    if (c.lattice->concat_positions_grad) flags |= PERMUTO_CONCAT_POSITIONS_GRAD;
+    Gradients g;
+    if (need_values)  // always fp32, whatever the storage type of the values
+        g.values = values_out.defined() ? values_out : at::empty(c.values.sizes(), c.positions.options());
+    if (need_positions) {
+        if (positions_out.defined()) {
+            g.positions = positions_out;
+            flags |= PERMUTO_KEEP_POSITIONS_GRAD;
+        } else {  // without ZERO_OUTPUTS nothing clears it natively
+            g.positions = zero ? at::empty({n, b.cfg.pos_dim}, c.positions.options())
+                               : at::zeros({n, b.cfg.pos_dim}, c.positions.options());
+        }
+    }
+    check(api.backward(&b.cfg, &b.in, data(c.order), grad.data_ptr<float>(),
+                       g.values.defined() ? g.values.data_ptr<float>() : nullptr,
+                       g.positions.defined() ? g.positions.data_ptr<float>() : nullptr, level_begin,
+                       level_end < 0 ? b.cfg.nr_levels : level_end, flags, stream_of(c.positions)));
+    return g;
+}
+
+struct SecondOrder {
+    Tensor values, features;
+};
+
+SecondOrder run_double_backward(const Call& c, const Tensor& double_positions_grad, const Tensor& grad, bool need_values,
+                                bool need_features) {
+    check_inputs(c);
+    const int64_t n = c.positions.size(0);
+    if (double_positions_grad.dim() != 2 || double_positions_grad.size(0) != n ||
+        double_positions_grad.size(1) != c.lattice->cfg.pos_dim)
+        fail("double_positions_grad should be nr_positions x pos_dim");
+    if (grad.dim() != 2 || grad.size(0) != n || grad.size(1) != c.lattice->width)
+        fail("The nr of positions should match between the input positions and the sliced values");
+    Bound b(c);
+    const Tensor dpg = double_positions_grad.contiguous(), gf = grad.contiguous();
+    SecondOrder s;
+    if (need_values) s.values = at::empty(c.values.sizes(), c.positions.options());
+    if (need_features) s.features = at::empty(gf.sizes(), c.positions.options());
+    check(api.double_backward(&b.cfg, &b.in, data(c.order), dpg.data_ptr<float>(), gf.data_ptr<float>(),
+                              need_values ? s.values.data_ptr<float>() : nullptr,
+                              need_features ? s.features.data_ptr<float>() : nullptr,
+                              PERMUTO_ZERO_OUTPUTS | (c.lattice->aggregate ? 0 : PERMUTO_NO_AGGREGATE),
+                              stream_of(c.positions)));
+    return s;
+}
+
+py::object as_python(const Tensor& t) { return t.defined() ? py::cast(t) : py::none(); }
+Tensor from_python(const py::handle& h) { return h.is_none() ? Tensor() : py::cast<Tensor>(h); }
+
+Gradients backward_or_hook(const Call& c, const Tensor& grad, bool need_values, bool need_positions) {
+    if (need_values && c.lattice->on_backward) {
+        py::gil_scoped_acquire gil;
+        const py::tuple r = c.lattice->on_backward(c.values, c.positions, c.window, as_python(c.half), as_python(c.order), grad,
+                                                   need_values, need_positions);
+        return {from_python(r[0]), from_python(r[1])};
+    }
+    return run_backward(c, grad, need_values, need_positions, {}, 0, -1, true, {});
+}
+
+// The first-order backward as a differentiable function of (upstream gradient, lattice values); its own
+// backward is the double backward from the position gradient.
+struct EncodeBackward : torch::autograd::Function<EncodeBackward> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& grad, const Tensor& values, const Tensor& positions,
+                                 const c10::intrusive_ptr<Call>& call, bool need_values, bool need_positions) {
+        const Gradients g = backward_or_hook(*call, grad, need_values, need_positions);
+        ctx->save_for_backward({grad, values, positions, call->window});
+        ctx->saved_data["call"] = c10::IValue::make_capsule(call);
+        ctx->saved_data["position_output"] = need_positions ? (need_values ? 1 : 0) : -1;
+        ctx->set_materialize_grads(false);
+        variable_list out;
+        if (need_values) out.push_back(g.values);
+        if (need_positions) out.push_back(g.positions);
+        return out;
+    }
+
+    static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+        // As in the reference, only the path through the position gradient is differentiated again; a
+        // second-order term through the lattice-value gradient is not propagated.
+        variable_list out(6);
+        const int64_t at = ctx->saved_data["position_output"].toInt();
+        if (at < 0 || !grads[at].defined()) return out;
+        const bool need_features = ctx->needs_input_grad(0), need_values = ctx->needs_input_grad(1);
+        if (!need_features && !need_values) return out;
+        const variable_list saved = ctx->get_saved_variables();
+        const auto call = c10::static_intrusive_pointer_cast<Call>(ctx->saved_data["call"].toCapsule());
+        SecondOrder s = run_double_backward(*call, grads[at], saved[0], need_values, need_features);
+        // data-parallel use: this second-order lattice gradient is summed over the ranks like the
+        // first-order one, otherwise the replicated tables drift apart
+        if (s.values.defined() && call->lattice->on_double_backward) {
+            py::gil_scoped_acquire gil;
+            s.values = from_python(call->lattice->on_double_backward(s.values));
+        }
+        out[0] = s.features;
+        out[1] = s.values;
+        return out;
+    }
+};
+
+struct Encode : torch::autograd::Function<Encode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& values, const Tensor& positions,
+                          const c10::intrusive_ptr<Call>& call) {
+        const Tensor out = run_forward(*call, true);
+        ctx->save_for_backward({values, positions, call->window});
+        ctx->saved_data["call"] = c10::IValue::make_capsule(call);
+        return out;
+    }
+
+    static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+        const variable_list saved = ctx->get_saved_variables();  // checks the version counters
+        const auto call = c10::static_intrusive_pointer_cast<Call>(ctx->saved_data["call"].toCapsule());
+        const bool need_values = call->need_values && ctx->needs_input_grad(0);
+        const bool need_positions = call->need_positions && ctx->needs_input_grad(1);
+        variable_list out(3);
+        if (!need_values && !need_positions) return out;
+        const Tensor grad = grads[0].contiguous();
+        if (at::GradMode::is_enabled()) {
+            const variable_list g = EncodeBackward::apply(grad, saved[0], saved[1], call, need_values, need_positions);
+            if (need_values) out[0] = g[0];
+            if (need_positions) out[1] = g[need_values ? 1 : 0];
+        } else {
+            const Gradients g = backward_or_hook(*call, grad, need_values, need_positions);
+            out[0] = g.values;
+            out[1] = g.positions;
+        }
+        return out;
+    }
+};
+
+c10::intrusive_ptr<Call> make_call(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, const Tensor& positions,
+                                   const Tensor& window, const Tensor& shift, const std::optional<Tensor>& half,
+                                   const std::optional<Tensor>& order, int levels_per_pass) {
+    auto c = c10::make_intrusive<Call>();
+    c->lattice = lattice;
+    c->values = values;
+    c->positions = positions;
+    c->window = window;
+    c->shift = shift;
+    if (half) c->half = *half;
+    if (order) c->order = *order;
+    c->levels_per_pass = levels_per_pass;
+    return c;
+}
+
+// the module's forward: with a graph where one is wanted
+Tensor encode(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, const Tensor& positions, const Tensor& window,
+              const Tensor& shift, const std::optional<Tensor>& half, int levels_per_pass) {
+    auto c = make_call(lattice, values, positions, window, shift, half, std::nullopt, levels_per_pass);
+    if (at::GradMode::is_enabled()) {
+        c->need_values = values.requires_grad();
+        c->need_positions = positions.requires_grad();
+    }
+    if (!c->need_values && !c->need_positions) return run_forward(*c, true);
+    return Encode::apply(values, positions, c);
+}
+
+Tensor forward_mlp(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, const Tensor& positions,
+                   const Tensor& window, const Tensor& shift, const std::optional<Tensor>& half,
+                   const std::optional<Tensor>& order, int levels_per_pass, const std::vector<Tensor>& weights,
+                   const std::vector<std::optional<Tensor>>& biases, int activation, const std::optional<Tensor>& status) {
+    auto c = make_call(lattice, values, positions, window, shift, half, order, levels_per_pass);
+    check_inputs(*c);
+    const c10::Device device = positions.device();
+    if (weights.empty() || weights.size() > 6)
+        fail("the fused network takes 1..6 layers, got " + std::to_string(weights.size()));
+    std::vector<permuto_mlp_layer> layers(weights.size());
+    std::vector<Tensor> keep;
+    int64_t width = lattice->width;
+    for (size_t i = 0; i < weights.size(); ++i) {
+        const std::string where = weights.size() == 1 ? "" : "layer " + std::to_string(i) + ": ";
+        if (weights[i].dim() != 2 || weights[i].size(1) != width)
+            fail(where + "weight should be out_features x " + std::to_string(width) + ", got " + sizes_of(weights[i]));
+        keep.push_back(plain(weights[i], device));
+        layers[i].weight = keep.back().data_ptr<float>();
+        layers[i].in_features = (int32_t)width;
+        width = weights[i].size(0);
+        layers[i].out_features = (int32_t)width;
+        layers[i].bias = nullptr;
+        if (biases[i]) {
+            if (biases[i]->dim() != 1 || biases[i]->size(0) != width)
+                fail(where + "bias should have " + std::to_string(width) + " entries");
+            keep.push_back(plain(*biases[i], device));
+            layers[i].bias = keep.back().data_ptr<float>();
+        }
+    }
+    if (status && (status->scalar_type() != at::kInt || status->device() != device || status->numel() != 1))
+        fail("status should be a one-element int32 tensor on the device of the positions");
+    Bound b(*c);
+    if (!c->order.defined() && api.order_pays(&b.cfg, b.in.nr_positions, 0)) c->order = make_order(*c, b);
+    Tensor out = at::empty({b.in.nr_positions, width}, positions.options());
+    check(api.forward_mlp(&b.cfg, &b.in, data(c->order), layers.data(), (int32_t)layers.size(), activation,
+                          out.data_ptr<float>(), status ? status->data_ptr<int32_t>() : nullptr, stream_of(positions)));
+    return out;
+}
+
+void adam_step(const Tensor& values, const Tensor& grad, const Tensor& exp_avg, const Tensor& exp_avg_sq, int64_t step, double lr,
+               double beta1, double beta2, double eps, double weight_decay, bool skip_untouched, bool zero_grad) {
+    const std::pair<const char*, const Tensor*> all[] = {
+        {"values", &values}, {"grad", &grad}, {"exp_avg", &exp_avg}, {"exp_avg_sq", &exp_avg_sq}};
+    for (const auto& [name, t] : all) {
+        if (!t->is_cuda()) fail(std::string(name) + " should be in GPU memory. There is no CPU path");
+        if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->sizes() != values.sizes() || t->device() != values.device())
+            fail(std::string(name) + " must be a contiguous float32 tensor of the shape and device of the values");
+    }
+    c10::cuda::OptionalCUDAGuard guard;
+    if (values.device().index() != c10::cuda::current_device()) guard.set_device(values.device());
+    check(api.adam_step(values.data_ptr<float>(), grad.data_ptr<float>(), exp_avg.data_ptr<float>(), exp_avg_sq.data_ptr<float>(),
+                        values.numel(), lr, beta1, beta2, eps, weight_decay, step,
+                        (skip_untouched ? PERMUTO_ADAM_SKIP_UNTOUCHED : 0) | (zero_grad ? PERMUTO_ADAM_ZERO_GRAD : 0),
+                        stream_of(values)));
+    // the kernel wrote through the raw pointer: tell autograd (and the module's fp16 copy) so
+    values.unsafeGetTensorImpl()->bump_version();
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    m.def("bind_api", &bind_api);
+    py::class_<Lattice, c10::intrusive_ptr<Lattice>>(m, "Lattice")
+        .def(py::init<int, int, int, int, bool, double, int64_t, Tensor>())
+        .def_readwrite("aggregate", &Lattice::aggregate)
+        .def_readwrite("concat_positions_grad", &Lattice::concat_positions_grad)
+        .def("scale_on", [](Lattice& l, const c10::Device& d) { return l.scale_on(d); })
+        .def("set_hooks", [](Lattice& l, const py::object& backward, const py::object& double_backward) {
+            l.on_backward = backward.is_none() ? py::object() : backward;
+            l.on_double_backward = double_backward.is_none() ? py::object() : double_backward;
+        });
+    m.def("encode", &encode);
+    m.def("forward", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w, const Tensor& s,
+                        const std::optional<Tensor>& half, const std::optional<Tensor>& order, int lpp) {
+        auto c = make_call(l, v, p, w, s, half, order, lpp);
+        return run_forward(*c, false);
+    });
+    m.def("check_inputs", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w,
+                             const Tensor& s, const std::optional<Tensor>& half) {
+        check_inputs(*make_call(l, v, p, w, s, half, std::nullopt, 0));
+    });
+    m.def("order", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w, const Tensor& s,
+                      const std::optional<Tensor>& half, int lpp, int purpose) -> std::optional<Tensor> {
+        auto c = make_call(l, v, p, w, s, half, std::nullopt, lpp);
+        check_inputs(*c);
+        Bound b(*c);
+        if (purpose >= 0 && !api.order_pays(&b.cfg, b.in.nr_positions, purpose)) return std::nullopt;
+        return make_order(*c, b);
+    });
+    m.def("backward", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w, const Tensor& s,
+                         const std::optional<Tensor>& half, const std::optional<Tensor>& order, int lpp, const Tensor& grad,
+                         bool need_values, bool need_positions, const std::optional<Tensor>& values_out, int level_begin,
+                         int level_end, bool zero, const std::optional<Tensor>& positions_out) {
+        auto c = make_call(l, v, p, w, s, half, order, lpp);
+        const Gradients g = run_backward(*c, grad, need_values, need_positions, values_out ? *values_out : Tensor(), level_begin,
+                                         level_end, zero, positions_out ? *positions_out : Tensor());
+        return py::make_tuple(as_python(g.values), as_python(g.positions));
+    });
+    m.def("double_backward", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w,
+                                const Tensor& s, const std::optional<Tensor>& half, const std::optional<Tensor>& order, int lpp,
+                                const Tensor& dpg, const Tensor& grad, bool need_values, bool need_features) {
+        auto c = make_call(l, v, p, w, s, half, order, lpp);
+        const SecondOrder r = run_double_backward(*c, dpg, grad, need_values, need_features);
+        return py::make_tuple(as_python(r.values), as_python(r.features));
+    });
+    m.def("forward_mlp", &forward_mlp);
+    m.def("adam_step", &adam_step);
+}

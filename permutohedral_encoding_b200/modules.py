@@ -5,7 +5,6 @@ import math
 import torch
 
 from . import _native as _C
-from .funcs import PermutoEncodingFunc
 from .utils import cosine_easing_window
 
 
@@ -117,18 +116,8 @@ class PermutoEncoding(torch.nn.Module):
         self.fixed_params.m_random_shift_per_level = self.random_shift_per_level
 
         half = self._half_copy() if getattr(self, "half_precision_table", False) else None
-        grad_mode = torch.is_grad_enabled()
-        require_lattice_values_grad = self.lattice_values.requires_grad and grad_mode
-        require_positions_grad = positions.requires_grad and grad_mode
-        if not (require_lattice_values_grad or require_positions_grad):
-            # inference: nothing to record, skip the autograd machinery (host overhead dominates
-            # README-sized batches)
-            return self.lattice.forward(_C.EncodingInput(self.lattice_values, positions, anneal_window, False, False,
-                                                         half))
-
         # [N, (L+extra)*F] already in the reference's output order: no permute/reshape copy
-        return PermutoEncodingFunc.apply(self.lattice, self.lattice_values, positions, anneal_window,
-                                         require_lattice_values_grad, require_positions_grad, half)
+        return self.lattice.encode(self.lattice_values, positions, anneal_window, half)
 
     def _half_copy(self):
         """fp16 copy of the lattice values the kernels gather from when ``half_precision_table`` is

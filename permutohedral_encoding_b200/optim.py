@@ -19,18 +19,8 @@ def adam_step(values: torch.Tensor, grad: torch.Tensor, exp_avg: torch.Tensor, e
               lr: float, betas=(0.9, 0.999), eps: float = 1e-8, weight_decay: float = 0.0, skip_untouched: bool = False,
               zero_grad: bool = False) -> None:
     """In-place AdamW step on raw tensors (all fp32, contiguous, same shape, same CUDA device)."""
-    for name, t in (("values", values), ("grad", grad), ("exp_avg", exp_avg), ("exp_avg_sq", exp_avg_sq)):
-        if not t.is_cuda:
-            raise RuntimeError(f"{name} should be in GPU memory. There is no CPU path")
-        if t.dtype != torch.float32 or not t.is_contiguous() or t.shape != values.shape or t.device != values.device:
-            raise RuntimeError(f"{name} must be a contiguous float32 tensor of the shape and device of the values")
-    flags = (_C.PERMUTO_ADAM_SKIP_UNTOUCHED if skip_untouched else 0) | (_C.PERMUTO_ADAM_ZERO_GRAD if zero_grad else 0)
-    with _C._guard(values.device):
-        _C.check(_C.lib.permuto_adam_step(values.data_ptr(), grad.data_ptr(), exp_avg.data_ptr(), exp_avg_sq.data_ptr(),
-                                          values.numel(), float(lr), float(betas[0]), float(betas[1]), float(eps),
-                                          float(weight_decay), int(step), flags, _C._stream(values.device)))
-    # the kernel wrote through the raw pointer: tell autograd (and the module's fp16 copy) so
-    torch.autograd.graph.increment_version(values)
+    _C._ext.adam_step(values, grad, exp_avg, exp_avg_sq, int(step), float(lr), float(betas[0]), float(betas[1]), float(eps),
+                      float(weight_decay), bool(skip_untouched), bool(zero_grad))
 
 
 class LatticeAdamW(torch.optim.Optimizer):

@@ -1,0 +1,84 @@
+"""What the C++ autograd nodes compute for each way of asking: only the gradients that the running
+backward needs, with the values of a full backward."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture()
+def setup():
+    from permutohedral_encoding_b200 import PermutoEncoding
+    torch.manual_seed(11)
+    m = PermutoEncoding(3, 2 ** 12, 6, 2, np.geomspace(1.0, 1e-2, 6))
+    with torch.no_grad():
+        m.lattice_values.uniform_(-1, 1)
+    pos = torch.rand(500, 3, device=DEV, requires_grad=True)
+    return m, pos, torch.randn(500, 12, device=DEV)
+
+
+def _close(a, b):
+    assert torch.all((a - b).abs() <= 1e-4 * b.abs().amax())
+
+
+def test_restricted_backwards_match_the_full_one(setup):
+    m, pos, go = setup
+    m(pos).backward(go)
+    want_v, want_p = m.lattice_values.grad.clone(), pos.grad.clone()
+    m.lattice_values.grad = pos.grad = None
+    (p,) = torch.autograd.grad(m(pos), pos, go)
+    _close(p, want_p)
+    (v,) = torch.autograd.grad(m(pos), m.lattice_values, go)
+    _close(v, want_v)
+    torch.autograd.backward([m(pos)], [go], inputs=[m.lattice_values])
+    _close(m.lattice_values.grad, want_v)
+    assert pos.grad is None
+
+
+def test_double_backward_and_hooks(setup):
+    """create_graph keeps the position gradient differentiable; hooks installed between forward and
+    backward are called, with the gradients they return used."""
+    m, pos, go = setup
+    go.requires_grad_(True)
+    dpg = torch.randn(500, 3, device=DEV)
+    (p,) = torch.autograd.grad(m(pos), pos, go, create_graph=True)
+    p.backward(dpg)
+    want_v, want_g = m.lattice_values.grad.clone(), go.grad.clone()
+    assert torch.count_nonzero(want_g) > 0
+    m.lattice_values.grad = go.grad = None
+    (p,) = torch.autograd.grad(m(pos), pos, go, create_graph=True)
+    m.lattice.double_backward_hook = lambda g: 2.0 * g
+    p.backward(dpg)
+    m.lattice.double_backward_hook = None
+    _close(m.lattice_values.grad, 2.0 * want_v)
+    _close(go.grad, want_g)
+
+    pos2 = pos.detach()
+    m.lattice_values.grad = None
+    m(pos2).backward(go.detach())
+    want = m.lattice_values.grad.clone()
+    m.lattice_values.grad = None
+    out = m(pos2)
+    seen = []
+
+    def hook(lattice, inp, grad):
+        seen.append(grad.shape)
+        g, p = lattice.backward(inp, grad)
+        return 3.0 * g, p
+
+    m.lattice.backward_hook = hook
+    out.backward(go.detach())
+    m.lattice.backward_hook = None
+    assert seen == [go.shape]
+    _close(m.lattice_values.grad, 3.0 * want)
+
+
+def test_saved_tensors_are_guarded(setup):
+    m, pos, go = setup
+    out = m(pos)
+    with torch.no_grad():
+        m.lattice_values.mul_(2.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.backward(go)

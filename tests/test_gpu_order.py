@@ -1,0 +1,91 @@
+"""Spatial order of a batch: it is a permutation that carries the coordinates, and every operation
+gives with it what it gives without it -- forward and per-point gradients bit for bit (a point's
+arithmetic does not depend on its neighbours), table gradients within the bound of summing the same
+fp32 addends in another order, 1e-4 * sum|addend|.  Sizes around the kernels' edges: one point, one
+thread's group of points, warps, blocks, several blocks; feature rows with and without 32-byte
+alignment; identical points and points far outside the bulk of the batch."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def nat():
+    from permutohedral_encoding_b200 import _native
+    return _native
+
+
+def _setup(nat, d, feat, levels, n, seed, concat=False, half=False, shape="box"):
+    gen = torch.Generator(device=DEV).manual_seed(seed)
+    cap = 2 ** 12 if d != 4 else 3001
+    shift = torch.randn((levels, d), device=DEV, generator=gen) * 10
+    fx = nat.EncodingFixedParams(d, cap, levels, feat, np.geomspace(1.0, 1e-3, levels), shift, concat, 0.5)
+    enc = nat.EncodingWrapper.create(d, feat, fx)
+    table = torch.randn((levels, cap, feat), device=DEV, generator=gen)
+    pos = torch.rand((n, d), device=DEV, generator=gen) * 2 - 1
+    if shape == "same":
+        pos[:] = pos[0].clone()
+    elif shape == "outliers":
+        pos[::97] *= 1e6
+        pos[1::101, 0] = float("inf")
+    elif shape == "flat":
+        pos[:, 1:] = 0.25
+    window = torch.rand(levels, device=DEV, generator=gen)
+    window[0] = 0.0
+    inp = nat.EncodingInput(table.half() if half else table, pos, window, True, True)
+    go = torch.randn((n, enc.output_width()), device=DEV, generator=gen)
+    return enc, inp, go, torch.randn((n, d), device=DEV, generator=gen)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 255, 257, 1025, 30011])
+@pytest.mark.parametrize("d,feat,levels,concat,half", [(2, 2, 7, False, False), (3, 2, 8, False, True), (3, 2, 5, True, False),
+                                                       (4, 4, 5, False, False), (6, 2, 12, False, False), (3, 8, 3, True, True),
+                                                       (7, 4, 34, False, False)])
+def test_ordered_equals_unordered(nat, n, d, feat, levels, concat, half):
+    enc, inp, go, dpg = _setup(nat, d, feat, levels, n, n + d, concat, half)
+    only_table = nat.EncodingInput(inp.m_lattice_values, inp.m_positions_raw, inp.m_anneal_window, True, False)
+    only_pos = nat.EncodingInput(inp.m_lattice_values, inp.m_positions_raw, inp.m_anneal_window, False, True)
+
+    def run(order):
+        inp.m_order = only_table.m_order = only_pos.m_order = order
+        tables = [enc.backward(only_table, go)[0], enc.backward(inp, go)[0], enc.double_backward_from_positions(inp, dpg, go)[0]]
+        rows = [enc.forward(inp), enc.double_backward_from_positions(inp, dpg, go)[1]]
+        points = [enc.backward(inp, go)[1], enc.backward(only_pos, go)[1]]
+        return tables, rows, points
+
+    plain, ordered = run(None), run(enc.order(inp))
+    magnitude = [enc.backward(only_table, go.abs())[0]] * 2 + [plain[0][2].abs().amax().expand_as(plain[0][2])]
+    for a, b, m in zip(plain[0], ordered[0], magnitude):
+        assert torch.all((a - b).abs() <= 1e-4 * m + 1e-6 * m.amax())
+    for a, b in zip(plain[1], ordered[1]):
+        assert torch.equal(a, b)
+    for a, b in zip(plain[2], ordered[2]):   # sums over sweeps of levels: same addends, another grouping
+        assert torch.all((a - b).abs() <= 1e-5 * a.abs().amax())
+
+
+@pytest.mark.parametrize("shape", ["box", "same", "outliers", "flat"])
+@pytest.mark.parametrize("d,n", [(2, 5000), (3, 1), (3, 4097), (5, 9000), (3, 2 ** 22 + 1025)])
+def test_order_is_a_permutation_with_coordinates(nat, shape, d, n):
+    enc, inp, _, _ = _setup(nat, d, 2, 4, n, 3, shape=shape)
+    words = 4 if d <= 3 else 8
+    rec = enc.order(inp)[:4 * words * n].view(torch.int32).view(n, words)
+    idx = rec[:, words - 1].long()
+    assert torch.equal(torch.sort(idx).values, torch.arange(n, device=DEV))
+    assert torch.equal(rec[:, :d].contiguous(), inp.m_positions_raw[idx].view(torch.int32))
+
+
+def test_module_orders_large_batches(nat):
+    """The module's own rule: above the threshold the batch is ordered, and nothing shows but time."""
+    from permutohedral_encoding_b200 import PermutoEncoding
+    torch.manual_seed(5)
+    m = PermutoEncoding(3, 2 ** 14, 8, 2, np.geomspace(1.0, 1e-3, 8))
+    pos = torch.rand(2 ** 19 + 77, 3, device=DEV)
+    inp = nat.EncodingInput(m.lattice_values.detach(), pos, m.anneal_window, False, False)
+    assert m.lattice.order(inp, nat.ORDER_TRAINING) is not None
+    with torch.no_grad():
+        assert torch.equal(m(pos), m.lattice.forward(inp))
+    small = nat.EncodingInput(m.lattice_values.detach(), pos[:1000], m.anneal_window, False, False)
+    assert m.lattice.order(small, nat.ORDER_TRAINING) is None
