@@ -141,6 +141,7 @@ def _load_torch_side():
 
 
 _ext = _load_torch_side()
+encode = _ext.encode
 
 
 def last_error() -> str:
@@ -304,13 +305,6 @@ class EncodingWrapper:
 
     def output_width(self) -> int:
         return self._width
-
-    def encode(self, lattice_values, positions, anneal_window, lattice_values_half=None) -> torch.Tensor:
-        """features [N, F*(L+extra)], recorded for autograd where the lattice values or the positions
-        require a gradient."""
-        fp = self.fixed
-        return _ext.encode(self._native, lattice_values, positions, anneal_window, fp.m_random_shift_per_level,
-                           lattice_values_half, fp.levels_per_pass)
 
     def order(self, inp: EncodingInput, purpose: int = ORDER_ALWAYS):
         """Spatial order of the positions (an opaque device buffer), or None where the batch is too

@@ -62,7 +62,7 @@ def _torch_command():
     return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_permuto_torch",
              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
             + [f for i in inc for f in ("-isystem", i)] + [TORCH_SOURCE, "-o", TORCH_PATH, "-L", os.path.join(root, "lib"),
-               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
+               "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"])
 
 
 def _run(cmd, verbose):

@@ -115,9 +115,9 @@ __device__ __forceinline__ void to_remainders(int s, T (&v)[D + 1]) {
 
 // ---- level constants in shared memory ---------------------------------------------------------
 // A level's weight, shift and scale are 2D+1 floats that every thread of a block reads: staged once
-// per block they cost a point one or two 16-byte shared loads per level instead of 2D+1 global ones
+// per block they cost a point two to four 16-byte shared loads per level instead of 2D+1 global ones
 // (7 of the 11 load instructions of a level at pos_dim 3).
-constexpr int kRecord = (2 * D + 1 + 3) / 4 * 4;
+constexpr int kRecord = (2 * D + 2 + 3) / 4 * 4;  // weight, shift, scale, reach
 constexpr int kStage = 32;  // levels staged at a time
 
 __device__ __forceinline__ void stage_levels(const Problem& p, int begin, int end, float* table) {
@@ -127,6 +127,7 @@ __device__ __forceinline__ void stage_levels(const Problem& p, int begin, int en
         if (c == 0) v = __ldg(p.anneal + l);
         else if (c <= D) v = __ldg(p.shift + l * D + c - 1);
         else if (c <= 2 * D) v = __ldg(p.scale + l * D + c - 1 - D);
+        else if (c == 2 * D + 1) v = exact_reach<D>(p.shift + l * D, p.scale + l * D);
         table[i] = v;
     }
 }
@@ -141,6 +142,7 @@ __device__ __forceinline__ void load_level(const float* table, int i, LevelConst
         v[4 * j + 3] = t.w;
     }
     lc.weight = v[0];
+    lc.reach = v[2 * D + 1];
 #pragma unroll
     for (int j = 0; j < D; ++j) {
         lc.shift[j] = v[1 + j];
@@ -318,8 +320,8 @@ __device__ __forceinline__ void store_row_segment(const Problem& p, float* rows,
 // One step of a point's feature row: LPS levels of F features (8 floats) starting at level l0;
 // levels at or beyond `end` give zeros (EncodingGPU.cuh:130-254 for one level).
 template <int F, int LPS, bool HALF>
-__device__ __forceinline__ void encode_step(const Problem& p, const float* levels, const float (&pos)[D], int l0, int end,
-                                            float (&out)[F * LPS]) {
+__device__ __forceinline__ void encode_step(const Problem& p, const float* levels, const float (&pos)[D], float largest,
+                                            int l0, int end, float (&out)[F * LPS]) {
 #pragma unroll
     for (int k = 0; k < LPS; ++k) {
         const int l = l0 + k;
@@ -331,7 +333,7 @@ __device__ __forceinline__ void encode_step(const Problem& p, const float* level
             load_level(levels, k, lc);
             if (lc.weight != 0.0f) {  // a closed coarse-to-fine window contributes exact zeros
                 Simplex<D> s;
-                locate_simplex<D>(pos, lc, s);
+                locate_simplex<D>(pos, largest, lc, s);
                 uint32_t slot[D + 1];
                 to_slots(p, s, slot);
                 float v[D + 1][F];
@@ -362,6 +364,7 @@ __global__ void __launch_bounds__(kThreads, (F == 2 ? PERMUTO_MIN_BLOCKS_FORWARD
 
     float pos[D];
     const int64_t n = load_point(p, active ? i_raw : p.n_points - 1, pos);  // idle threads shadow the last point
+    const float largest = largest_coordinate<D>(pos);
 
 #pragma unroll 1
     for (int begin = pass_begin; begin < pass_end; begin += kStage) {
@@ -376,7 +379,7 @@ __global__ void __launch_bounds__(kThreads, (F == 2 ? PERMUTO_MIN_BLOCKS_FORWARD
             const int l0 = begin + step * LPS;
             step = (step + 1 == nsteps) ? 0 : step + 1;
             float out[F * LPS];
-            encode_step<F, LPS, HALF>(p, levels + (l0 - begin) * kRecord, pos, l0, end, out);
+            encode_step<F, LPS, HALF>(p, levels + (l0 - begin) * kRecord, pos, largest, l0, end, out);
             if (active) store_row_segment<F, LPS>(p, a.features, n, l0, out);
         }
     }
@@ -644,6 +647,7 @@ forward_mlp_kernel(const ForwardLinearArgs a) {
     {
         float pos[D];
         n = load_point(p, active ? i_raw : p.n_points - 1, pos);  // idle rows shadow the last point and are not stored
+        const float largest = largest_coordinate<D>(pos);
         const int lattice_cols = F * p.nr_levels;
         // a column past the lattice levels: a concatenated raw coordinate (EncodingGPU.cuh:105-121) or padding
         auto tail_value = [&](int c) -> float {
@@ -662,7 +666,7 @@ forward_mlp_kernel(const ForwardLinearArgs a) {
             float out[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) out[i] = 0.f;
-            if (s < nsteps) encode_step<F, LPS, HALF>(p, levels + s * LPS * kRecord, pos, s * LPS, p.nr_levels, out);
+            if (s < nsteps) encode_step<F, LPS, HALF>(p, levels + s * LPS * kRecord, pos, largest, s * LPS, p.nr_levels, out);
             if (8 * s + 8 > lattice_cols) {  // block-uniform: only the last step(s) reach past the lattice levels
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
@@ -911,6 +915,29 @@ __device__ __forceinline__ void scatter_level(Scatter& sc, float* level_base, in
     }
 }
 
+// d loss / d barycentric weight of every vertex, times the level weight (EncodingGPU.cuh:1187-1218)
+__device__ __forceinline__ void second_order_weights(const Simplex<D>& s, const LevelConst<D>& lc, const float (&dpg)[D],
+                                                     float (&dBw)[D + 1]) {
+    float gsd[D], dE[D + 1];  // d loss / d elevated
+#pragma unroll
+    for (int i = 0; i < D; ++i) gsd[i] = dpg[i] * lc.scale[i];
+#pragma unroll
+    for (int j = 0; j <= D; ++j) dE[j] = 0.f;
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+#pragma unroll
+        for (int j = 0; j <= i; ++j) dE[j] += gsd[i];
+    }
+#pragma unroll
+    for (int i = 0; i < D; ++i) dE[i + 1] -= gsd[i] * (float)(i + 1);
+#pragma unroll
+    for (int i = 0; i <= D; ++i) dE[i] *= 1.0f / (D + 1);
+    to_ranks(s, dE);  // the gaps of dE in rank order
+#pragma unroll
+    for (int m = 1; m <= D; ++m) dBw[m] = (dE[D - m] - dE[D + 1 - m]) * lc.weight;
+    dBw[0] = (dE[D] - dE[0]) * lc.weight;
+}
+
 // ------------------------------------------------------------------------------------------
 // first-order backward: table gradient (scatter) and/or position gradient (gather)
 // ------------------------------------------------------------------------------------------
@@ -928,6 +955,7 @@ backward_kernel(const BackwardArgs a) {
 
     float pos[D];
     const int64_t n = load_point(p, active ? i_raw : p.n_points - 1, pos);  // idle lanes shadow the last point
+    const float largest = largest_coordinate<D>(pos);
 
     float dpos[D];
 #pragma unroll
@@ -963,7 +991,7 @@ backward_kernel(const BackwardArgs a) {
                 load_level(levels, l - begin, lc);
                 if (lc.weight == 0.0f) continue;  // every addend of this level is an exact zero
                 Simplex<D> s;
-                locate_simplex<D>(pos, lc, s);
+                locate_simplex<D>(pos, largest, lc, s);
                 uint32_t slot[D + 1];
                 to_slots(p, s, slot);
 
@@ -1036,18 +1064,107 @@ backward_kernel(const BackwardArgs a) {
 constexpr int kRunPoints = PERMUTO_RUN_POINTS;
 constexpr int kRunThreads = PERMUTO_RUN_THREADS;
 constexpr int kPosVec = D <= 3 ? 1 : 2;  // float4s per point: coordinates, row index last
+// D floats kept as kPosVec float4s, kRunThreads apart
+__device__ __forceinline__ void load_vec(const float4* src, float (&x)[D]) {
+#pragma unroll
+    for (int i = 0; i < kPosVec; ++i) {
+        const float4 v = src[i * kRunThreads];
+        x[4 * i] = v.x;
+        if (4 * i + 1 < D) x[(4 * i + 1) % D] = v.y;
+        if (4 * i + 2 < D) x[(4 * i + 2) % D] = v.z;
+        if (4 * i + 3 < D) x[(4 * i + 3) % D] = v.w;
+    }
+}
+template <bool DOUBLE>
 struct RunStage {
     float levels[kStage * kRecord];
     float4 point[kRunPoints][kPosVec][kRunThreads];
+    float4 dpg[DOUBLE ? kRunPoints : 1][DOUBLE ? kPosVec : 1][DOUBLE ? kRunThreads : 1];
     float4 grad[kRunPoints][2][kRunThreads];  // gradient row segments: [point][4 floats of the step][thread]
 };
+// Sum over the warp of CNT vertices' addends by recursive halving: at each step a lane keeps one half of
+// the vertices and hands the other half to its partner, so CNT = 4 vertices take 4+2+1 exchanges of F
+// values where a butterfly per value takes 20.  The last step's owners add their vertex to the table.
+template <int F, int CNT>
+__device__ __forceinline__ void reduce_vertices(float* level_base, unsigned lane, int bit, int vertex, uint32_t (&slot)[CNT],
+                                                float (&v)[CNT][F]) {
+    if constexpr (CNT == 1) {
+        for (int b = bit; b > 0; b >>= 1) {
+#pragma unroll
+            for (int f = 0; f < F; ++f) v[0][f] += __shfl_xor_sync(kFullMask, v[0][f], b);
+        }
+        if ((lane & (2u * bit - 1u)) == 0u && vertex <= D) red_add<F>(level_base, slot[0], v[0]);
+    } else {
+        constexpr int H = (CNT + 1) / 2;
+        const bool up = (lane & bit) != 0u;
+        uint32_t s[H];
+        float k[H][F];
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+            const bool pair = i + H < CNT;
+            s[i] = (up && pair) ? slot[pair ? i + H : i] : slot[i];
+#pragma unroll
+            for (int f = 0; f < F; ++f) {
+                const float a = v[i][f], b = pair ? v[pair ? i + H : i][f] : 0.f;
+                k[i][f] = (up ? b : a) + __shfl_xor_sync(kFullMask, up ? a : b, bit);
+            }
+        }
+        reduce_vertices<F, H>(level_base, lane, bit >> 1, up ? vertex + H : vertex, s, k);
+    }
+}
+
+// The addends of a warp whose lanes sit in at most kFewSimplices simplices (coarse levels): one reduction
+// per simplex.  False, with nothing done, otherwise.
+#ifndef PERMUTO_FEW_SIMPLICES
+#define PERMUTO_FEW_SIMPLICES 3
+#endif
+constexpr int kFewSimplices = PERMUTO_FEW_SIMPLICES;
 template <int F>
-__global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_kernel(const BackwardArgs a) {
+__device__ __forceinline__ bool merge_simplices(float* level_base, unsigned lane, const uint32_t (&slot)[D + 1],
+                                                const float (&add)[D + 1][F]) {
+    uint32_t key = slot[0];
+#pragma unroll
+    for (int r = 1; r <= D; ++r) key = key * 0x9E3779B1u + slot[r];
+    const int leader = __ffs(__match_any_sync(kFullMask, key)) - 1;
+    bool same = true;  // equal keys have to mean equal slots
+#pragma unroll
+    for (int r = 0; r <= D; ++r) same = (__shfl_sync(kFullMask, slot[r], leader) == slot[r]) && same;
+    unsigned leaders = __ballot_sync(kFullMask, leader == (int)lane);
+    if (!__all_sync(kFullMask, same) || __popc(leaders) > kFewSimplices) return false;
+#pragma unroll 1
+    do {
+        const int of = __ffs(leaders) - 1;
+        leaders &= leaders - 1u;
+        uint32_t s[D + 1];
+        float v[D + 1][F];
+#pragma unroll
+        for (int r = 0; r <= D; ++r) {
+            s[r] = __shfl_sync(kFullMask, slot[r], of);
+#pragma unroll
+            for (int f = 0; f < F; ++f) v[r][f] = leader == of ? add[r][f] : 0.f;
+        }
+        reduce_vertices<F, D + 1>(level_base, lane, 16, 0, s, v);
+    } while (leaders);
+    return true;
+}
+
+struct RunArgs {
+    Problem p;
+    const float* grad_features;
+    const float* double_positions_grad;  // double backward only
+    float* lattice_grad;
+    int32_t aggregate;
+};
+
+// DOUBLE: the addends are those of the double backward, weight d loss / d barycentric instead of the
+// barycentric weight
+template <int F, bool DOUBLE>
+__global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_kernel(const RunArgs a) {
     constexpr int P = kRunPoints;
     constexpr int LPS = 8 / F;
     const Problem& p = a.p;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    RunStage& sm = *reinterpret_cast<RunStage*>(smem_raw);
+    RunStage<DOUBLE>& sm = *reinterpret_cast<RunStage<DOUBLE>*>(smem_raw);
     const int t = threadIdx.x;
     const int pass_begin = p.level_begin + (int)blockIdx.y * p.levels_per_pass;
     const int pass_end = min(pass_begin + p.levels_per_pass, p.level_end);
@@ -1065,6 +1182,12 @@ __global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_
         r[4 * kPosVec - 1] = __uint_as_float((uint32_t)n);
 #pragma unroll
         for (int i = 0; i < kPosVec; ++i) sm.point[j][i][t] = make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+        if (DOUBLE) {
+#pragma unroll
+            for (int i = 0; i < 4 * kPosVec; ++i) r[i] = i < D ? __ldg(a.double_positions_grad + n * D + i) : 0.f;
+#pragma unroll
+            for (int i = 0; i < kPosVec; ++i) sm.dpg[j][i][t] = make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+        }
     }
     Scatter sc{threadIdx.x & 31u, true, a.aggregate != 0};
 
@@ -1114,14 +1237,7 @@ __global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_
 #pragma unroll 1
                 for (int j = 0; j < P; ++j) {
                     float x[D], g[F];
-#pragma unroll
-                    for (int i = 0; i < kPosVec; ++i) {
-                        const float4 v = sm.point[j][i][t];
-                        x[4 * i] = v.x;
-                        x[4 * i + 1] = v.y;
-                        if (4 * i + 2 < D) x[(4 * i + 2) % D] = v.z;
-                        if (4 * i + 3 < D) x[(4 * i + 3) % D] = v.w;
-                    }
+                    load_vec(&sm.point[j][0][t], x);
                     {
                         const float4* src = &sm.grad[j][F * k / 4][t];
                         if (F == 2) {
@@ -1140,11 +1256,17 @@ __global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_
                         }
                     }
                     Simplex<D> s;
-                    locate_simplex<D>(x, lc, s);
+                    locate_simplex<D>(x, largest_coordinate<D>(x), lc, s);
                     uint32_t slot[D + 1];
                     to_slots(p, s, slot);
                     float w[D + 1];
-                    vertex_weights<D>(s, lc.weight * kInv, w);
+                    if (DOUBLE) {
+                        float dpg[D];
+                        load_vec(&sm.dpg[j][0][t], dpg);
+                        second_order_weights(s, lc, dpg, w);
+                    } else {
+                        vertex_weights<D>(s, lc.weight * kInv, w);
+                    }
                     if (runs) {
                         to_remainders(s.s, slot);
                         to_remainders(s.s, w);
@@ -1171,6 +1293,7 @@ __global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_
                     const unsigned lane = sc.lane;
                     const unsigned group0 = __match_any_sync(kFullMask, cur[0]);
                     const int distinct = __popc(__ballot_sync(kFullMask, (group0 & ((1u << lane) - 1u)) == 0u));
+                    if (distinct <= 2 && merge_simplices<F>(gbase, lane, cur, acc)) continue;
                     if (distinct <= kMergeBelow) {
                         merge_from<F, 0>(sc, gbase, cur, acc, group0);
                     } else {
@@ -1197,10 +1320,10 @@ __global__ void __launch_bounds__(kThreads, min_blocks(F, false)) double_backwar
     const int pass_begin = p.level_begin + (int)blockIdx.y * p.levels_per_pass;
     const int pass_end = min(pass_begin + p.levels_per_pass, p.level_end);
     const unsigned lane = threadIdx.x & 31u;
-    constexpr float kInv = 1.0f / (D + 1);
 
     float pos[D], dpg[D];
     const int64_t n = load_point(p, active ? i_raw : p.n_points - 1, pos);
+    const float largest = largest_coordinate<D>(pos);
 #pragma unroll
     for (int i = 0; i < D; ++i) dpg[i] = __ldg(a.double_positions_grad + n * D + i);
     Scatter sc{lane, active, a.aggregate != 0};  // as in backward_kernel
@@ -1238,31 +1361,12 @@ __global__ void __launch_bounds__(kThreads, min_blocks(F, false)) double_backwar
                     load_level(levels, l - begin, lc);
                     if (lc.weight != 0.0f) {
                         Simplex<D> s;
-                        locate_simplex<D>(pos, lc, s);
+                        locate_simplex<D>(pos, largest, lc, s);
                         uint32_t slot[D + 1];
                         to_slots(p, s, slot);
 
-                        // d loss / d elevated (EncodingGPU.cuh:1187-1199)
-                        float gsd[D], dE[D + 1];
-#pragma unroll
-                        for (int i = 0; i < D; ++i) gsd[i] = dpg[i] * lc.scale[i];
-#pragma unroll
-                        for (int j = 0; j <= D; ++j) dE[j] = 0.f;
-#pragma unroll
-                        for (int i = 0; i < D; ++i) {
-#pragma unroll
-                            for (int j = 0; j <= i; ++j) dE[j] += gsd[i];
-                        }
-#pragma unroll
-                        for (int i = 0; i < D; ++i) dE[i + 1] -= gsd[i] * (float)(i + 1);
-                        // d loss / d barycentric (EncodingGPU.cuh:1213-1218): the gaps of dE in rank order
-#pragma unroll
-                        for (int i = 0; i <= D; ++i) dE[i] *= kInv;
-                        to_ranks(s, dE);
-                        float dBw[D + 1];  // dB * level weight
-#pragma unroll
-                        for (int m = 1; m <= D; ++m) dBw[m] = (dE[D - m] - dE[D + 1 - m]) * lc.weight;
-                        dBw[0] = (dE[D] - dE[0]) * lc.weight;
+                        float dBw[D + 1];
+                        second_order_weights(s, lc, dpg, dBw);
 
                         if (GGF) {
 #pragma unroll
@@ -1306,13 +1410,15 @@ __global__ void __launch_bounds__(kThreads) debug_kernel(const DebugArgs a) {
     load_pos(p, n, pos);
     LevelConst<D> lc;
     lc.weight = 1.0f;
+    lc.reach = exact_reach<D>(p.shift + l * D, p.scale + l * D);
+    const float largest = largest_coordinate<D>(pos);
 #pragma unroll
     for (int i = 0; i < D; ++i) {
         lc.shift[i] = __ldg(p.shift + l * D + i);
         lc.scale[i] = __ldg(p.scale + l * D + i);
     }
     Simplex<D> s;
-    locate_simplex<D>(pos, lc, s);
+    locate_simplex<D>(pos, largest, lc, s);
     uint32_t slot[D + 1];
     to_slots(p, s, slot);
     float w[D + 1];
@@ -1356,7 +1462,7 @@ enum class Traffic { Gather, Scatter, Both };
 inline int pick_levels_per_pass(const Problem& p, int requested, Traffic t, int lps) {
     const int levels = p.level_end - p.level_begin;
     int lpp = requested;
-    if (lpp <= 0 && p.order != nullptr && t != Traffic::Both) {
+    if (lpp <= 0 && p.order != nullptr) {
         lpp = levels;
     } else if (lpp <= 0) {
         const double slice = (p.table_half ? 2.0 : 4.0) * p.nr_feat * p.capacity;
@@ -1412,8 +1518,6 @@ inline bool use_single_level(const Problem& p) {
     return lps > 1 && blocks < 2 * (sms > 0 ? sms : 148);
 }
 
-// table gradient alone of a batch in spatial order
-inline bool use_runs(const BackwardArgs& a) { return a.p.order != nullptr && a.lattice_grad != nullptr && a.positions_grad == nullptr; }
 
 template <class Args>
 inline Args with_schedule(const Args& in, bool single, Traffic t) {
@@ -1466,11 +1570,6 @@ cudaError_t launch_backward(const BackwardArgs& a, cudaStream_t st) {
     if (a.lattice_grad && a.positions_grad) {
         if (h) backward_kernel<F, LPS, true, true, true><<<g, kThreads, 0, st>>>(a);
         else backward_kernel<F, LPS, true, true, false><<<g, kThreads, 0, st>>>(a);
-    } else if (use_runs(a)) {
-        const dim3 gr((unsigned)((a.p.n_points + kRunThreads * kRunPoints - 1) / (kRunThreads * kRunPoints)), g.y);
-        const cudaError_t e = cudaFuncSetAttribute(scatter_runs_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RunStage));
-        if (e != cudaSuccess) return e;
-        scatter_runs_kernel<F><<<gr, kRunThreads, sizeof(RunStage), st>>>(a);
     } else if (a.lattice_grad) {
         backward_kernel<F, LPS, true, false, false><<<g, kThreads, 0, st>>>(a);
     } else if (a.positions_grad) {
@@ -1494,6 +1593,27 @@ cudaError_t launch_double(const DoubleBackwardArgs& a, cudaStream_t st) {
         else double_backward_kernel<F, LPS, false, true, false><<<g, kThreads, 0, st>>>(a);
     }
     return cudaGetLastError();
+}
+
+// whole steps of 8 floats whatever the size of the batch
+template <int F, bool DOUBLE>
+cudaError_t launch_runs(const RunArgs& a, cudaStream_t st) {
+    constexpr int smem = (int)sizeof(RunStage<DOUBLE>);
+    const cudaError_t e = cudaFuncSetAttribute(scatter_runs_kernel<F, DOUBLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    dim3 g = grid_for(a.p);
+    g.x = (unsigned)((a.p.n_points + kRunThreads * kRunPoints - 1) / (kRunThreads * kRunPoints));
+    scatter_runs_kernel<F, DOUBLE><<<g, kRunThreads, smem, st>>>(a);
+    return cudaGetLastError();
+}
+template <bool DOUBLE>
+cudaError_t launch_runs_by_width(const RunArgs& a, cudaStream_t st) {
+    switch (a.p.nr_feat) {
+        case 2: return launch_runs<2, DOUBLE>(a, st);
+        case 4: return launch_runs<4, DOUBLE>(a, st);
+        case 8: return launch_runs<8, DOUBLE>(a, st);
+        default: return cudaErrorInvalidValue;
+    }
 }
 
 // feature width and step size are compile-time: pick the instantiation
@@ -1525,21 +1645,39 @@ cudaError_t PERMUTO_CAT(launch_forward_linear_dim, PERMUTO_DIM)(const ForwardLin
     }
 }
 
+// A batch in spatial order takes its table gradient and what it gathers in two launches: the scatter has a
+// kernel of its own, and the gather alone runs with more warps per SM (pos_dim 3, 24 levels, 2^20 points:
+// 207 + 300 us against 596 fused; without an order the fused kernel is the faster one).
 cudaError_t PERMUTO_CAT(launch_backward_dim, PERMUTO_DIM)(const BackwardArgs& a0, cudaStream_t st) {
-    // the runs kernel takes whole steps of 8 floats, so its sweeps have to start on a step
-    const bool single = use_single_level(a0.p) && !use_runs(a0);
-    const Traffic t = (a0.lattice_grad && a0.positions_grad) ? Traffic::Both
-                                                             : (a0.lattice_grad ? Traffic::Scatter : Traffic::Gather);
-    const BackwardArgs a = with_schedule(a0, single, t);
+    BackwardArgs in = a0;
+    if (in.p.order && in.lattice_grad) {
+        RunArgs r{in.p, in.grad_features, nullptr, in.lattice_grad, in.aggregate};
+        r = with_schedule(r, false, Traffic::Scatter);
+        const cudaError_t e = launch_runs_by_width<false>(r, st);
+        if (e != cudaSuccess || !in.positions_grad) return e;
+        in.lattice_grad = nullptr;
+    }
+    const bool single = use_single_level(in.p);
+    const Traffic t = (in.lattice_grad && in.positions_grad) ? Traffic::Both
+                                                             : (in.lattice_grad ? Traffic::Scatter : Traffic::Gather);
+    const BackwardArgs a = with_schedule(in, single, t);
     PERMUTO_BY_WIDTH(launch_backward, a, single, st)
 }
 
 cudaError_t PERMUTO_CAT(launch_double_backward_dim, PERMUTO_DIM)(const DoubleBackwardArgs& a0, cudaStream_t st) {
-    const bool single = use_single_level(a0.p);
-    const Traffic t = (a0.lattice_grad && a0.grad_grad_features)
+    DoubleBackwardArgs in = a0;
+    if (in.p.order && in.lattice_grad) {
+        RunArgs r{in.p, in.grad_features, in.double_positions_grad, in.lattice_grad, in.aggregate};
+        r = with_schedule(r, false, Traffic::Scatter);
+        const cudaError_t e = launch_runs_by_width<true>(r, st);
+        if (e != cudaSuccess || !in.grad_grad_features) return e;
+        in.lattice_grad = nullptr;
+    }
+    const bool single = use_single_level(in.p);
+    const Traffic t = (in.lattice_grad && in.grad_grad_features)
                           ? Traffic::Both
-                          : (a0.lattice_grad ? Traffic::Scatter : Traffic::Gather);
-    const DoubleBackwardArgs a = with_schedule(a0, single, t);
+                          : (in.lattice_grad ? Traffic::Scatter : Traffic::Gather);
+    const DoubleBackwardArgs a = with_schedule(in, single, t);
     PERMUTO_BY_WIDTH(launch_double, a, single, st)
 }
 

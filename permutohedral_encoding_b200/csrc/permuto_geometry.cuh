@@ -35,14 +35,37 @@ __host__ __device__ constexpr uint32_t hash_step(int i) {
     return hash_all<D>() - (i < D ? (uint32_t)(D + 1) * hash_pow(D - i) : 0u);
 }
 
-// One level's constants.  Kernels keep the records of the levels of a sweep in shared memory
-// (kRecord floats each, moved as 16-byte vectors): weight, then shift and scale of coordinate 0, 1, ...
+// One level's constants.
 template <int D>
 struct LevelConst {
     float weight;
     float shift[D];
     float scale[D];
+    float reach;  // points with every |coordinate| below it elevate to less than 2^22 (exact_reach)
 };
+
+// Largest coordinate for which every elevated coordinate of the level stays below 2^22:
+// |e_i| <= sum_j j * scale_j * (|pos_j| + |shift_j|), j = 1..D, with a margin for the roundings.
+// Testing a point's largest coordinate once against this replaces D+1 maxima per level.
+template <int D>
+__device__ __forceinline__ float exact_reach(const float* __restrict__ shift, const float* __restrict__ scale) {
+    float a = 0.f, b = 0.f;
+#pragma unroll
+    for (int j = 1; j <= D; ++j) {
+        const float s = (float)j * fabsf(__ldg(scale + j - 1));
+        a += s;
+        b = fmaf(s, fabsf(__ldg(shift + j - 1)), b);
+    }
+    return (4194304.0f * 0.9999f - b) / a;  // negative or NaN: no point qualifies
+}
+
+template <int D>
+__device__ __forceinline__ float largest_coordinate(const float (&pos)[D]) {
+    float r = 0.f;
+#pragma unroll
+    for (int i = 0; i < D; ++i) r = fmaxf(r, fabsf(pos[i]));
+    return r;
+}
 
 // The simplex around a point, its vertices numbered q = 0..D along the walk that leaves the
 // *unwrapped* nearest remainder-0 point:
@@ -120,15 +143,19 @@ __device__ __forceinline__ void to_ranks(const Simplex<D>& s, T (&v)[D + 1]) {
 // low mantissa bits, read as an integer for the hash and, after subtracting it again, as a float.
 //  * D+1 a power of two: both additions round upwards, so rounding never crosses a multiple of D+1
 //    from above (the multiple itself is representable) and the ceiling is exact.
-//  * otherwise the reciprocal is inexact: round to nearest, then move by one where the residual is
-//    outside (-(D+1)/2, (D+1)/2].
+//  * otherwise the reciprocal is inexact: round to nearest, then move by ceil((residual - (D+1)/2) /
+//    (D+1)), which is not zero where the residual is outside (-(D+1)/2, (D+1)/2].  The fp32 reciprocals
+//    of 3, 5, 6 and 7 are rounded upwards by 0.25 to 0.75 * 2^-24 of their value: a residual of
+//    -(D+1)/2 gives -1, and the next one above it, rounded upwards by the subtraction to a multiple of
+//    2^-22 or 2^-21, already 0.
 // The residual e - (D+1)*r is exact in both cases (r*(D+1) <= 2|e| or r = 0), which is the
-// reference's -(up - e) or e - down.  From 2^22 on the reference's own expressions are used.
+// reference's -(up - e) or e - down.  Where 2^22 may be exceeded (`largest`, the point's largest
+// coordinate, against the level's reach) the reference's own expressions are used.
 //
 // Instructions per point and level, pos_dim 3: about 110 against 245 for a version with floor,
 // rank counting, rank wrap and select-by-rank.
 template <int D>
-__device__ __forceinline__ void locate_simplex(const float (&pos)[D], const LevelConst<D>& lc, Simplex<D>& s) {
+__device__ __forceinline__ void locate_simplex(const float (&pos)[D], float largest, const LevelConst<D>& lc, Simplex<D>& s) {
     constexpr float kInv = 1.0f / (D + 1);
     constexpr float kDp1 = (float)(D + 1);
     constexpr float kHalf = 0.5f * (D + 1);
@@ -158,13 +185,9 @@ __device__ __forceinline__ void locate_simplex(const float (&pos)[D], const Leve
     }
     e[0] = sm;
 
-    float biggest = 0.0f;
-#pragma unroll
-    for (int i = 0; i <= D; ++i) biggest = fmaxf(biggest, fabsf(e[i]));
-
     float res[D + 1];
     int rint[D + 1];  // R_i / (D+1)
-    if (biggest < 4194304.0f) {
+    if (largest < lc.reach) {
         uint32_t h = 0u;
         int sum = 0;
 #pragma unroll
@@ -178,7 +201,7 @@ __device__ __forceinline__ void locate_simplex(const float (&pos)[D], const Leve
                 w = __fmaf_rn(e[i], kInv, kMagic);
                 r = __fsub_rn(w, kMagic);
                 res[i] = __fmaf_rn(-kDp1, r, e[i]);
-                const float fix = (res[i] > kHalf ? 1.0f : 0.0f) - (res[i] <= -kHalf ? 1.0f : 0.0f);
+                const float fix = __fsub_rn(__fmaf_ru(__fadd_ru(res[i], -kHalf), kInv, kMagic), kMagic);
                 w = __fadd_rn(w, fix);
                 res[i] = __fmaf_rn(-kDp1, fix, res[i]);
             }

@@ -27,7 +27,7 @@ namespace permuto {
 namespace {
 
 #ifndef PERMUTO_CHUNK_BITS
-#define PERMUTO_CHUNK_BITS 22
+#define PERMUTO_CHUNK_BITS 21
 #endif
 #ifndef PERMUTO_CELL_POINTS_BITS
 #define PERMUTO_CELL_POINTS_BITS 3
@@ -36,7 +36,7 @@ constexpr int kChunkBits = PERMUTO_CHUNK_BITS;
 constexpr int kCellBits = PERMUTO_CELL_POINTS_BITS;  // about 2^kCellBits points per cell
 constexpr int kScanBins = 1024;     // cells per block of the scan
 constexpr int kThreads = 256;
-constexpr int kPerThread = 4;       // points per thread, so that a batch of 2^20 is one wave of blocks
+constexpr int kPerThread = 4;       // consecutive points of a thread: whole 16-byte vectors of any row length
 constexpr int kPerBlock = kThreads * kPerThread;
 constexpr int kNibbles = 6;         // a cell coordinate has at most 24 bits
 
@@ -45,6 +45,8 @@ struct OrderArgs {
     int64_t stride_n, stride_d;
     uint32_t n;
     int bits;            // cells per chunk: 2^bits, at least kScanBins
+    int rounds;          // tiles of kPerBlock points per block
+    int vec_ok;          // contiguous rows on a 16-byte boundary
     uint32_t* cursors;   // one per chunk: records handed out
     uint32_t* counters;  // 2^bits per chunk
     uint2* arrival;      // per point: cell, arrival number
@@ -57,25 +59,35 @@ __device__ __forceinline__ void load(const OrderArgs& a, int64_t n, float (&pos)
     for (int i = 0; i < D; ++i) pos[i] = __ldg(a.positions + n * a.stride_n + i * a.stride_d);
 }
 
-// sum over the block of M values per thread; every thread gets it
-template <int M>
-__device__ __forceinline__ void block_sum(float (&v)[M], float* scratch) {
-    constexpr int kWarps = kThreads / 32;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// the kPerThread points from n on; where the batch ends, its last point again
+template <int D>
+__device__ __forceinline__ void load_points(const OrderArgs& a, uint32_t n, float (&x)[kPerThread][D]) {
+    if (a.vec_ok && n + kPerThread <= a.n) {
+        const float4* src = reinterpret_cast<const float4*>(a.positions) + (size_t)n / kPerThread * D;
+        float v[kPerThread * D];
 #pragma unroll
-    for (int i = 0; i < M; ++i) {
+        for (int q = 0; q < D; ++q) {
+            const float4 f = __ldg(src + q);
+            v[4 * q] = f.x;
+            v[4 * q + 1] = f.y;
+            v[4 * q + 2] = f.z;
+            v[4 * q + 3] = f.w;
+        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
-        if (lane == 0) scratch[warp * M + i] = v[i];
+        for (int k = 0; k < kPerThread; ++k) {
+#pragma unroll
+            for (int i = 0; i < D; ++i) x[k][i] = v[k * D + i];
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < kPerThread; ++k) load<D>(a, min(n + k, a.n - 1u), x[k]);
     }
-    __syncthreads();
+}
+
+__device__ __forceinline__ float warp_sum_all(float v) {
 #pragma unroll
-    for (int i = 0; i < M; ++i) {
-        v[i] = scratch[i];
-#pragma unroll
-        for (int w = 1; w < kWarps; ++w) v[i] += scratch[w * M + i];
-    }
-    __syncthreads();
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // Cell of a point: `bits` halvings of the batch's extent, each of the dimension whose cells are widest
@@ -84,46 +96,56 @@ __device__ __forceinline__ void block_sum(float (&v)[M], float* scratch) {
 // from the same 256 points, with the same result.
 template <int D>
 __global__ void __launch_bounds__(kThreads) order_count_kernel(const OrderArgs a) {
-    __shared__ float scratch[kThreads / 32 * (D + 1)];
+    constexpr int kWarps = kThreads / 32;
+    __shared__ float part[2 * D][kWarps];
     __shared__ float lo[D], inv_cell[D];
     __shared__ int halvings[D];
     __shared__ uint8_t key_bit[D][24];                // of a dimension's k-th halving
     __shared__ uint32_t spread[D][kNibbles][16];      // coordinate nibble -> its key bits
-    const uint32_t first = blockIdx.x * (uint32_t)kPerBlock;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t first = blockIdx.x * (uint32_t)a.rounds * kPerBlock;
     const uint32_t chunk = first >> kChunkBits;
     const uint32_t chunk_begin = chunk << kChunkBits;
     const uint32_t chunk_n = min(a.n - chunk_begin, 1u << kChunkBits);
 
     float s[D];
-    load<D>(a, (int64_t)chunk_begin + (int64_t)((uint64_t)threadIdx.x * chunk_n / kThreads), s);
+    load<D>(a, (int64_t)chunk_begin + (int64_t)((uint64_t)t * chunk_n / kThreads), s);
     float x[kPerThread][D];
-#pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        const uint32_t n = first + k * kThreads + threadIdx.x;
-        load<D>(a, min(n, a.n - 1u), x[k]);
-    }
+    load_points<D>(a, first + t * kPerThread, x);
     {
         bool ok = true;  // what is not finite does not take part
 #pragma unroll
         for (int i = 0; i < D; ++i) ok = ok && fabsf(s[i]) < 1e30f;
-        float sum[D + 1], dev[D];
+        const float inv = 1.f / fmaxf((float)__popc(__ballot_sync(0xffffffffu, ok)), 1.f);
 #pragma unroll
-        for (int i = 0; i < D; ++i) sum[i] = ok ? s[i] : 0.f;
-        sum[D] = ok ? 1.f : 0.f;
-        block_sum<D + 1>(sum, scratch);
-        const float inv = 1.f / fmaxf(sum[D], 1.f);
+        for (int i = 0; i < D; ++i) {
+            const float mean = warp_sum_all(ok ? s[i] : 0.f) * inv;
+            const float dev = warp_sum_all(ok ? fabsf(s[i] - mean) : 0.f) * inv;
+            if (lane == 0) {
+                part[i][warp] = mean;
+                part[D + i][warp] = dev;
+            }
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        // mean, and mean absolute deviation (inside a warp's samples plus of its mean), over the warps
+        float mean[D], dev[D];
 #pragma unroll
-        for (int i = 0; i < D; ++i) dev[i] = ok ? fabsf(s[i] - sum[i] * inv) : 0.f;
-        block_sum<D>(dev, scratch);
-        if (threadIdx.x == 0) {
+        for (int i = 0; i < D; ++i) {
+            const float m = lane < kWarps ? part[i][lane] : 0.f, d = lane < kWarps ? part[D + i][lane] : 0.f;
+            mean[i] = warp_sum_all(m) * (1.f / kWarps);
+            dev[i] = warp_sum_all(lane < kWarps ? d + fabsf(m - mean[i]) : 0.f) * (1.f / kWarps);
+        }
+        if (lane == 0) {
             float cell[D];
             int halved[D];
 #pragma unroll
             for (int i = 0; i < D; ++i) {
                 // 4.4 mean absolute deviations hold a uniform box with a margin; what lies outside
                 // goes to the edge cells
-                cell[i] = fmaxf(4.4f * dev[i] * inv, 1e-30f);
-                lo[i] = sum[i] * inv - 0.5f * cell[i];
+                cell[i] = fmaxf(4.4f * dev[i], 1e-30f);
+                lo[i] = mean[i] - 0.5f * cell[i];
                 halved[i] = 0;
             }
             for (int b = a.bits - 1; b >= 0; --b) {
@@ -150,39 +172,49 @@ __global__ void __launch_bounds__(kThreads) order_count_kernel(const OrderArgs a
         }
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < D * kNibbles * 16; e += kThreads) {
+    for (int e = t; e < D * kNibbles * 16; e += kThreads) {
         const int dim = e / (kNibbles * 16), nibble = e / 16 % kNibbles, v = e % 16;
         uint32_t r = 0u;
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            const int k = halvings[dim] - 1 - (4 * nibble + t);  // the top bit is halving 0
-            if ((v >> t & 1) && k >= 0) r |= 1u << key_bit[dim][k];
+        for (int b = 0; b < 4; ++b) {
+            const int k = halvings[dim] - 1 - (4 * nibble + b);  // the top bit is halving 0
+            if ((v >> b & 1) && k >= 0) r |= 1u << key_bit[dim][k];
         }
         spread[dim][nibble][v] = r;
     }
     __syncthreads();
-    uint32_t key[kPerThread];
+#pragma unroll 1
+    for (int round = 0; round < a.rounds; ++round) {
+        const uint32_t n = first + round * (uint32_t)kPerBlock + t * kPerThread;
+        if (n >= a.n) return;
+        if (round > 0) load_points<D>(a, n, x);
+        uint32_t key[kPerThread], arrived[kPerThread];
 #pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        key[k] = chunk << a.bits;
+        for (int k = 0; k < kPerThread; ++k) key[k] = chunk << a.bits;
 #pragma unroll
         for (int i = 0; i < D; ++i) {
             const int h = halvings[i];
-            const float top = (float)((1 << h) - 1);
-            const int c = (int)fminf(fmaxf((x[k][i] - lo[i]) * inv_cell[i], 0.f), top);  // NaN: cell 0
-            for (int nibble = 0; 4 * nibble < h; ++nibble) key[k] |= spread[i][nibble][c >> (4 * nibble) & 15];
+            const float top = (float)((1 << h) - 1), l = lo[i], ic = inv_cell[i];
+            int c[kPerThread];
+#pragma unroll
+            for (int k = 0; k < kPerThread; ++k) c[k] = (int)fminf(fmaxf((x[k][i] - l) * ic, 0.f), top);  // NaN: cell 0
+            for (int nibble = 0; 4 * nibble < h; ++nibble) {
+#pragma unroll
+                for (int k = 0; k < kPerThread; ++k) key[k] |= spread[i][nibble][c[k] >> (4 * nibble) & 15];
+            }
         }
-    }
-    uint32_t arrived[kPerThread];
 #pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        const uint32_t n = first + k * kThreads + threadIdx.x;
-        if (n < a.n) arrived[k] = atomicAdd(a.counters + key[k], 1u);
-    }
+        for (int k = 0; k < kPerThread; ++k)
+            if (n + k < a.n) arrived[k] = atomicAdd(a.counters + key[k], 1u);
+        if (n + kPerThread <= a.n) {
+            uint4* dst = reinterpret_cast<uint4*>(a.arrival + n);
+            dst[0] = make_uint4(key[0], arrived[0], key[1], arrived[1]);
+            dst[1] = make_uint4(key[2], arrived[2], key[3], arrived[3]);
+        } else {
 #pragma unroll
-    for (int k = 0; k < kPerThread; ++k) {
-        const uint32_t n = first + k * kThreads + threadIdx.x;
-        if (n < a.n) a.arrival[n] = make_uint2(key[k], arrived[k]);
+            for (int k = 0; k < kPerThread; ++k)
+                if (n + k < a.n) a.arrival[n + k] = make_uint2(key[k], arrived[k]);
+        }
     }
 }
 
@@ -219,27 +251,35 @@ __global__ void __launch_bounds__(256) order_scan_kernel(const OrderArgs a) {
 
 template <int D>
 __global__ void __launch_bounds__(kThreads) order_scatter_kernel(const OrderArgs a) {
-    const uint32_t first = blockIdx.x * (uint32_t)kPerBlock + threadIdx.x;
+    const uint32_t n = (blockIdx.x * (uint32_t)kThreads + threadIdx.x) * kPerThread;
+    if (n >= a.n) return;
     float x[kPerThread][D];
-#pragma unroll
-    for (int k = 0; k < kPerThread; ++k) load<D>(a, min(first + k * kThreads, a.n - 1u), x[k]);
+    load_points<D>(a, n, x);
     cudaGridDependencySynchronize();
     uint2 at[kPerThread];
+    if (n + kPerThread <= a.n) {
+        const uint4* src = reinterpret_cast<const uint4*>(a.arrival + n);
+        const uint4 u = src[0], v = src[1];
+        at[0] = make_uint2(u.x, u.y);
+        at[1] = make_uint2(u.z, u.w);
+        at[2] = make_uint2(v.x, v.y);
+        at[3] = make_uint2(v.z, v.w);
+    } else {
 #pragma unroll
-    for (int k = 0; k < kPerThread; ++k) at[k] = a.arrival[min(first + k * kThreads, a.n - 1u)];
+        for (int k = 0; k < kPerThread; ++k) at[k] = a.arrival[min(n + k, a.n - 1u)];
+    }
 #pragma unroll
     for (int k = 0; k < kPerThread; ++k) at[k].y += a.counters[at[k].x];
 #pragma unroll
     for (int k = 0; k < kPerThread; ++k) {
-        const uint32_t n = first + k * kThreads;
-        if (n >= a.n) break;
+        if (n + k >= a.n) break;
         if (D <= 3) {
-            a.records[at[k].y] = make_float4(x[k][0], x[k][1], D == 3 ? x[k][D - 1] : 0.f, __uint_as_float(n));
+            a.records[at[k].y] = make_float4(x[k][0], x[k][1], D == 3 ? x[k][D - 1] : 0.f, __uint_as_float(n + k));
         } else {
             float r[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int i = 0; i < D; ++i) r[i] = x[k][i];
-            r[7] = __uint_as_float(n);
+            r[7] = __uint_as_float(n + k);
             asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(a.records + 2 * (size_t)at[k].y),
                          "f"(r[0]), "f"(r[1]), "f"(r[2]), "f"(r[3]), "f"(r[4]), "f"(r[5]), "f"(r[6]), "f"(r[7])
                          : "memory");
@@ -277,9 +317,10 @@ cudaError_t launch_early(K kernel, unsigned blocks, unsigned threads, const Orde
 template <int D>
 cudaError_t launch(const OrderArgs& a, cudaStream_t st) {
     const unsigned points = (a.n + kPerBlock - 1) / kPerBlock;
+    const unsigned counting = (points + a.rounds - 1) / a.rounds;
     cudaError_t e = cudaMemsetAsync(a.cursors, 0, cursor_bytes(a.n) + counter_bytes(a.n), st);
     if (e != cudaSuccess) return e;
-    order_count_kernel<D><<<points, kThreads, 0, st>>>(a);
+    order_count_kernel<D><<<counting, kThreads, 0, st>>>(a);
     e = launch_early(order_scan_kernel, (order_chunks(a.n) << a.bits) / kScanBins, 256, a, st);
     if (e != cudaSuccess) return e;
     e = launch_early(order_scatter_kernel<D>, points, kThreads, a, st);
@@ -299,8 +340,9 @@ int64_t permuto_order_bytes(int32_t pos_dim, int64_t nr_positions) {
 }
 
 int permuto_order_pays(const permuto_config* cfg, int64_t nr_positions, int32_t with_gradients) {
-    (void)with_gradients;
-    return cfg && nr_positions >= (1 << 18) ? 1 : 0;
+    if (!cfg) return 0;
+    if (with_gradients) return nr_positions >= (1 << 17) ? 1 : 0;
+    return nr_positions >= (cfg->pos_dim <= 4 ? 1 << 18 : 1 << 20) ? 1 : 0;
 }
 
 int permuto_order_points(const permuto_config* cfg, const permuto_inputs* in, void* order, int64_t order_bytes, void* stream) {
@@ -317,6 +359,10 @@ int permuto_order_points(const permuto_config* cfg, const permuto_inputs* in, vo
     a.stride_d = in->pos_stride_d;
     a.n = (uint32_t)in->nr_positions;
     a.bits = order_bits(a.n);
+    // a block's grid of cells serves several tiles once there are more tiles than resident blocks
+    a.rounds = 1;
+    while (a.rounds < 8 && a.n / kPerBlock / (2 * a.rounds) >= 1024) a.rounds *= 2;
+    a.vec_ok = in->pos_stride_d == 1 && in->pos_stride_n == cfg->pos_dim && (reinterpret_cast<uintptr_t>(in->positions) & 15u) == 0;
     char* at = static_cast<char*>(order);
     a.records = reinterpret_cast<float4*>(at);
     at += align256(a.n * record_bytes(cfg->pos_dim));

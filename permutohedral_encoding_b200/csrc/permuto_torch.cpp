@@ -13,6 +13,7 @@
 // The C ABI is called through the pointers of the library the Python side has loaded.
 #include <torch/extension.h>
 
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -79,6 +80,11 @@ void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.devi
 Tensor plain(const Tensor& t, const c10::Device& device) {
     if (t.device() == device && t.scalar_type() == at::kFloat && t.is_contiguous()) return t;
     return t.detach().to(t.options().device(device).dtype(at::kFloat).requires_grad(false)).contiguous();
+}
+
+// fp32 (or byte) tensor on the device of `like`, straight from the allocator: the dispatcher is a third of at::empty
+Tensor empty(at::IntArrayRef sizes, const Tensor& like, at::ScalarType type = at::kFloat) {
+    return Tensor(at::detail::empty_cuda(sizes, type, like.device(), std::nullopt));
 }
 
 const void* data(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
@@ -190,7 +196,7 @@ struct Bound {
 
 Tensor make_order(const Call& c, Bound& b) {
     const int64_t bytes = api.order_bytes(b.cfg.pos_dim, b.in.nr_positions);
-    Tensor order = at::empty({bytes}, c.positions.options().dtype(at::kByte));
+    Tensor order = empty({bytes}, c.positions, at::kByte);
     check(api.order_points(&b.cfg, &b.in, order.data_ptr(), bytes, stream_of(c.positions)));
     return order;
 }
@@ -202,7 +208,7 @@ Tensor run_forward(Call& c, bool may_order) {
     Bound b(c);
     if (may_order && !c.order.defined() && api.order_pays(&b.cfg, b.in.nr_positions, c.need_values || c.need_positions ? 1 : 0))
         c.order = make_order(c, b);
-    Tensor out = at::empty({b.in.nr_positions, c.lattice->width}, c.positions.options());
+    Tensor out = empty({b.in.nr_positions, c.lattice->width}, c.positions);
     check(api.forward(&b.cfg, &b.in, data(c.order), out.data_ptr<float>(), stream_of(c.positions)));
     return out;
 }
@@ -225,13 +231,13 @@ Gradients run_backward(const Call& c, const Tensor& grad, bool need_values, bool
     if (c.lattice->concat_positions_grad) flags |= PERMUTO_CONCAT_POSITIONS_GRAD;
     Gradients g;
     if (need_values)  // always fp32, whatever the storage type of the values
-        g.values = values_out.defined() ? values_out : at::empty(c.values.sizes(), c.positions.options());
+        g.values = values_out.defined() ? values_out : empty(c.values.sizes(), c.positions);
     if (need_positions) {
         if (positions_out.defined()) {
             g.positions = positions_out;
             flags |= PERMUTO_KEEP_POSITIONS_GRAD;
         } else {  // without ZERO_OUTPUTS nothing clears it natively
-            g.positions = zero ? at::empty({n, b.cfg.pos_dim}, c.positions.options())
+            g.positions = zero ? empty({n, b.cfg.pos_dim}, c.positions)
                                : at::zeros({n, b.cfg.pos_dim}, c.positions.options());
         }
     }
@@ -258,8 +264,8 @@ SecondOrder run_double_backward(const Call& c, const Tensor& double_positions_gr
     Bound b(c);
     const Tensor dpg = double_positions_grad.contiguous(), gf = grad.contiguous();
     SecondOrder s;
-    if (need_values) s.values = at::empty(c.values.sizes(), c.positions.options());
-    if (need_features) s.features = at::empty(gf.sizes(), c.positions.options());
+    if (need_values) s.values = empty(c.values.sizes(), c.positions);
+    if (need_features) s.features = empty(gf.sizes(), c.positions);
     check(api.double_backward(&b.cfg, &b.in, data(c.order), dpg.data_ptr<float>(), gf.data_ptr<float>(),
                               need_values ? s.values.data_ptr<float>() : nullptr,
                               need_features ? s.features.data_ptr<float>() : nullptr,
@@ -409,8 +415,10 @@ Tensor forward_mlp(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& val
     if (status && (status->scalar_type() != at::kInt || status->device() != device || status->numel() != 1))
         fail("status should be a one-element int32 tensor on the device of the positions");
     Bound b(*c);
-    if (!c->order.defined() && api.order_pays(&b.cfg, b.in.nr_positions, 0)) c->order = make_order(*c, b);
-    Tensor out = at::empty({b.in.nr_positions, width}, positions.options());
+    // One layer behind the encoding gains 18 % from an order on 2^20 independent points (349 -> 285 us); with
+    // a whole network behind it the gathers are less of the time, and the gain (4 %) is what ray samples lose.
+    if (!c->order.defined() && layers.size() == 1 && api.order_pays(&b.cfg, b.in.nr_positions, 0)) c->order = make_order(*c, b);
+    Tensor out = empty({b.in.nr_positions, width}, positions);
     check(api.forward_mlp(&b.cfg, &b.in, data(c->order), layers.data(), (int32_t)layers.size(), activation,
                           out.data_ptr<float>(), status ? status->data_ptr<int32_t>() : nullptr, stream_of(positions)));
     return out;

@@ -81,6 +81,7 @@ class PermutoEncoding(torch.nn.Module):
 
     def __setstate__(self, state):
         self.__dict__.update(state)
+        self.__dict__.setdefault("half_precision_table", False)   # pickles from before the switch existed
         self.fixed_params, self.lattice = self._make_lattice_wrapper()
 
     def _apply(self, fn, *args, **kwargs):
@@ -110,14 +111,15 @@ class PermutoEncoding(torch.nn.Module):
     def forward(self, positions, anneal_window=None):
         if anneal_window is None:
             anneal_window = self.anneal_window
-        if anneal_window.device != positions.device:
-            anneal_window = anneal_window.to(positions.device)
-        # the shift parameter may have been replaced (load_state_dict(assign=True), .to())
-        self.fixed_params.m_random_shift_per_level = self.random_shift_per_level
-
-        half = self._half_copy() if getattr(self, "half_precision_table", False) else None
+        # straight from the dict: nn.Module's attribute lookup of a parameter is most of a microsecond
+        values, shift = self._parameters.get("lattice_values"), self._parameters.get("random_shift_per_level")
+        if values is None or shift is None:   # replaced by something else, e.g. a parametrization
+            values, shift = self.lattice_values, self.random_shift_per_level
+        fixed = self.fixed_params
+        fixed.m_random_shift_per_level = shift   # may have been replaced (load_state_dict(assign=True), .to())
         # [N, (L+extra)*F] already in the reference's output order: no permute/reshape copy
-        return self.lattice.encode(self.lattice_values, positions, anneal_window, half)
+        return _C.encode(self.lattice._native, values, positions, anneal_window, shift,
+                         self._half_copy() if self.half_precision_table else None, fixed.levels_per_pass)
 
     def _half_copy(self):
         """fp16 copy of the lattice values the kernels gather from when ``half_precision_table`` is
@@ -144,7 +146,7 @@ class PermutoEncoding(torch.nn.Module):
             anneal_window = anneal_window.to(positions.device)
         self.fixed_params.m_random_shift_per_level = self.random_shift_per_level
         weight, bias = (linear.weight, linear.bias) if hasattr(linear, "weight") else linear
-        half = self._half_copy() if getattr(self, "half_precision_table", False) else None
+        half = self._half_copy() if self.half_precision_table else None
         inp = _C.EncodingInput(self.lattice_values, positions, anneal_window, False, False, half)
         return self.lattice.forward_linear(inp, weight, bias, status)
 
@@ -183,7 +185,7 @@ class PermutoEncoding(torch.nn.Module):
         if len(kinds) > 1:
             raise RuntimeError(f"one kind of activation between the layers, got {sorted(kinds)}")
         activation = kinds.pop() if kinds else "none"
-        half = self._half_copy() if getattr(self, "half_precision_table", False) else None
+        half = self._half_copy() if self.half_precision_table else None
         inp = _C.EncodingInput(self.lattice_values, positions, anneal_window, False, False, half)
         return self.lattice.forward_mlp(inp, layers, activation, status)
 
