@@ -202,6 +202,15 @@ int permuto_double_backward_ordered(const permuto_config *cfg, const permuto_inp
                                     float *lattice_grad, float *grad_grad_features, uint32_t flags,
                                     void *stream);
 
+/* lattice_grad (+)= the table gradient of permuto_backward_ordered(grad_features) plus that of
+ * permuto_double_backward_ordered(double_positions_grad, second_grad_features), for a loss that reaches
+ * the features and the position gradient of the same points (an SDF's data and eikonal terms).  One pass
+ * over the points when there is an order: a vertex receives both addends in one reduction. */
+int permuto_backward_combined(const permuto_config *cfg, const permuto_inputs *in, const void *order,
+                              const float *grad_features, const float *double_positions_grad,
+                              const float *second_grad_features, float *lattice_grad, uint32_t flags,
+                              void *stream);
+
 /* Debug view of the lattice geometry (the reference has no counterpart; it exists so that
  * keys and hash slots can be compared bit for bit).  Any output may be NULL.
  *   keys  int32 [N, L, pos_dim+1, pos_dim]   slots int32 [N, L, pos_dim+1]

@@ -50,7 +50,7 @@ EXPORTED_SYMBOLS = (
     "permuto_forward", "permuto_backward", "permuto_double_backward", "permuto_debug_lattice",
     "permuto_probe_random_access", "permuto_adam_step", "permuto_forward_linear", "permuto_forward_mlp",
     "permuto_order_pays", "permuto_order_bytes", "permuto_order_points", "permuto_forward_ordered", "permuto_forward_mlp_ordered",
-    "permuto_backward_ordered", "permuto_double_backward_ordered",
+    "permuto_backward_ordered", "permuto_double_backward_ordered", "permuto_backward_combined",
 )
 
 

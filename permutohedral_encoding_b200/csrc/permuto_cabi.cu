@@ -217,12 +217,9 @@ int permuto_forward_mlp_ordered(const permuto_config* cfg, const permuto_inputs*
     a.activation = activation;
     a.out = out;
     a.k_pad = (a.p.width + 7) / 8 * 8;
-    int half = 16;  // two accumulator ranges for the hidden layers to alternate between
-    while (half < widest) half <<= 1;
     int cols = 32;  // allocation granularity of tensor memory: a power of two, at least 32 columns
-    while (cols < (nr_layers == 1 ? widest : 2 * half)) cols <<= 1;
+    while (cols < widest) cols <<= 1;
     a.tmem_cols = cols;
-    a.tmem_half = half;
     a.status = status;
     a.out_vec8_ok = (last_out % 16 == 0 && aligned(out, 32)) ? 1 : 0;
     cudaError_t err;
@@ -312,6 +309,35 @@ int permuto_double_backward_ordered(const permuto_config* cfg, const permuto_inp
     cudaError_t err;
     PERMUTO_DISPATCH(launch_double_backward, a, st)
     if (err != cudaSuccess) return cuda_fail(err, "permuto_double_backward launch");
+    return PERMUTO_OK;
+}
+
+int permuto_backward_combined(const permuto_config* cfg, const permuto_inputs* in, const void* order,
+                              const float* grad_features, const float* double_positions_grad,
+                              const float* second_grad_features, float* lattice_grad, uint32_t flags, void* stream) {
+    permuto::CombinedArgs a;
+    if (int rc = build_problem(cfg, in, order, a.p)) return rc;
+    if (!grad_features || !double_positions_grad || !second_grad_features || !lattice_grad)
+        return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "grad_features, double_positions_grad, second_grad_features and "
+                                                       "lattice_grad must not be NULL");
+    if (!aligned(grad_features, row_align(a.p)) || !aligned(second_grad_features, row_align(a.p)) ||
+        !aligned(lattice_grad, row_align(a.p)))
+        return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "grad_features, second_grad_features and lattice_grad must be %d-byte aligned",
+                         (int)row_align(a.p));
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    a.grad_features = grad_features;
+    a.double_positions_grad = double_positions_grad;
+    a.second_grad_features = second_grad_features;
+    a.lattice_grad = lattice_grad;
+    a.aggregate = (flags & PERMUTO_NO_AGGREGATE) ? 0 : 1;
+    a.p.rows_vec8_ok = rows_vec8(a.p, grad_features, second_grad_features);
+    if (flags & PERMUTO_ZERO_OUTPUTS) {
+        cudaError_t e = cudaMemsetAsync(lattice_grad, 0, (size_t)a.p.nr_levels * a.p.capacity * a.p.nr_feat * sizeof(float), st);
+        if (e != cudaSuccess) return cuda_fail(e, "permuto_backward_combined clearing outputs");
+    }
+    cudaError_t err;
+    PERMUTO_DISPATCH(launch_combined, a, st)
+    if (err != cudaSuccess) return cuda_fail(err, "permuto_backward_combined launch");
     return PERMUTO_OK;
 }
 

@@ -46,7 +46,7 @@ constexpr int D = PERMUTO_DIM;
 // The forward kernel is bound by the LSU pipe, not by instruction-level parallelism: at 60
 // registers (what a cap of 64 invites) it runs 4 % slower than at 32 with twice the resident warps.
 #ifndef PERMUTO_MIN_BLOCKS_FORWARD
-#define PERMUTO_MIN_BLOCKS_FORWARD (PERMUTO_DIM <= 3 ? 8 : (PERMUTO_DIM == 4 ? 6 : 4))
+#define PERMUTO_MIN_BLOCKS_FORWARD (PERMUTO_DIM <= 3 ? 8 : (PERMUTO_DIM <= 5 ? 6 : 4))
 #endif
 #ifndef PERMUTO_FWD_STAGGER
 #define PERMUTO_FWD_STAGGER 1
@@ -505,7 +505,9 @@ struct SliceRing {
         *reinterpret_cast<float4*>(dst + 128) =
             make_float4(umma::to_tf32(v[4]), umma::to_tf32(v[5]), umma::to_tf32(v[6]), umma::to_tf32(v[7]));
         // the block's writes -> visible to the tensor core (async proxy); then one thread issues the slice's MMA
+        // (and what the threads have read from tensor memory is ordered before it may be overwritten)
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncthreads();
         if (threadIdx.x == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -563,30 +565,68 @@ __device__ __forceinline__ void tmem_load16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// erf to 1.5e-7 absolute (Abramowitz & Stegun 7.1.26) in about 15 instructions: the hidden
-// activations are rounded to tf32 (5e-4 relative) right afterwards, and erff() itself would be
-// most of the instructions of a hidden layer
-__device__ __forceinline__ float erf_fast(float x) {
-    const float ax = fabsf(x);
-    const float t = __frcp_rn(fmaf(0.3275911f, ax, 1.0f));
-    const float poly = t * fmaf(t, fmaf(t, fmaf(t, fmaf(t, 1.061405429f, -1.453152027f), 1.421413741f), -0.284496736f), 0.254829592f);
-    return copysignf(1.0f - poly * __expf(-ax * ax), x);
+// Packed fp32 pairs: one instruction, the IEEE result in each half.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
-__device__ __forceinline__ float activate(float x, int kind) {
-    if (kind == PERMUTO_ACT_RELU) return fmaxf(x, 0.f);
-    if (kind == PERMUTO_ACT_GELU) return 0.5f * x * (1.0f + erf_fast(x * 0.70710678118654752f));  // torch.nn.GELU()
-    return x;
+// torch.nn.GELU() of two values: x * Phi(x) = max(x, 0) - |x| * Q(t) * exp(-x^2 / 2), t = 1 / (1 + p |x|).
+// Q is the degree-6 polynomial (no constant term) with the smallest largest error of erfc against
+// erfcx(x) * exp(-x^2) on [0, 6], p = 0.4 / sqrt(2): 2.8e-8 before rounding, 2.4e-7 absolute in fp32 with
+// the approximate reciprocal and exponential (the form through 1 + erf had 4.7e-7).  About ten issue
+// slots a value instead of 25: a hidden layer was mostly this.
+__device__ __forceinline__ void gelu2(float& x, float& y) {
+    const uint64_t v = pack2(x, y);
+    const float ax = fminf(fabsf(x), 1e18f), ay = fminf(fabsf(y), 1e18f);  // infinity times zero otherwise
+    const uint64_t a = pack2(ax, ay);
+    float dx, dy, sx, sy;
+    unpack2(fma2(a, pack2(0.282842712f, 0.282842712f), pack2(1.f, 1.f)), dx, dy);
+    asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(dx));
+    asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(dy));
+    const uint64_t t = pack2(dx, dy);
+    uint64_t q = fma2(t, pack2(-0.100129196f, -0.100129196f), pack2(0.354571956f, 0.354571956f));
+    q = fma2(t, q, pack2(-0.1854512479f, -0.1854512479f));
+    q = fma2(t, q, pack2(0.2341349315f, 0.2341349315f));
+    q = fma2(t, q, pack2(0.08091262737f, 0.08091262737f));
+    q = fma2(t, q, pack2(0.1159609153f, 0.1159609153f));
+    q = mul2(t, q);
+    unpack2(mul2(mul2(v, pack2(-0.72134752f, -0.72134752f)), v), sx, sy);  // -x^2 / 2 * log2(e)
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(sx));
+    asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(sy));
+    const uint64_t m = mul2(pack2(-ax, -ay), pack2(sx, sy));
+    unpack2(fma2(m, q, pack2(fmaxf(x, 0.f), fmaxf(y, 0.f))), x, y);
 }
 
-#ifndef PERMUTO_FUSED_MIN_BLOCKS
-#define PERMUTO_FUSED_MIN_BLOCKS 8
+#ifndef FB0
+#define FB0 10
+#endif
+#ifndef FB32
+#define FB32 6
 #endif
 // HMAX = 0: the encoding followed by ONE linear layer (out = features @ W^T + b).
 // HMAX = 32 / 64: a whole small MLP behind the encoding; hidden widths are multiples of 16 up to
 // HMAX (a thread holds its row of hidden activations in registers between two layers).
+constexpr int fused_blocks(int feats, int hmax) { return feats == 2 && hmax <= 32 ? (hmax ? FB32 : FB0) : 4; }
 template <int F, int LPS, bool HALF, int HMAX>
-__global__ void __launch_bounds__(kTileRows, (F == 2 && HMAX <= 32 ? PERMUTO_FUSED_MIN_BLOCKS : 4))
+__global__ void __launch_bounds__(kTileRows, fused_blocks(F, HMAX))
 forward_mlp_kernel(const ForwardLinearArgs a) {
     const Problem& p = a.p;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -615,6 +655,22 @@ forward_mlp_kernel(const ForwardLinearArgs a) {
     unsigned char* tile_w = smem_raw + kRing * kSliceBytes;
     const int chunks0 = a.k_pad / 4;
     float* levels = reinterpret_cast<float*>(smem_raw + a.levels_offset);  // behind the weights
+    float* biases = levels + p.nr_levels * kRecord;  // one layer after the other, zeros where there is none
+    float* narrow = nullptr;                         // weight rows of a narrow last layer
+    {
+        int at = 0;
+        for (int i = 0; i < a.nr_layers; ++i) {
+            const MlpLayer& ly = a.layer[i];
+            const int padded = (ly.out_features + 3) / 4 * 4;
+            for (int k = t; k < padded; k += kTileRows) biases[at + k] = ly.bias && k < ly.out_features ? __ldg(ly.bias + k) : 0.f;
+            at += padded;
+        }
+        const MlpLayer& ly = a.layer[a.nr_layers - 1];
+        if (HMAX > 0 && ly.out_features % 16 != 0) {
+            narrow = biases + at;
+            for (int k = t; k < ly.out_features * ly.in_features; k += kTileRows) narrow[k] = __ldg(ly.weight + k);
+        }
+    }
     stage_levels(p, 0, p.nr_levels, levels);
     stage_weight(tile_w, a.layer[0].weight, H0, p.width, chunks0);
     if (HMAX > 0) {
@@ -640,135 +696,148 @@ forward_mlp_kernel(const ForwardLinearArgs a) {
     ring.pushed = 0;
     ring.ok = true;
 
-    // ---- layer 0: this thread's point -> row t of every slice ----------------------------------
-    const int64_t i_raw = (int64_t)blockIdx.x * kTileRows + t;
-    const bool active = i_raw < p.n_points;
-    int64_t n;
-    {
-        float pos[D];
-        n = load_point(p, active ? i_raw : p.n_points - 1, pos);  // idle rows shadow the last point and are not stored
-        const float largest = largest_coordinate<D>(pos);
-        const int lattice_cols = F * p.nr_levels;
-        // a column past the lattice levels: a concatenated raw coordinate (EncodingGPU.cuh:105-121) or padding
-        auto tail_value = [&](int c) -> float {
-            float v = 0.f;
-            const int i = c - lattice_cols;
-#pragma unroll
-            for (int j = 0; j < D; ++j) v = (i == j && c < p.width) ? pos[j] * p.points_scaling : v;
-            return v;
-        };
-        const int nsteps = (p.nr_levels + LPS - 1) / LPS;  // steps that hold lattice levels
-        const int ksteps = a.k_pad / 8;                    // all steps: one tcgen05.mma each
-        const uint32_t idesc = umma::instr_desc_tf32(kTileRows, H0);
-        const uint32_t addr_w = umma::smem_u32(tile_w);
-#pragma unroll 1
-        for (int s = 0; s < ksteps; ++s) {
-            float out[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) out[i] = 0.f;
-            if (s < nsteps) encode_step<F, LPS, HALF>(p, levels + s * LPS * kRecord, pos, largest, s * LPS, p.nr_levels, out);
-            if (8 * s + 8 > lattice_cols) {  // block-uniform: only the last step(s) reach past the lattice levels
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int c = 8 * s + i;
-                    out[i] = (c >= lattice_cols) ? tail_value(c) : out[i];
-                }
-            }
-            ring.push(out, tmem, addr_w + (uint32_t)s * 256u, (uint32_t)chunks0 * 128u, idesc, s > 0);
-        }
-    }
-
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);  // tensor-memory lane = 32*warp + lane = row t
     bool ok = true;
-    int last = 0;          // layer whose accumulators are in tensor memory
-    uint32_t col = 0;      // ... starting at this column
-
-    // ---- hidden layers: accumulators -> registers (+bias, activation) -> slices -> next product ----
-    if (HMAX > 0) {
-        constexpr int HM = HMAX > 0 ? HMAX : 16;
-        uint32_t w_addr = umma::smem_u32(tile_w) + (uint32_t)H0 * (uint32_t)a.k_pad * 4u;
-        for (int i = 1; i < a.nr_layers; ++i) {
-            const MlpLayer& ly = a.layer[i];
-            const int width = ly.in_features;  // = out_features of layer i-1, a multiple of 16 up to HMAX
-            ok = ring.drain() && ok;
-            float h[HM];
-            const float* bias = a.layer[i - 1].bias;
-            const int kind = a.activation;
+    // A block walks over tiles of 128 points: what stands above -- tensor memory, barriers, weights -- is
+    // set up once per resident block, not once per tile (355 -> FILLIN us on 10^6 ray samples).
+    const int64_t tiles = (p.n_points + kTileRows - 1) / kTileRows;
+#pragma unroll 1
+    for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        // ---- layer 0: this thread's point -> row t of every slice ----------------------------------
+        const int64_t i_raw = tile * kTileRows + t;
+        const bool active = i_raw < p.n_points;
+        int64_t n;
+        {
+            float pos[D];
+            n = load_point(p, active ? i_raw : p.n_points - 1, pos);  // idle rows shadow the last point and are not stored
+            const float largest = largest_coordinate<D>(pos);
+            const int lattice_cols = F * p.nr_levels;
+            // a column past the lattice levels: a concatenated raw coordinate (EncodingGPU.cuh:105-121) or padding
+            auto tail_value = [&](int c) -> float {
+                float v = 0.f;
+                const int i = c - lattice_cols;
 #pragma unroll
-            for (int c = 0; c < HM / 16; ++c) {
-                if (16 * c < width) {
-                    float v[16];
-                    tmem_load16(lane_base + col + 16u * c, v);
-                    if (bias) {  // 64-byte aligned groups of a tensor allocated by the caller: vector loads when possible
+                for (int j = 0; j < D; ++j) v = (i == j && c < p.width) ? pos[j] * p.points_scaling : v;
+                return v;
+            };
+            const int nsteps = (p.nr_levels + LPS - 1) / LPS;  // steps that hold lattice levels
+            const int ksteps = a.k_pad / 8;                    // all steps: one tcgen05.mma each
+            const uint32_t idesc = umma::instr_desc_tf32(kTileRows, H0);
+            const uint32_t addr_w = umma::smem_u32(tile_w);
+#pragma unroll 1
+            for (int s = 0; s < ksteps; ++s) {
+                float out[8];
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) v[k] += __ldg(bias + 16 * c + k);
+                for (int i = 0; i < 8; ++i) out[i] = 0.f;
+                if (s < nsteps) encode_step<F, LPS, HALF>(p, levels + s * LPS * kRecord, pos, largest, s * LPS, p.nr_levels, out);
+                if (8 * s + 8 > lattice_cols) {  // block-uniform: only the last step(s) reach past the lattice levels
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int c = 8 * s + i;
+                        out[i] = (c >= lattice_cols) ? tail_value(c) : out[i];
                     }
-                    // one uniform branch per group, not one per element
-                    if (kind == PERMUTO_ACT_GELU) {
+                }
+                ring.push(out, tmem, addr_w + (uint32_t)s * 256u, (uint32_t)chunks0 * 128u, idesc, s > 0);
+            }
+        }
+
+        int last = 0;          // layer whose accumulators are in tensor memory
+        const float* bias = biases;  // of that layer
+
+        // ---- hidden layers: accumulators -> registers (+bias, activation) -> slices -> next product ----
+        if (HMAX > 0) {
+            constexpr int HM = HMAX > 0 ? HMAX : 16;
+            uint32_t w_addr = umma::smem_u32(tile_w) + (uint32_t)H0 * (uint32_t)a.k_pad * 4u;
+            for (int i = 1; i < a.nr_layers; ++i) {
+                const MlpLayer& ly = a.layer[i];
+                const int width = ly.in_features;  // = out_features of layer i-1, a multiple of 16 up to HMAX
+                ok = ring.drain() && ok;
+                float h[HM];
+                const int kind = a.activation;
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) h[16 * c + k] = activate(v[k], PERMUTO_ACT_GELU);
-                    } else if (kind == PERMUTO_ACT_RELU) {
+                for (int c = 0; c < HM / 16; ++c) {
+                    if (16 * c < width) {
+                        float v[16];
+                        tmem_load16(lane_base + 16u * c, v);
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) h[16 * c + k] = fmaxf(v[k], 0.f);
-                    } else {
+                        for (int k = 0; k < 16; k += 4) {
+                            const float4 b = *reinterpret_cast<const float4*>(bias + 16 * c + k);
+                            unpack2(add2(pack2(v[k], v[k + 1]), pack2(b.x, b.y)), v[k], v[k + 1]);
+                            unpack2(add2(pack2(v[k + 2], v[k + 3]), pack2(b.z, b.w)), v[k + 2], v[k + 3]);
+                        }
+                        // one uniform branch per group, not one per element
+                        if (kind == PERMUTO_ACT_GELU) {
+#pragma unroll
+                            for (int k = 0; k < 16; k += 2) gelu2(v[k], v[k + 1]);
+                        } else if (kind == PERMUTO_ACT_RELU) {
+#pragma unroll
+                            for (int k = 0; k < 16; ++k) v[k] = fmaxf(v[k], 0.f);
+                        }
 #pragma unroll
                         for (int k = 0; k < 16; ++k) h[16 * c + k] = v[k];
                     }
                 }
-            }
-            if (ly.out_features % 16 != 0) {
-                // narrow last layer (e.g. one output): plain fp32 dot products in registers
-                if (active && ok) {
-                    for (int o = 0; o < ly.out_features; ++o) {
-                        float acc = ly.bias ? __ldg(ly.bias + o) : 0.f;
-                        const float* w = ly.weight + (size_t)o * width;
+                bias += width;  // a multiple of 16
+                if (ly.out_features % 16 != 0) {
+                    // narrow last layer (e.g. one output): plain fp32 dot products in registers
+                    if (active && ok) {
+                        for (int o = 0; o < ly.out_features; ++o) {
+                            float acc = bias[o];
+                            const float4* w = reinterpret_cast<const float4*>(narrow + o * width);
 #pragma unroll
-                        for (int k = 0; k < HM; ++k)
-                            if (k < width) acc = fmaf(h[k], __ldg(w + k), acc);
-                        a.out[n * ly.out_features + o] = acc;
+                            for (int k = 0; k < HM; k += 4) {
+                                if (k < width) {
+                                    const float4 u = w[k / 4];
+                                    acc = fmaf(h[k], u.x, acc);
+                                    acc = fmaf(h[k + 1], u.y, acc);
+                                    acc = fmaf(h[k + 2], u.z, acc);
+                                    acc = fmaf(h[k + 3], u.w, acc);
+                                }
+                            }
+                            a.out[n * ly.out_features + o] = acc;
+                        }
+                    }
+                    last = -1;  // everything is written
+                    break;
+                }
+                // the product goes to the columns it came from: every row is in registers when the block meets
+                // in the first push, before its MMA is issued
+                const uint32_t idesc = umma::instr_desc_tf32(kTileRows, ly.out_features);
+#pragma unroll
+                for (int j = 0; j < HM / 8; ++j) {
+                    if (8 * j < width) {
+                        float v[8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) v[k] = h[8 * j + k];
+                        ring.push(v, tmem, w_addr + (uint32_t)j * 256u, (uint32_t)(width / 4) * 128u, idesc, j > 0);
                     }
                 }
-                last = -1;  // everything is written
-                break;
+                w_addr += (uint32_t)ly.out_features * (uint32_t)width * 4u;
+                last = i;
             }
-            const uint32_t dst_col = col ^ (uint32_t)a.tmem_half;  // ping-pong between the two halves
-            const uint32_t idesc = umma::instr_desc_tf32(kTileRows, ly.out_features);
-#pragma unroll
-            for (int j = 0; j < HM / 8; ++j) {
-                if (8 * j < width) {
-                    float v[8];
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) v[k] = h[8 * j + k];
-                    ring.push(v, tmem + dst_col, w_addr + (uint32_t)j * 256u, (uint32_t)(width / 4) * 128u, idesc, j > 0);
-                }
-            }
-            w_addr += (uint32_t)ly.out_features * (uint32_t)width * 4u;
-            col = dst_col;
-            last = i;
         }
-    }
 
-    // ---- last tensor-core layer: accumulators + bias -> out[N, out_features] -------------------------
-    if (last >= 0) {
-        ok = ring.drain() && ok;
-        const int H = a.layer[last].out_features;
-        const float* bias = a.layer[last].bias;
-        if (ok) {
-            float* dst = a.out + n * H;
-            for (int c = 0; c < H; c += 16) {
-                float v[16];
-                tmem_load16(lane_base + col + (uint32_t)c, v);
-                if (active) {
+        // ---- last tensor-core layer: accumulators + bias -> out[N, out_features] -------------------------
+        if (last >= 0) {
+            ok = ring.drain() && ok;
+            const int H = a.layer[last].out_features;
+            if (ok) {
+                float* dst = a.out + n * H;
+                for (int c = 0; c < H; c += 16) {
+                    float v[16];
+                    tmem_load16(lane_base + (uint32_t)c, v);
+                    if (active) {
 #pragma unroll
-                    for (int h8 = 0; h8 < 2; ++h8) {
-                        float o[8];
+                        for (int h8 = 0; h8 < 2; ++h8) {
+                            float o[8];
 #pragma unroll
-                        for (int k = 0; k < 8; ++k) o[k] = v[8 * h8 + k] + (bias ? __ldg(bias + c + 8 * h8 + k) : 0.f);
-                        if (a.out_vec8_ok) {
-                            store8(dst + c + 8 * h8, o);
-                        } else {
-                            reinterpret_cast<float4*>(dst + c + 8 * h8)[0] = make_float4(o[0], o[1], o[2], o[3]);
-                            reinterpret_cast<float4*>(dst + c + 8 * h8)[1] = make_float4(o[4], o[5], o[6], o[7]);
+                            for (int k = 0; k < 8; ++k) o[k] = v[8 * h8 + k] + bias[c + 8 * h8 + k];
+                            if (a.out_vec8_ok) {
+                                store8(dst + c + 8 * h8, o);
+                            } else {
+                                reinterpret_cast<float4*>(dst + c + 8 * h8)[0] = make_float4(o[0], o[1], o[2], o[3]);
+                                reinterpret_cast<float4*>(dst + c + 8 * h8)[1] = make_float4(o[4], o[5], o[6], o[7]);
+                            }
                         }
                     }
                 }
@@ -1052,17 +1121,28 @@ backward_kernel(const BackwardArgs a) {
 // ------------------------------------------------------------------------------------------
 // table gradient of a coherent batch: P consecutive points per thread
 // ------------------------------------------------------------------------------------------
+#ifndef RUNS_IF
+#define RUNS_IF(p) ((p).order != nullptr)
+#endif
 #ifndef PERMUTO_RUN_POINTS
 #define PERMUTO_RUN_POINTS 2
-#endif
-#ifndef PERMUTO_RUN_BLOCKS
-#define PERMUTO_RUN_BLOCKS 8
 #endif
 #ifndef PERMUTO_RUN_THREADS
 #define PERMUTO_RUN_THREADS 128
 #endif
 constexpr int kRunPoints = PERMUTO_RUN_POINTS;
 constexpr int kRunThreads = PERMUTO_RUN_THREADS;
+#ifndef RB2
+#define RB2 5
+#define RB3 4
+#define RB4 3
+#endif
+// Resident blocks the registers have to allow: the D+1 running sums of F features and their slots stay
+// live over the points of a thread, and spilling them costs more than the warps they displace.
+constexpr int run_blocks(int feats) {
+    const int live = (D + 1) * (feats + 1);
+    return live <= 18 ? 8 : (live <= 26 ? RB2 : (live <= 45 ? RB3 : RB4));
+}
 constexpr int kPosVec = D <= 3 ? 1 : 2;  // float4s per point: coordinates, row index last
 // D floats kept as kPosVec float4s, kRunThreads apart
 __device__ __forceinline__ void load_vec(const float4* src, float (&x)[D]) {
@@ -1075,12 +1155,16 @@ __device__ __forceinline__ void load_vec(const float4* src, float (&x)[D]) {
         if (4 * i + 3 < D) x[(4 * i + 3) % D] = v.w;
     }
 }
-template <bool DOUBLE>
+// what the table receives: the addends of the first-order backward, of the double backward, or their sum
+enum class Order { First, Second, Both };
+template <Order ORDER>
 struct RunStage {
+    static constexpr bool kSecond = ORDER != Order::First;
     float levels[kStage * kRecord];
     float4 point[kRunPoints][kPosVec][kRunThreads];
-    float4 dpg[DOUBLE ? kRunPoints : 1][DOUBLE ? kPosVec : 1][DOUBLE ? kRunThreads : 1];
-    float4 grad[kRunPoints][2][kRunThreads];  // gradient row segments: [point][4 floats of the step][thread]
+    float4 dpg[kSecond ? kRunPoints : 1][kSecond ? kPosVec : 1][kSecond ? kRunThreads : 1];
+    // gradient row segments: [first, second order][point][4 floats of the step][thread]
+    float4 grad[ORDER == Order::Both ? 2 : 1][kRunPoints][2][kRunThreads];
 };
 // Sum over the warp of CNT vertices' addends by recursive halving: at each step a lane keeps one half of
 // the vertices and hands the other half to its partner, so CNT = 4 vertices take 4+2+1 exchanges of F
@@ -1148,23 +1232,14 @@ __device__ __forceinline__ bool merge_simplices(float* level_base, unsigned lane
     return true;
 }
 
-struct RunArgs {
-    Problem p;
-    const float* grad_features;
-    const float* double_positions_grad;  // double backward only
-    float* lattice_grad;
-    int32_t aggregate;
-};
-
-// DOUBLE: the addends are those of the double backward, weight d loss / d barycentric instead of the
-// barycentric weight
-template <int F, bool DOUBLE>
-__global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_kernel(const RunArgs a) {
+template <int F, Order ORDER>
+__global__ void __launch_bounds__(kRunThreads, run_blocks(F)) scatter_runs_kernel(const CombinedArgs a) {
     constexpr int P = kRunPoints;
     constexpr int LPS = 8 / F;
     const Problem& p = a.p;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    RunStage<DOUBLE>& sm = *reinterpret_cast<RunStage<DOUBLE>*>(smem_raw);
+    constexpr bool kSecond = ORDER != Order::First;
+    RunStage<ORDER>& sm = *reinterpret_cast<RunStage<ORDER>*>(smem_raw);
     const int t = threadIdx.x;
     const int pass_begin = p.level_begin + (int)blockIdx.y * p.levels_per_pass;
     const int pass_end = min(pass_begin + p.levels_per_pass, p.level_end);
@@ -1182,7 +1257,7 @@ __global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_
         r[4 * kPosVec - 1] = __uint_as_float((uint32_t)n);
 #pragma unroll
         for (int i = 0; i < kPosVec; ++i) sm.point[j][i][t] = make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
-        if (DOUBLE) {
+        if (kSecond) {
 #pragma unroll
             for (int i = 0; i < 4 * kPosVec; ++i) r[i] = i < D ? __ldg(a.double_positions_grad + n * D + i) : 0.f;
 #pragma unroll
@@ -1204,17 +1279,19 @@ __global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_
             const int l0 = begin + step * LPS;
             step = (step + 1 == nsteps) ? 0 : step + 1;
             if (l0 == begin) sc.probe = a.aggregate != 0;
-            {
+#pragma unroll
+            for (int o = 0; o < (ORDER == Order::Both ? 2 : 1); ++o) {
+                const float* rows = (ORDER == Order::Second || o == 1) ? a.second_grad_features : a.grad_features;
                 float g[P][8];
 #pragma unroll
                 for (int j = 0; j < P; ++j)
-                    load_row_segment<F, LPS>(p, a.grad_features, __float_as_uint(sm.point[j][kPosVec - 1][t].w), l0, g[j]);
+                    load_row_segment<F, LPS>(p, rows, __float_as_uint(sm.point[j][kPosVec - 1][t].w), l0, g[j]);
 #pragma unroll
                 for (int j = 0; j < P; ++j) {
 #pragma unroll
                     for (int q = 0; q < 2; ++q)
-                        sm.grad[j][q][t] = j < count ? make_float4(g[j][4 * q], g[j][4 * q + 1], g[j][4 * q + 2], g[j][4 * q + 3])
-                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+                        sm.grad[o][j][q][t] = j < count ? make_float4(g[j][4 * q], g[j][4 * q + 1], g[j][4 * q + 2], g[j][4 * q + 3])
+                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             }
 #pragma unroll 1
@@ -1236,10 +1313,14 @@ __global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_
                 }
 #pragma unroll 1
                 for (int j = 0; j < P; ++j) {
-                    float x[D], g[F];
+                    float x[D], add[D + 1][F];
                     load_vec(&sm.point[j][0][t], x);
-                    {
-                        const float4* src = &sm.grad[j][F * k / 4][t];
+                    Simplex<D> s;
+                    locate_simplex<D>(x, largest_coordinate<D>(x), lc, s);
+                    uint32_t slot[D + 1];
+                    to_slots(p, s, slot);
+                    auto load_grad = [&](int o, float (&g)[F]) {
+                        const float4* src = &sm.grad[o][j][F * k / 4][t];
                         if (F == 2) {
                             const float2 v = reinterpret_cast<const float2*>(src)[k & 1];
                             g[0] = v.x;
@@ -1254,39 +1335,51 @@ __global__ void __launch_bounds__(kRunThreads, PERMUTO_RUN_BLOCKS) scatter_runs_
                                 g[(4 * q + 3) % F] = v.w;
                             }
                         }
+                    };
+                    if (ORDER != Order::Second) {
+                        float w[D + 1], g[F];
+                        vertex_weights<D>(s, lc.weight * kInv, w);
+                        load_grad(0, g);
+#pragma unroll
+                        for (int r = 0; r <= D; ++r) {
+#pragma unroll
+                            for (int f = 0; f < F; ++f) add[r][f] = w[r] * g[f];
+                        }
                     }
-                    Simplex<D> s;
-                    locate_simplex<D>(x, largest_coordinate<D>(x), lc, s);
-                    uint32_t slot[D + 1];
-                    to_slots(p, s, slot);
-                    float w[D + 1];
-                    if (DOUBLE) {
-                        float dpg[D];
+                    if (kSecond) {
+                        float w[D + 1], g[F], dpg[D];
                         load_vec(&sm.dpg[j][0][t], dpg);
                         second_order_weights(s, lc, dpg, w);
-                    } else {
-                        vertex_weights<D>(s, lc.weight * kInv, w);
+                        load_grad(ORDER == Order::Both ? 1 : 0, g);
+#pragma unroll
+                        for (int r = 0; r <= D; ++r) {
+#pragma unroll
+                            for (int f = 0; f < F; ++f) add[r][f] = ORDER == Order::Both ? fmaf(w[r], g[f], add[r][f]) : w[r] * g[f];
+                        }
                     }
                     if (runs) {
                         to_remainders(s.s, slot);
-                        to_remainders(s.s, w);
+#pragma unroll
+                        for (int f = 0; f < F; ++f) {
+                            float c[D + 1];
+#pragma unroll
+                            for (int r = 0; r <= D; ++r) c[r] = add[r][f];
+                            to_remainders(s.s, c);
+#pragma unroll
+                            for (int r = 0; r <= D; ++r) add[r][f] = c[r];
+                        }
 #pragma unroll
                         for (int r = 0; r <= D; ++r) {
                             const bool same = slot[r] == cur[r];
                             if (j > 0 && !same) red_add<F>(gbase, cur[r], acc[r]);
                             cur[r] = slot[r];
 #pragma unroll
-                            for (int f = 0; f < F; ++f) acc[r][f] = fmaf(w[r], g[f], same ? acc[r][f] : 0.f);
+                            for (int f = 0; f < F; ++f) acc[r][f] = add[r][f] + (same ? acc[r][f] : 0.f);
                             if (r == 0) kept += same ? 1 : 0;
                         }
                     } else if (j < count) {
 #pragma unroll
-                        for (int r = 0; r <= D; ++r) {
-                            float add[F];
-#pragma unroll
-                            for (int f = 0; f < F; ++f) add[f] = w[r] * g[f];
-                            red_add<F>(gbase, slot[r], add);
-                        }
+                        for (int r = 0; r <= D; ++r) red_add<F>(gbase, slot[r], add[r]);
                     }
                 }
                 if (runs) {
@@ -1519,10 +1612,35 @@ inline bool use_single_level(const Problem& p) {
 }
 
 
+#ifndef SPREAD_G
+#define SPREAD_G 2
+#endif
+#ifndef SPREAD_S
+#define SPREAD_S 2
+#endif
+// A batch too small to fill the multiprocessors with one block per 256 points has its levels split
+// over more blocks, as far as whole steps go.
+inline int spread_levels(const Problem& p, int lpp, Traffic t, int lps) {
+    const int levels = p.level_end - p.level_begin;
+    const int64_t points = (p.n_points + kThreads - 1) / kThreads;
+    const int64_t passes = sm_count() * (t == Traffic::Gather ? SPREAD_G : SPREAD_S) / points;
+    const int steps = (levels + lps - 1) / lps;
+    if (passes <= 1) return lpp;
+    const int each = (int)((steps + passes - 1) / passes) * lps;
+    return each < lpp ? each : lpp;
+}
+
 template <class Args>
 inline Args with_schedule(const Args& in, bool single, Traffic t) {
     Args a = in;
-    a.p.levels_per_pass = single ? 1 : pick_levels_per_pass(a.p, a.p.levels_per_pass, t, 8 / a.p.nr_feat);
+    const int lps = 8 / a.p.nr_feat;
+    if (single) {
+        a.p.levels_per_pass = 1;
+    } else {
+        const int requested = a.p.levels_per_pass;
+        a.p.levels_per_pass = pick_levels_per_pass(a.p, requested, t, lps);
+        if (requested <= 0) a.p.levels_per_pass = spread_levels(a.p, a.p.levels_per_pass, t, lps);
+    }
     return a;
 }
 
@@ -1546,7 +1664,15 @@ cudaError_t launch_forward_linear(const ForwardLinearArgs& in, cudaStream_t st) 
     }
     a.levels_offset = (int32_t)smem;
     smem += (size_t)a.p.nr_levels * kRecord * sizeof(float);
-    const dim3 g((unsigned)((a.p.n_points + kTileRows - 1) / kTileRows));
+    for (int i = 0; i < a.nr_layers; ++i) smem += (size_t)(a.layer[i].out_features + 3) / 4 * 4 * sizeof(float);
+    const MlpLayer& tail = a.layer[a.nr_layers - 1];
+    if (tail.out_features % 16 != 0) smem += (size_t)tail.out_features * tail.in_features * sizeof(float);
+    // as many blocks as an SM holds (launch bounds, shared and tensor memory), each walking over several tiles
+    const int64_t tiles = (a.p.n_points + kTileRows - 1) / kTileRows;
+    const int fits = (int)((size_t)(227 * 1024) / (smem + 2048));
+    const int resident = min(min(fused_blocks(F, hmax), 512 / a.tmem_cols), fits > 0 ? fits : 1);
+    const int64_t blocks = min(tiles, (int64_t)max(sm_count(), 1) * resident);
+    const dim3 g((unsigned)blocks);
     auto launch = [&](auto kernel) -> cudaError_t {
         if (smem + 1024 > 48 * 1024) {  // the kernel's few static shared words count against the default limit
             const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1596,22 +1722,23 @@ cudaError_t launch_double(const DoubleBackwardArgs& a, cudaStream_t st) {
 }
 
 // whole steps of 8 floats whatever the size of the batch
-template <int F, bool DOUBLE>
-cudaError_t launch_runs(const RunArgs& a, cudaStream_t st) {
-    constexpr int smem = (int)sizeof(RunStage<DOUBLE>);
-    const cudaError_t e = cudaFuncSetAttribute(scatter_runs_kernel<F, DOUBLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+template <int F, Order ORDER>
+cudaError_t launch_runs(const CombinedArgs& a, cudaStream_t st) {
+    constexpr int smem = (int)sizeof(RunStage<ORDER>);
+    const cudaError_t e = cudaFuncSetAttribute(scatter_runs_kernel<F, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     dim3 g = grid_for(a.p);
     g.x = (unsigned)((a.p.n_points + kRunThreads * kRunPoints - 1) / (kRunThreads * kRunPoints));
-    scatter_runs_kernel<F, DOUBLE><<<g, kRunThreads, smem, st>>>(a);
+    scatter_runs_kernel<F, ORDER><<<g, kRunThreads, smem, st>>>(a);
     return cudaGetLastError();
 }
-template <bool DOUBLE>
-cudaError_t launch_runs_by_width(const RunArgs& a, cudaStream_t st) {
+template <Order ORDER>
+cudaError_t launch_runs_by_width(const CombinedArgs& in, cudaStream_t st) {
+    const CombinedArgs a = with_schedule(in, false, Traffic::Scatter);
     switch (a.p.nr_feat) {
-        case 2: return launch_runs<2, DOUBLE>(a, st);
-        case 4: return launch_runs<4, DOUBLE>(a, st);
-        case 8: return launch_runs<8, DOUBLE>(a, st);
+        case 2: return launch_runs<2, ORDER>(a, st);
+        case 4: return launch_runs<4, ORDER>(a, st);
+        case 8: return launch_runs<8, ORDER>(a, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -1650,10 +1777,9 @@ cudaError_t PERMUTO_CAT(launch_forward_linear_dim, PERMUTO_DIM)(const ForwardLin
 // 207 + 300 us against 596 fused; without an order the fused kernel is the faster one).
 cudaError_t PERMUTO_CAT(launch_backward_dim, PERMUTO_DIM)(const BackwardArgs& a0, cudaStream_t st) {
     BackwardArgs in = a0;
-    if (in.p.order && in.lattice_grad) {
-        RunArgs r{in.p, in.grad_features, nullptr, in.lattice_grad, in.aggregate};
-        r = with_schedule(r, false, Traffic::Scatter);
-        const cudaError_t e = launch_runs_by_width<false>(r, st);
+    if (RUNS_IF(in.p) && in.lattice_grad) {
+        const CombinedArgs r{in.p, in.grad_features, nullptr, nullptr, in.lattice_grad, in.aggregate};
+        const cudaError_t e = launch_runs_by_width<Order::First>(r, st);
         if (e != cudaSuccess || !in.positions_grad) return e;
         in.lattice_grad = nullptr;
     }
@@ -1666,10 +1792,9 @@ cudaError_t PERMUTO_CAT(launch_backward_dim, PERMUTO_DIM)(const BackwardArgs& a0
 
 cudaError_t PERMUTO_CAT(launch_double_backward_dim, PERMUTO_DIM)(const DoubleBackwardArgs& a0, cudaStream_t st) {
     DoubleBackwardArgs in = a0;
-    if (in.p.order && in.lattice_grad) {
-        RunArgs r{in.p, in.grad_features, in.double_positions_grad, in.lattice_grad, in.aggregate};
-        r = with_schedule(r, false, Traffic::Scatter);
-        const cudaError_t e = launch_runs_by_width<true>(r, st);
+    if (RUNS_IF(in.p) && in.lattice_grad) {
+        const CombinedArgs r{in.p, nullptr, in.double_positions_grad, in.grad_features, in.lattice_grad, in.aggregate};
+        const cudaError_t e = launch_runs_by_width<Order::Second>(r, st);
         if (e != cudaSuccess || !in.grad_grad_features) return e;
         in.lattice_grad = nullptr;
     }
@@ -1679,6 +1804,16 @@ cudaError_t PERMUTO_CAT(launch_double_backward_dim, PERMUTO_DIM)(const DoubleBac
                           : (in.lattice_grad ? Traffic::Scatter : Traffic::Gather);
     const DoubleBackwardArgs a = with_schedule(in, single, t);
     PERMUTO_BY_WIDTH(launch_double, a, single, st)
+}
+
+cudaError_t PERMUTO_CAT(launch_combined_dim, PERMUTO_DIM)(const CombinedArgs& a, cudaStream_t st) {
+    if (a.p.order) return launch_runs_by_width<Order::Both>(a, st);
+    // small batches: two launches onto the same table
+    const BackwardArgs first{a.p, a.grad_features, a.lattice_grad, nullptr, a.aggregate, 0};
+    const cudaError_t e = PERMUTO_CAT(launch_backward_dim, PERMUTO_DIM)(first, st);
+    if (e != cudaSuccess) return e;
+    const DoubleBackwardArgs second{a.p, a.double_positions_grad, a.second_grad_features, a.lattice_grad, nullptr, a.aggregate};
+    return PERMUTO_CAT(launch_double_backward_dim, PERMUTO_DIM)(second, st);
 }
 
 cudaError_t PERMUTO_CAT(launch_debug_dim, PERMUTO_DIM)(const DebugArgs& a, cudaStream_t st) {

@@ -57,7 +57,6 @@ struct ForwardLinearArgs {
     float* out;            // [N, out_features of the last layer]
     int32_t k_pad;         // p.width rounded up to a multiple of 8 (one tf32 MMA consumes 8)
     int32_t tmem_cols;     // tensor-memory columns per block: a power of two >= 32
-    int32_t tmem_half;     // column offset of the second accumulator range (hidden layers ping-pong)
     int32_t* status;       // device word set non-zero when a wait on the tensor core ran out
     int32_t levels_offset; // shared-memory offset of the level constants (set by the launcher)
     int32_t out_vec8_ok;   // out rows can be written with 256-bit stores
@@ -78,6 +77,16 @@ struct DoubleBackwardArgs {
     const float* grad_features;
     float* lattice_grad;        // may be null
     float* grad_grad_features;  // may be null
+    int32_t aggregate;
+};
+
+// table gradient of a first-order and a double backward of the same points, summed
+struct CombinedArgs {
+    Problem p;
+    const float* grad_features;          // upstream gradient of the features
+    const float* double_positions_grad;
+    const float* second_grad_features;   // upstream gradient the differentiated backward received
+    float* lattice_grad;
     int32_t aggregate;
 };
 
@@ -102,6 +111,7 @@ int sm_count();
     cudaError_t launch_forward_linear_dim##d(const ForwardLinearArgs&, cudaStream_t); \
     cudaError_t launch_backward_dim##d(const BackwardArgs&, cudaStream_t);            \
     cudaError_t launch_double_backward_dim##d(const DoubleBackwardArgs&, cudaStream_t); \
+    cudaError_t launch_combined_dim##d(const CombinedArgs&, cudaStream_t);              \
     cudaError_t launch_debug_dim##d(const DebugArgs&, cudaStream_t);
 PERMUTO_DECLARE_DIM(2)
 PERMUTO_DECLARE_DIM(3)

@@ -339,10 +339,17 @@ int64_t permuto_order_bytes(int32_t pos_dim, int64_t nr_positions) {
     return (int64_t)(align256(n * record_bytes(pos_dim)) + align256(n * sizeof(uint2)) + cursor_bytes(n) + counter_bytes(n));
 }
 
+// Where the order's own time comes back, measured on 16-24 levels (us without -> with order, the order
+// itself included).  Training, 2 features: pos_dim 3, 2^16 points 73 -> 84, 2^17 125 -> 115, 2^20
+// 745 -> 533; pos_dim 6, 2^17 140 -> 147, 2^18 243 -> 234.  Wider entries have fewer levels to gain on and
+// ray samples of 3*10^5 points lose (119 -> 131), 2^20 points 431 -> 381.  Inference, 2 features:
+// 2^18 points 82 -> 78 but ray samples 64 -> 74, 2^19 149 -> 133, 2^20 288 -> 235; pos_dim 6, 2^20
+// 347 -> 340; 4 features, 2^20 174 -> 178; 8 levels, 2^18 21 -> 32.
 int permuto_order_pays(const permuto_config* cfg, int64_t nr_positions, int32_t with_gradients) {
     if (!cfg) return 0;
-    if (with_gradients) return nr_positions >= (1 << 17) ? 1 : 0;
-    return nr_positions >= (cfg->pos_dim <= 4 ? 1 << 18 : 1 << 20) ? 1 : 0;
+    const bool pairs = cfg->nr_feat_per_level == 2;
+    if (with_gradients) return nr_positions >= (!pairs ? 1 << 19 : (cfg->pos_dim <= 4 ? 1 << 17 : 1 << 18)) ? 1 : 0;
+    return pairs && cfg->nr_levels >= 12 && nr_positions >= (cfg->pos_dim <= 5 ? 1 << 19 : 1 << 20) ? 1 : 0;
 }
 
 int permuto_order_points(const permuto_config* cfg, const permuto_inputs* in, void* order, int64_t order_bytes, void* stream) {

@@ -17,8 +17,11 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <map>
+#include <memory>
 #include <mutex>
 #include <optional>
+#include <set>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -40,6 +43,7 @@ struct Api {
     decltype(&permuto_forward_mlp_ordered) forward_mlp;
     decltype(&permuto_backward_ordered) backward;
     decltype(&permuto_double_backward_ordered) double_backward;
+    decltype(&permuto_backward_combined) backward_combined;
     decltype(&permuto_adam_step) adam_step;
 } api = {};
 
@@ -59,6 +63,7 @@ void bind_api(const std::unordered_map<std::string, uintptr_t>& t) {
     take(api.forward_mlp, t, "permuto_forward_mlp_ordered");
     take(api.backward, t, "permuto_backward_ordered");
     take(api.double_backward, t, "permuto_double_backward_ordered");
+    take(api.backward_combined, t, "permuto_backward_combined");
     take(api.adam_step, t, "permuto_adam_step");
 }
 
@@ -137,6 +142,67 @@ struct Call : torch::CustomClassHolder {
     Tensor values, positions, window, shift, half, order;
     int levels_per_pass = 0;
     bool need_values = false, need_positions = false;
+
+    // A loss that reaches both the features and the position gradient gives the lattice values two
+    // gradients in one backward, from the first-order node and from a second-order one (EncodeBackward).
+    // Whichever of the two runs first leaves its part to the other, which adds both to the table in one
+    // pass -- instead of two passes, two cleared tables and their sum.  It only does so when the engine
+    // is certain to run the other one later in the same backward.
+    struct Part {
+        Tensor double_positions_grad;  // undefined: the first-order part
+        Tensor grad;
+    };
+    static constexpr int kFirst = 0;  // number of the first-order node; the others are second-order ones
+
+    int reserve_node() {
+        std::lock_guard<std::mutex> lock(mutex_);
+        nodes_.emplace_back();
+        return (int)nodes_.size() - 1;
+    }
+    void set_node(int number, const std::shared_ptr<torch::autograd::Node>& node) {
+        std::lock_guard<std::mutex> lock(mutex_);
+        nodes_[number] = node;
+    }
+
+    // from the node `number` of the running backward: true when another node has taken over `p`
+    bool leave(int number, Part p) {
+        const int task = torch::autograd::get_current_graph_task_id();
+        const auto* in_graph = torch::autograd::get_current_graph_task_nodes_in_graph();
+        if (task < 0 || !in_graph) return false;
+        const auto* info = torch::autograd::get_current_graph_task_exec_info();
+        std::lock_guard<std::mutex> lock(mutex_);
+        const int begin = number == kFirst ? 1 : kFirst, end = number == kFirst ? (int)nodes_.size() : kFirst + 1;
+        for (int to = begin; to < end; ++to) {
+            const auto node = nodes_[to].lock();
+            if (!node || in_graph->count(node.get()) == 0 || ran_.count({task, to}) || parts_.count({task, to})) continue;
+            if (info && !info->empty()) {  // a backward restricted to some inputs
+                const auto it = info->find(node.get());
+                if (it == info->end() || !it->second.should_execute()) continue;
+            }
+            parts_.emplace(std::make_pair(task, to), std::move(p));
+            return true;
+        }
+        return false;
+    }
+    // what was left for the node `number` in the running backward; nothing is left for it from here on
+    std::optional<Part> collect(int number) {
+        const auto key = std::make_pair(torch::autograd::get_current_graph_task_id(), number);
+        std::lock_guard<std::mutex> lock(mutex_);
+        ran_.insert(key);  // task numbers are never used again
+        std::optional<Part> p;
+        const auto it = parts_.find(key);
+        if (it != parts_.end()) {
+            p = std::move(it->second);
+            parts_.erase(it);
+        }
+        return p;
+    }
+
+  private:
+    std::mutex mutex_;
+    std::vector<std::weak_ptr<torch::autograd::Node>> nodes_ = std::vector<std::weak_ptr<torch::autograd::Node>>(1);
+    std::map<std::pair<int, int>, Part> parts_;
+    std::set<std::pair<int, int>> ran_;
 };
 
 // Same checks and messages as the reference (src/Encoding.cu:37-45, :63-66, :119-125).
@@ -274,6 +340,17 @@ SecondOrder run_double_backward(const Call& c, const Tensor& double_positions_gr
     return s;
 }
 
+// table gradient of both orders in one buffer
+Tensor run_combined(const Call& c, const Tensor& grad, const Call::Part& second) {
+    Bound b(c);
+    const Tensor dpg = second.double_positions_grad.contiguous();
+    Tensor values = empty(c.values.sizes(), c.positions);
+    check(api.backward_combined(&b.cfg, &b.in, data(c.order), grad.data_ptr<float>(), dpg.data_ptr<float>(),
+                                second.grad.data_ptr<float>(), values.data_ptr<float>(),
+                                PERMUTO_ZERO_OUTPUTS | (c.lattice->aggregate ? 0 : PERMUTO_NO_AGGREGATE), stream_of(c.positions)));
+    return values;
+}
+
 py::object as_python(const Tensor& t) { return t.defined() ? py::cast(t) : py::none(); }
 Tensor from_python(const py::handle& h) { return h.is_none() ? Tensor() : py::cast<Tensor>(h); }
 
@@ -287,14 +364,20 @@ Gradients backward_or_hook(const Call& c, const Tensor& grad, bool need_values, 
     return run_backward(c, grad, need_values, need_positions, {}, 0, -1, true, {});
 }
 
+// parts of one backward may be merged: no second differentiation, no data-parallel hooks
+bool may_merge(const Call& c) {
+    return !at::GradMode::is_enabled() && !c.lattice->on_backward && !c.lattice->on_double_backward;
+}
+
 // The first-order backward as a differentiable function of (upstream gradient, lattice values); its own
 // backward is the double backward from the position gradient.
 struct EncodeBackward : torch::autograd::Function<EncodeBackward> {
     static variable_list forward(AutogradContext* ctx, const Tensor& grad, const Tensor& values, const Tensor& positions,
-                                 const c10::intrusive_ptr<Call>& call, bool need_values, bool need_positions) {
+                                 const c10::intrusive_ptr<Call>& call, bool need_values, bool need_positions, int64_t number) {
         const Gradients g = backward_or_hook(*call, grad, need_values, need_positions);
         ctx->save_for_backward({grad, values, positions, call->window});
         ctx->saved_data["call"] = c10::IValue::make_capsule(call);
+        ctx->saved_data["number"] = number;
         ctx->saved_data["position_output"] = need_positions ? (need_values ? 1 : 0) : -1;
         ctx->set_materialize_grads(false);
         variable_list out;
@@ -304,16 +387,24 @@ struct EncodeBackward : torch::autograd::Function<EncodeBackward> {
     }
 
     static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
+        variable_list out(7);
+        const variable_list saved = ctx->get_saved_variables();  // checks the version counters
+        const auto call = c10::static_intrusive_pointer_cast<Call>(ctx->saved_data["call"].toCapsule());
+        const int number = (int)ctx->saved_data["number"].toInt();
+        const bool need_features = ctx->needs_input_grad(0), need_values = ctx->needs_input_grad(1);
+        const auto first = call->collect(number);
         // As in the reference, only the path through the position gradient is differentiated again; a
         // second-order term through the lattice-value gradient is not propagated.
-        variable_list out(6);
         const int64_t at = ctx->saved_data["position_output"].toInt();
-        if (at < 0 || !grads[at].defined()) return out;
-        const bool need_features = ctx->needs_input_grad(0), need_values = ctx->needs_input_grad(1);
-        if (!need_features && !need_values) return out;
-        const variable_list saved = ctx->get_saved_variables();
-        const auto call = c10::static_intrusive_pointer_cast<Call>(ctx->saved_data["call"].toCapsule());
-        SecondOrder s = run_double_backward(*call, grads[at], saved[0], need_values, need_features);
+        const bool second = at >= 0 && grads[at].defined();
+        if (first) {
+            out[1] = second ? run_combined(*call, first->grad, {grads[at], saved[0]})
+                            : run_backward(*call, first->grad, true, false, {}, 0, -1, true, {}).values;
+        }
+        if (!second) return out;
+        const bool own_values = need_values && !first && !(may_merge(*call) && call->leave(number, {grads[at], saved[0]}));
+        if (!need_features && !own_values) return out;
+        SecondOrder s = run_double_backward(*call, grads[at], saved[0], own_values, need_features);
         // data-parallel use: this second-order lattice gradient is summed over the ranks like the
         // first-order one, otherwise the replicated tables drift apart
         if (s.values.defined() && call->lattice->on_double_backward) {
@@ -321,7 +412,7 @@ struct EncodeBackward : torch::autograd::Function<EncodeBackward> {
             s.values = from_python(call->lattice->on_double_backward(s.values));
         }
         out[0] = s.features;
-        out[1] = s.values;
+        if (own_values) out[1] = s.values;
         return out;
     }
 };
@@ -344,12 +435,19 @@ struct Encode : torch::autograd::Function<Encode> {
         if (!need_values && !need_positions) return out;
         const Tensor grad = grads[0].contiguous();
         if (at::GradMode::is_enabled()) {
-            const variable_list g = EncodeBackward::apply(grad, saved[0], saved[1], call, need_values, need_positions);
+            const int number = call->reserve_node();
+            const variable_list g = EncodeBackward::apply(grad, saved[0], saved[1], call, need_values, need_positions, number);
+            call->set_node(number, g[0].grad_fn());
             if (need_values) out[0] = g[0];
             if (need_positions) out[1] = g[need_values ? 1 : 0];
-        } else {
-            const Gradients g = backward_or_hook(*call, grad, need_values, need_positions);
-            out[0] = g.values;
+            return out;
+        }
+        const auto second = call->collect(Call::kFirst);
+        if (second) out[0] = run_combined(*call, grad, *second);
+        const bool own_values = need_values && !second && !(may_merge(*call) && call->leave(Call::kFirst, {{}, grad}));
+        if (own_values || need_positions) {
+            const Gradients g = backward_or_hook(*call, grad, own_values, need_positions);
+            if (own_values) out[0] = g.values;
             out[1] = g.positions;
         }
         return out;
@@ -380,7 +478,9 @@ Tensor encode(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, 
         c->need_positions = positions.requires_grad();
     }
     if (!c->need_values && !c->need_positions) return run_forward(*c, true);
-    return Encode::apply(values, positions, c);
+    Tensor out = Encode::apply(values, positions, c);
+    c->set_node(Call::kFirst, out.grad_fn());
+    return out;
 }
 
 Tensor forward_mlp(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, const Tensor& positions,

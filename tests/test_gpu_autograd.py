@@ -82,3 +82,52 @@ def test_saved_tensors_are_guarded(setup):
         m.lattice_values.mul_(2.0)
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         out.backward(go)
+
+
+@pytest.mark.parametrize("n", [33, 2 ** 19 + 77])
+@pytest.mark.parametrize("d,feat,levels", [(2, 2, 3), (3, 2, 9), (3, 4, 5), (4, 8, 3), (6, 2, 5), (7, 4, 2)])
+def test_both_orders_in_one_backward(d, feat, levels, n):
+    """A loss on the features and on the position gradient: the table gradient of one backward is the
+    sum of the two separate ones (1e-4 * sum|addend|, as for any order of the fp32 sums), whichever
+    node runs first, restricted or not, and again when the graph is kept."""
+    from permutohedral_encoding_b200 import PermutoEncoding
+    torch.manual_seed(d)
+    m = PermutoEncoding(d, 2 ** 10, levels, feat, np.geomspace(1.0, 1e-2, levels))
+    with torch.no_grad():
+        m.lattice_values.uniform_(-1, 1)
+    pos = torch.rand(n, d, device=DEV, requires_grad=True)
+    go = torch.randn(n, m.output_dims(), device=DEV)
+    up = torch.randn(n, m.output_dims(), device=DEV, requires_grad=True)
+    dpg = torch.randn(n, d, device=DEV)
+
+    def graph():
+        out = m(pos)
+        (normal,) = torch.autograd.grad(out, pos, up, create_graph=True)
+        return out, normal
+
+    out, normal = graph()
+    first = torch.autograd.grad(out, m.lattice_values, go, retain_graph=True)[0]
+    second, want_up = torch.autograd.grad(normal, [m.lattice_values, up], dpg)
+    want = first + second
+    bound = 1e-4 * (first.abs() + second.abs()) + 1e-5 * want.abs().amax()
+
+    def check(got, got_up):
+        assert torch.all((got - want).abs() <= bound)
+        assert torch.all((got_up - want_up).abs() <= 1e-5 * want_up.abs().amax())
+
+    check(*torch.autograd.grad(graph(), [m.lattice_values, up], [go, dpg]))
+    out, normal = graph()
+    for _ in range(2):
+        m.lattice_values.grad = up.grad = None
+        torch.autograd.backward([out, normal], [go, dpg], inputs=[m.lattice_values, up], retain_graph=True)
+        check(m.lattice_values.grad, up.grad)
+    m.lattice_values.grad = up.grad = pos.grad = None
+    torch.autograd.backward([normal, out], [dpg, go])          # everything, the position gradient of `out` too
+    check(m.lattice_values.grad, up.grad)
+    assert pos.grad is not None
+    # the features' part runs first when the other part hangs on it
+    out, normal = graph()
+    m.lattice_values.grad = up.grad = None
+    (normal * dpg).sum().backward()
+    out2, _ = graph()
+    check(m.lattice_values.grad + torch.autograd.grad(out2, m.lattice_values, go)[0], up.grad)
