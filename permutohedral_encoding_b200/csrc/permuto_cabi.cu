@@ -88,7 +88,7 @@ int build_problem(const permuto_config* cfg, const permuto_inputs* in, const voi
     p.nr_levels = cfg->nr_levels;
     p.capacity = (uint32_t)cfg->capacity;
     p.cap_is_pow2 = (cfg->capacity & (cfg->capacity - 1)) == 0;
-    p.cap_magic = ~0ull / (uint64_t)cfg->capacity + 1ull;
+    p.cap_magic = (uint32_t)((1ull << 32) / (uint64_t)cfg->capacity);  // 0 for capacity 1, a power of two
     p.nr_feat = F;
     p.table_half = cfg->table_dtype == PERMUTO_TABLE_F16 ? 1 : 0;
     p.width = F * (cfg->nr_levels + extra);

@@ -84,11 +84,12 @@ __device__ __forceinline__ void load_pos(const Problem& p, int64_t n, float (&po
     for (int i = 0; i < D; ++i) pos[i] = __ldg(src + i * p.pos_stride_d);
 }
 
-// Hash modulo the capacity (EncodingGPU.cuh:34-36): a mask when it is a power of two, else an exact
-// remainder by multiplication with the host-computed 2^64 / capacity (Lemire, Kaser, Kurz 2019).
+// Hash modulo the capacity (EncodingGPU.cuh:34-36): a mask when it is a power of two, else the remainder
+// from the quotient estimate h * floor(2^32 / capacity) / 2^32, which is at most one too small.
 __device__ __forceinline__ uint32_t to_slot(const Problem& p, uint32_t h) {
     if (p.cap_is_pow2) return h & (p.capacity - 1u);
-    return (uint32_t)__umul64hi(p.cap_magic * h, (uint64_t)p.capacity);
+    const uint32_t r = h - __umulhi(h, p.cap_magic) * p.capacity;
+    return min(r, r - p.capacity);  // r - capacity wraps around to a larger number when r is the remainder
 }
 __device__ __forceinline__ void to_slots(const Problem& p, const Simplex<D>& s, uint32_t (&slot)[D + 1]) {
     uint32_t h[D + 1];

@@ -22,7 +22,7 @@ struct Problem {
     int32_t nr_levels;
     uint32_t capacity;
     int32_t cap_is_pow2;
-    uint64_t cap_magic;   // 2^64 / capacity rounded up (modulo 2^64), for the exact remainder by multiplication
+    uint32_t cap_magic;   // floor(2^32 / capacity), for the remainder by multiplication
     int32_t table_half;   // the value table is stored as fp16 (gathers only; gradients stay fp32)
     int32_t nr_feat;      // F: features per level, 2, 4 or 8
     int32_t width;        // F * (L + extra): row length of features / gradients

@@ -30,7 +30,7 @@ namespace {
 #define PERMUTO_CHUNK_BITS 21
 #endif
 #ifndef PERMUTO_CELL_POINTS_BITS
-#define PERMUTO_CELL_POINTS_BITS 3
+#define PERMUTO_CELL_POINTS_BITS 1
 #endif
 constexpr int kChunkBits = PERMUTO_CHUNK_BITS;
 constexpr int kCellBits = PERMUTO_CELL_POINTS_BITS;  // about 2^kCellBits points per cell
