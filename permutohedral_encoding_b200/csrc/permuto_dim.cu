@@ -48,9 +48,6 @@ constexpr int D = PERMUTO_DIM;
 #ifndef PERMUTO_MIN_BLOCKS_FORWARD
 #define PERMUTO_MIN_BLOCKS_FORWARD (PERMUTO_DIM <= 3 ? 8 : (PERMUTO_DIM <= 5 ? 6 : 4))
 #endif
-#ifndef PERMUTO_FWD_STAGGER
-#define PERMUTO_FWD_STAGGER 1
-#endif
 constexpr int kThreads = PERMUTO_THREADS;
 // wider table entries keep more addends live per vertex: leave them more registers
 constexpr int min_blocks(int feats, bool gather_only) {
@@ -315,6 +312,54 @@ __device__ __forceinline__ void store_row_segment(const Problem& p, float* rows,
     }
 }
 
+// Rows that do not start on a 32-byte boundary (level counts that are no multiple of four at F = 2, of two
+// at F = 4): the row's values, handed over 8 at a time, go out as whole 32-byte sectors shifted by the
+// row's misalignment, and only the ends of the row as 8-byte pieces.  Four 8-byte stores per step touch
+// every sector four times (18 levels, 2^19 points: forward 134 -> 118 us, in spatial order 108 -> 91).
+struct ShiftedRow {
+    float* at;       // sector the next 8 values start in
+    int m;           // values of that sector before them, 0, 2, 4 or 6
+    int left;        // values still held in `held` when the row ends
+    bool first;
+    float held[8];   // the last 8 values, rotated by m: the first m are still to be written
+
+    __device__ __forceinline__ explicit ShiftedRow(float* row) {
+        m = (int)((reinterpret_cast<uintptr_t>(row) >> 2) & 7u);
+        at = row - m;
+        left = 0;
+        first = true;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) held[i] = 0.f;
+    }
+    __device__ __forceinline__ void push(const float (&v)[8], int valid) {
+        float a[8], r[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] = (m & 4) ? v[(i + 4) & 7] : v[i];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = (m & 2) ? a[(i + 6) & 7] : a[i];
+        float out[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out[i] = i < m ? held[i] : r[i];
+        left = m + valid - 8;
+        if (left >= 0 && (!first || m == 0)) {
+            store8(at, out);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 8; q += 2)
+                if ((!first || q >= m) && q < m + valid) *reinterpret_cast<float2*>(at + q) = make_float2(out[q], out[q + 1]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) held[i] = r[i];
+        at += 8;
+        first = false;
+    }
+    __device__ __forceinline__ void finish() {
+#pragma unroll
+        for (int q = 0; q < 8; q += 2)
+            if (q < left) *reinterpret_cast<float2*>(at + q) = make_float2(held[q], held[q + 1]);
+    }
+};
+
 // ------------------------------------------------------------------------------------------
 // forward
 // ------------------------------------------------------------------------------------------
@@ -354,8 +399,14 @@ __device__ __forceinline__ void encode_step(const Problem& p, const float* level
     }
 }
 
-template <int F, int LPS, bool HALF>
-__global__ void __launch_bounds__(kThreads, (F == 2 ? PERMUTO_MIN_BLOCKS_FORWARD : min_blocks(F, false))) forward_kernel(const ForwardArgs a) {
+// SHIFTED: rows off the 32-byte grid, written by a ShiftedRow.  Its held values spill at the occupancy of
+// the plain kernel, which costs more than the warps (17 levels, 2^19 points, 8 / 6 / 5 / 4 blocks per SM:
+// 149 / 126 / 115 / 115 us).
+constexpr int forward_blocks(int feats, bool shifted) {
+    return feats == 2 ? (shifted ? (D <= 5 ? 5 : 4) : PERMUTO_MIN_BLOCKS_FORWARD) : min_blocks(feats, false);
+}
+template <int F, int LPS, bool HALF, bool SHIFTED>
+__global__ void __launch_bounds__(kThreads, forward_blocks(F, SHIFTED)) forward_kernel(const ForwardArgs a) {
     const Problem& p = a.p;
     __shared__ __align__(16) float levels[kStage * kRecord];
     const int64_t i_raw = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -366,6 +417,7 @@ __global__ void __launch_bounds__(kThreads, (F == 2 ? PERMUTO_MIN_BLOCKS_FORWARD
     float pos[D];
     const int64_t n = load_point(p, active ? i_raw : p.n_points - 1, pos);  // idle threads shadow the last point
     const float largest = largest_coordinate<D>(pos);
+    ShiftedRow row(a.features + n * p.width + F * pass_begin);  // used by SHIFTED only
 
 #pragma unroll 1
     for (int begin = pass_begin; begin < pass_end; begin += kStage) {
@@ -374,16 +426,22 @@ __global__ void __launch_bounds__(kThreads, (F == 2 ? PERMUTO_MIN_BLOCKS_FORWARD
         stage_levels(p, begin, end, levels);
         __syncthreads();
         const int nsteps = (end - begin + LPS - 1) / LPS;
-        int step = (PERMUTO_FWD_STAGGER && p.order == nullptr) ? (int)(blockIdx.x % (unsigned)nsteps) : 0;
+        // without an order, blocks start at different steps as in the scatter kernels (1 %)
+        int step = (!SHIFTED && p.order == nullptr) ? (int)(blockIdx.x % (unsigned)nsteps) : 0;
 #pragma unroll 1
         for (int it = 0; it < nsteps; ++it) {
             const int l0 = begin + step * LPS;
             step = (step + 1 == nsteps) ? 0 : step + 1;
             float out[F * LPS];
             encode_step<F, LPS, HALF>(p, levels + (l0 - begin) * kRecord, pos, largest, l0, end, out);
-            if (active) store_row_segment<F, LPS>(p, a.features, n, l0, out);
+            if (SHIFTED) {
+                if (active) row.push(reinterpret_cast<const float(&)[8]>(out), F * min(LPS, end - l0));
+            } else if (active) {
+                store_row_segment<F, LPS>(p, a.features, n, l0, out);
+            }
         }
     }
+    if (SHIFTED && active) row.finish();
 
     // raw points appended after the lattice levels (EncodingGPU.cuh:105-121)
     if (active && p.extra_levels > 0 && blockIdx.y == 0 && p.level_begin == 0) {
@@ -616,16 +674,13 @@ __device__ __forceinline__ void gelu2(float& x, float& y) {
     unpack2(fma2(m, q, pack2(fmaxf(x, 0.f), fmaxf(y, 0.f))), x, y);
 }
 
-#ifndef FB0
-#define FB0 10
-#endif
-#ifndef FB32
-#define FB32 6
-#endif
 // HMAX = 0: the encoding followed by ONE linear layer (out = features @ W^T + b).
 // HMAX = 32 / 64: a whole small MLP behind the encoding; hidden widths are multiples of 16 up to
 // HMAX (a thread holds its row of hidden activations in registers between two layers).
-constexpr int fused_blocks(int feats, int hmax) { return feats == 2 && hmax <= 32 ? (hmax ? FB32 : FB0) : 4; }
+// Resident blocks per SM: ten of the one-layer kernel, and six of the small MLP, whose row of 32 hidden
+// activations would spill at eight (pos_dim 4: 469 -> 400 us); more blocks also leave too little L1 beside
+// their shared memory for the gathers (one layer at eleven or twelve: 285 -> 297 us on 10^6 ray samples).
+constexpr int fused_blocks(int feats, int hmax) { return feats == 2 && hmax <= 32 ? (hmax ? 6 : 10) : 4; }
 template <int F, int LPS, bool HALF, int HMAX>
 __global__ void __launch_bounds__(kTileRows, fused_blocks(F, HMAX))
 forward_mlp_kernel(const ForwardLinearArgs a) {
@@ -700,7 +755,7 @@ forward_mlp_kernel(const ForwardLinearArgs a) {
     const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);  // tensor-memory lane = 32*warp + lane = row t
     bool ok = true;
     // A block walks over tiles of 128 points: what stands above -- tensor memory, barriers, weights -- is
-    // set up once per resident block, not once per tile (355 -> FILLIN us on 10^6 ray samples).
+    // set up once per resident block, not once per tile (355 -> 307 us on 10^6 ray samples).
     const int64_t tiles = (p.n_points + kTileRows - 1) / kTileRows;
 #pragma unroll 1
     for (int64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
@@ -1120,29 +1175,30 @@ backward_kernel(const BackwardArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------
-// table gradient of a coherent batch: P consecutive points per thread
+// table gradient of a batch in spatial order: two consecutive points per thread
 // ------------------------------------------------------------------------------------------
-#ifndef RUNS_IF
-#define RUNS_IF(p) ((p).order != nullptr)
-#endif
-#ifndef PERMUTO_RUN_POINTS
-#define PERMUTO_RUN_POINTS 2
-#endif
-#ifndef PERMUTO_RUN_THREADS
-#define PERMUTO_RUN_THREADS 128
-#endif
-constexpr int kRunPoints = PERMUTO_RUN_POINTS;
-constexpr int kRunThreads = PERMUTO_RUN_THREADS;
-#ifndef RB2
-#define RB2 5
-#define RB3 4
-#define RB4 3
-#endif
+// Consecutive points of an ordered batch share vertices on every level whose cells are wider than the
+// distance between points: a thread first sums what its two points add to the same vertex, in
+// registers; then the warp merges its lanes (scatter_level above), and a warp that sits in at most three
+// simplices -- coarse levels -- adds each simplex's D+1 vertices by recursive halving instead.
+//
+// What bounds it: on fine levels the rate of L2 reductions (pos_dim 3, levels 16-23 of 2^20 points:
+// 33 M reductions in 175 us, 190 G/s of the 220 G/s the device sustains), on coarse ones instruction issue
+// (levels 0-7: 77 % of the slots).  Coordinates and gradient rows wait in shared memory so that level
+// and point loops need not be unrolled: unrolled over 4 levels and 4 points four of five issue slots
+// waited for instructions (384 us against 309).  Two points per thread: 3, 4 and 8 take 309, 325 and
+// 378 us against 302.  Row segments go through registers as one 32-byte load; copied asynchronously as
+// two 16-byte ones they cost twice the L2 requests (2^24 points: 5257 us against 4410).
+// Against the fused scatter of an unordered batch: 2^20 points and 24 levels 440 -> 300 us, 2^24 points
+// 6300 -> 4230, pos_dim 6 545 -> 480, double backward 660 -> 540.
+constexpr int kRunPoints = 2;
+constexpr int kRunThreads = 128;
 // Resident blocks the registers have to allow: the D+1 running sums of F features and their slots stay
-// live over the points of a thread, and spilling them costs more than the warps they displace.
+// live over the points of a thread, and spilling them costs more than the warps they displace (pos_dim 6
+// at eight blocks 552 us, at five 490; 8 features, 2^20 points, at eight 236, at four 204).
 constexpr int run_blocks(int feats) {
     const int live = (D + 1) * (feats + 1);
-    return live <= 18 ? 8 : (live <= 26 ? RB2 : (live <= 45 ? RB3 : RB4));
+    return live <= 18 ? 8 : (live <= 26 ? 5 : (live <= 45 ? 4 : 3));
 }
 constexpr int kPosVec = D <= 3 ? 1 : 2;  // float4s per point: coordinates, row index last
 // D floats kept as kPosVec float4s, kRunThreads apart
@@ -1200,10 +1256,7 @@ __device__ __forceinline__ void reduce_vertices(float* level_base, unsigned lane
 
 // The addends of a warp whose lanes sit in at most kFewSimplices simplices (coarse levels): one reduction
 // per simplex.  False, with nothing done, otherwise.
-#ifndef PERMUTO_FEW_SIMPLICES
-#define PERMUTO_FEW_SIMPLICES 3
-#endif
-constexpr int kFewSimplices = PERMUTO_FEW_SIMPLICES;
+constexpr int kFewSimplices = 3;  // 0 (never) / 1 / 3 / 6: 313 / 301 / 300 / 303 us
 template <int F>
 __device__ __forceinline__ bool merge_simplices(float* level_base, unsigned lane, const uint32_t (&slot)[D + 1],
                                                 const float (&add)[D + 1][F]) {
@@ -1405,7 +1458,7 @@ __global__ void __launch_bounds__(kRunThreads, run_blocks(F)) scatter_runs_kerne
 // ------------------------------------------------------------------------------------------
 // double backward of the position gradient
 // ------------------------------------------------------------------------------------------
-template <int F, int LPS, bool TABLE, bool GGF, bool HALF>
+template <int F, int LPS, bool TABLE, bool GGF, bool HALF, bool SHIFTED>
 __global__ void __launch_bounds__(kThreads, min_blocks(F, false)) double_backward_kernel(const DoubleBackwardArgs a) {
     const Problem& p = a.p;
     __shared__ __align__(16) float levels[kStage * kRecord];
@@ -1421,6 +1474,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks(F, false)) double_backwar
 #pragma unroll
     for (int i = 0; i < D; ++i) dpg[i] = __ldg(a.double_positions_grad + n * D + i);
     Scatter sc{lane, active, a.aggregate != 0};  // as in backward_kernel
+    ShiftedRow row(a.grad_grad_features + n * p.width + F * pass_begin);  // used by SHIFTED only, as in forward_kernel
 
 #pragma unroll 1
     for (int begin = pass_begin; begin < pass_end; begin += kStage) {
@@ -1483,9 +1537,14 @@ __global__ void __launch_bounds__(kThreads, min_blocks(F, false)) double_backwar
 #pragma unroll
                 for (int f = 0; f < F; ++f) out[F * k + f] = o[f];
             }
-            if (GGF && active) store_row_segment<F, LPS>(p, a.grad_grad_features, n, l0, out);
+            if (SHIFTED) {
+                if (active) row.push(reinterpret_cast<const float(&)[8]>(out), F * min(LPS, end - l0));
+            } else if (GGF && active) {
+                store_row_segment<F, LPS>(p, a.grad_grad_features, n, l0, out);
+            }
         }
     }
+    if (SHIFTED && active) row.finish();
     if (GGF && active && p.extra_levels > 0 && blockIdx.y == 0 && p.level_begin == 0) {  // EncodingGPU.cuh:1290-1295
         float* dst = a.grad_grad_features + n * p.width + F * p.nr_levels;
         for (int c = 0; c < F * p.extra_levels; ++c) dst[c] = 0.f;
@@ -1557,7 +1616,7 @@ inline int pick_levels_per_pass(const Problem& p, int requested, Traffic t, int 
     const int levels = p.level_end - p.level_begin;
     int lpp = requested;
     if (lpp <= 0 && p.order != nullptr) {
-        lpp = levels;
+        lpp = levels;  // neighbouring points share their lines: nothing to split (pos_dim 3, 2^20 points: 201 us, two sweeps 224)
     } else if (lpp <= 0) {
         const double slice = (p.table_half ? 2.0 : 4.0) * p.nr_feat * p.capacity;
         const double mb = 1024.0 * 1024.0;
@@ -1613,18 +1672,13 @@ inline bool use_single_level(const Problem& p) {
 }
 
 
-#ifndef SPREAD_G
-#define SPREAD_G 2
-#endif
-#ifndef SPREAD_S
-#define SPREAD_S 2
-#endif
-// A batch too small to fill the multiprocessors with one block per 256 points has its levels split
-// over more blocks, as far as whole steps go.
-inline int spread_levels(const Problem& p, int lpp, Traffic t, int lps) {
+// A batch with fewer than two blocks of 256 points per multiprocessor has its levels split over more
+// blocks, as far as whole steps go (2^14 points: table gradient 31 -> 25 us, forward 12.7 -> 10.7).
+// Aiming for a full wave instead makes 2^15 and 2^16 points slower (position gradient 16.7 -> 20.8 us).
+inline int spread_levels(const Problem& p, int lpp, int lps) {
     const int levels = p.level_end - p.level_begin;
     const int64_t points = (p.n_points + kThreads - 1) / kThreads;
-    const int64_t passes = sm_count() * (t == Traffic::Gather ? SPREAD_G : SPREAD_S) / points;
+    const int64_t passes = 2 * sm_count() / points;
     const int steps = (levels + lps - 1) / lps;
     if (passes <= 1) return lpp;
     const int each = (int)((steps + passes - 1) / passes) * lps;
@@ -1640,18 +1694,24 @@ inline Args with_schedule(const Args& in, bool single, Traffic t) {
     } else {
         const int requested = a.p.levels_per_pass;
         a.p.levels_per_pass = pick_levels_per_pass(a.p, requested, t, lps);
-        if (requested <= 0) a.p.levels_per_pass = spread_levels(a.p, a.p.levels_per_pass, t, lps);
+        if (requested <= 0) a.p.levels_per_pass = spread_levels(a.p, a.p.levels_per_pass, lps);
     }
     return a;
 }
 
+template <int F, int LPS, bool SHIFTED>
+cudaError_t launch_forward_rows(const ForwardArgs& a, cudaStream_t st) {
+    if (a.p.table_half)
+        forward_kernel<F, LPS, true, SHIFTED><<<grid_for(a.p), kThreads, 0, st>>>(a);
+    else
+        forward_kernel<F, LPS, false, SHIFTED><<<grid_for(a.p), kThreads, 0, st>>>(a);
+    return cudaGetLastError();
+}
 template <int F, int LPS>
 cudaError_t launch_forward(const ForwardArgs& a, cudaStream_t st) {
-    if (a.p.table_half)
-        forward_kernel<F, LPS, true><<<grid_for(a.p), kThreads, 0, st>>>(a);
-    else
-        forward_kernel<F, LPS, false><<<grid_for(a.p), kThreads, 0, st>>>(a);
-    return cudaGetLastError();
+    if constexpr (F * LPS == 8 && F < 8)
+        if (!a.p.rows_vec8_ok) return launch_forward_rows<F, LPS, true>(a, st);
+    return launch_forward_rows<F, LPS, false>(a, st);
 }
 
 template <int F, int LPS>
@@ -1711,13 +1771,20 @@ cudaError_t launch_double(const DoubleBackwardArgs& a, cudaStream_t st) {
     const dim3 g = grid_for(a.p);
     const bool h = a.p.table_half != 0;
     if (a.lattice_grad && a.grad_grad_features) {
-        if (h) double_backward_kernel<F, LPS, true, true, true><<<g, kThreads, 0, st>>>(a);
-        else double_backward_kernel<F, LPS, true, true, false><<<g, kThreads, 0, st>>>(a);
+        if (h) double_backward_kernel<F, LPS, true, true, true, false><<<g, kThreads, 0, st>>>(a);
+        else double_backward_kernel<F, LPS, true, true, false, false><<<g, kThreads, 0, st>>>(a);
     } else if (a.lattice_grad) {
-        double_backward_kernel<F, LPS, true, false, false><<<g, kThreads, 0, st>>>(a);
+        double_backward_kernel<F, LPS, true, false, false, false><<<g, kThreads, 0, st>>>(a);
     } else if (a.grad_grad_features) {
-        if (h) double_backward_kernel<F, LPS, false, true, true><<<g, kThreads, 0, st>>>(a);
-        else double_backward_kernel<F, LPS, false, true, false><<<g, kThreads, 0, st>>>(a);
+        if constexpr (F * LPS == 8 && F < 8) {
+            if (!a.p.rows_vec8_ok) {
+                if (h) double_backward_kernel<F, LPS, false, true, true, true><<<g, kThreads, 0, st>>>(a);
+                else double_backward_kernel<F, LPS, false, true, false, true><<<g, kThreads, 0, st>>>(a);
+                return cudaGetLastError();
+            }
+        }
+        if (h) double_backward_kernel<F, LPS, false, true, true, false><<<g, kThreads, 0, st>>>(a);
+        else double_backward_kernel<F, LPS, false, true, false, false><<<g, kThreads, 0, st>>>(a);
     }
     return cudaGetLastError();
 }
@@ -1778,7 +1845,7 @@ cudaError_t PERMUTO_CAT(launch_forward_linear_dim, PERMUTO_DIM)(const ForwardLin
 // 207 + 300 us against 596 fused; without an order the fused kernel is the faster one).
 cudaError_t PERMUTO_CAT(launch_backward_dim, PERMUTO_DIM)(const BackwardArgs& a0, cudaStream_t st) {
     BackwardArgs in = a0;
-    if (RUNS_IF(in.p) && in.lattice_grad) {
+    if (in.p.order && in.lattice_grad) {
         const CombinedArgs r{in.p, in.grad_features, nullptr, nullptr, in.lattice_grad, in.aggregate};
         const cudaError_t e = launch_runs_by_width<Order::First>(r, st);
         if (e != cudaSuccess || !in.positions_grad) return e;
@@ -1793,7 +1860,7 @@ cudaError_t PERMUTO_CAT(launch_backward_dim, PERMUTO_DIM)(const BackwardArgs& a0
 
 cudaError_t PERMUTO_CAT(launch_double_backward_dim, PERMUTO_DIM)(const DoubleBackwardArgs& a0, cudaStream_t st) {
     DoubleBackwardArgs in = a0;
-    if (RUNS_IF(in.p) && in.lattice_grad) {
+    if (in.p.order && in.lattice_grad) {
         const CombinedArgs r{in.p, nullptr, in.double_positions_grad, in.grad_features, in.lattice_grad, in.aggregate};
         const cudaError_t e = launch_runs_by_width<Order::Second>(r, st);
         if (e != cudaSuccess || !in.grad_grad_features) return e;

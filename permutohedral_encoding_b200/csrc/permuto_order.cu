@@ -14,9 +14,13 @@
 //   order_scan_kernel      exclusive sums over each group of kScanBins cells, plus the group's place
 //   order_scatter_kernel   record {coordinates, index} to cell base + arrival number
 // Only neighbouring cells have to stay together, so groups take their place in the order they arrive
-// (one atomic on a cursor) and no sum over all cells is needed.  Batches above kChunk points are
-// sorted chunk by chunk: the records of a chunk (64 MB) and the rows it touches stay within reach of
-// L2 and of the address translation caches.
+// (one atomic on a cursor) and no sum over all cells is needed.  Large batches are sorted chunk by
+// chunk, so that the records and counters of a chunk (32 and 4 MB) stay in L2.
+//
+// What bounds it: the counters' returning atomics (about 92 G/s) and the scattered 16-byte records; 34 us
+// for 2^20 points, 520 us for 2^24, where reading and writing its data once would take 5 and 75 us.
+// Tried: counting with reductions and taking the places in the scatter kernel (34 -> 38 us, 2^24 points
+// 520 -> 432), counters 16 or 32 bytes apart (no change).
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -26,14 +30,10 @@
 namespace permuto {
 namespace {
 
-#ifndef PERMUTO_CHUNK_BITS
-#define PERMUTO_CHUNK_BITS 21
-#endif
-#ifndef PERMUTO_CELL_POINTS_BITS
-#define PERMUTO_CELL_POINTS_BITS 1
-#endif
-constexpr int kChunkBits = PERMUTO_CHUNK_BITS;
-constexpr int kCellBits = PERMUTO_CELL_POINTS_BITS;  // about 2^kCellBits points per cell
+constexpr int kChunkBits = 21;      // points per chunk; 2^20 / 2^22 / 2^23 / 2^24 points: order 461 / 568 / 675 / 772 us
+                                    // against 520, but the forward after it 3160 / 3085 / 3064 / 3018 against 3080
+constexpr int kCellBits = 1;        // about two points per cell: more share counters, whose atomics then collide
+                                    // (8 / 32 / 128 / 512 points per cell, 2^20 points: 34 / 37 / 39 / 72 us)
 constexpr int kScanBins = 1024;     // cells per block of the scan
 constexpr int kThreads = 256;
 constexpr int kPerThread = 4;       // consecutive points of a thread: whole 16-byte vectors of any row length
@@ -340,16 +340,16 @@ int64_t permuto_order_bytes(int32_t pos_dim, int64_t nr_positions) {
 }
 
 // Where the order's own time comes back, measured on 16-24 levels (us without -> with order, the order
-// itself included).  Training, 2 features: pos_dim 3, 2^16 points 73 -> 84, 2^17 125 -> 115, 2^20
-// 745 -> 533; pos_dim 6, 2^17 140 -> 147, 2^18 243 -> 234.  Wider entries have fewer levels to gain on and
+// itself included).  Training, 2 features: pos_dim 3, 2^17 points 125 -> 115 but ray
+// samples 85 -> 99, 2^18 216 -> 170 (rays 170 -> 167), 2^20 745 -> 533; pos_dim 6, 2^17 140 -> 147, 2^18 243 -> 234.  Wider entries have fewer levels to gain on and
 // ray samples of 3*10^5 points lose (119 -> 131), 2^20 points 431 -> 381.  Inference, 2 features:
 // 2^18 points 82 -> 78 but ray samples 64 -> 74, 2^19 149 -> 133, 2^20 288 -> 235; pos_dim 6, 2^20
 // 347 -> 340; 4 features, 2^20 174 -> 178; 8 levels, 2^18 21 -> 32.
 int permuto_order_pays(const permuto_config* cfg, int64_t nr_positions, int32_t with_gradients) {
     if (!cfg) return 0;
     const bool pairs = cfg->nr_feat_per_level == 2;
-    if (with_gradients) return nr_positions >= (!pairs ? 1 << 19 : (cfg->pos_dim <= 4 ? 1 << 17 : 1 << 18)) ? 1 : 0;
-    return pairs && cfg->nr_levels >= 12 && nr_positions >= (cfg->pos_dim <= 5 ? 1 << 19 : 1 << 20) ? 1 : 0;
+    if (with_gradients) return nr_positions >= (pairs ? 1 << 18 : 1 << 19) ? 1 : 0;
+    return pairs && cfg->nr_levels >= 16 && nr_positions >= (cfg->pos_dim <= 5 ? 1 << 19 : 1 << 20) ? 1 : 0;
 }
 
 int permuto_order_points(const permuto_config* cfg, const permuto_inputs* in, void* order, int64_t order_bytes, void* stream) {
