@@ -203,7 +203,10 @@ class OursStep:
         self.hook = LatticeGradAllReduce(self.m, nr_buckets=buckets, policy=ARGS.bucket_policy, multimem=mm,
                                          copy_out=ARGS.copy_out, clear=ARGS.clear) if world > 1 else None
         self.collective = None if self.hook is None else ("multimem" if self.hook._symm is not None else "nccl")
-        self.launches_per_step = 2 if world == 1 else 1 + len(self.hook.buckets)
+        # the three kernels of the spatial order (batches from 2^18 points on), the forward, and the table
+        # gradient once or once per bucket
+        order = 3 if w["total_points"] // world >= 2 ** 18 else 0
+        self.launches_per_step = order + (2 if world == 1 else 1 + len(self.hook.buckets))
         self.opt = None
 
     @property
@@ -228,6 +231,7 @@ class OursStep:
         from permutohedral_encoding_b200 import _native as nat
         I = nat.EncodingInput(self.m.lattice_values.detach(), pos, self.m.anneal_window, True, False)
         lat = self.m.lattice
+        I.m_order = lat.order(I, nat.ORDER_TRAINING)   # what the module does for a batch of this size
         buf = torch.empty_like(self.m.lattice_values)
         return (lambda: lat.forward(I)), (lambda: lat.backward(I, grad_out, lattice_grad_out=buf))
 

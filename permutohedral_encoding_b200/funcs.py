@@ -7,6 +7,10 @@ eikonal term) can be differentiated again into the lattice values and into the u
 gradient.  Differences from the reference, all internal: tensors are kept with
 ``save_for_backward`` (version-counter checks apply), exactly as many gradients are returned as
 there are inputs, and features are ``[N, 2*(L+extra)]`` so no transposing copy happens here.
+
+The module's own graph is the same pair as C++ nodes (csrc/permuto_torch.cpp), which cost less per call
+and compute only the gradients the running backward needs; this Python form takes any object with
+the wrapper's methods.
 """
 import torch
 
