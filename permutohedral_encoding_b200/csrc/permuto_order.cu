@@ -9,7 +9,7 @@
 // writes its rows to the point's own index, which travels in the record.
 //
 // A counting sort over curve cells:
-//   (counters cleared)
+//   order_clear_kernel     zero counters
 //   order_count_kernel     cell of every point, its arrival number inside the cell (atomic counter)
 //   order_scan_kernel      exclusive sums over each group of kScanBins cells, plus the group's place
 //   order_scatter_kernel   record {coordinates, index} to cell base + arrival number
@@ -17,8 +17,8 @@
 // (one atomic on a cursor) and no sum over all cells is needed.  Large batches are sorted chunk by
 // chunk, so that the records and counters of a chunk (32 and 4 MB) stay in L2.
 //
-// What bounds it: the counters' returning atomics (about 92 G/s) and the scattered 16-byte records; 34 us
-// for 2^20 points, 520 us for 2^24, where reading and writing its data once would take 5 and 75 us.
+// What bounds it: the counters' returning atomics (about 92 G/s) and the scattered 16-byte records; 32 us
+// for 2^20 points (34 with a separate clear and a serial grid), 520-540 us for 2^24, where reading and writing its data once would take 5 and 75 us.
 // Tried: counting with reductions and taking the places in the scatter kernel (34 -> 38 us, 2^24 points
 // 520 -> 432), counters 16 or 32 bytes apart (no change).
 #include <cstdint>
@@ -90,6 +90,13 @@ __device__ __forceinline__ float warp_sum_all(float v) {
     return v;
 }
 
+// clears the counters and cursors while the blocks of the count kernel already work out their grid
+__global__ void __launch_bounds__(256) order_clear_kernel(uint4* words, uint32_t n) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    for (uint32_t i = blockIdx.x * 1024u + threadIdx.x, end = min(n, blockIdx.x * 1024u + 1024u); i < end; i += 256u)
+        words[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // Cell of a point: `bits` halvings of the batch's extent, each of the dimension whose cells are widest
 // at that moment -- cells stay near cubes whatever the aspect of the batch, flat dimensions get none --
 // and the coordinate bits interleaved in that sequence.  Every block derives the grid of its chunk
@@ -98,7 +105,7 @@ template <int D>
 __global__ void __launch_bounds__(kThreads) order_count_kernel(const OrderArgs a) {
     constexpr int kWarps = kThreads / 32;
     __shared__ float part[2 * D][kWarps];
-    __shared__ float lo[D], inv_cell[D];
+    __shared__ float lo[D], width[D], inv_cell[D];
     __shared__ int halvings[D];
     __shared__ uint8_t key_bit[D][24];                // of a dimension's k-th halving
     __shared__ uint32_t spread[D][kNibbles][16];      // coordinate nibble -> its key bits
@@ -138,40 +145,36 @@ __global__ void __launch_bounds__(kThreads) order_count_kernel(const OrderArgs a
             dev[i] = warp_sum_all(lane < kWarps ? d + fabsf(m - mean[i]) : 0.f) * (1.f / kWarps);
         }
         if (lane == 0) {
-            float cell[D];
-            int halved[D];
 #pragma unroll
             for (int i = 0; i < D; ++i) {
                 // 4.4 mean absolute deviations hold a uniform box with a margin; what lies outside
                 // goes to the edge cells
-                cell[i] = fmaxf(4.4f * dev[i], 1e-30f);
-                lo[i] = mean[i] - 0.5f * cell[i];
-                halved[i] = 0;
-            }
-            for (int b = a.bits - 1; b >= 0; --b) {
-                int best = 0;
-                float widest = cell[0];
-#pragma unroll
-                for (int i = 1; i < D; ++i)
-                    if (cell[i] > widest) {
-                        widest = cell[i];
-                        best = i;
-                    }
-#pragma unroll
-                for (int i = 0; i < D; ++i)
-                    if (i == best) {
-                        cell[i] *= 0.5f;
-                        key_bit[i][halved[i]++] = (uint8_t)b;
-                    }
-            }
-#pragma unroll
-            for (int i = 0; i < D; ++i) {
-                halvings[i] = halved[i];
-                inv_cell[i] = 1.f / cell[i];
+                width[i] = fmaxf(4.4f * dev[i], 1e-30f);
+                lo[i] = mean[i] - 0.5f * width[i];
+                halvings[i] = 0;
             }
         }
     }
     __syncthreads();
+    // Halving k of dimension i splits cells of width[i] / 2^k.  Its place in the sequence is the number of
+    // halvings of wider cells, counted from the widths' exponents and mantissas (all places at once: taking
+    // the widest dimension `bits` times in one thread was a microsecond of every block).
+    if (t < D * 24) {
+        const int i = t / 24, k = t % 24, mine = __float_as_int(width[i]);
+        int place = 0;
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            const int other = __float_as_int(width[j]);
+            const int a0 = other & 0x7fffff, b0 = mine & 0x7fffff;
+            place += max(0, (other >> 23) - (mine >> 23) + k + ((a0 > b0 || (a0 == b0 && j < i)) ? 1 : 0));
+        }
+        if (place < a.bits) {
+            key_bit[i][k] = (uint8_t)(a.bits - 1 - place);
+            atomicMax(&halvings[i], k + 1);
+        }
+    }
+    __syncthreads();
+    if (t < D) inv_cell[t] = ldexpf(1.f / width[t], halvings[t]);
     for (int e = t; e < D * kNibbles * 16; e += kThreads) {
         const int dim = e / (kNibbles * 16), nibble = e / 16 % kNibbles, v = e % 16;
         uint32_t r = 0u;
@@ -183,6 +186,7 @@ __global__ void __launch_bounds__(kThreads) order_count_kernel(const OrderArgs a
         spread[dim][nibble][v] = r;
     }
     __syncthreads();
+    cudaGridDependencySynchronize();  // the counters are cleared
 #pragma unroll 1
     for (int round = 0; round < a.rounds; ++round) {
         const uint32_t n = first + round * (uint32_t)kPerBlock + t * kPerThread;
@@ -318,9 +322,10 @@ template <int D>
 cudaError_t launch(const OrderArgs& a, cudaStream_t st) {
     const unsigned points = (a.n + kPerBlock - 1) / kPerBlock;
     const unsigned counting = (points + a.rounds - 1) / a.rounds;
-    cudaError_t e = cudaMemsetAsync(a.cursors, 0, cursor_bytes(a.n) + counter_bytes(a.n), st);
+    const uint32_t words = (uint32_t)((cursor_bytes(a.n) + counter_bytes(a.n)) / sizeof(uint4));
+    order_clear_kernel<<<(words + 1023u) / 1024u, 256, 0, st>>>(reinterpret_cast<uint4*>(a.cursors), words);
+    cudaError_t e = launch_early(order_count_kernel<D>, counting, kThreads, a, st);
     if (e != cudaSuccess) return e;
-    order_count_kernel<D><<<counting, kThreads, 0, st>>>(a);
     e = launch_early(order_scan_kernel, (order_chunks(a.n) << a.bits) / kScanBins, 256, a, st);
     if (e != cudaSuccess) return e;
     e = launch_early(order_scatter_kernel<D>, points, kThreads, a, st);
