@@ -17,8 +17,6 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
-#include <algorithm>
-#include <cmath>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -123,19 +121,6 @@ struct Lattice : torch::CustomClassHolder {
             on_backward.release();
             on_double_backward.release();
         }
-    }
-
-    // Leading levels (whole steps) on which a slot receives more than 2^18 addends from n points in a unit
-    // box: lattice vertices have the density sigma^-d / ((d+1)^(d-1) * sqrt(d+1)).
-    int heavy_levels(int64_t n) const {
-        const int d = cfg.pos_dim, step = 8 / cfg.nr_feat_per_level;
-        const float* scale = scale_host_.data_ptr<float>();  // [L, d]; scale[l, 0] = 1 / (sigma_l * sqrt(2))
-        int l = 0;
-        for (; l < cfg.nr_levels; ++l) {
-            const double vertices = std::pow(scale[l * d] * std::sqrt(2.0), d) / (std::pow(d + 1.0, d - 1) * std::sqrt(d + 1.0));
-            if (n * (d + 1.0) <= 262144.0 * std::max(vertices, 1.0)) break;
-        }
-        return std::min((l + step / 2) / step * step, (int)cfg.nr_levels);
     }
 
     Tensor scale_on(const c10::Device& device) {
@@ -294,6 +279,16 @@ Tensor run_forward(Call& c, bool may_order) {
     return out;
 }
 
+// Up to this many points the table gradients are summed in spatial order, beyond it in the sequence of the
+// batch.  A slot of a coarse level receives up to a million fp32 addends and more, and what their sum rounds
+// to follows the sequence and the merging inside the warps.  Two runs of one sequence differ in the 2-norm by
+// 2-3e-6 at 2^22 and 2.4-4e-6 at 2^24 points, the two sequences by about 2.5e-9 * sqrt(points): 2-3e-6 at 2^20,
+// 3-7e-6 at 2^22, 6.6-11e-6 at 2^24 (pos_dim 2, 3 and 6, 6 to 24 levels).  The line keeps that below 1e-5, on a
+// measured size: whether a batch is ordered does not show in its gradient.  Spatial order is closer to a
+// float64 sum of the same addends (1.3-3.4e-6 against 2-6.5e-6 at 2^22).
+constexpr int64_t kOrderedSums = 1 << 22;
+bool ordered_sums(const Call& c) { return c.order.defined() && c.positions.size(0) <= kOrderedSums; }
+
 struct Gradients {
     Tensor values, positions;
 };
@@ -323,23 +318,16 @@ Gradients run_backward(const Call& c, const Tensor& grad, bool need_values, bool
         }
     }
     const int end = level_end < 0 ? b.cfg.nr_levels : level_end;
-    auto launch = [&](const void* order, float* values, float* positions, int from, int to) {
-        if (from < to)
-            check(api.backward(&b.cfg, &b.in, order, grad.data_ptr<float>(), values, positions, from, to, flags,
-                               stream_of(c.positions)));
+    auto launch = [&](const void* order, const Tensor& values, const Tensor& positions) {
+        check(api.backward(&b.cfg, &b.in, order, grad.data_ptr<float>(), values.defined() ? values.data_ptr<float>() : nullptr,
+                           positions.defined() ? positions.data_ptr<float>() : nullptr, level_begin, end, flags,
+                           stream_of(c.positions)));
     };
-    float* values = g.values.defined() ? g.values.data_ptr<float>() : nullptr;
-    float* positions = g.positions.defined() ? g.positions.data_ptr<float>() : nullptr;
-    if (c.order.defined() && values && n > (1 << 22)) {
-        // fp32 sums of 10^5 and more addends depend on their sequence by up to 1e-3 of a cancelling entry
-        // (2^24 points): such levels are summed in the sequence of the batch, as without an order, so that
-        // the order does not show in the gradient (2^24 points, 24 levels: 5450 us, all in order 4210)
-        const int heavy = std::min(std::max(c.lattice->heavy_levels(n), level_begin), end);
-        launch(nullptr, values, nullptr, level_begin, heavy);
-        launch(data(c.order), values, nullptr, heavy, end);
-        if (positions) launch(data(c.order), nullptr, positions, level_begin, end);
+    if (c.order.defined() && need_values && !ordered_sums(c)) {
+        launch(nullptr, g.values, {});
+        if (need_positions) launch(data(c.order), {}, g.positions);
     } else {
-        launch(data(c.order), values, positions, level_begin, end);
+        launch(data(c.order), g.values, g.positions);
     }
     return g;
 }
@@ -362,11 +350,19 @@ SecondOrder run_double_backward(const Call& c, const Tensor& double_positions_gr
     SecondOrder s;
     if (need_values) s.values = empty(c.values.sizes(), c.positions);
     if (need_features) s.features = empty(gf.sizes(), c.positions);
-    check(api.double_backward(&b.cfg, &b.in, data(c.order), dpg.data_ptr<float>(), gf.data_ptr<float>(),
-                              need_values ? s.values.data_ptr<float>() : nullptr,
-                              need_features ? s.features.data_ptr<float>() : nullptr,
-                              PERMUTO_ZERO_OUTPUTS | (c.lattice->aggregate ? 0 : PERMUTO_NO_AGGREGATE),
-                              stream_of(c.positions)));
+    auto launch = [&](const void* order, const Tensor& values, const Tensor& features) {
+        check(api.double_backward(&b.cfg, &b.in, order, dpg.data_ptr<float>(), gf.data_ptr<float>(),
+                                  values.defined() ? values.data_ptr<float>() : nullptr,
+                                  features.defined() ? features.data_ptr<float>() : nullptr,
+                                  PERMUTO_ZERO_OUTPUTS | (c.lattice->aggregate ? 0 : PERMUTO_NO_AGGREGATE),
+                                  stream_of(c.positions)));
+    };
+    if (c.order.defined() && need_values && !ordered_sums(c)) {
+        launch(nullptr, s.values, {});
+        if (need_features) launch(data(c.order), {}, s.features);
+    } else {
+        launch(data(c.order), s.values, s.features);
+    }
     return s;
 }
 
@@ -394,9 +390,11 @@ Gradients backward_or_hook(const Call& c, const Tensor& grad, bool need_values, 
     return run_backward(c, grad, need_values, need_positions, {}, 0, -1, true, {});
 }
 
-// parts of one backward may be merged: no second differentiation, no data-parallel hooks
+// parts of one backward may be merged: no second differentiation, no data-parallel hooks, and not where each
+// part is summed in the sequence of the batch (the two sums stay separate there, as without an order)
 bool may_merge(const Call& c) {
-    return !at::GradMode::is_enabled() && !c.lattice->on_backward && !c.lattice->on_double_backward;
+    return !at::GradMode::is_enabled() && !c.lattice->on_backward && !c.lattice->on_double_backward &&
+           c.positions.size(0) <= kOrderedSums;
 }
 
 // The first-order backward as a differentiable function of (upstream gradient, lattice values); its own
