@@ -184,11 +184,18 @@ int permuto_double_backward(const permuto_config *cfg, const permuto_inputs *in,
  * 256-byte aligned, for in->positions; the *_ordered entry points below take it together with the SAME
  * positions (NULL = no order, which is what the plain entry points pass).  One order serves the forward,
  * backward and double backward of a batch; it holds a copy of the coordinates, so it is only valid
- * while the positions are unchanged. */
+ * while the positions are unchanged.
+ * permuto_order_records does the same with two buffers, each 256-byte aligned: the order itself, of
+ * permuto_order_record_bytes(pos_dim, N) bytes (one record per point, and pos_dim bytes more, so that the
+ * size tells pos_dim and N), and scratch of permuto_order_scratch_bytes(pos_dim, N) bytes that is free again
+ * once the sort has run on `stream`.  All sizes are 0 for a pos_dim or N out of range. */
 int permuto_order_pays(const permuto_config *cfg, int64_t nr_positions, int32_t with_gradients); /* 1: worth it */
 int64_t permuto_order_bytes(int32_t pos_dim, int64_t nr_positions);
 int permuto_order_points(const permuto_config *cfg, const permuto_inputs *in, void *order, int64_t order_bytes,
                          void *stream);
+int64_t permuto_order_record_bytes(int32_t pos_dim, int64_t nr_positions);
+int64_t permuto_order_scratch_bytes(int32_t pos_dim, int64_t nr_positions);
+int permuto_order_records(const permuto_config *cfg, const permuto_inputs *in, void *records, void *scratch, void *stream);
 int permuto_forward_ordered(const permuto_config *cfg, const permuto_inputs *in, const void *order,
                             float *features, void *stream);
 int permuto_forward_mlp_ordered(const permuto_config *cfg, const permuto_inputs *in, const void *order,

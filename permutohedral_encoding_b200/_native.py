@@ -49,7 +49,8 @@ EXPORTED_SYMBOLS = (
     "permuto_abi_version", "permuto_last_error", "permuto_extra_levels", "permuto_scale_factor",
     "permuto_forward", "permuto_backward", "permuto_double_backward", "permuto_debug_lattice",
     "permuto_probe_random_access", "permuto_adam_step", "permuto_forward_linear", "permuto_forward_mlp",
-    "permuto_order_pays", "permuto_order_bytes", "permuto_order_points", "permuto_forward_ordered", "permuto_forward_mlp_ordered",
+    "permuto_order_pays", "permuto_order_bytes", "permuto_order_points", "permuto_order_record_bytes",
+    "permuto_order_scratch_bytes", "permuto_order_records", "permuto_forward_ordered", "permuto_forward_mlp_ordered",
     "permuto_backward_ordered", "permuto_double_backward_ordered", "permuto_backward_combined",
 )
 
@@ -101,6 +102,12 @@ def _load() -> C.CDLL:
     lib.permuto_order_pays.argtypes = [cfgp, C.c_int64, C.c_int32]
     lib.permuto_order_bytes.restype = C.c_int64
     lib.permuto_order_bytes.argtypes = [C.c_int32, C.c_int64]
+    lib.permuto_order_record_bytes.restype = C.c_int64
+    lib.permuto_order_record_bytes.argtypes = [C.c_int32, C.c_int64]
+    lib.permuto_order_scratch_bytes.restype = C.c_int64
+    lib.permuto_order_scratch_bytes.argtypes = [C.c_int32, C.c_int64]
+    lib.permuto_order_records.restype = C.c_int
+    lib.permuto_order_records.argtypes = [cfgp, inp, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.permuto_order_points.restype = C.c_int
     lib.permuto_order_points.argtypes = [cfgp, inp, C.c_void_p, C.c_int64, C.c_void_p]
     lib.permuto_forward_ordered.restype = C.c_int

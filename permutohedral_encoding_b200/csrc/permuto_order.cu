@@ -302,6 +302,7 @@ size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 size_t record_bytes(int pos_dim) { return pos_dim <= 3 ? 16 : 32; }
 size_t cursor_bytes(uint32_t n) { return align256(sizeof(uint32_t) * order_chunks(n)); }
 size_t counter_bytes(uint32_t n) { return (sizeof(uint32_t) * order_chunks(n)) << order_bits(n); }
+bool order_sizes_ok(int32_t pos_dim, int64_t n) { return pos_dim >= 2 && pos_dim <= 7 && n >= 1 && n <= (int64_t)0x7fffffff; }
 
 // launched while the kernel before it drains; the kernel waits for it itself
 template <class K>
@@ -337,11 +338,23 @@ cudaError_t launch(const OrderArgs& a, cudaStream_t st) {
 
 extern "C" {
 
+int64_t permuto_order_record_bytes(int32_t pos_dim, int64_t nr_positions) {
+    using namespace permuto;
+    if (!order_sizes_ok(pos_dim, nr_positions)) return 0;
+    return nr_positions * (int64_t)record_bytes(pos_dim) + pos_dim;
+}
+
+int64_t permuto_order_scratch_bytes(int32_t pos_dim, int64_t nr_positions) {
+    using namespace permuto;
+    if (!order_sizes_ok(pos_dim, nr_positions)) return 0;
+    const uint32_t n = (uint32_t)nr_positions;
+    return (int64_t)(align256(n * sizeof(uint2)) + cursor_bytes(n) + counter_bytes(n));
+}
+
 int64_t permuto_order_bytes(int32_t pos_dim, int64_t nr_positions) {
     using namespace permuto;
-    if (pos_dim < 2 || pos_dim > 7 || nr_positions < 1 || nr_positions > (int64_t)0x7fffffff) return 0;
-    const uint32_t n = (uint32_t)nr_positions;
-    return (int64_t)(align256(n * record_bytes(pos_dim)) + align256(n * sizeof(uint2)) + cursor_bytes(n) + counter_bytes(n));
+    if (!order_sizes_ok(pos_dim, nr_positions)) return 0;
+    return (int64_t)align256((size_t)nr_positions * record_bytes(pos_dim)) + permuto_order_scratch_bytes(pos_dim, nr_positions);
 }
 
 // Where the order's own time comes back, measured on 16-24 levels (us without -> with order, the order
@@ -359,12 +372,22 @@ int permuto_order_pays(const permuto_config* cfg, int64_t nr_positions, int32_t 
 
 int permuto_order_points(const permuto_config* cfg, const permuto_inputs* in, void* order, int64_t order_bytes, void* stream) {
     using namespace permuto;
-    if (!cfg || !in || !in->positions || !order)
-        return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "cfg, in, positions and order must not be NULL");
+    if (!cfg || !in || !order) return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "cfg, in, positions and order must not be NULL");
     const int64_t need = permuto_order_bytes(cfg->pos_dim, in->nr_positions);
     if (need == 0) return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "order: pos_dim must be 2..7 and nr_positions in 1..2^31-1");
-    if (order_bytes < need || (reinterpret_cast<uintptr_t>(order) & 255u) != 0)
-        return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "order: needs %lld bytes on a 256-byte boundary", (long long)need);
+    if (order_bytes < need) return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "order: needs %lld bytes on a 256-byte boundary", (long long)need);
+    void* scratch = static_cast<char*>(order) + align256((size_t)in->nr_positions * record_bytes(cfg->pos_dim));
+    return permuto_order_records(cfg, in, order, scratch, stream);
+}
+
+int permuto_order_records(const permuto_config* cfg, const permuto_inputs* in, void* records, void* scratch, void* stream) {
+    using namespace permuto;
+    if (!cfg || !in || !in->positions || !records || !scratch)
+        return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "cfg, in, positions and order must not be NULL");
+    if (!order_sizes_ok(cfg->pos_dim, in->nr_positions))
+        return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "order: pos_dim must be 2..7 and nr_positions in 1..2^31-1");
+    if (((reinterpret_cast<uintptr_t>(records) | reinterpret_cast<uintptr_t>(scratch)) & 255u) != 0)
+        return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "order: records and scratch need a 256-byte boundary");
     OrderArgs a;
     a.positions = in->positions;
     a.stride_n = in->pos_stride_n;
@@ -375,9 +398,8 @@ int permuto_order_points(const permuto_config* cfg, const permuto_inputs* in, vo
     a.rounds = 1;
     while (a.rounds < 8 && a.n / kPerBlock / (2 * a.rounds) >= 1024) a.rounds *= 2;
     a.vec_ok = in->pos_stride_d == 1 && in->pos_stride_n == cfg->pos_dim && (reinterpret_cast<uintptr_t>(in->positions) & 15u) == 0;
-    char* at = static_cast<char*>(order);
-    a.records = reinterpret_cast<float4*>(at);
-    at += align256(a.n * record_bytes(cfg->pos_dim));
+    a.records = static_cast<float4*>(records);
+    char* at = static_cast<char*>(scratch);
     a.arrival = reinterpret_cast<uint2*>(at);
     at += align256(a.n * sizeof(uint2));
     a.cursors = reinterpret_cast<uint32_t*>(at);

@@ -37,8 +37,9 @@ using torch::autograd::variable_list;
 struct Api {
     decltype(&permuto_last_error) last_error;
     decltype(&permuto_order_pays) order_pays;
-    decltype(&permuto_order_bytes) order_bytes;
-    decltype(&permuto_order_points) order_points;
+    decltype(&permuto_order_record_bytes) order_record_bytes;
+    decltype(&permuto_order_scratch_bytes) order_scratch_bytes;
+    decltype(&permuto_order_records) order_records;
     decltype(&permuto_forward_ordered) forward;
     decltype(&permuto_forward_mlp_ordered) forward_mlp;
     decltype(&permuto_backward_ordered) backward;
@@ -57,8 +58,9 @@ void take(F& slot, const std::unordered_map<std::string, uintptr_t>& table, cons
 void bind_api(const std::unordered_map<std::string, uintptr_t>& t) {
     take(api.last_error, t, "permuto_last_error");
     take(api.order_pays, t, "permuto_order_pays");
-    take(api.order_bytes, t, "permuto_order_bytes");
-    take(api.order_points, t, "permuto_order_points");
+    take(api.order_record_bytes, t, "permuto_order_record_bytes");
+    take(api.order_scratch_bytes, t, "permuto_order_scratch_bytes");
+    take(api.order_records, t, "permuto_order_records");
     take(api.forward, t, "permuto_forward_ordered");
     take(api.forward_mlp, t, "permuto_forward_mlp_ordered");
     take(api.backward, t, "permuto_backward_ordered");
@@ -260,10 +262,11 @@ struct Bound {
     }
 };
 
+// The records alone: the scratch of the sort, a third of it all, goes back to the allocator right away.
 Tensor make_order(const Call& c, Bound& b) {
-    const int64_t bytes = api.order_bytes(b.cfg.pos_dim, b.in.nr_positions);
-    Tensor order = empty({bytes}, c.positions, at::kByte);
-    check(api.order_points(&b.cfg, &b.in, order.data_ptr(), bytes, stream_of(c.positions)));
+    Tensor order = empty({api.order_record_bytes(b.cfg.pos_dim, b.in.nr_positions)}, c.positions, at::kByte);
+    const Tensor scratch = empty({api.order_scratch_bytes(b.cfg.pos_dim, b.in.nr_positions)}, c.positions, at::kByte);
+    check(api.order_records(&b.cfg, &b.in, order.data_ptr(), scratch.data_ptr(), stream_of(c.positions)));
     return order;
 }
 

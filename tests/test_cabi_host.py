@@ -146,3 +146,22 @@ def test_header_is_plain_c_and_library_links_from_c(tmp_path, nat):
     want = nat.scale_factor([1.0, 0.5], 3)
     assert np.float32(a) == want[0, 0] and np.float32(b) == want[1, 2]
     assert "NULL" in res.stdout
+
+
+def test_order_sizes(nat):
+    """The records' size tells the number of points and pos_dim; the one-buffer form has room for both parts."""
+    lib, sizes = nat.lib, {}
+    for d in range(2, 8):
+        for n in (1, 2, 15, 16, 17, 4096, 2 ** 21, 2 ** 21 + 1, 2 ** 31 - 1):
+            rec, scratch = lib.permuto_order_record_bytes(d, n), lib.permuto_order_scratch_bytes(d, n)
+            assert sizes.setdefault(rec, (d, n)) == (d, n)
+            assert rec == n * (16 if d <= 3 else 32) + d and scratch >= 8 * n
+            assert lib.permuto_order_bytes(d, n) >= rec - d + scratch
+    for d, n in ((1, 5), (8, 5), (3, 0), (3, 2 ** 31)):
+        assert lib.permuto_order_record_bytes(d, n) == lib.permuto_order_scratch_bytes(d, n) == lib.permuto_order_bytes(d, n) == 0
+    cfg = nat.PermutoConfig(3, 2, 4, 1024, 0, 1.0, 0, 0)
+    ins = nat.PermutoInputs(10, 4096, 3, 1, 4096, 4096, 4096, 4096)
+    for records, scratch in ((None, 4096), (4096, None), (4097, 4096), (4096, 4100)):
+        assert lib.permuto_order_records(C.byref(cfg), C.byref(ins), records, scratch, None) == nat.PERMUTO_ERR_INVALID_ARGUMENT
+    for ins in (nat.PermutoInputs(0, 4096, 3, 1, 8, 8, 8, 8), nat.PermutoInputs(2 ** 31, 4096, 3, 1, 8, 8, 8, 8)):
+        assert lib.permuto_order_records(C.byref(cfg), C.byref(ins), 4096, 4096, None) == nat.PERMUTO_ERR_INVALID_ARGUMENT

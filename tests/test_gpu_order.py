@@ -133,3 +133,13 @@ def test_large_batches_sum_as_without_an_order(nat):
         assert torch.all(counts >= 1000)
         ratio = off(got, want) / off(plain(), want)
         assert torch.all(ratio <= 1.3), ratio
+
+
+@pytest.mark.parametrize("d,n", [(2, 2 ** 18 + 1), (7, 2 ** 20 - 3)])
+def test_order_keeps_its_records_only(nat, d, n):
+    """What an order holds on to is one record per point (the allocator rounds up to 512 bytes)."""
+    enc, inp, _, _ = _setup(nat, d, 2, 4, n, 3)
+    before = torch.cuda.memory_allocated()
+    order = enc.order(inp)
+    assert torch.cuda.memory_allocated() - before <= (16 if d <= 3 else 32) * n + 1024
+    assert order is not None
