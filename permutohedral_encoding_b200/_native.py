@@ -316,7 +316,9 @@ class EncodingWrapper:
     def order(self, inp: EncodingInput, purpose: int = ORDER_ALWAYS):
         """Spatial order of the positions (an opaque device buffer), or None where the batch is too
         small for it to pay for ``purpose``: attached to ``inp.m_order`` it makes the operations below
-        visit neighbouring points together.  Results do not depend on it."""
+        visit neighbouring points together.  Results do not depend on it.  It holds a copy of the
+        coordinates: an order of another number of points or pos_dim is refused, one made before the
+        positions were changed gives the results of the old ones."""
         return _ext.order(*self._args(inp), self.fixed.levels_per_pass, purpose)
 
     def forward(self, inp: EncodingInput) -> torch.Tensor:

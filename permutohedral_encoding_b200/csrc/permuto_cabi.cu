@@ -71,6 +71,7 @@ int build_problem(const permuto_config* cfg, const permuto_inputs* in, const voi
     if (cfg->table_dtype != PERMUTO_TABLE_F32 && cfg->table_dtype != PERMUTO_TABLE_F16)
         return set_error(PERMUTO_ERR_UNSUPPORTED, "table_dtype must be PERMUTO_TABLE_F32 or PERMUTO_TABLE_F16 (got %d)",
                          cfg->table_dtype);
+    if (!aligned(order, 256)) return set_error(PERMUTO_ERR_INVALID_ARGUMENT, "order must be 256-byte aligned");
     const int entry_bytes = (cfg->table_dtype == PERMUTO_TABLE_F16 ? 2 : 4) * F;
     if (!aligned(in->lattice_values, (size_t)entry_bytes))
         return set_error(PERMUTO_ERR_INVALID_ARGUMENT,

@@ -190,7 +190,8 @@ __device__ __forceinline__ void store8(float* dst, const float (&v)[8]) {
 }
 
 // Point number i of the sweep and the row it belongs to: i itself, or, when the batch has been put
-// into spatial order, the i-th record {coordinates, row} (16 bytes up to pos_dim 3, else 32).
+// into spatial order, the i-th record {coordinates, row} (16 bytes up to pos_dim 3, else 32).  The row is
+// an index into every row-shaped operand, so it is held inside the batch whatever the buffer contains.
 __device__ __forceinline__ int64_t load_point(const Problem& p, int64_t i, float (&pos)[D]) {
     if (p.order == nullptr) {
         load_pos(p, i, pos);
@@ -201,13 +202,13 @@ __device__ __forceinline__ int64_t load_point(const Problem& p, int64_t i, float
         pos[0] = t.x;
         pos[1] = t.y;
         if (D == 3) pos[D - 1] = t.z;
-        return (int64_t)__float_as_uint(t.w);
+        return (int64_t)min(__float_as_uint(t.w), (uint32_t)p.n_points - 1u);
     }
     float r[8];
     load8(reinterpret_cast<const float*>(p.order) + 8 * i, r);
 #pragma unroll
     for (int j = 0; j < D; ++j) pos[j] = r[j];
-    return (int64_t)__float_as_uint(r[7]);
+    return (int64_t)min(__float_as_uint(r[7]), (uint32_t)p.n_points - 1u);
 }
 
 // Aligned gather of one table entry (all F features) through the read-only path.  HALF: the

@@ -37,6 +37,7 @@ using torch::autograd::variable_list;
 struct Api {
     decltype(&permuto_last_error) last_error;
     decltype(&permuto_order_pays) order_pays;
+    decltype(&permuto_order_bytes) order_bytes;
     decltype(&permuto_order_record_bytes) order_record_bytes;
     decltype(&permuto_order_scratch_bytes) order_scratch_bytes;
     decltype(&permuto_order_records) order_records;
@@ -58,6 +59,7 @@ void take(F& slot, const std::unordered_map<std::string, uintptr_t>& table, cons
 void bind_api(const std::unordered_map<std::string, uintptr_t>& t) {
     take(api.last_error, t, "permuto_last_error");
     take(api.order_pays, t, "permuto_order_pays");
+    take(api.order_bytes, t, "permuto_order_bytes");
     take(api.order_record_bytes, t, "permuto_order_record_bytes");
     take(api.order_scratch_bytes, t, "permuto_order_scratch_bytes");
     take(api.order_records, t, "permuto_order_records");
@@ -233,6 +235,17 @@ void check_inputs(const Call& c) {
         fail("Random shift should be nr of resolutions x pos dim");
     if (c.window.dim() != 1 || c.window.size(0) != cfg.nr_levels)
         fail("anneal_window should have the first dimension the same as the nr of resolutions");
+    if (c.order.defined()) {
+        // one of EncodingWrapper.order, whose size tells pos_dim and the number of points, or a buffer of
+        // permuto_order_points
+        const Tensor& o = c.order;
+        const int64_t n = pos.size(0);
+        if (o.device() != pos.device() || o.scalar_type() != at::kByte || o.dim() != 1 || !o.is_contiguous() ||
+            (o.numel() != api.order_record_bytes(cfg.pos_dim, n) && o.numel() != api.order_bytes(cfg.pos_dim, n)) ||
+            reinterpret_cast<uintptr_t>(o.data_ptr()) % 256 != 0)
+            fail("the spatial order does not belong to " + std::to_string(n) + " positions of pos dim " +
+                 std::to_string(cfg.pos_dim) + " on their device");
+    }
 }
 
 // The C ABI's view of a checked call.

@@ -143,3 +143,44 @@ def test_order_keeps_its_records_only(nat, d, n):
     order = enc.order(inp)
     assert torch.cuda.memory_allocated() - before <= (16 if d <= 3 else 32) * n + 1024
     assert order is not None
+
+
+@pytest.mark.parametrize("d", [3, 6])
+def test_an_order_of_another_batch_is_refused(nat, d):
+    n = 5000
+    enc, inp, go, dpg = _setup(nat, d, 2, 4, n, 3)
+    good = enc.order(inp)
+    wide = torch.empty(2 * good.numel(), dtype=torch.uint8, device=DEV)
+    wrong = [enc.order(_setup(nat, d, 2, 4, m, 3)[1]) for m in (n - 1, n + 1, 2 * n, n // 2)]
+    wrong += [enc_.order(i) for enc_, i, _, _ in (_setup(nat, e, 2, 4, n, 3) for e in (2, 5))]
+    wrong += [good.cpu(), good.view(torch.int8), good.float(), wide[16:16 + good.numel()], wide[::2], good[:-1]]
+    weight = torch.randn(32, enc.output_width(), device=DEV)
+    for order in wrong:
+        inp.m_order = order
+        for call in (lambda: enc.forward(inp), lambda: enc.forward_linear(inp, weight), lambda: enc.backward(inp, go),
+                     lambda: enc.double_backward_from_positions(inp, dpg, go)):
+            with pytest.raises(RuntimeError, match="spatial order does not belong"):
+                call()
+    whole = torch.empty(nat.lib.permuto_order_bytes(d, n), dtype=torch.uint8, device=DEV)   # filled by permuto_order_points
+    whole[:good.numel()] = good
+    want = enc.forward(nat.EncodingInput(inp.m_lattice_values, inp.m_positions_raw, inp.m_anneal_window, True, True))
+    for order in (good, whole):
+        inp.m_order = order
+        assert torch.equal(enc.forward(inp), want)
+
+
+@pytest.mark.parametrize("d,feat", [(2, 2), (3, 4), (6, 2)])
+def test_rows_of_an_order_stay_inside_the_batch(nat, d, feat):
+    """Whatever the buffer holds, no operation writes past the batch's rows."""
+    n, room = 3001, 4096
+    enc, inp, go, _ = _setup(nat, d, feat, 5, n, 9)
+    gen = torch.Generator(device=DEV).manual_seed(4)
+    for fill in (torch.full_like(enc.order(inp), 255),
+                 torch.randint(0, 256, enc.order(inp).shape, device=DEV, generator=gen, dtype=torch.uint8)):
+        inp.m_order = fill
+        rows = torch.zeros((n + room, d), device=DEV)
+        enc.backward(inp, go, positions_grad_out=rows[:n])
+        torch.cuda.synchronize()
+        assert torch.count_nonzero(rows[n:]) == 0
+        assert enc.forward(inp).shape == (n, enc.output_width())
+        torch.cuda.synchronize()
