@@ -13,6 +13,7 @@
 // The C ABI is called through the pointers of the library the Python side has loaded.
 #include <torch/extension.h>
 
+#include <ATen/SavedTensorHooks.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -140,12 +141,21 @@ struct Lattice : torch::CustomClassHolder {
     std::unordered_map<int, Tensor> scale_;
 };
 
-// One call's inputs, checked; holds what the pointers of `in` refer to.
-struct Call : torch::CustomClassHolder {
+// One call's inputs.
+struct Inputs {
     c10::intrusive_ptr<Lattice> lattice;
     Tensor values, positions, window, shift, half, order;
     int levels_per_pass = 0;
+};
+
+// What the nodes of one call share.  The tensors of the graph are not here: nodes keep them with
+// save_for_backward, so that the engine frees them with the graph and saved-tensor hooks see them.
+struct Call : torch::CustomClassHolder {
+    c10::intrusive_ptr<Lattice> lattice;
+    Tensor shift, half;
+    int levels_per_pass = 0;
     bool need_values = false, need_positions = false;
+    bool ordered = false;  // the forward ran in spatial order
 
     // A loss that reaches both the features and the position gradient gives the lattice values two
     // gradients in one backward, from the first-order node and from a second-order one (EncodeBackward).
@@ -210,7 +220,7 @@ struct Call : torch::CustomClassHolder {
 };
 
 // Same checks and messages as the reference (src/Encoding.cu:37-45, :63-66, :119-125).
-void check_inputs(const Call& c) {
+void check_inputs(const Inputs& c) {
     const permuto_config& cfg = c.lattice->cfg;
     const Tensor& pos = c.positions;
     if (!pos.is_cuda()) fail("positions should be in GPU memory. Please call .cuda() on the tensor");
@@ -255,7 +265,7 @@ struct Bound {
     c10::cuda::OptionalCUDAGuard guard;
     Tensor scale, shift, window;
 
-    explicit Bound(const Call& c) : cfg(c.lattice->cfg) {
+    explicit Bound(const Inputs& c) : cfg(c.lattice->cfg) {
         const c10::Device device = c.positions.device();
         if (device.index() != c10::cuda::current_device()) guard.set_device(device);
         scale = c.lattice->scale_on(device);
@@ -276,20 +286,22 @@ struct Bound {
 };
 
 // The records alone: the scratch of the sort, a third of it all, goes back to the allocator right away.
-Tensor make_order(const Call& c, Bound& b) {
+Tensor make_order(const Inputs& c, Bound& b) {
     Tensor order = empty({api.order_record_bytes(b.cfg.pos_dim, b.in.nr_positions)}, c.positions, at::kByte);
     const Tensor scratch = empty({api.order_scratch_bytes(b.cfg.pos_dim, b.in.nr_positions)}, c.positions, at::kByte);
     check(api.order_records(&b.cfg, &b.in, order.data_ptr(), scratch.data_ptr(), stream_of(c.positions)));
     return order;
 }
 
+// What a call is ordered for: an order is made where order_pays says so.
+enum Purpose { kAsGiven = -1, kInference = 0, kTraining = 1 };
+
 // features [N, W]; where the batch is large enough to be worth it the points are put into spatial order
-// first, and the order stays with the call for its backward passes
-Tensor run_forward(Call& c, bool may_order) {
+// first, and the order is left in `c` for the backward passes
+Tensor run_forward(Inputs& c, Purpose purpose) {
     check_inputs(c);
     Bound b(c);
-    if (may_order && !c.order.defined() && api.order_pays(&b.cfg, b.in.nr_positions, c.need_values || c.need_positions ? 1 : 0))
-        c.order = make_order(c, b);
+    if (purpose != kAsGiven && !c.order.defined() && api.order_pays(&b.cfg, b.in.nr_positions, purpose)) c.order = make_order(c, b);
     Tensor out = empty({b.in.nr_positions, c.lattice->width}, c.positions);
     check(api.forward(&b.cfg, &b.in, data(c.order), out.data_ptr<float>(), stream_of(c.positions)));
     return out;
@@ -303,13 +315,13 @@ Tensor run_forward(Call& c, bool may_order) {
 // measured size: whether a batch is ordered does not show in its gradient.  Spatial order is closer to a
 // float64 sum of the same addends (1.3-3.4e-6 against 2-6.5e-6 at 2^22).
 constexpr int64_t kOrderedSums = 1 << 22;
-bool ordered_sums(const Call& c) { return c.order.defined() && c.positions.size(0) <= kOrderedSums; }
+bool ordered_sums(const Inputs& c) { return c.order.defined() && c.positions.size(0) <= kOrderedSums; }
 
 struct Gradients {
     Tensor values, positions;
 };
 
-Gradients run_backward(const Call& c, const Tensor& grad, bool need_values, bool need_positions, const Tensor& values_out,
+Gradients run_backward(const Inputs& c, const Tensor& grad, bool need_values, bool need_positions, const Tensor& values_out,
                        int level_begin, int level_end, bool zero, const Tensor& positions_out) {
     check_inputs(c);
     const int64_t n = c.positions.size(0);
@@ -352,7 +364,7 @@ struct SecondOrder {
     Tensor values, features;
 };
 
-SecondOrder run_double_backward(const Call& c, const Tensor& double_positions_grad, const Tensor& grad, bool need_values,
+SecondOrder run_double_backward(const Inputs& c, const Tensor& double_positions_grad, const Tensor& grad, bool need_values,
                                 bool need_features) {
     check_inputs(c);
     const int64_t n = c.positions.size(0);
@@ -383,7 +395,7 @@ SecondOrder run_double_backward(const Call& c, const Tensor& double_positions_gr
 }
 
 // table gradient of both orders in one buffer
-Tensor run_combined(const Call& c, const Tensor& grad, const Call::Part& second) {
+Tensor run_combined(const Inputs& c, const Tensor& grad, const Call::Part& second) {
     Bound b(c);
     const Tensor dpg = second.double_positions_grad.contiguous();
     Tensor values = empty(c.values.sizes(), c.positions);
@@ -396,7 +408,7 @@ Tensor run_combined(const Call& c, const Tensor& grad, const Call::Part& second)
 py::object as_python(const Tensor& t) { return t.defined() ? py::cast(t) : py::none(); }
 Tensor from_python(const py::handle& h) { return h.is_none() ? Tensor() : py::cast<Tensor>(h); }
 
-Gradients backward_or_hook(const Call& c, const Tensor& grad, bool need_values, bool need_positions) {
+Gradients backward_or_hook(const Inputs& c, const Tensor& grad, bool need_values, bool need_positions) {
     if (need_values && c.lattice->on_backward) {
         py::gil_scoped_acquire gil;
         const py::tuple r = c.lattice->on_backward(c.values, c.positions, c.window, as_python(c.half), as_python(c.order), grad,
@@ -408,18 +420,35 @@ Gradients backward_or_hook(const Call& c, const Tensor& grad, bool need_values, 
 
 // parts of one backward may be merged: no second differentiation, no data-parallel hooks, and not where each
 // part is summed in the sequence of the batch (the two sums stay separate there, as without an order)
-bool may_merge(const Call& c) {
+bool may_merge(const Inputs& c) {
     return !at::GradMode::is_enabled() && !c.lattice->on_backward && !c.lattice->on_double_backward &&
            c.positions.size(0) <= kOrderedSums;
+}
+
+// The order goes with the saved tensors, unless hooks look at those: they get what a node without an order
+// saves, and the backward makes the order again from the positions that they hand back.
+Tensor order_to_save(const Inputs& in) { return at::SavedTensorDefaultHooks::get_tls_state().stack.empty() ? in.order : Tensor(); }
+
+// a node's inputs out of its saved tensors, which start at `first`: values, positions, window, order
+Inputs saved_inputs(const Call& call, const variable_list& saved, size_t first) {
+    Inputs in{call.lattice, saved[first], saved[first + 1], saved[first + 2], call.shift, call.half, saved[first + 3],
+              call.levels_per_pass};
+    if (call.ordered && !in.order.defined()) {
+        check_inputs(in);
+        Bound b(in);
+        in.order = make_order(in, b);
+    }
+    return in;
 }
 
 // The first-order backward as a differentiable function of (upstream gradient, lattice values); its own
 // backward is the double backward from the position gradient.
 struct EncodeBackward : torch::autograd::Function<EncodeBackward> {
     static variable_list forward(AutogradContext* ctx, const Tensor& grad, const Tensor& values, const Tensor& positions,
-                                 const c10::intrusive_ptr<Call>& call, bool need_values, bool need_positions, int64_t number) {
-        const Gradients g = backward_or_hook(*call, grad, need_values, need_positions);
-        ctx->save_for_backward({grad, values, positions, call->window});
+                                 const Inputs& in, const c10::intrusive_ptr<Call>& call, bool need_values, bool need_positions,
+                                 int64_t number) {
+        const Gradients g = backward_or_hook(in, grad, need_values, need_positions);
+        ctx->save_for_backward({grad, values, positions, in.window, order_to_save(in)});
         ctx->saved_data["call"] = c10::IValue::make_capsule(call);
         ctx->saved_data["number"] = number;
         ctx->saved_data["position_output"] = need_positions ? (need_values ? 1 : 0) : -1;
@@ -431,7 +460,7 @@ struct EncodeBackward : torch::autograd::Function<EncodeBackward> {
     }
 
     static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
-        variable_list out(7);
+        variable_list out(8);
         const variable_list saved = ctx->get_saved_variables();  // checks the version counters
         const auto call = c10::static_intrusive_pointer_cast<Call>(ctx->saved_data["call"].toCapsule());
         const int number = (int)ctx->saved_data["number"].toInt();
@@ -441,14 +470,16 @@ struct EncodeBackward : torch::autograd::Function<EncodeBackward> {
         // second-order term through the lattice-value gradient is not propagated.
         const int64_t at = ctx->saved_data["position_output"].toInt();
         const bool second = at >= 0 && grads[at].defined();
+        if (!first && !(second && (need_features || need_values))) return out;
+        const Inputs in = saved_inputs(*call, saved, 1);
         if (first) {
-            out[1] = second ? run_combined(*call, first->grad, {grads[at], saved[0]})
-                            : run_backward(*call, first->grad, true, false, {}, 0, -1, true, {}).values;
+            out[1] = second ? run_combined(in, first->grad, {grads[at], saved[0]})
+                            : run_backward(in, first->grad, true, false, {}, 0, -1, true, {}).values;
         }
         if (!second) return out;
-        const bool own_values = need_values && !first && !(may_merge(*call) && call->leave(number, {grads[at], saved[0]}));
+        const bool own_values = need_values && !first && !(may_merge(in) && call->leave(number, {grads[at], saved[0]}));
         if (!need_features && !own_values) return out;
-        SecondOrder s = run_double_backward(*call, grads[at], saved[0], own_values, need_features);
+        SecondOrder s = run_double_backward(in, grads[at], saved[0], own_values, need_features);
         // data-parallel use: this second-order lattice gradient is summed over the ranks like the
         // first-order one, otherwise the replicated tables drift apart
         if (s.values.defined() && call->lattice->on_double_backward) {
@@ -462,10 +493,11 @@ struct EncodeBackward : torch::autograd::Function<EncodeBackward> {
 };
 
 struct Encode : torch::autograd::Function<Encode> {
-    static Tensor forward(AutogradContext* ctx, const Tensor& values, const Tensor& positions,
+    static Tensor forward(AutogradContext* ctx, const Tensor& values, const Tensor& positions, Inputs& in,
                           const c10::intrusive_ptr<Call>& call) {
-        const Tensor out = run_forward(*call, true);
-        ctx->save_for_backward({values, positions, call->window});
+        const Tensor out = run_forward(in, kTraining);
+        call->ordered = in.order.defined();
+        ctx->save_for_backward({values, positions, in.window, order_to_save(in)});
         ctx->saved_data["call"] = c10::IValue::make_capsule(call);
         return out;
     }
@@ -475,22 +507,23 @@ struct Encode : torch::autograd::Function<Encode> {
         const auto call = c10::static_intrusive_pointer_cast<Call>(ctx->saved_data["call"].toCapsule());
         const bool need_values = call->need_values && ctx->needs_input_grad(0);
         const bool need_positions = call->need_positions && ctx->needs_input_grad(1);
-        variable_list out(3);
+        variable_list out(4);
         if (!need_values && !need_positions) return out;
         const Tensor grad = grads[0].contiguous();
+        const Inputs in = saved_inputs(*call, saved, 0);
         if (at::GradMode::is_enabled()) {
             const int number = call->reserve_node();
-            const variable_list g = EncodeBackward::apply(grad, saved[0], saved[1], call, need_values, need_positions, number);
+            const variable_list g = EncodeBackward::apply(grad, saved[0], saved[1], in, call, need_values, need_positions, number);
             call->set_node(number, g[0].grad_fn());
             if (need_values) out[0] = g[0];
             if (need_positions) out[1] = g[need_values ? 1 : 0];
             return out;
         }
         const auto second = call->collect(Call::kFirst);
-        if (second) out[0] = run_combined(*call, grad, *second);
-        const bool own_values = need_values && !second && !(may_merge(*call) && call->leave(Call::kFirst, {{}, grad}));
+        if (second) out[0] = run_combined(in, grad, *second);
+        const bool own_values = need_values && !second && !(may_merge(in) && call->leave(Call::kFirst, {{}, grad}));
         if (own_values || need_positions) {
-            const Gradients g = backward_or_hook(*call, grad, own_values, need_positions);
+            const Gradients g = backward_or_hook(in, grad, own_values, need_positions);
             if (own_values) out[0] = g.values;
             out[1] = g.positions;
         }
@@ -498,32 +531,28 @@ struct Encode : torch::autograd::Function<Encode> {
     }
 };
 
-c10::intrusive_ptr<Call> make_call(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, const Tensor& positions,
-                                   const Tensor& window, const Tensor& shift, const std::optional<Tensor>& half,
-                                   const std::optional<Tensor>& order, int levels_per_pass) {
-    auto c = c10::make_intrusive<Call>();
-    c->lattice = lattice;
-    c->values = values;
-    c->positions = positions;
-    c->window = window;
-    c->shift = shift;
-    if (half) c->half = *half;
-    if (order) c->order = *order;
-    c->levels_per_pass = levels_per_pass;
-    return c;
+Inputs make_inputs(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, const Tensor& positions, const Tensor& window,
+                   const Tensor& shift, const std::optional<Tensor>& half, const std::optional<Tensor>& order,
+                   int levels_per_pass) {
+    return {lattice, values, positions, window, shift, half ? *half : Tensor(), order ? *order : Tensor(), levels_per_pass};
 }
 
 // the module's forward: with a graph where one is wanted
 Tensor encode(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, const Tensor& positions, const Tensor& window,
               const Tensor& shift, const std::optional<Tensor>& half, int levels_per_pass) {
-    auto c = make_call(lattice, values, positions, window, shift, half, std::nullopt, levels_per_pass);
-    if (at::GradMode::is_enabled()) {
-        c->need_values = values.requires_grad();
-        c->need_positions = positions.requires_grad();
-    }
-    if (!c->need_values && !c->need_positions) return run_forward(*c, true);
-    Tensor out = Encode::apply(values, positions, c);
-    c->set_node(Call::kFirst, out.grad_fn());
+    Inputs in = make_inputs(lattice, values, positions, window, shift, half, std::nullopt, levels_per_pass);
+    const bool graph = at::GradMode::is_enabled();
+    const bool need_values = graph && values.requires_grad(), need_positions = graph && positions.requires_grad();
+    if (!need_values && !need_positions) return run_forward(in, kInference);
+    auto call = c10::make_intrusive<Call>();
+    call->lattice = lattice;
+    call->shift = in.shift;
+    call->half = in.half;
+    call->levels_per_pass = levels_per_pass;
+    call->need_values = need_values;
+    call->need_positions = need_positions;
+    Tensor out = Encode::apply(values, positions, in, call);
+    call->set_node(Call::kFirst, out.grad_fn());
     return out;
 }
 
@@ -531,8 +560,8 @@ Tensor forward_mlp(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& val
                    const Tensor& window, const Tensor& shift, const std::optional<Tensor>& half,
                    const std::optional<Tensor>& order, int levels_per_pass, const std::vector<Tensor>& weights,
                    const std::vector<std::optional<Tensor>>& biases, int activation, const std::optional<Tensor>& status) {
-    auto c = make_call(lattice, values, positions, window, shift, half, order, levels_per_pass);
-    check_inputs(*c);
+    Inputs c = make_inputs(lattice, values, positions, window, shift, half, order, levels_per_pass);
+    check_inputs(c);
     const c10::Device device = positions.device();
     if (weights.empty() || weights.size() > 6)
         fail("the fused network takes 1..6 layers, got " + std::to_string(weights.size()));
@@ -558,12 +587,12 @@ Tensor forward_mlp(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& val
     }
     if (status && (status->scalar_type() != at::kInt || status->device() != device || status->numel() != 1))
         fail("status should be a one-element int32 tensor on the device of the positions");
-    Bound b(*c);
+    Bound b(c);
     // One layer behind the encoding gains 18 % from an order on 2^20 independent points (349 -> 285 us); with
     // a whole network behind it the gathers are less of the time, and the gain (4 %) is what ray samples lose.
-    if (!c->order.defined() && layers.size() == 1 && api.order_pays(&b.cfg, b.in.nr_positions, 0)) c->order = make_order(*c, b);
+    if (!c.order.defined() && layers.size() == 1 && api.order_pays(&b.cfg, b.in.nr_positions, kInference)) c.order = make_order(c, b);
     Tensor out = empty({b.in.nr_positions, width}, positions);
-    check(api.forward_mlp(&b.cfg, &b.in, data(c->order), layers.data(), (int32_t)layers.size(), activation,
+    check(api.forward_mlp(&b.cfg, &b.in, data(c.order), layers.data(), (int32_t)layers.size(), activation,
                           out.data_ptr<float>(), status ? status->data_ptr<int32_t>() : nullptr, stream_of(positions)));
     return out;
 }
@@ -603,35 +632,35 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("encode", &encode);
     m.def("forward", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w, const Tensor& s,
                         const std::optional<Tensor>& half, const std::optional<Tensor>& order, int lpp) {
-        auto c = make_call(l, v, p, w, s, half, order, lpp);
-        return run_forward(*c, false);
+        Inputs c = make_inputs(l, v, p, w, s, half, order, lpp);
+        return run_forward(c, kAsGiven);
     });
     m.def("check_inputs", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w,
                              const Tensor& s, const std::optional<Tensor>& half) {
-        check_inputs(*make_call(l, v, p, w, s, half, std::nullopt, 0));
+        check_inputs(make_inputs(l, v, p, w, s, half, std::nullopt, 0));
     });
     m.def("order", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w, const Tensor& s,
                       const std::optional<Tensor>& half, int lpp, int purpose) -> std::optional<Tensor> {
-        auto c = make_call(l, v, p, w, s, half, std::nullopt, lpp);
-        check_inputs(*c);
-        Bound b(*c);
+        Inputs c = make_inputs(l, v, p, w, s, half, std::nullopt, lpp);
+        check_inputs(c);
+        Bound b(c);
         if (purpose >= 0 && !api.order_pays(&b.cfg, b.in.nr_positions, purpose)) return std::nullopt;
-        return make_order(*c, b);
+        return make_order(c, b);
     });
     m.def("backward", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w, const Tensor& s,
                          const std::optional<Tensor>& half, const std::optional<Tensor>& order, int lpp, const Tensor& grad,
                          bool need_values, bool need_positions, const std::optional<Tensor>& values_out, int level_begin,
                          int level_end, bool zero, const std::optional<Tensor>& positions_out) {
-        auto c = make_call(l, v, p, w, s, half, order, lpp);
-        const Gradients g = run_backward(*c, grad, need_values, need_positions, values_out ? *values_out : Tensor(), level_begin,
+        Inputs c = make_inputs(l, v, p, w, s, half, order, lpp);
+        const Gradients g = run_backward(c, grad, need_values, need_positions, values_out ? *values_out : Tensor(), level_begin,
                                          level_end, zero, positions_out ? *positions_out : Tensor());
         return py::make_tuple(as_python(g.values), as_python(g.positions));
     });
     m.def("double_backward", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w,
                                 const Tensor& s, const std::optional<Tensor>& half, const std::optional<Tensor>& order, int lpp,
                                 const Tensor& dpg, const Tensor& grad, bool need_values, bool need_features) {
-        auto c = make_call(l, v, p, w, s, half, order, lpp);
-        const SecondOrder r = run_double_backward(*c, dpg, grad, need_values, need_features);
+        Inputs c = make_inputs(l, v, p, w, s, half, order, lpp);
+        const SecondOrder r = run_double_backward(c, dpg, grad, need_values, need_features);
         return py::make_tuple(as_python(r.values), as_python(r.features));
     });
     m.def("forward_mlp", &forward_mlp);

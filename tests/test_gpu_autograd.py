@@ -131,3 +131,84 @@ def test_both_orders_in_one_backward(d, feat, levels, n):
     (normal * dpg).sum().backward()
     out2, _ = graph()
     check(m.lattice_values.grad + torch.autograd.grad(out2, m.lattice_values, go)[0], up.grad)
+
+
+def _large(n=2 ** 18 + 5, levels=16):
+    from permutohedral_encoding_b200 import PermutoEncoding
+    torch.manual_seed(3)
+    m = PermutoEncoding(3, 2 ** 10, levels, 2, np.geomspace(1.0, 1e-2, levels))
+    with torch.no_grad():
+        m.lattice_values.uniform_(-1, 1)
+    return m, torch.rand(n, 3, device=DEV, requires_grad=True), torch.randn(n, 2 * levels, device=DEV)
+
+
+def test_a_backward_frees_what_the_graph_kept():
+    """The engine frees the saved tensors, the spatial order among them, with a backward that does not keep
+    the graph, even while its output lives; the pose case runs both nodes of a create_graph backward."""
+    m, pos, go = _large()
+    out = m(pos)
+    held = torch.cuda.memory_allocated()
+    out.backward(go, inputs=[m.lattice_values])
+    m.lattice_values.grad = None
+    assert held - torch.cuda.memory_allocated() >= 16 * pos.shape[0]
+    with pytest.raises(RuntimeError, match="second time"):
+        out.backward(go)
+    before = torch.cuda.memory_allocated()
+    out2 = m(pos)
+    (normal,) = torch.autograd.grad(out2, pos, go, create_graph=True)
+    torch.autograd.backward([out2, normal], [go, torch.ones_like(normal)], inputs=[m.lattice_values])
+    kept = sum(t.numel() * 4 for t in (out2, normal, m.lattice_values.grad))
+    assert torch.cuda.memory_allocated() - before <= kept + 4096
+
+
+@pytest.mark.parametrize("large", [False, True])
+def test_saved_tensor_hooks_see_and_replace_what_a_node_keeps(setup, large):
+    m, pos, go = _large() if large else setup
+    window = torch.rand(m.nr_levels, device=DEV)
+
+    def grads(out):
+        return torch.autograd.grad(out, [m.lattice_values, pos], go)
+
+    want_v, want_p = grads(m(pos, window))
+    seen = []
+
+    def keep(t):
+        seen.append(t)
+        return t
+
+    def same(ts):
+        return sorted((tuple(t.shape), t.dtype) for t in ts)
+
+    with torch.autograd.graph.saved_tensors_hooks(keep, lambda t: t):
+        out = m(pos, window)
+    assert same(seen) == same([m.lattice_values, pos, window])
+    got_v, got_p = grads(out)
+    _close(got_v, want_v)
+    _close(got_p, want_p)
+    # the table gradient is linear in the window, the position gradient in window and values
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t * 2 if t.shape != pos.shape else t):
+        out = m(pos, window)
+    got_v, got_p = grads(out)
+    _close(got_v, 2 * want_v)
+    _close(got_p, 4 * want_p)
+    # moved points, first order and second order
+    where = (pos.detach() + 0.25).requires_grad_(True)
+    (want_n,) = torch.autograd.grad(m(where, window), where, go, create_graph=True)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t + 0.25 if t.shape == pos.shape else t):
+        (normal,) = torch.autograd.grad(m(pos, window), pos, go, create_graph=False)
+        _close(normal, want_n.detach())
+    with torch.autograd.graph.save_on_cpu():
+        (normal,) = torch.autograd.grad(m(where, window), where, go.requires_grad_(True), create_graph=True)
+        got = torch.autograd.grad(normal.sum(), [m.lattice_values, go])
+    want = torch.autograd.grad(torch.autograd.grad(m(where, window), where, go, create_graph=True)[0].sum(), [m.lattice_values, go])
+    for a, b in zip(got, want):
+        _close(a, b)
+
+
+def test_checkpointed_batches_match():
+    from torch.utils.checkpoint import checkpoint
+    m, pos, go = _large()
+    want = torch.autograd.grad(m(pos), [m.lattice_values, pos], go)
+    got = torch.autograd.grad(checkpoint(m, pos, use_reentrant=False), [m.lattice_values, pos], go)
+    for a, b in zip(got, want):
+        _close(a, b)
