@@ -296,13 +296,23 @@ Tensor make_order(const Inputs& c, Bound& b) {
 // What a call is ordered for: an order is made where order_pays says so.
 enum Purpose { kAsGiven = -1, kInference = 0, kTraining = 1 };
 
+// An order that a call can do without: where there is no room for its 24 to 44 bytes a point the call runs
+// as it would without one (callers allocate their outputs first).
+void try_order(Inputs& c, Bound& b, Purpose purpose) {
+    if (c.order.defined() || !api.order_pays(&b.cfg, b.in.nr_positions, purpose)) return;
+    try {
+        c.order = make_order(c, b);
+    } catch (const c10::OutOfMemoryError&) {
+    }
+}
+
 // features [N, W]; where the batch is large enough to be worth it the points are put into spatial order
 // first, and the order is left in `c` for the backward passes
 Tensor run_forward(Inputs& c, Purpose purpose) {
     check_inputs(c);
     Bound b(c);
-    if (purpose != kAsGiven && !c.order.defined() && api.order_pays(&b.cfg, b.in.nr_positions, purpose)) c.order = make_order(c, b);
     Tensor out = empty({b.in.nr_positions, c.lattice->width}, c.positions);
+    if (purpose != kAsGiven) try_order(c, b, purpose);
     check(api.forward(&b.cfg, &b.in, data(c.order), out.data_ptr<float>(), stream_of(c.positions)));
     return out;
 }
@@ -436,7 +446,7 @@ Inputs saved_inputs(const Call& call, const variable_list& saved, size_t first) 
     if (call.ordered && !in.order.defined()) {
         check_inputs(in);
         Bound b(in);
-        in.order = make_order(in, b);
+        try_order(in, b, kTraining);
     }
     return in;
 }
@@ -590,8 +600,8 @@ Tensor forward_mlp(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& val
     Bound b(c);
     // One layer behind the encoding gains 18 % from an order on 2^20 independent points (349 -> 285 us); with
     // a whole network behind it the gathers are less of the time, and the gain (4 %) is what ray samples lose.
-    if (!c.order.defined() && layers.size() == 1 && api.order_pays(&b.cfg, b.in.nr_positions, kInference)) c.order = make_order(c, b);
     Tensor out = empty({b.in.nr_positions, width}, positions);
+    if (layers.size() == 1) try_order(c, b, kInference);
     check(api.forward_mlp(&b.cfg, &b.in, data(c.order), layers.data(), (int32_t)layers.size(), activation,
                           out.data_ptr<float>(), status ? status->data_ptr<int32_t>() : nullptr, stream_of(positions)));
     return out;

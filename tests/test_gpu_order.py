@@ -184,3 +184,39 @@ def test_rows_of_an_order_stay_inside_the_batch(nat, d, feat):
         assert torch.count_nonzero(rows[n:]) == 0
         assert enc.forward(inp).shape == (n, enc.output_width())
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("n,d,levels", [(2 ** 21 + 1, 7, 1), (2 ** 18 + 1, 3, 8)])
+def test_a_call_without_room_for_an_order_runs_without_one(nat, n, d, levels):
+    """The order is an aid: a batch whose outputs fit runs whether or not the order fits beside them (rows of 8
+    and records of 32 bytes: the order alone does not fit; 64 and 16: it fits, but not beside the rows)."""
+    from permutohedral_encoding_b200 import PermutoEncoding
+    m = PermutoEncoding(d, 2 ** 10, levels, 2, np.ones(levels))
+    pos = torch.rand(n, d, device=DEV)
+    go = torch.randn(n, 2 * levels, device=DEV)
+    inp = nat.EncodingInput(m.lattice_values.detach(), pos, m.anneal_window, True, False)
+    want, want_grad = m.lattice.forward(inp), m.lattice.backward(inp, go)[0]
+    assert m.lattice.order(inp, nat.ORDER_TRAINING) is not None
+    total = torch.cuda.get_device_properties(0).total_memory
+    room, held = torch.empty(20 * 2 ** 20, dtype=torch.uint8, device=DEV), []   # the rows take 16 MB
+
+    def limit(extra):
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + extra) / total)
+
+    try:
+        limit(0)
+        with pytest.raises(torch.cuda.OutOfMemoryError):   # nothing free but `room` and 8 MB
+            while True:
+                held.append(torch.empty(4 * 2 ** 20, dtype=torch.uint8, device=DEV))
+        limit(8 * 2 ** 20)
+        del room
+        if d == 7:
+            with pytest.raises(torch.cuda.OutOfMemoryError):
+                m.lattice.order(inp)
+        out = m(pos)
+        out.backward(go)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        held.clear()
+    assert torch.equal(out, want)
+    assert torch.all((m.lattice_values.grad - want_grad).abs() <= 1e-4 * want_grad.abs().amax())
