@@ -188,8 +188,14 @@ int permuto_double_backward(const permuto_config *cfg, const permuto_inputs *in,
  * permuto_order_records does the same with two buffers, each 256-byte aligned: the order itself, of
  * permuto_order_record_bytes(pos_dim, N) bytes (one record per point, and pos_dim bytes more, so that the
  * size tells pos_dim and N), and scratch of permuto_order_scratch_bytes(pos_dim, N) bytes that is free again
- * once the sort has run on `stream`.  All sizes are 0 for a pos_dim or N out of range. */
-int permuto_order_pays(const permuto_config *cfg, int64_t nr_positions, int32_t with_gradients); /* 1: worth it */
+ * once the sort has run on `stream`.  All sizes are 0 for a pos_dim or N out of range.
+ * permuto_order_pays is 1 where a sort comes back in what follows it (purpose), with every level open. */
+enum {
+    PERMUTO_ORDER_FEATURES = 0,   /* forward only                                          */
+    PERMUTO_ORDER_TABLE_GRAD = 1, /* forward, and a gradient of the table                  */
+    PERMUTO_ORDER_POS_GRAD = 2    /* forward, and a gradient of the positions or of both   */
+};
+int permuto_order_pays(const permuto_config *cfg, int64_t nr_positions, int32_t purpose);
 int64_t permuto_order_bytes(int32_t pos_dim, int64_t nr_positions);
 int permuto_order_points(const permuto_config *cfg, const permuto_inputs *in, void *order, int64_t order_bytes,
                          void *stream);

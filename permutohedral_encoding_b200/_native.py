@@ -40,7 +40,7 @@ PERMUTO_ZERO_OUTPUTS = 1
 PERMUTO_NO_AGGREGATE = 2
 PERMUTO_KEEP_POSITIONS_GRAD = 4
 PERMUTO_CONCAT_POSITIONS_GRAD = 8
-ORDER_ALWAYS, ORDER_INFERENCE, ORDER_TRAINING = -1, 0, 1   # when EncodingWrapper.order makes an order
+ORDER_ALWAYS, ORDER_INFERENCE, ORDER_TRAINING, ORDER_POSITIONS = -1, 0, 1, 2   # when EncodingWrapper.order makes an order
 PERMUTO_ACT = {"none": 0, "relu": 1, "gelu": 2}
 PERMUTO_ADAM_SKIP_UNTOUCHED = 1
 PERMUTO_ADAM_ZERO_GRAD = 2
@@ -197,6 +197,7 @@ class EncodingInput:
         self.m_require_lattice_values_grad = bool(require_lattice_values_grad)
         self.m_require_positions_grad = bool(require_positions_grad)
         self.m_order = None   # spatial order of these positions (EncodingWrapper.order), or None
+        self.m_all_open = True   # no level is closed by the window (decides about ordering, never about results)
 
 
 class EncodingFixedParams:
@@ -314,8 +315,8 @@ class EncodingWrapper:
         return self._width
 
     def order(self, inp: EncodingInput, purpose: int = ORDER_ALWAYS):
-        """Spatial order of the positions (an opaque device buffer), or None where the batch is too
-        small for it to pay for ``purpose``: attached to ``inp.m_order`` it makes the operations below
+        """Spatial order of the positions (an opaque device buffer), or None where the batch or the number
+        of levels is too small for it to pay for ``purpose``: attached to ``inp.m_order`` it makes the operations below
         visit neighbouring points together.  Results do not depend on it.  It holds a copy of the
         coordinates: an order of another number of points or pos_dim is refused, one made before the
         positions were changed gives the results of the old ones."""
@@ -344,8 +345,8 @@ class EncodingWrapper:
         (examples/train_toy_example.py:18-26) is the model case."""
         if activation not in PERMUTO_ACT:
             raise RuntimeError(f"activation must be one of {sorted(PERMUTO_ACT)}, got {activation!r}")
-        return _ext.forward_mlp(*self._args(inp), inp.m_order, self.fixed.levels_per_pass, [w for w, _ in layers],
-                                [b for _, b in layers], PERMUTO_ACT[activation], status)
+        return _ext.forward_mlp(*self._args(inp), inp.m_order, self.fixed.levels_per_pass, inp.m_all_open,
+                                [w for w, _ in layers], [b for _, b in layers], PERMUTO_ACT[activation], status)
 
     def backward(self, inp: EncodingInput, grad_features: torch.Tensor, lattice_grad_out=None,
                  level_begin=None, level_end=None, zero=True, positions_grad_out=None):

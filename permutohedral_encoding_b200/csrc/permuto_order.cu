@@ -357,17 +357,41 @@ int64_t permuto_order_bytes(int32_t pos_dim, int64_t nr_positions) {
     return (int64_t)align256((size_t)nr_positions * record_bytes(pos_dim)) + permuto_order_scratch_bytes(pos_dim, nr_positions);
 }
 
-// Where the order's own time comes back, measured on 16-24 levels (us without -> with order, the order
-// itself included).  Training, 2 features: pos_dim 3, 2^17 points 125 -> 115 but ray
-// samples 85 -> 99, 2^18 216 -> 170 (rays 170 -> 167), 2^20 745 -> 533; pos_dim 6, 2^17 140 -> 147, 2^18 243 -> 234.  Wider entries have fewer levels to gain on and
-// ray samples of 3*10^5 points lose (119 -> 131), 2^20 points 431 -> 381.  Inference, 2 features:
-// 2^18 points 82 -> 78 but ray samples 64 -> 74, 2^19 149 -> 133, 2^20 288 -> 235; pos_dim 6, 2^20
-// 347 -> 340; 4 features, 2^20 174 -> 178; 8 levels, 2^18 21 -> 32.
-int permuto_order_pays(const permuto_config* cfg, int64_t nr_positions, int32_t with_gradients) {
-    if (!cfg) return 0;
-    const bool pairs = cfg->nr_feat_per_level == 2;
-    if (with_gradients) return nr_positions >= (pairs ? 1 << 18 : 1 << 19) ? 1 : 0;
-    return pairs && cfg->nr_levels >= 16 && nr_positions >= (cfg->pos_dim <= 5 ? 1 << 19 : 1 << 20) ? 1 : 0;
+// Where the order's own time comes back: the number of levels from which on it is used, by what follows it.  A
+// line lies where neither independent points nor ray samples (half in order already) get slower than on the
+// kernels of the build that knew no order ("before").  us without -> with the order, itself included:
+//  features only, F = 2: 2^19 points 24 levels 156 -> 141 (pos_dim 2: 115 -> 98), rays 121 -> 135 (before 147), 16
+//    levels 115 -> 106, but rays 90 -> 100 (before 97); 2^20: 24 levels 293 -> 250, rays 228 -> 240 (before 282), 16
+//    levels 211 -> 186, rays 161 -> 180 (before 172), 12 levels 148 -> 150; pos_dim 6, 16 levels 369 -> 371.
+//    F = 4, 2^20 points 174 -> 178.
+//  table gradient, F = 2: 2^18: 12 levels 118 -> 108, rays 95 -> 111 (before 112), 8 levels 75 -> 76; pos_dim 4, 16
+//    levels 202 -> 188, 12 levels 146 -> 156.  2^19: 8 levels 128 -> 117, rays 112 -> 115, pos_dim 6 218 -> 219; 4 levels 95
+//    -> 104 at pos_dim 4.  2^20: 4 levels 157 -> 131, pos_dim 2 122 -> 113, rays 110 -> 127 (before 132), but pos_dim 4
+//    173 -> 184; 8 levels of pos_dim 6 404 -> 397.
+//    F = 4, 2^19: 8 levels 163 -> 147, rays 134 -> 145 (before 160), 4 levels rays 79 -> 94 (before 89); pos_dim 4, 8 / 16
+//    levels 181 -> 188 / 372 -> 356.  F = 8, 2^19: 4 levels 146 -> 132, pos_dim 6, 4 / 8 levels 212 -> 229 / 390 -> 389.
+//  position gradient, alone or with the table's, F = 2: 2^18: both, 16 levels 198 -> 194, 12 levels 148 -> 152; pos_dim 4,
+//    24 levels 345 -> 356.  2^19: 12 levels 265 -> 248, rays 210 -> 236 (before 263), 8 levels 146 -> 156; pos_dim 6, 12 /
+//    16 levels 462 -> 492 / 620 -> 631 (2^20: 1185 -> 1167).  F = 4: 2^19: 16 levels 414 -> 408, rays 359 -> 397 (before 402);
+//    pos_dim 4 503 -> 510, 2^20 949 -> 932; pos_dim 6 1330 -> 1366.  F = 8: 8 levels 341 -> 276, pos_dim 6 534 -> 533, 4
+//    levels rays 138 -> 164 (before 150).
+int permuto_order_pays(const permuto_config* cfg, int64_t nr_positions, int32_t purpose) {
+    if (!cfg || nr_positions > (int64_t)0x7fffffff) return 0;
+    const int F = cfg->nr_feat_per_level, d = cfg->pos_dim;
+    const bool n18 = nr_positions >= 1 << 18, n19 = nr_positions >= 1 << 19, n20 = nr_positions >= 1 << 20;
+    int levels = 0;  // never
+    if (purpose == PERMUTO_ORDER_FEATURES) {
+        if (F == 2 && (d <= 5 ? n19 : n20)) levels = 18;
+    } else if (purpose == PERMUTO_ORDER_TABLE_GRAD) {
+        if (F == 2 && n18) levels = n20 ? (d <= 3 ? 4 : 8) : (n19 ? 8 : (d <= 3 ? 10 : 16));
+        if (F == 4 && n19) levels = d <= 3 ? 8 : 16;
+        if (F == 8 && n19) levels = d <= 5 ? 4 : 8;
+    } else {
+        if (F == 2 && n18) levels = n19 ? (d <= 5 ? 12 : 16) : (d <= 3 ? 16 : 0);
+        if (F == 4 && n19) levels = d <= 3 || (d <= 5 && n20) ? 12 : 0;
+        if (F == 8 && n19) levels = 8;
+    }
+    return levels > 0 && cfg->nr_levels >= levels ? 1 : 0;
 }
 
 int permuto_order_points(const permuto_config* cfg, const permuto_inputs* in, void* order, int64_t order_bytes, void* stream) {

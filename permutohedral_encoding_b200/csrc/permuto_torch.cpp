@@ -18,6 +18,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <algorithm>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -146,6 +147,7 @@ struct Inputs {
     c10::intrusive_ptr<Lattice> lattice;
     Tensor values, positions, window, shift, half, order;
     int levels_per_pass = 0;
+    bool all_open = false;  // the caller knows the window to be open on every level
 };
 
 // What the nodes of one call share.  The tensors of the graph are not here: nodes keep them with
@@ -155,7 +157,8 @@ struct Call : torch::CustomClassHolder {
     Tensor shift, half;
     int levels_per_pass = 0;
     bool need_values = false, need_positions = false;
-    bool ordered = false;  // the forward ran in spatial order
+    bool all_open = false;  // as in Inputs
+    bool ordered = false;   // the forward ran in spatial order
 
     // A loss that reaches both the features and the position gradient gives the lattice values two
     // gradients in one backward, from the first-order node and from a second-order one (EncodeBackward).
@@ -294,12 +297,35 @@ Tensor make_order(const Inputs& c, Bound& b) {
 }
 
 // What a call is ordered for: an order is made where order_pays says so.
-enum Purpose { kAsGiven = -1, kInference = 0, kTraining = 1 };
+enum Purpose {
+    kAsGiven = -1,
+    kInference = PERMUTO_ORDER_FEATURES,
+    kTable = PERMUTO_ORDER_TABLE_GRAD,
+    kPositions = PERMUTO_ORDER_POS_GRAD
+};
+
+// Whether to order a call, as far as the host knows its open levels.  What a closed level takes is far less than
+// its share of the order (24 levels with 7 open, 2^20 points: features 74 -> 102 us, both gradients 269 -> 297), so
+// a call whose window is on the device, unless it is the module's own, is not ordered.  Letting the sort count
+// the open levels there and stand aside was measured too: 10-15 us a call (91 -> 106), and no gain at 0.3.
+// Half of the levels have to be open, since rows are read out of order whether their levels are open or not
+// (table gradient of 2^21 points, 7 of 24 levels open: 421 -> 477; 14 of 24: 862 -> 649).
+bool order_pays(const Inputs& c, const Bound& b, Purpose purpose) {
+    permuto_config cfg = b.cfg;
+    if (!c.all_open) {
+        if (!c.window.is_cpu()) return false;
+        const Tensor w = plain(c.window, c.window.device());
+        const float* v = w.data_ptr<float>();
+        cfg.nr_levels = (int)std::count_if(v, v + w.numel(), [](float x) { return x != 0.f; });
+        if (2 * cfg.nr_levels < b.cfg.nr_levels) return false;
+    }
+    return api.order_pays(&cfg, b.in.nr_positions, purpose) != 0;
+}
 
 // An order that a call can do without: where there is no room for its 24 to 44 bytes a point the call runs
 // as it would without one (callers allocate their outputs first).
 void try_order(Inputs& c, Bound& b, Purpose purpose) {
-    if (c.order.defined() || !api.order_pays(&b.cfg, b.in.nr_positions, purpose)) return;
+    if (c.order.defined() || !order_pays(c, b, purpose)) return;
     try {
         c.order = make_order(c, b);
     } catch (const c10::OutOfMemoryError&) {
@@ -442,11 +468,11 @@ Tensor order_to_save(const Inputs& in) { return at::SavedTensorDefaultHooks::get
 // a node's inputs out of its saved tensors, which start at `first`: values, positions, window, order
 Inputs saved_inputs(const Call& call, const variable_list& saved, size_t first) {
     Inputs in{call.lattice, saved[first], saved[first + 1], saved[first + 2], call.shift, call.half, saved[first + 3],
-              call.levels_per_pass};
+              call.levels_per_pass, call.all_open};
     if (call.ordered && !in.order.defined()) {
         check_inputs(in);
         Bound b(in);
-        try_order(in, b, kTraining);
+        try_order(in, b, call.need_positions ? kPositions : kTable);
     }
     return in;
 }
@@ -505,7 +531,7 @@ struct EncodeBackward : torch::autograd::Function<EncodeBackward> {
 struct Encode : torch::autograd::Function<Encode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& values, const Tensor& positions, Inputs& in,
                           const c10::intrusive_ptr<Call>& call) {
-        const Tensor out = run_forward(in, kTraining);
+        const Tensor out = run_forward(in, call->need_positions ? kPositions : kTable);
         call->ordered = in.order.defined();
         ctx->save_for_backward({values, positions, in.window, order_to_save(in)});
         ctx->saved_data["call"] = c10::IValue::make_capsule(call);
@@ -543,14 +569,15 @@ struct Encode : torch::autograd::Function<Encode> {
 
 Inputs make_inputs(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, const Tensor& positions, const Tensor& window,
                    const Tensor& shift, const std::optional<Tensor>& half, const std::optional<Tensor>& order,
-                   int levels_per_pass) {
-    return {lattice, values, positions, window, shift, half ? *half : Tensor(), order ? *order : Tensor(), levels_per_pass};
+                   int levels_per_pass, bool all_open) {
+    return {lattice, values, positions, window, shift, half ? *half : Tensor(), order ? *order : Tensor(), levels_per_pass,
+            all_open};
 }
 
 // the module's forward: with a graph where one is wanted
 Tensor encode(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, const Tensor& positions, const Tensor& window,
-              const Tensor& shift, const std::optional<Tensor>& half, int levels_per_pass) {
-    Inputs in = make_inputs(lattice, values, positions, window, shift, half, std::nullopt, levels_per_pass);
+              const Tensor& shift, const std::optional<Tensor>& half, int levels_per_pass, bool all_open) {
+    Inputs in = make_inputs(lattice, values, positions, window, shift, half, std::nullopt, levels_per_pass, all_open);
     const bool graph = at::GradMode::is_enabled();
     const bool need_values = graph && values.requires_grad(), need_positions = graph && positions.requires_grad();
     if (!need_values && !need_positions) return run_forward(in, kInference);
@@ -559,6 +586,7 @@ Tensor encode(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, 
     call->shift = in.shift;
     call->half = in.half;
     call->levels_per_pass = levels_per_pass;
+    call->all_open = all_open;
     call->need_values = need_values;
     call->need_positions = need_positions;
     Tensor out = Encode::apply(values, positions, in, call);
@@ -568,9 +596,9 @@ Tensor encode(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, 
 
 Tensor forward_mlp(const c10::intrusive_ptr<Lattice>& lattice, const Tensor& values, const Tensor& positions,
                    const Tensor& window, const Tensor& shift, const std::optional<Tensor>& half,
-                   const std::optional<Tensor>& order, int levels_per_pass, const std::vector<Tensor>& weights,
+                   const std::optional<Tensor>& order, int levels_per_pass, bool all_open, const std::vector<Tensor>& weights,
                    const std::vector<std::optional<Tensor>>& biases, int activation, const std::optional<Tensor>& status) {
-    Inputs c = make_inputs(lattice, values, positions, window, shift, half, order, levels_per_pass);
+    Inputs c = make_inputs(lattice, values, positions, window, shift, half, order, levels_per_pass, all_open);
     check_inputs(c);
     const c10::Device device = positions.device();
     if (weights.empty() || weights.size() > 6)
@@ -642,16 +670,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("encode", &encode);
     m.def("forward", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w, const Tensor& s,
                         const std::optional<Tensor>& half, const std::optional<Tensor>& order, int lpp) {
-        Inputs c = make_inputs(l, v, p, w, s, half, order, lpp);
+        Inputs c = make_inputs(l, v, p, w, s, half, order, lpp, true);
         return run_forward(c, kAsGiven);
     });
     m.def("check_inputs", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w,
                              const Tensor& s, const std::optional<Tensor>& half) {
-        check_inputs(make_inputs(l, v, p, w, s, half, std::nullopt, 0));
+        check_inputs(make_inputs(l, v, p, w, s, half, std::nullopt, 0, true));
     });
     m.def("order", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w, const Tensor& s,
                       const std::optional<Tensor>& half, int lpp, int purpose) -> std::optional<Tensor> {
-        Inputs c = make_inputs(l, v, p, w, s, half, std::nullopt, lpp);
+        Inputs c = make_inputs(l, v, p, w, s, half, std::nullopt, lpp, true);
         check_inputs(c);
         Bound b(c);
         if (purpose >= 0 && !api.order_pays(&b.cfg, b.in.nr_positions, purpose)) return std::nullopt;
@@ -661,7 +689,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
                          const std::optional<Tensor>& half, const std::optional<Tensor>& order, int lpp, const Tensor& grad,
                          bool need_values, bool need_positions, const std::optional<Tensor>& values_out, int level_begin,
                          int level_end, bool zero, const std::optional<Tensor>& positions_out) {
-        Inputs c = make_inputs(l, v, p, w, s, half, order, lpp);
+        Inputs c = make_inputs(l, v, p, w, s, half, order, lpp, true);
         const Gradients g = run_backward(c, grad, need_values, need_positions, values_out ? *values_out : Tensor(), level_begin,
                                          level_end, zero, positions_out ? *positions_out : Tensor());
         return py::make_tuple(as_python(g.values), as_python(g.positions));
@@ -669,7 +697,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("double_backward", [](const c10::intrusive_ptr<Lattice>& l, const Tensor& v, const Tensor& p, const Tensor& w,
                                 const Tensor& s, const std::optional<Tensor>& half, const std::optional<Tensor>& order, int lpp,
                                 const Tensor& dpg, const Tensor& grad, bool need_values, bool need_features) {
-        Inputs c = make_inputs(l, v, p, w, s, half, order, lpp);
+        Inputs c = make_inputs(l, v, p, w, s, half, order, lpp, true);
         const SecondOrder r = run_double_backward(c, dpg, grad, need_values, need_features);
         return py::make_tuple(as_python(r.values), as_python(r.features));
     });

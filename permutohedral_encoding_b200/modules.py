@@ -109,7 +109,8 @@ class PermutoEncoding(torch.nn.Module):
         return super()._load_from_state_dict(state_dict, prefix, *args, **kwargs)
 
     def forward(self, positions, anneal_window=None):
-        if anneal_window is None:
+        all_open = anneal_window is None
+        if all_open:
             anneal_window = self.anneal_window
         # straight from the dict: nn.Module's attribute lookup of a parameter is most of a microsecond
         values, shift = self._parameters.get("lattice_values"), self._parameters.get("random_shift_per_level")
@@ -119,7 +120,7 @@ class PermutoEncoding(torch.nn.Module):
         fixed.m_random_shift_per_level = shift   # may have been replaced (load_state_dict(assign=True), .to())
         # [N, (L+extra)*F] already in the reference's output order: no permute/reshape copy
         return _C.encode(self.lattice._native, values, positions, anneal_window, shift,
-                         self._half_copy() if self.half_precision_table else None, fixed.levels_per_pass)
+                         self._half_copy() if self.half_precision_table else None, fixed.levels_per_pass, all_open)
 
     def _half_copy(self):
         """fp16 copy of the lattice values the kernels gather from when ``half_precision_table`` is
@@ -140,7 +141,8 @@ class PermutoEncoding(torch.nn.Module):
         the ``[N, output_dims()]`` features stay on chip and the product runs on the tensor cores
         (operands rounded to tf32, fp32 accumulation -- about 1e-3 relative to the magnitude of
         the summed terms).  No gradients are recorded; train through ``forward``."""
-        if anneal_window is None:
+        all_open = anneal_window is None
+        if all_open:
             anneal_window = self.anneal_window
         if anneal_window.device != positions.device:
             anneal_window = anneal_window.to(positions.device)
@@ -148,6 +150,7 @@ class PermutoEncoding(torch.nn.Module):
         weight, bias = (linear.weight, linear.bias) if hasattr(linear, "weight") else linear
         half = self._half_copy() if self.half_precision_table else None
         inp = _C.EncodingInput(self.lattice_values, positions, anneal_window, False, False, half)
+        inp.m_all_open = all_open
         return self.lattice.forward_linear(inp, weight, bias, status)
 
     @torch.no_grad()
@@ -158,7 +161,8 @@ class PermutoEncoding(torch.nn.Module):
         (examples/train_toy_example.py:18-26).  One kernel: neither the features nor the hidden
         activations are written to memory; see ``EncodingWrapper.forward_mlp`` for the limits
         (hidden widths multiples of 16 up to 64) and the precision (tf32 operands)."""
-        if anneal_window is None:
+        all_open = anneal_window is None
+        if all_open:
             anneal_window = self.anneal_window
         if anneal_window.device != positions.device:
             anneal_window = anneal_window.to(positions.device)
@@ -187,6 +191,7 @@ class PermutoEncoding(torch.nn.Module):
         activation = kinds.pop() if kinds else "none"
         half = self._half_copy() if self.half_precision_table else None
         inp = _C.EncodingInput(self.lattice_values, positions, anneal_window, False, False, half)
+        inp.m_all_open = all_open
         return self.lattice.forward_mlp(inp, layers, activation, status)
 
     def output_dims(self):

@@ -165,3 +165,28 @@ def test_order_sizes(nat):
         assert lib.permuto_order_records(C.byref(cfg), C.byref(ins), records, scratch, None) == nat.PERMUTO_ERR_INVALID_ARGUMENT
     for ins in (nat.PermutoInputs(0, 4096, 3, 1, 8, 8, 8, 8), nat.PermutoInputs(2 ** 31, 4096, 3, 1, 8, 8, 8, 8)):
         assert lib.permuto_order_records(C.byref(cfg), C.byref(ins), 4096, 4096, None) == nat.PERMUTO_ERR_INVALID_ARGUMENT
+
+
+def test_order_is_used_where_it_was_measured_to_pay(nat):
+    """Few levels, small batches and wide entries stay unordered (each of these was slower with an order
+    than without); more levels than the limit, or a larger batch, never change that back."""
+    def pays(d, feat, levels, n, purpose):
+        return nat.lib.permuto_order_pays(nat.PermutoConfig(d, feat, levels, 2 ** 18, 0, 1.0, 0, 0), n, purpose)
+
+    for d, feat, levels, n, purpose in (
+            (3, 2, 4, 2 ** 18, 1), (4, 2, 4, 2 ** 20, 1), (6, 2, 4, 2 ** 19, 1), (4, 4, 4, 2 ** 20, 1), (3, 2, 8, 2 ** 18, 2),
+            (3, 2, 4, 2 ** 20, 2), (2, 2, 8, 2 ** 20, 2), (4, 2, 8, 2 ** 20, 2), (3, 4, 8, 2 ** 20, 2), (3, 8, 4, 2 ** 19, 2),
+            (6, 4, 16, 2 ** 20, 2), (3, 2, 16, 2 ** 19, 0), (3, 2, 16, 2 ** 20, 0), (3, 4, 24, 2 ** 20, 0), (3, 2, 24, 2 ** 18, 0)):
+        assert pays(d, feat, levels, n, purpose) == 0, (d, feat, levels, n, purpose)
+    for d, feat, levels, n, purpose in (
+            (3, 2, 24, 2 ** 20, 0), (3, 2, 24, 2 ** 18, 1), (6, 2, 16, 2 ** 20, 1), (3, 2, 24, 2 ** 18, 2), (3, 4, 16, 2 ** 20, 2),
+            (3, 8, 4, 2 ** 19, 1)):
+        assert pays(d, feat, levels, n, purpose) == 1, (d, feat, levels, n, purpose)
+    for d in range(2, 8):
+        for feat in (2, 4, 8):
+            for purpose in range(3):
+                for levels in range(1, 40):
+                    got = [pays(d, feat, levels, n, purpose) for n in (2 ** 17, 2 ** 18, 2 ** 19, 2 ** 20, 2 ** 24, 2 ** 31 - 1)]
+                    assert got == sorted(got) and got[0] == 0
+                    assert pays(d, feat, levels + 1, 2 ** 20, purpose) >= got[3]
+    assert pays(3, 2, 24, 2 ** 31, 1) == 0

@@ -164,7 +164,7 @@ def test_a_backward_frees_what_the_graph_kept():
 @pytest.mark.parametrize("large", [False, True])
 def test_saved_tensor_hooks_see_and_replace_what_a_node_keeps(setup, large):
     m, pos, go = _large() if large else setup
-    window = torch.rand(m.nr_levels, device=DEV)
+    window = None if large else torch.rand(m.nr_levels, device=DEV)   # with a window on the device nothing is ordered
 
     def grads(out):
         return torch.autograd.grad(out, [m.lattice_values, pos], go)
@@ -181,7 +181,7 @@ def test_saved_tensor_hooks_see_and_replace_what_a_node_keeps(setup, large):
 
     with torch.autograd.graph.saved_tensors_hooks(keep, lambda t: t):
         out = m(pos, window)
-    assert same(seen) == same([m.lattice_values, pos, window])
+    assert same(seen) == same([m.lattice_values, pos, m.anneal_window if large else window])
     got_v, got_p = grads(out)
     _close(got_v, want_v)
     _close(got_p, want_p)
@@ -212,3 +212,12 @@ def test_checkpointed_batches_match():
     got = torch.autograd.grad(checkpoint(m, pos, use_reentrant=False), [m.lattice_values, pos], go)
     for a, b in zip(got, want):
         _close(a, b)
+
+
+@pytest.mark.parametrize("d,feat,levels", [(2, 2, 13), (3, 4, 12), (4, 8, 8), (6, 2, 16), (7, 8, 8)])
+def test_both_orders_in_one_backward_of_an_ordered_batch(d, feat, levels):
+    """The same on batches that the module puts into spatial order."""
+    from permutohedral_encoding_b200 import _native as nat
+    n = 2 ** 19 + 77
+    assert nat.lib.permuto_order_pays(nat.PermutoConfig(d, feat, levels, 2 ** 10, 0, 1.0, 0, 0), n, nat.ORDER_POSITIONS)
+    test_both_orders_in_one_backward(d, feat, levels, n)

@@ -98,7 +98,7 @@ def test_large_batches_sum_as_without_an_order(nat):
     thousand slots or more, which varies by a few per cent (0.97-1.12 measured); sums in spatial order are
     at 1.6-2.3."""
     from permutohedral_encoding_b200 import PermutoEncoding
-    n, levels = 2 ** 22 + 2051, 8
+    n, levels = 2 ** 22 + 2051, 12
     torch.manual_seed(21)
     m = PermutoEncoding(3, 2 ** 15, levels, 2, np.geomspace(0.035, 1e-3, levels))
     with torch.no_grad():
@@ -106,7 +106,7 @@ def test_large_batches_sum_as_without_an_order(nat):
     pos = (torch.rand(n, 3, device=DEV) - 0.5).requires_grad_(True)
     go, dpg = torch.randn(n, 2 * levels, device=DEV), torch.randn(n, 3, device=DEV)
     inp = nat.EncodingInput(m.lattice_values.detach(), pos.detach(), m.anneal_window, True, False)
-    assert m.lattice.order(inp, nat.ORDER_TRAINING) is not None
+    assert m.lattice.order(inp, nat.ORDER_POSITIONS) is not None
 
     def first():
         return m.lattice.backward(inp, go)[0]
@@ -186,33 +186,31 @@ def test_rows_of_an_order_stay_inside_the_batch(nat, d, feat):
         torch.cuda.synchronize()
 
 
-@pytest.mark.parametrize("n,d,levels", [(2 ** 21 + 1, 7, 1), (2 ** 18 + 1, 3, 8)])
-def test_a_call_without_room_for_an_order_runs_without_one(nat, n, d, levels):
-    """The order is an aid: a batch whose outputs fit runs whether or not the order fits beside them (rows of 8
-    and records of 32 bytes: the order alone does not fit; 64 and 16: it fits, but not beside the rows)."""
+def test_a_call_without_room_for_an_order_runs_without_one(nat):
+    """The order is an aid: a batch whose outputs fit runs whether or not the order fits beside them."""
     from permutohedral_encoding_b200 import PermutoEncoding
-    m = PermutoEncoding(d, 2 ** 10, levels, 2, np.ones(levels))
-    pos = torch.rand(n, d, device=DEV)
+    n, levels = 2 ** 18 + 1, 16                                 # rows of 32 MB, records of 4 MB, scratch of 3 MB
+    m = PermutoEncoding(3, 2 ** 10, levels, 2, np.ones(levels))
+    pos = torch.rand(n, 3, device=DEV)
     go = torch.randn(n, 2 * levels, device=DEV)
     inp = nat.EncodingInput(m.lattice_values.detach(), pos, m.anneal_window, True, False)
     want, want_grad = m.lattice.forward(inp), m.lattice.backward(inp, go)[0]
     assert m.lattice.order(inp, nat.ORDER_TRAINING) is not None
     total = torch.cuda.get_device_properties(0).total_memory
-    room, held = torch.empty(20 * 2 ** 20, dtype=torch.uint8, device=DEV), []   # the rows take 16 MB
+    room, held = torch.empty(36 * 2 ** 20, dtype=torch.uint8, device=DEV), []
 
     def limit(extra):
         torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + extra) / total)
 
     try:
         limit(0)
-        with pytest.raises(torch.cuda.OutOfMemoryError):   # nothing free but `room` and 8 MB
+        with pytest.raises(torch.cuda.OutOfMemoryError):   # nothing free but `room` and 2 MB
             while True:
-                held.append(torch.empty(4 * 2 ** 20, dtype=torch.uint8, device=DEV))
-        limit(8 * 2 ** 20)
+                held.append(torch.empty(2 ** 21, dtype=torch.uint8, device=DEV))
+        limit(2 ** 21)
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            m.lattice.order(inp)
         del room
-        if d == 7:
-            with pytest.raises(torch.cuda.OutOfMemoryError):
-                m.lattice.order(inp)
         out = m(pos)
         out.backward(go)
     finally:
@@ -220,3 +218,40 @@ def test_a_call_without_room_for_an_order_runs_without_one(nat, n, d, levels):
         held.clear()
     assert torch.equal(out, want)
     assert torch.all((m.lattice_values.grad - want_grad).abs() <= 1e-4 * want_grad.abs().amax())
+
+
+@pytest.mark.parametrize("share", [0.0, 0.2, 0.9])
+@pytest.mark.parametrize("where", ["cuda", "cpu"])
+def test_module_with_a_window(nat, share, where):
+    """The module's calls with a mostly closed, a mostly open and a closed window, on a batch that is ordered
+    when all levels are open: results as without an order."""
+    from permutohedral_encoding_b200 import PermutoEncoding
+    torch.manual_seed(8)
+    n, levels = 2 ** 19 + 3, 16
+    m = PermutoEncoding(3, 2 ** 10, levels, 2, np.geomspace(1.0, 1e-2, levels))
+    with torch.no_grad():
+        m.lattice_values.uniform_(-1, 1)
+    window = torch.rand(levels) + 0.1
+    window[int(levels * share):] = 0.0
+    pos = torch.rand(n, 3, device=DEV, requires_grad=True)
+    go, dpg = torch.randn(n, 2 * levels, device=DEV, requires_grad=True), torch.randn(n, 3, device=DEV)
+    inp = nat.EncodingInput(m.lattice_values.detach(), pos.detach(), window.cuda(), True, True)
+    want, (want_v, want_p) = m.lattice.forward(inp), m.lattice.backward(inp, go.detach())
+    want_v2, want_g = m.lattice.double_backward_from_positions(inp, dpg, go.detach())
+
+    def close(a, b):
+        assert torch.all((a - b).abs() <= 1e-4 * b.abs().amax())
+
+    w = window.to(where)
+    with torch.no_grad():
+        assert torch.equal(m(pos, w), want)
+    out = m(pos, w)
+    assert torch.equal(out, want)
+    for a, b in zip(torch.autograd.grad(out, [m.lattice_values, pos], go), (want_v, want_p)):
+        close(a, b)
+    out = m(pos, w)
+    (normal,) = torch.autograd.grad(out, pos, go, create_graph=True)
+    got = torch.autograd.grad([out, normal], [m.lattice_values, go], [go.detach(), dpg])
+    close(got[0], want_v + want_v2)
+    close(got[1], want_g)
+    close(torch.autograd.grad(m(pos.detach(), w), m.lattice_values, go)[0], want_v)
