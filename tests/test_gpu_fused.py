@@ -258,3 +258,43 @@ def test_forward_mlp_module_with_the_toy_example_network(nat):
         enc.forward_mlp(pts, torch.nn.Sequential(torch.nn.Linear(48, 32), torch.nn.Tanh(), torch.nn.Linear(32, 1)).to(DEV))
     with pytest.raises(RuntimeError, match="hidden width"):
         enc.forward_mlp(pts, torch.nn.Sequential(torch.nn.Linear(48, 24), torch.nn.ReLU(), torch.nn.Linear(24, 1)).to(DEV))
+
+
+@pytest.mark.parametrize("sizes,activation", [((32,), None), ((32, 32, 1), torch.nn.GELU), ((64, 16), torch.nn.ReLU)])
+def test_more_tiles_than_resident_blocks(nat, sizes, activation):
+    """A block walks over tiles of 128 points: with more than twice the tiles that can be resident (at most ten
+    blocks on each multiprocessor) every block takes several, the last one ragged.  The rows equal, bit for bit,
+    those of the batch in pieces that leave a block one tile (a row does not depend on the others), with and
+    without a spatial order, and the unfused network within the bound of its tf32 roundings."""
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    sms, levels = torch.cuda.get_device_properties(0).multi_processor_count, 9
+    piece = 128 * sms
+    n = 2 * 10 * piece + 77
+    fx = nat.EncodingFixedParams(3, 2 ** 12, levels, 2, np.geomspace(1.0, 1e-2, levels),
+                                 torch.randn((levels, 3), device=DEV, generator=gen) * 10, False, 1.0)
+    enc = nat.EncodingWrapper.create(3, 2, fx)
+    table = torch.randn((levels, 2 ** 12, 2), device=DEV, generator=gen)
+    pos, window = torch.rand((n, 3), device=DEV, generator=gen), torch.ones(levels, device=DEV)
+    widths = (enc.output_width(),) + sizes
+    layers = [(torch.randn((b, a), device=DEV, generator=gen) / a ** 0.5, torch.randn(b, device=DEV, generator=gen))
+              for a, b in zip(widths, widths[1:])]
+    kind = {None: "none", torch.nn.GELU: "gelu", torch.nn.ReLU: "relu"}[activation]
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(x, ordered):
+        inp = nat.EncodingInput(table, x, window, False, False)
+        inp.m_order = enc.order(inp) if ordered else None
+        return enc.forward_mlp(inp, layers, kind, status=status)
+
+    whole = run(pos, False)
+    for b in range(0, n, piece):
+        assert torch.equal(run(pos[b:b + piece], False), whole[b:b + piece])
+    assert torch.equal(run(pos, True), whole)
+    assert int(status.item()) == 0
+    x = enc.forward(nat.EncodingInput(table, pos, window, False, False)).double()
+    for i, (w, bias) in enumerate(layers):
+        last = (x.abs() @ w.double().abs().t()).amax()
+        x = x @ w.double().t() + bias.double()
+        if activation and i + 1 < len(layers):
+            x = activation()(x)
+    assert (whole.double() - x).abs().amax() <= len(layers) * TF32_RTOL * last
