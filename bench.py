@@ -203,11 +203,11 @@ class OursStep:
         self.hook = LatticeGradAllReduce(self.m, nr_buckets=buckets, policy=ARGS.bucket_policy, multimem=mm,
                                          copy_out=ARGS.copy_out, clear=ARGS.clear) if world > 1 else None
         self.collective = None if self.hook is None else ("multimem" if self.hook._symm is not None else "nccl")
-        # the four kernels of the spatial order (batches from 2^18 points on), the forward, and the table
-        # gradient once, twice (beyond 2^22 points) or once per bucket
-        local = w["total_points"] // world
-        table = len(self.hook.buckets) if world > 1 else (2 if local > 2 ** 22 else 1)
-        self.launches_per_step = (4 if local >= 2 ** 18 else 0) + 1 + table
+        # the four kernels of the spatial order where the module makes one, the forward, and the table gradient
+        # once or once per bucket
+        from permutohedral_encoding_b200 import _native as nat
+        ordered = nat.lib.permuto_order_pays(self.m.fixed_params.config(), w["total_points"] // world, nat.ORDER_TRAINING)
+        self.launches_per_step = (4 if ordered else 0) + 1 + (len(self.hook.buckets) if world > 1 else 1)
         self.opt = None
 
     @property

@@ -179,7 +179,8 @@ int permuto_double_backward(const permuto_config *cfg, const permuto_inputs *in,
 
 /* Spatial order of a batch.  Sorting the points along a space-filling curve first puts neighbours
  * into the same warp, which is what the gathers and reductions of a large batch of independent samples
- * gain from (no counterpart in the reference; results do not depend on it, rows keep their place).
+ * gain from (no counterpart in the reference; rows keep their place and their values, table
+ * gradients are the same fp32 sums in another sequence).
  * permuto_order_points fills a caller-owned device buffer of permuto_order_bytes(pos_dim, N) bytes,
  * 256-byte aligned, for in->positions; the *_ordered entry points below take it together with the SAME
  * positions (NULL = no order, which is what the plain entry points pass).  One order serves the forward,

@@ -1190,8 +1190,9 @@ backward_kernel(const BackwardArgs a) {
 // waited for instructions (384 us against 309).  Two points per thread: 3, 4 and 8 take 309, 325 and
 // 378 us against 302.  Row segments go through registers as one 32-byte load; copied asynchronously as
 // two 16-byte ones they cost twice the L2 requests (2^24 points: 5257 us against 4410).
-// Against the fused scatter of an unordered batch: 2^20 points and 24 levels 440 -> 300 us, 2^24 points
-// 6300 -> 4230, pos_dim 6 545 -> 480, double backward 660 -> 540.
+// Against the fused scatter of an unordered batch: 2^20 points and 24 levels 440 -> 300 us, pos_dim 6
+// 545 -> 480, double backward 660 -> 540; 2^24 points 6300 -> 4230, but batches of that size are summed in
+// their own sequence (kOrderedSums on the PyTorch side).
 constexpr int kRunPoints = 2;
 constexpr int kRunThreads = 128;
 // Resident blocks the registers have to allow: the D+1 running sums of F features and their slots stay
@@ -1447,6 +1448,9 @@ __global__ void __launch_bounds__(kRunThreads, run_blocks(F)) scatter_runs_kerne
                     } else {
 #pragma unroll
                         for (int r = 0; r <= D; ++r) red_add<F>(gbase, cur[r], acc[r]);
+                        // less than a quarter of the warp's points shared their vertex 0 with another: the finer
+                        // levels of this walk go without the merge (2^20 points; an eighth / a quarter / a half / never:
+                        // 306 / 305 / 304 / 314 us)
                         kept = __reduce_add_sync(kFullMask, kept);
                         if (kept + 32 - distinct < 8 * P) sc.probe = false;
                     }

@@ -33,7 +33,9 @@ namespace {
 constexpr int kChunkBits = 21;      // points per chunk; 2^20 / 2^22 / 2^23 / 2^24 points: order 461 / 568 / 675 / 772 us
                                     // against 520, but the forward after it 3160 / 3085 / 3064 / 3018 against 3080
 constexpr int kCellBits = 1;        // about two points per cell: more share counters, whose atomics then collide
-                                    // (8 / 32 / 128 / 512 points per cell, 2^20 points: 34 / 37 / 39 / 72 us)
+                                    // (8 / 32 / 128 / 512 points per cell, 2^20 points: 34 / 37 / 39 / 72 us).  1 / 2 / 4
+                                    // / 8 points out of a cold L2: order 43 / 42 / 42 / 42, table gradient after it 304 /
+                                    // 305 / 305 / 309; 2^24 points, order 552 / 534 / 527 / 523
 constexpr int kScanBins = 1024;     // cells per block of the scan
 constexpr int kThreads = 256;
 constexpr int kPerThread = 4;       // consecutive points of a thread: whole 16-byte vectors of any row length
