@@ -1176,287 +1176,218 @@ backward_kernel(const BackwardArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------
-// table gradient of a batch in spatial order: two consecutive points per thread
+// table gradient of a batch in spatial order: one level per thread, points one after the other
 // ------------------------------------------------------------------------------------------
-// Consecutive points of an ordered batch share vertices on every level whose cells are wider than the
-// distance between points: a thread first sums what its two points add to the same vertex, in
-// registers; then the warp merges its lanes (scatter_level above), and a warp that sits in at most three
-// simplices -- coarse levels -- adds each simplex's D+1 vertices by recursive halving instead.
+// A strand is a run of consecutive points of the ordered batch.  The levels of a sweep are dealt to consecutive
+// threads; each walks the strand for its own level and keeps the sums of the D+1 vertices it is at in
+// registers (a vertex keeps its remainder from one simplex to the next, which is where its sum is looked for).
+// A sum goes to the table when the walk has left its vertex.  A warp reads a gradient row as whole sectors, and
+// no lane has to look at another: with two points per thread and the lanes of a warp merged by match and
+// shuffles (the kernel before) 40 % of the instructions were merging, and coarse and fine levels
+// took turns at the two limits.  Here every warp carries all levels at all times.
 //
-// What bounds it: on fine levels the rate of L2 reductions (pos_dim 3, levels 16-23 of 2^20 points:
-// 33 M reductions in 175 us, 190 G/s of the 220 G/s the device sustains), on coarse ones instruction issue
-// (levels 0-7: 77 % of the slots).  Coordinates and gradient rows wait in shared memory so that level
-// and point loops need not be unrolled: unrolled over 4 levels and 4 points four of five issue slots
-// waited for instructions (384 us against 309).  Two points per thread: 3, 4 and 8 take 309, 325 and
-// 378 us against 302.  Row segments go through registers as one 32-byte load; copied asynchronously as
-// two 16-byte ones they cost twice the L2 requests (2^24 points: 5257 us against 4410).
-// Against the fused scatter of an unordered batch: 2^20 points and 24 levels 440 -> 300 us, pos_dim 6
-// 545 -> 480, double backward 660 -> 540; 2^24 points 6300 -> 4230, but batches of that size are summed in
-// their own sequence (kOrderedSums on the PyTorch side).
-constexpr int kRunPoints = 2;
-constexpr int kRunThreads = 128;
-// Resident blocks the registers have to allow: the D+1 running sums of F features and their slots stay
-// live over the points of a thread, and spilling them costs more than the warps they displace (pos_dim 6
-// at eight blocks 552 us, at five 490; 8 features, 2^20 points, at eight 236, at four 204).
-constexpr int run_blocks(int feats) {
-    const int live = (D + 1) * (feats + 1);
-    return live <= 18 ? 8 : (live <= 26 ? 5 : (live <= 45 ? 4 : 3));
-}
-constexpr int kPosVec = D <= 3 ? 1 : 2;  // float4s per point: coordinates, row index last
-// D floats kept as kPosVec float4s, kRunThreads apart
-__device__ __forceinline__ void load_vec(const float4* src, float (&x)[D]) {
-#pragma unroll
-    for (int i = 0; i < kPosVec; ++i) {
-        const float4 v = src[i * kRunThreads];
-        x[4 * i] = v.x;
-        if (4 * i + 1 < D) x[(4 * i + 1) % D] = v.y;
-        if (4 * i + 2 < D) x[(4 * i + 2) % D] = v.z;
-        if (4 * i + 3 < D) x[(4 * i + 3) % D] = v.w;
-    }
-}
-// what the table receives: the addends of the first-order backward, of the double backward, or their sum
+// What bounds it: the rate of L2 reductions (pos_dim 3, 24 levels, 2^20 points: 44 M in 220 us of 250, the rest
+// clearing the table and the ends of the launch; 174 to 200 M instructions against 212 M) and the integer
+// and select pipe (75 % with two vertices kept).  Records wait in shared memory because a load takes its turn
+// behind the reductions: with records and rows requested one point ahead from memory 280 us, through a
+// per-thread ring of asynchronous copies 310 (the copies themselves).  Before -> now, first order / second
+// order / both in one, us: pos_dim 3, 24 levels, 2^19 points 174 / 185 / 229 -> 138 / 150 / 164, 2^20 points 306 / 327 ->
+// 250 / 269, 2^22 1080 -> 917; 2^20 points and 16 levels of pos_dim 4 328 / 358 / 448 -> 241 / 267 / 304, of pos_dim 6
+// 482 / 521 / 622 -> 425 / 480 / 523; 11 levels of 4 features 224 -> 157, 6 of 8 features 210 -> 189.  A warp of 4 levels
+// and 8 strands, which can drop the sums on levels that share nothing, takes 228 at pos_dim 4 and 854 for 2^22
+// points, but 144 for 2^19, 459 at pos_dim 6 and 213 with 8 features.
+//
+// What the table receives: the addends of the first-order backward, of the double backward, or their sum.
 enum class Order { First, Second, Both };
-template <Order ORDER>
-struct RunStage {
-    static constexpr bool kSecond = ORDER != Order::First;
-    float levels[kStage * kRecord];
-    float4 point[kRunPoints][kPosVec][kRunThreads];
-    float4 dpg[kSecond ? kRunPoints : 1][kSecond ? kPosVec : 1][kSecond ? kRunThreads : 1];
-    // gradient row segments: [first, second order][point][4 floats of the step][thread]
-    float4 grad[ORDER == Order::Both ? 2 : 1][kRunPoints][2][kRunThreads];
-};
-// Sum over the warp of CNT vertices' addends by recursive halving: at each step a lane keeps one half of
-// the vertices and hands the other half to its partner, so CNT = 4 vertices take 4+2+1 exchanges of F
-// values where a butterfly per value takes 20.  The last step's owners add their vertex to the table.
-template <int F, int CNT>
-__device__ __forceinline__ void reduce_vertices(float* level_base, unsigned lane, int bit, int vertex, uint32_t (&slot)[CNT],
-                                                float (&v)[CNT][F]) {
-    if constexpr (CNT == 1) {
-        for (int b = bit; b > 0; b >>= 1) {
+
+constexpr int kStrandLength = 16;  // points of a strand, at least: 8 / 16 / 32 points, 2^19 points 169 / 147 / 163 us
+// a block's points: what its shared memory holds where a sweep has few levels
+constexpr int kStrandPoints = D <= 3 ? 2048 : 1024;
+// Sums kept per remainder.  With TWO the vertex before the last one is kept too, which catches walks that go to
+// and fro between neighbouring simplices: 10 to 14 % fewer reductions for a quarter more instructions.
+constexpr int strand_live(int feats, bool two) { return (D + 1) * (feats + 1) * (two ? 2 : 1); }
+constexpr int strand_left(int feats) { return (D + 1) * (feats + 1); }  // words a thread leaves at its strand's end
+constexpr int strand_threads(int feats) { return strand_left(feats) * 4 * 256 <= 48 * 1024 ? 256 : 128; }  // of a block, at most
+// warps per SM that the registers have to allow: the sums and their slots stay live over the walk
+constexpr int strand_warps(int feats, bool two) {
+    return strand_live(feats, two) <= 24 ? 32 : (strand_live(feats, two) <= 30 ? 24 : (strand_live(feats, two) <= 60 ? 16 : 12));
+}
+constexpr int kRecordVec = D <= 3 ? 1 : 2;  // float4s of a record
+
+template <int F, Order ORDER, bool TWO>
+__global__ void __launch_bounds__(strand_threads(F), strand_warps(F, TWO) * 32 / strand_threads(F))
+scatter_strands_kernel(const CombinedArgs a) {
+    constexpr bool kSecond = ORDER != Order::First;
+    constexpr bool kBoth = ORDER == Order::Both;
+    constexpr float kInv = 1.0f / (D + 1);
+    constexpr uint32_t kNone = 0xffffffffu;  // no slot: capacities are below 2^31
+    const Problem& p = a.p;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    const int pass_begin = p.level_begin + (int)blockIdx.y * p.levels_per_pass;
+    const int levels = min(p.levels_per_pass, p.level_end - pass_begin);
+    const int strands = (int)blockDim.x / levels;
+    const int strand = (int)threadIdx.x / levels;
+    const int l = pass_begin + (int)threadIdx.x - strand * levels;
+    const int64_t block_first = (int64_t)blockIdx.x * a.points_per_block;
+    const int block_points = (int)min((int64_t)a.points_per_block, p.n_points - block_first);
+    const int each = (a.points_per_block + strands - 1) / strands;
+    const int first = strand * each, last = min(first + each, block_points);
+    const bool merge = a.aggregate != 0;
+    float* gbase = a.lattice_grad + (size_t)l * p.capacity * F;
+
+    // the block's records, and what else it needs of each point
+    float4* record = reinterpret_cast<float4*>(smem_raw);
+    float* dpgs = reinterpret_cast<float*>(record + kRecordVec * a.points_per_block);
+    for (int i = threadIdx.x; i < block_points; i += blockDim.x) {
+        float x[D];
+        const int64_t n = load_point(p, block_first + i, x);
+        float r[4 * kRecordVec];
 #pragma unroll
-            for (int f = 0; f < F; ++f) v[0][f] += __shfl_xor_sync(kFullMask, v[0][f], b);
+        for (int j = 0; j < 4 * kRecordVec; ++j) r[j] = j < D ? x[j < D ? j : 0] : 0.f;
+        r[4 * kRecordVec - 1] = __uint_as_float((uint32_t)n);
+#pragma unroll
+        for (int v = 0; v < kRecordVec; ++v) record[i * kRecordVec + v] = make_float4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+        if constexpr (kSecond) {
+#pragma unroll
+            for (int j = 0; j < D; ++j) dpgs[i * D + j] = __ldg(a.double_positions_grad + n * D + j);
         }
-        if ((lane & (2u * bit - 1u)) == 0u && vertex <= D) red_add<F>(level_base, slot[0], v[0]);
-    } else {
-        constexpr int H = (CNT + 1) / 2;
-        const bool up = (lane & bit) != 0u;
-        uint32_t s[H];
-        float k[H][F];
+    }
+    __syncthreads();
+
+    uint32_t cur[D + 1];
+    float acc[D + 1][F];
 #pragma unroll
-        for (int i = 0; i < H; ++i) {
-            const bool pair = i + H < CNT;
-            s[i] = (up && pair) ? slot[pair ? i + H : i] : slot[i];
+    for (int r = 0; r <= D; ++r) {
+        cur[r] = kNone;
+#pragma unroll
+        for (int f = 0; f < F; ++f) acc[r][f] = 0.f;
+    }
+    if (strand < strands && first < last && __ldg(p.anneal + l) != 0.0f) {  // a closed level's addends are exact zeros
+        const float* rows1 = (ORDER == Order::Second ? a.second_grad_features : a.grad_features) + F * l;
+        const float* rows2 = a.second_grad_features + F * l;  // Both
+        float next1[F], next2[kBoth ? F : 1];
+        auto request = [&](int i) {  // the rows of a point, while the point before it is worked on
+            const int64_t n = (int64_t)__float_as_uint(record[min(i, last - 1) * kRecordVec + kRecordVec - 1].w);
+            load_feats<F>(rows1 + n * p.width, next1);
+            if constexpr (kBoth) load_feats<F>(rows2 + n * p.width, next2);
+        };
+        request(first);
+        LevelConst<D> lc;
+        lc.weight = __ldg(p.anneal + l);
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            lc.shift[i] = __ldg(p.shift + l * D + i);
+            lc.scale[i] = __ldg(p.scale + l * D + i);
+        }
+        lc.reach = exact_reach<D>(p.shift + l * D, p.scale + l * D);
+        uint32_t old[TWO ? D + 1 : 1];
+        float old_sum[TWO ? D + 1 : 1][F];
+        if constexpr (TWO) {
+#pragma unroll
+            for (int r = 0; r <= D; ++r) {
+                old[r] = kNone;
+#pragma unroll
+                for (int f = 0; f < F; ++f) old_sum[r][f] = 0.f;
+            }
+        }
+#pragma unroll 1
+        for (int i = first; i < last; ++i) {
+            float g1[F], g2[kBoth ? F : 1];
 #pragma unroll
             for (int f = 0; f < F; ++f) {
-                const float a = v[i][f], b = pair ? v[pair ? i + H : i][f] : 0.f;
-                k[i][f] = (up ? b : a) + __shfl_xor_sync(kFullMask, up ? a : b, bit);
+                g1[f] = next1[f];
+                if (kBoth) g2[kBoth ? f : 0] = next2[kBoth ? f : 0];
+            }
+            request(i + 1);
+            float v[4 * kRecordVec], x[D];
+#pragma unroll
+            for (int q = 0; q < kRecordVec; ++q) {
+                const float4 t = record[i * kRecordVec + q];
+                v[4 * q] = t.x;
+                v[4 * q + 1] = t.y;
+                v[4 * q + 2] = t.z;
+                v[4 * q + 3] = t.w;
+            }
+#pragma unroll
+            for (int j = 0; j < D; ++j) x[j] = v[j];
+            Simplex<D> s;
+            locate_simplex<D>(x, largest_coordinate<D>(x), lc, s);
+            uint32_t slot[D + 1];
+            to_slots(p, s, slot);
+            to_remainders(s.s, slot);
+            float w1[D + 1], w2[kBoth ? D + 1 : 1], dpg[kSecond ? D : 1];
+            if constexpr (kSecond) {
+#pragma unroll
+                for (int j = 0; j < D; ++j) dpg[j] = dpgs[i * D + j];
+            }
+            if constexpr (ORDER != Order::Second)
+                vertex_weights<D>(s, lc.weight * kInv, w1);
+            else
+                second_order_weights(s, lc, dpg, w1);
+            to_remainders(s.s, w1);
+            if constexpr (kBoth) {
+                second_order_weights(s, lc, dpg, w2);
+                to_remainders(s.s, w2);
+            }
+#pragma unroll
+            for (int r = 0; r <= D; ++r) {
+                const bool same = merge && slot[r] == cur[r];
+                float sum[F];
+                if constexpr (TWO) {
+                    const bool back = merge && slot[r] == old[r];
+                    if (!same && !back && old[r] != kNone) red_add<F>(gbase, old[r], old_sum[r]);
+#pragma unroll
+                    for (int f = 0; f < F; ++f) {
+                        sum[f] = same ? acc[r][f] : (back ? old_sum[r][f] : 0.f);
+                        old_sum[r][f] = same ? old_sum[r][f] : acc[r][f];
+                    }
+                    old[r] = same ? old[r] : cur[r];
+                } else {
+                    if (!same && i > first) red_add<F>(gbase, cur[r], acc[r]);
+#pragma unroll
+                    for (int f = 0; f < F; ++f) sum[f] = same ? acc[r][f] : 0.f;
+                }
+                cur[r] = slot[r];
+#pragma unroll
+                for (int f = 0; f < F; ++f) {
+                    acc[r][f] = fmaf(w1[r], g1[f], sum[f]);
+                    if constexpr (kBoth) acc[r][f] = fmaf(w2[r], g2[f], acc[r][f]);
+                }
             }
         }
-        reduce_vertices<F, H>(level_base, lane, bit >> 1, up ? vertex + H : vertex, s, k);
-    }
-}
-
-// The addends of a warp whose lanes sit in at most kFewSimplices simplices (coarse levels): one reduction
-// per simplex.  False, with nothing done, otherwise.
-constexpr int kFewSimplices = 3;  // 0 (never) / 1 / 3 / 6: 313 / 301 / 300 / 303 us
-template <int F>
-__device__ __forceinline__ bool merge_simplices(float* level_base, unsigned lane, const uint32_t (&slot)[D + 1],
-                                                const float (&add)[D + 1][F]) {
-    uint32_t key = slot[0];
+        if constexpr (TWO) {
 #pragma unroll
-    for (int r = 1; r <= D; ++r) key = key * 0x9E3779B1u + slot[r];
-    const int leader = __ffs(__match_any_sync(kFullMask, key)) - 1;
-    bool same = true;  // equal keys have to mean equal slots
-#pragma unroll
-    for (int r = 0; r <= D; ++r) same = (__shfl_sync(kFullMask, slot[r], leader) == slot[r]) && same;
-    unsigned leaders = __ballot_sync(kFullMask, leader == (int)lane);
-    if (!__all_sync(kFullMask, same) || __popc(leaders) > kFewSimplices) return false;
-#pragma unroll 1
-    do {
-        const int of = __ffs(leaders) - 1;
-        leaders &= leaders - 1u;
-        uint32_t s[D + 1];
-        float v[D + 1][F];
-#pragma unroll
-        for (int r = 0; r <= D; ++r) {
-            s[r] = __shfl_sync(kFullMask, slot[r], of);
-#pragma unroll
-            for (int f = 0; f < F; ++f) v[r][f] = leader == of ? add[r][f] : 0.f;
-        }
-        reduce_vertices<F, D + 1>(level_base, lane, 16, 0, s, v);
-    } while (leaders);
-    return true;
-}
-
-template <int F, Order ORDER>
-__global__ void __launch_bounds__(kRunThreads, run_blocks(F)) scatter_runs_kernel(const CombinedArgs a) {
-    constexpr int P = kRunPoints;
-    constexpr int LPS = 8 / F;
-    const Problem& p = a.p;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr bool kSecond = ORDER != Order::First;
-    RunStage<ORDER>& sm = *reinterpret_cast<RunStage<ORDER>*>(smem_raw);
-    const int t = threadIdx.x;
-    const int pass_begin = p.level_begin + (int)blockIdx.y * p.levels_per_pass;
-    const int pass_end = min(pass_begin + p.levels_per_pass, p.level_end);
-    constexpr float kInv = 1.0f / (D + 1);
-
-    const int64_t first = ((int64_t)blockIdx.x * kRunThreads + t) * P;
-    const int count = (int)max((int64_t)0, min((int64_t)P, p.n_points - first));  // points this thread owns
-#pragma unroll
-    for (int j = 0; j < P; ++j) {
-        float x[D];
-        const int64_t n = load_point(p, min(first + j, p.n_points - 1), x);
-        float r[4 * kPosVec];
-#pragma unroll
-        for (int i = 0; i < 4 * kPosVec; ++i) r[i] = i < D ? x[i < D ? i : 0] : 0.f;
-        r[4 * kPosVec - 1] = __uint_as_float((uint32_t)n);
-#pragma unroll
-        for (int i = 0; i < kPosVec; ++i) sm.point[j][i][t] = make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
-        if (kSecond) {
-#pragma unroll
-            for (int i = 0; i < 4 * kPosVec; ++i) r[i] = i < D ? __ldg(a.double_positions_grad + n * D + i) : 0.f;
-#pragma unroll
-            for (int i = 0; i < kPosVec; ++i) sm.dpg[j][i][t] = make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+            for (int r = 0; r <= D; ++r)
+                if (old[r] != kNone) red_add<F>(gbase, old[r], old_sum[r]);
         }
     }
-    Scatter sc{threadIdx.x & 31u, true, a.aggregate != 0};
 
-#pragma unroll 1
-    for (int begin = pass_begin; begin < pass_end; begin += kStage) {
-        const int end = min(begin + kStage, pass_end);
-        const int nsteps = (end - begin + LPS - 1) / LPS;
-        int step = kStagger ? (int)(blockIdx.x % (unsigned)nsteps) : 0;
-        if (begin != pass_begin) __syncthreads();
-        stage_levels(p, begin, end, sm.levels);
-        __syncthreads();
-#pragma unroll 1
-        for (int it = 0; it < nsteps; ++it) {
-            const int l0 = begin + step * LPS;
-            step = (step + 1 == nsteps) ? 0 : step + 1;
-            if (l0 == begin) sc.probe = a.aggregate != 0;
+    // Neighbouring strands end at the same vertices on coarse levels, whose few slots take one reduction per
+    // 4 ns each: what the strands are left with is summed along the block first.
+    uint32_t* left_slot = reinterpret_cast<uint32_t*>(smem_raw);                   // [vertex][thread]
+    float* left_sum = reinterpret_cast<float*>(left_slot + (D + 1) * blockDim.x);  // [vertex][feature][thread]
+    __syncthreads();  // the records are done with
 #pragma unroll
-            for (int o = 0; o < (ORDER == Order::Both ? 2 : 1); ++o) {
-                const float* rows = (ORDER == Order::Second || o == 1) ? a.second_grad_features : a.grad_features;
-                float g[P][8];
+    for (int r = 0; r <= D; ++r) {
+        left_slot[r * blockDim.x + threadIdx.x] = cur[r];
 #pragma unroll
-                for (int j = 0; j < P; ++j)
-                    load_row_segment<F, LPS>(p, rows, __float_as_uint(sm.point[j][kPosVec - 1][t].w), l0, g[j]);
+        for (int f = 0; f < F; ++f) left_sum[(r * F + f) * blockDim.x + threadIdx.x] = acc[r][f];
+    }
+    __syncthreads();
+    if (strand >= strands) return;
+    for (int r = strand; r <= D; r += strands) {
+        uint32_t at = kNone;
+        float sum[F];
+        for (int j = (int)threadIdx.x - strand * levels; j < strands * levels; j += levels) {
+            const uint32_t slot = left_slot[r * blockDim.x + j];
+            if (slot == kNone) continue;
+            const bool same = merge && slot == at;
+            if (!same && at != kNone) red_add<F>(gbase, at, sum);
+            at = slot;
 #pragma unroll
-                for (int j = 0; j < P; ++j) {
-#pragma unroll
-                    for (int q = 0; q < 2; ++q)
-                        sm.grad[o][j][q][t] = j < count ? make_float4(g[j][4 * q], g[j][4 * q + 1], g[j][4 * q + 2], g[j][4 * q + 3])
-                                                        : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
-#pragma unroll 1
-            for (int k = 0; k < LPS && l0 + k < end; ++k) {
-                const int l = l0 + k;
-                LevelConst<D> lc;
-                load_level(sm.levels, l - begin, lc);
-                if (lc.weight == 0.0f) continue;
-                float* gbase = a.lattice_grad + (size_t)l * p.capacity * F;
-                uint32_t cur[D + 1];
-                float acc[D + 1][F];
-                int kept = 0;
-                const bool runs = sc.probe;
-#pragma unroll
-                for (int r = 0; r <= D; ++r) {
-                    cur[r] = 0u;
-#pragma unroll
-                    for (int f = 0; f < F; ++f) acc[r][f] = 0.f;
-                }
-#pragma unroll 1
-                for (int j = 0; j < P; ++j) {
-                    float x[D], add[D + 1][F];
-                    load_vec(&sm.point[j][0][t], x);
-                    Simplex<D> s;
-                    locate_simplex<D>(x, largest_coordinate<D>(x), lc, s);
-                    uint32_t slot[D + 1];
-                    to_slots(p, s, slot);
-                    auto load_grad = [&](int o, float (&g)[F]) {
-                        const float4* src = &sm.grad[o][j][F * k / 4][t];
-                        if (F == 2) {
-                            const float2 v = reinterpret_cast<const float2*>(src)[k & 1];
-                            g[0] = v.x;
-                            g[1] = v.y;
-                        } else {
-#pragma unroll
-                            for (int q = 0; q < F / 4; ++q) {
-                                const float4 v = src[q * kRunThreads];
-                                g[(4 * q) % F] = v.x;
-                                g[(4 * q + 1) % F] = v.y;
-                                g[(4 * q + 2) % F] = v.z;
-                                g[(4 * q + 3) % F] = v.w;
-                            }
-                        }
-                    };
-                    if (ORDER != Order::Second) {
-                        float w[D + 1], g[F];
-                        vertex_weights<D>(s, lc.weight * kInv, w);
-                        load_grad(0, g);
-#pragma unroll
-                        for (int r = 0; r <= D; ++r) {
-#pragma unroll
-                            for (int f = 0; f < F; ++f) add[r][f] = w[r] * g[f];
-                        }
-                    }
-                    if (kSecond) {
-                        float w[D + 1], g[F], dpg[D];
-                        load_vec(&sm.dpg[j][0][t], dpg);
-                        second_order_weights(s, lc, dpg, w);
-                        load_grad(ORDER == Order::Both ? 1 : 0, g);
-#pragma unroll
-                        for (int r = 0; r <= D; ++r) {
-#pragma unroll
-                            for (int f = 0; f < F; ++f) add[r][f] = ORDER == Order::Both ? fmaf(w[r], g[f], add[r][f]) : w[r] * g[f];
-                        }
-                    }
-                    if (runs) {
-                        to_remainders(s.s, slot);
-#pragma unroll
-                        for (int f = 0; f < F; ++f) {
-                            float c[D + 1];
-#pragma unroll
-                            for (int r = 0; r <= D; ++r) c[r] = add[r][f];
-                            to_remainders(s.s, c);
-#pragma unroll
-                            for (int r = 0; r <= D; ++r) add[r][f] = c[r];
-                        }
-#pragma unroll
-                        for (int r = 0; r <= D; ++r) {
-                            const bool same = slot[r] == cur[r];
-                            if (j > 0 && !same) red_add<F>(gbase, cur[r], acc[r]);
-                            cur[r] = slot[r];
-#pragma unroll
-                            for (int f = 0; f < F; ++f) acc[r][f] = add[r][f] + (same ? acc[r][f] : 0.f);
-                            if (r == 0) kept += same ? 1 : 0;
-                        }
-                    } else if (j < count) {
-#pragma unroll
-                        for (int r = 0; r <= D; ++r) red_add<F>(gbase, slot[r], add[r]);
-                    }
-                }
-                if (runs) {
-                    const unsigned lane = sc.lane;
-                    const unsigned group0 = __match_any_sync(kFullMask, cur[0]);
-                    const int distinct = __popc(__ballot_sync(kFullMask, (group0 & ((1u << lane) - 1u)) == 0u));
-                    if (distinct <= 2 && merge_simplices<F>(gbase, lane, cur, acc)) continue;
-                    if (distinct <= kMergeBelow) {
-                        merge_from<F, 0>(sc, gbase, cur, acc, group0);
-                    } else {
-#pragma unroll
-                        for (int r = 0; r <= D; ++r) red_add<F>(gbase, cur[r], acc[r]);
-                        // less than a quarter of the warp's points shared their vertex 0 with another: the finer
-                        // levels of this walk go without the merge (2^20 points; an eighth / a quarter / a half / never:
-                        // 306 / 305 / 304 / 314 us)
-                        kept = __reduce_add_sync(kFullMask, kept);
-                        if (kept + 32 - distinct < 8 * P) sc.probe = false;
-                    }
-                }
-            }
+            for (int f = 0; f < F; ++f) sum[f] = left_sum[(r * F + f) * blockDim.x + j] + (same ? sum[f] : 0.f);
         }
+        if (at != kNone) red_add<F>(gbase, at, sum);
     }
 }
 
@@ -1794,24 +1725,55 @@ cudaError_t launch_double(const DoubleBackwardArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// whole steps of 8 floats whatever the size of the batch
-template <int F, Order ORDER>
-cudaError_t launch_runs(const CombinedArgs& a, cudaStream_t st) {
-    constexpr int smem = (int)sizeof(RunStage<ORDER>);
-    const cudaError_t e = cudaFuncSetAttribute(scatter_runs_kernel<F, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    dim3 g = grid_for(a.p);
-    g.x = (unsigned)((a.p.n_points + kRunThreads * kRunPoints - 1) / (kRunThreads * kRunPoints));
-    scatter_runs_kernel<F, ORDER><<<g, kRunThreads, smem, st>>>(a);
+// Two vertices per remainder (F = 2) where reductions are what there is too much of: the more dimensions, the
+// more vertices a walk comes back to, and the more points, the fewer it leaves.  us, one -> two, at 2^18 / 2^19 / 2^20
+// / 2^21 points: pos_dim 2 64 -> 69 / 102 -> 112 / 188 -> 206 / 351 -> 388; 3 95 -> 87 / 146 -> 138 / 261 -> 249 / 479 -> 472; 4 120 -> 99 /
+// 161 -> 148 / 241 -> 254 / 417 -> 462; 5 165 -> 130 / 221 -> 200 / 363 -> 344 / 612 -> 628; 6 202 -> 163 / 294 -> 254 / 480 -> 425 /
+// 863 -> 767; 7 242 -> 186 / 348 -> 299 / 609 -> 512 / 1079 -> 917.  Second order: 3 97 -> 89 / 150 -> 151 / 269 -> 288; 5 166 -> 139 / 231 ->
+// 220 / 380 -> 394; others as first order.
+template <Order ORDER>
+bool keep_two_vertices(int64_t points) {
+    constexpr bool kFirst = ORDER == Order::First;
+    switch (D) {
+        case 2: return false;
+        case 3: return kFirst || points < 3 << 17;
+        case 4: return points < 3 << 18;
+        case 5: return points < (kFirst ? 3 << 19 : 3 << 18);
+        default: return true;
+    }
+}
+
+template <int F, Order ORDER, bool TWO>
+cudaError_t launch_strands(const CombinedArgs& in, cudaStream_t st) {
+    CombinedArgs a = in;
+    const int levels = a.p.level_end - a.p.level_begin;
+    const int lpp = min(a.p.levels_per_pass > 0 ? min(a.p.levels_per_pass, levels) : levels, strand_threads(F));
+    a.p.levels_per_pass = lpp;
+    // the levels of a sweep are dealt to threads: the largest block among those that leave the fewest idle
+    int threads = (lpp + 31) / 32 * 32;
+    for (int t = threads; t <= strand_threads(F); t += 32)
+        if (t / lpp * threads >= threads / lpp * t) threads = t;
+    const int strands = threads / lpp;
+    // whole waves of resident blocks, as many as strands of the least length allow
+    const int64_t resident = (int64_t)max(sm_count(), 1) * max(strand_warps(F, TWO) * 32 / threads, 1);
+    const int64_t waves = max((int64_t)1, a.p.n_points / (resident * strands * kStrandLength));
+    a.points_per_block = (int32_t)min((int64_t)kStrandPoints, (a.p.n_points + resident * waves - 1) / (resident * waves));
+    const dim3 g((unsigned)((a.p.n_points + a.points_per_block - 1) / a.points_per_block), (unsigned)((levels + lpp - 1) / lpp));
+    const int point_words = 4 * kRecordVec + (ORDER != Order::First ? D : 0);
+    const int smem = max(strand_left(F) * threads, point_words * a.points_per_block) * (int)sizeof(float);
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(scatter_strands_kernel<F, ORDER, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+    }
+    scatter_strands_kernel<F, ORDER, TWO><<<g, threads, smem, st>>>(a);
     return cudaGetLastError();
 }
 template <Order ORDER>
-cudaError_t launch_runs_by_width(const CombinedArgs& in, cudaStream_t st) {
-    const CombinedArgs a = with_schedule(in, false, Traffic::Scatter);
+cudaError_t launch_strands_by_width(const CombinedArgs& a, cudaStream_t st) {
     switch (a.p.nr_feat) {
-        case 2: return launch_runs<2, ORDER>(a, st);
-        case 4: return launch_runs<4, ORDER>(a, st);
-        case 8: return launch_runs<8, ORDER>(a, st);
+        case 2: return keep_two_vertices<ORDER>(a.p.n_points) ? launch_strands<2, ORDER, true>(a, st) : launch_strands<2, ORDER, false>(a, st);
+        case 4: return launch_strands<4, ORDER, false>(a, st);
+        case 8: return launch_strands<8, ORDER, false>(a, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -1852,7 +1814,7 @@ cudaError_t PERMUTO_CAT(launch_backward_dim, PERMUTO_DIM)(const BackwardArgs& a0
     BackwardArgs in = a0;
     if (in.p.order && in.lattice_grad) {
         const CombinedArgs r{in.p, in.grad_features, nullptr, nullptr, in.lattice_grad, in.aggregate};
-        const cudaError_t e = launch_runs_by_width<Order::First>(r, st);
+        const cudaError_t e = launch_strands_by_width<Order::First>(r, st);
         if (e != cudaSuccess || !in.positions_grad) return e;
         in.lattice_grad = nullptr;
     }
@@ -1867,7 +1829,7 @@ cudaError_t PERMUTO_CAT(launch_double_backward_dim, PERMUTO_DIM)(const DoubleBac
     DoubleBackwardArgs in = a0;
     if (in.p.order && in.lattice_grad) {
         const CombinedArgs r{in.p, nullptr, in.double_positions_grad, in.grad_features, in.lattice_grad, in.aggregate};
-        const cudaError_t e = launch_runs_by_width<Order::Second>(r, st);
+        const cudaError_t e = launch_strands_by_width<Order::Second>(r, st);
         if (e != cudaSuccess || !in.grad_grad_features) return e;
         in.lattice_grad = nullptr;
     }
@@ -1880,7 +1842,7 @@ cudaError_t PERMUTO_CAT(launch_double_backward_dim, PERMUTO_DIM)(const DoubleBac
 }
 
 cudaError_t PERMUTO_CAT(launch_combined_dim, PERMUTO_DIM)(const CombinedArgs& a, cudaStream_t st) {
-    if (a.p.order) return launch_runs_by_width<Order::Both>(a, st);
+    if (a.p.order) return launch_strands_by_width<Order::Both>(a, st);
     // small batches: two launches onto the same table
     const BackwardArgs first{a.p, a.grad_features, a.lattice_grad, nullptr, a.aggregate, 0};
     const cudaError_t e = PERMUTO_CAT(launch_backward_dim, PERMUTO_DIM)(first, st);

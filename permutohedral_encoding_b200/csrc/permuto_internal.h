@@ -88,6 +88,7 @@ struct CombinedArgs {
     const float* second_grad_features;   // upstream gradient the differentiated backward received
     float* lattice_grad;
     int32_t aggregate;
+    int32_t points_per_block;  // set by the launcher
 };
 
 struct DebugArgs {

@@ -339,3 +339,26 @@ def test_an_ordered_step_can_be_replayed_from_a_cuda_graph(nat):
     assert torch.equal(out, want[0])
     for a, b in zip((m.lattice_values.grad, static.grad), want[1:]):
         assert torch.all((a - b).abs() <= 1e-4 * b.abs().amax())
+
+
+@pytest.mark.parametrize("d,feat,levels,n", [
+    (3, 2, 1, 700), (3, 2, 33, 17), (2, 2, 24, 4111), (4, 4, 11, 2 ** 15 + 1), (7, 8, 130, 300),   # strands of one point and
+    # more, blocks with idle threads, more levels than a block has threads; below: either side of the lines between
+    # one and two vertices per remainder
+    (3, 2, 6, 3 * 2 ** 17 - 1), (3, 2, 6, 3 * 2 ** 17), (4, 2, 5, 3 * 2 ** 18 - 1), (4, 2, 5, 3 * 2 ** 18),
+    (5, 2, 4, 3 * 2 ** 18), (5, 2, 4, 3 * 2 ** 19), (6, 2, 5, 2 ** 18 + 3)])
+def test_table_gradients_of_strands(nat, d, feat, levels, n):
+    """Every form of the ordered table gradient against the unordered kernels: the same fp32 addends in another
+    sequence, with and without merging, with levels closed; bound as above."""
+    enc, inp, go, dpg = _setup(nat, d, feat, levels, n, 5 * d + levels)
+    inp = nat.EncodingInput(inp.m_lattice_values, inp.m_positions_raw, inp.m_anneal_window, True, False)
+
+    def run(order):
+        inp.m_order = order
+        return [enc.backward(inp, go)[0], enc.double_backward_from_positions(inp, dpg, go, need_grad_grad_features=False)[0]]
+
+    plain, order = run(None), enc.order(inp)
+    magnitude = enc.backward(nat.EncodingInput(inp.m_lattice_values, inp.m_positions_raw, inp.m_anneal_window, True, False), go.abs())[0]
+    for enc.aggregate_collisions in (True, False) if n < 2 ** 16 else (True,):
+        for a, b, m in zip(plain, run(order), (magnitude, plain[1].abs().amax().expand_as(plain[1]))):
+            assert torch.all((a - b).abs() <= 1e-4 * m + 1e-6 * m.amax())
