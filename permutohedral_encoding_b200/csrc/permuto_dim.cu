@@ -111,6 +111,12 @@ __device__ __forceinline__ void to_remainders(int s, T (&v)[D + 1]) {
     }
 }
 
+// and back to the numbers of the walk
+template <class T>
+__device__ __forceinline__ void from_remainders(int s, T (&v)[D + 1]) {
+    to_remainders(s == 0 ? 0 : (s < 0 ? -s : D + 1 - s), v);
+}
+
 // ---- level constants in shared memory ---------------------------------------------------------
 // A level's weight, shift and scale are 2D+1 floats that every thread of a block reads: staged once
 // per block they cost a point two to four 16-byte shared loads per level instead of 2D+1 global ones
@@ -1214,9 +1220,23 @@ constexpr int strand_warps(int feats, bool two) {
 }
 constexpr int kRecordVec = D <= 3 ? 1 : 2;  // float4s of a record
 
-template <int F, Order ORDER, bool TWO>
-__global__ void __launch_bounds__(strand_threads(F), strand_warps(F, TWO) * 32 / strand_threads(F))
+// With a position gradient in the same pass (F = 2): the entry of a vertex is gathered when the walk arrives at it, a
+// thread leaves its level's part of a point's gradient in shared memory, and every kPosBatch points the block sums
+// the parts over the levels.  The geometry of a point is worked out once for both gradients, and entries are
+// gathered through the same walk (one_walk has the figures).  Bound like the table gradient alone, with the
+// gathers in the queue of the reductions.
+constexpr int kPosBatch = D <= 3 ? 8 : 4;
+constexpr int pos_stage_words(int threads) { return kPosBatch * D * (threads + 1); }  // rows shifted by a bank
+
+enum class Extra { None, Positions, PositionsHalf };  // Half: of an fp16 table
+constexpr int strand_blocks(int feats, bool two, Extra extra) {
+    return (extra == Extra::None ? strand_warps(feats, two) : (D <= 4 ? 24 : 16)) * 32 / strand_threads(feats);
+}
+
+template <int F, Order ORDER, bool TWO, Extra EXTRA>
+__global__ void __launch_bounds__(strand_threads(F), strand_blocks(F, TWO, EXTRA))
 scatter_strands_kernel(const CombinedArgs a) {
+    constexpr bool kPos = EXTRA != Extra::None;
     constexpr bool kSecond = ORDER != Order::First;
     constexpr bool kBoth = ORDER == Order::Both;
     constexpr float kInv = 1.0f / (D + 1);
@@ -1256,13 +1276,45 @@ scatter_strands_kernel(const CombinedArgs a) {
 
     uint32_t cur[D + 1];
     float acc[D + 1][F];
+    float entry[kPos ? D + 1 : 1][F];
 #pragma unroll
     for (int r = 0; r <= D; ++r) {
         cur[r] = kNone;
 #pragma unroll
-        for (int f = 0; f < F; ++f) acc[r][f] = 0.f;
+        for (int f = 0; f < F; ++f) {
+            acc[r][f] = 0.f;
+            if (kPos) entry[kPos ? r : 0][f] = 0.f;
+        }
     }
-    if (strand < strands && first < last && __ldg(p.anneal + l) != 0.0f) {  // a closed level's addends are exact zeros
+    // a closed level's addends are exact zeros
+    const bool works = strand < strands && first < last && __ldg(p.anneal + l) != 0.0f;
+    float* stage = reinterpret_cast<float*>(smem_raw) + kRecordVec * 4 * a.points_per_block;  // kPos
+    const int pitch = (int)blockDim.x + 1;
+    int batch = 0;
+    if constexpr (kPos) {
+        if (!works) {
+            for (int k = 0; k < kPosBatch * D; ++k) stage[k * pitch + threadIdx.x] = 0.f;
+        }
+    }
+    // the block's position gradients of points batch .. batch + kPosBatch of every strand
+    auto sum_positions = [&]() {
+        __syncthreads();
+        for (int u = threadIdx.x; u < strands * kPosBatch * D; u += blockDim.x) {
+            const int of = u % strands, k = u / strands;  // k = point of the batch * D + coordinate
+            const int i = batch + k / D, at = of * each + i;
+            if (i < each && at < block_points) {
+                const float* src = stage + k * pitch + of * levels;
+                float sum = 0.f;
+                for (int j = 0; j < levels; ++j) sum += src[j];
+                const int64_t n = (int64_t)__float_as_uint(record[at * kRecordVec + kRecordVec - 1].w);
+                if (a.concat_grad && p.extra_levels > 0 && blockIdx.y == 0 && p.level_begin == 0)  // as in backward_kernel
+                    sum = fmaf(__ldg(a.grad_features + n * p.width + F * p.nr_levels + k % D), p.points_scaling, sum);
+                red_add1(a.positions_grad + n * D + k % D, sum);
+            }
+        }
+        __syncthreads();
+    };
+    if (kPos || works) {
         const float* rows1 = (ORDER == Order::Second ? a.second_grad_features : a.grad_features) + F * l;
         const float* rows2 = a.second_grad_features + F * l;  // Both
         float next1[F], next2[kBoth ? F : 1];
@@ -1271,15 +1323,17 @@ scatter_strands_kernel(const CombinedArgs a) {
             load_feats<F>(rows1 + n * p.width, next1);
             if constexpr (kBoth) load_feats<F>(rows2 + n * p.width, next2);
         };
-        request(first);
         LevelConst<D> lc;
-        lc.weight = __ldg(p.anneal + l);
+        if (works) {
+            request(first);
+            lc.weight = __ldg(p.anneal + l);
 #pragma unroll
-        for (int i = 0; i < D; ++i) {
-            lc.shift[i] = __ldg(p.shift + l * D + i);
-            lc.scale[i] = __ldg(p.scale + l * D + i);
+            for (int i = 0; i < D; ++i) {
+                lc.shift[i] = __ldg(p.shift + l * D + i);
+                lc.scale[i] = __ldg(p.scale + l * D + i);
+            }
+            lc.reach = exact_reach<D>(p.shift + l * D, p.scale + l * D);
         }
-        lc.reach = exact_reach<D>(p.shift + l * D, p.scale + l * D);
         uint32_t old[TWO ? D + 1 : 1];
         float old_sum[TWO ? D + 1 : 1][F];
         if constexpr (TWO) {
@@ -1290,8 +1344,11 @@ scatter_strands_kernel(const CombinedArgs a) {
                 for (int f = 0; f < F; ++f) old_sum[r][f] = 0.f;
             }
         }
+        int i = first;
+        do {
+        const int end = !works ? first : (kPos ? min(first + batch + kPosBatch, last) : last);
 #pragma unroll 1
-        for (int i = first; i < last; ++i) {
+        for (; i < end; ++i) {
             float g1[F], g2[kBoth ? F : 1];
 #pragma unroll
             for (int f = 0; f < F; ++f) {
@@ -1315,6 +1372,30 @@ scatter_strands_kernel(const CombinedArgs a) {
             uint32_t slot[D + 1];
             to_slots(p, s, slot);
             to_remainders(s.s, slot);
+            if constexpr (kPos) {
+                // as in backward_kernel (EncodingGPU.cuh:671-749)
+                float dB[D + 1];
+#pragma unroll
+                for (int r = 0; r <= D; ++r) {
+                    if (slot[r] != cur[r]) gather<F, EXTRA == Extra::PositionsHalf>(p.table, l, p.capacity, slot[r], entry[kPos ? r : 0]);
+                    float t = entry[kPos ? r : 0][0] * (g1[0] * lc.weight * kInv);
+#pragma unroll
+                    for (int f = 1; f < F; ++f) t = fmaf(entry[kPos ? r : 0][f], g1[f] * lc.weight * kInv, t);
+                    dB[r] = t;
+                }
+                from_remainders(s.s, dB);
+                float dE[D + 1];
+#pragma unroll
+                for (int k = 0; k <= D; ++k) dE[k] = dB[D - k] - dB[k == 0 ? 0 : D + 1 - k];
+                to_coordinates(s, dE);
+                float* dst = stage + (i - first - batch) * D * pitch + threadIdx.x;
+                float run = 0.f;
+#pragma unroll
+                for (int j = 0; j < D; ++j) {
+                    run += dE[j];
+                    dst[j * pitch] = lc.scale[j] * (run - (float)(j + 1) * dE[j + 1]);
+                }
+            }
             float w1[D + 1], w2[kBoth ? D + 1 : 1], dpg[kSecond ? D : 1];
             if constexpr (kSecond) {
 #pragma unroll
@@ -1355,6 +1436,11 @@ scatter_strands_kernel(const CombinedArgs a) {
                 }
             }
         }
+        if constexpr (kPos) {
+            sum_positions();
+            batch += kPosBatch;
+        }
+        } while (kPos && batch < each);
         if constexpr (TWO) {
 #pragma unroll
             for (int r = 0; r <= D; ++r)
@@ -1743,7 +1829,7 @@ bool keep_two_vertices(int64_t points) {
     }
 }
 
-template <int F, Order ORDER, bool TWO>
+template <int F, Order ORDER, bool TWO, Extra EXTRA = Extra::None>
 cudaError_t launch_strands(const CombinedArgs& in, cudaStream_t st) {
     CombinedArgs a = in;
     const int levels = a.p.level_end - a.p.level_begin;
@@ -1755,17 +1841,18 @@ cudaError_t launch_strands(const CombinedArgs& in, cudaStream_t st) {
         if (t / lpp * threads >= threads / lpp * t) threads = t;
     const int strands = threads / lpp;
     // whole waves of resident blocks, as many as strands of the least length allow
-    const int64_t resident = (int64_t)max(sm_count(), 1) * max(strand_warps(F, TWO) * 32 / threads, 1);
+    const int64_t resident = (int64_t)max(sm_count(), 1) * max(strand_blocks(F, TWO, EXTRA) * strand_threads(F) / threads, 1);
     const int64_t waves = max((int64_t)1, a.p.n_points / (resident * strands * kStrandLength));
     a.points_per_block = (int32_t)min((int64_t)kStrandPoints, (a.p.n_points + resident * waves - 1) / (resident * waves));
     const dim3 g((unsigned)((a.p.n_points + a.points_per_block - 1) / a.points_per_block), (unsigned)((levels + lpp - 1) / lpp));
     const int point_words = 4 * kRecordVec + (ORDER != Order::First ? D : 0);
-    const int smem = max(strand_left(F) * threads, point_words * a.points_per_block) * (int)sizeof(float);
+    const int stage_words = EXTRA == Extra::None ? 0 : pos_stage_words(threads);
+    const int smem = max(strand_left(F) * threads, point_words * a.points_per_block + stage_words) * (int)sizeof(float);
     if (smem > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(scatter_strands_kernel<F, ORDER, TWO>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const cudaError_t e = cudaFuncSetAttribute(scatter_strands_kernel<F, ORDER, TWO, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return e;
     }
-    scatter_strands_kernel<F, ORDER, TWO><<<g, threads, smem, st>>>(a);
+    scatter_strands_kernel<F, ORDER, TWO, EXTRA><<<g, threads, smem, st>>>(a);
     return cudaGetLastError();
 }
 template <Order ORDER>
@@ -1807,11 +1894,29 @@ cudaError_t PERMUTO_CAT(launch_forward_linear_dim, PERMUTO_DIM)(const ForwardLin
     }
 }
 
-// A batch in spatial order takes its table gradient and what it gathers in two launches: the scatter has a
-// kernel of its own, and the gather alone runs with more warps per SM (pos_dim 3, 24 levels, 2^20 points:
-// 207 + 300 us against 596 fused; without an order the fused kernel is the faster one).
+// Both gradients in one walk: two features, pos_dim 2 and 3 (with more dimensions a thread's registers hold too
+// little), and values and gradient of a sweep within reach of L2 together -- a gather that misses waits behind
+// the reductions.  us, two launches -> one, at 2^18 / 2^19 / 2^20 / 2^21 points: pos_dim 2 123 -> 99 / 193 -> 167 / 338 -> 310 /
+// 635 -> 585; 3 167 -> 142 / 267 -> 245 / 471 -> 443 / 887 -> 826; 4 145 -> 138 / 242 -> 245 / 420 -> 456 / 773 -> 869; 6 219 -> 217 / 390 ->
+// 399 / 732 -> 777; pos_dim 3 with tables of 201 MB 320 -> 427 / 504 -> 718 / 876 -> 1248.
+inline bool one_walk(const Problem& p) {
+    const double slice = ((p.table_half ? 2.0 : 4.0) + 4.0) * p.nr_feat * p.capacity;
+    return D <= 3 && p.nr_feat == 2 && slice * (p.level_end - p.level_begin) <= 112.0 * 1024 * 1024;
+}
+
+// Else a batch in spatial order takes its table gradient and what it gathers in two launches: the scatter has
+// a kernel of its own, and the gather alone runs with more warps per SM.
 cudaError_t PERMUTO_CAT(launch_backward_dim, PERMUTO_DIM)(const BackwardArgs& a0, cudaStream_t st) {
     BackwardArgs in = a0;
+    if constexpr (D <= 3) {
+        if (in.p.order && in.lattice_grad && in.positions_grad && one_walk(in.p)) {
+            CombinedArgs r{in.p, in.grad_features, nullptr, nullptr, in.lattice_grad, in.aggregate};
+            r.positions_grad = in.positions_grad;
+            r.concat_grad = in.concat_grad;
+            return in.p.table_half ? launch_strands<2, Order::First, false, Extra::PositionsHalf>(r, st)
+                                   : launch_strands<2, Order::First, false, Extra::Positions>(r, st);
+        }
+    }
     if (in.p.order && in.lattice_grad) {
         const CombinedArgs r{in.p, in.grad_features, nullptr, nullptr, in.lattice_grad, in.aggregate};
         const cudaError_t e = launch_strands_by_width<Order::First>(r, st);

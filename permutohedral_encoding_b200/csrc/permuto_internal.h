@@ -89,6 +89,8 @@ struct CombinedArgs {
     float* lattice_grad;
     int32_t aggregate;
     int32_t points_per_block;  // set by the launcher
+    float* positions_grad;     // of the first order, added to; may be null
+    int32_t concat_grad;       // as in BackwardArgs
 };
 
 struct DebugArgs {

@@ -362,3 +362,24 @@ def test_table_gradients_of_strands(nat, d, feat, levels, n):
     for enc.aggregate_collisions in (True, False) if n < 2 ** 16 else (True,):
         for a, b, m in zip(plain, run(order), (magnitude, plain[1].abs().amax().expand_as(plain[1]))):
             assert torch.all((a - b).abs() <= 1e-4 * m + 1e-6 * m.amax())
+
+
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("d,levels,n,concat", [(3, 24, 2 ** 15 + 5, False), (2, 9, 31, True), (3, 33, 4111, True), (3, 1, 700, False)])
+def test_both_gradients_in_one_walk(nat, d, levels, n, concat, half):
+    """The position gradient that comes with the ordered table gradient: batches of points that end inside a
+    strand, closed levels, concatenated points, accumulation onto a given gradient, level ranges.  The same fp32
+    terms summed level by level: bound as for other groupings of the levels."""
+    enc, inp, go, _ = _setup(nat, d, 2, levels, n, levels, concat=concat, half=half)
+    enc.concat_positions_grad = True
+    plain = enc.backward(inp, go)
+    magnitude = enc.backward(nat.EncodingInput(inp.m_lattice_values, inp.m_positions_raw, inp.m_anneal_window, True, False), go.abs())[0]
+    inp.m_order = enc.order(inp)
+    got = enc.backward(inp, go)
+    assert torch.all((got[0] - plain[0]).abs() <= 1e-4 * magnitude + 1e-6 * magnitude.amax())
+    assert torch.all((got[1] - plain[1]).abs() <= 1e-5 * plain[1].abs().amax())
+    table, points = torch.zeros_like(got[0]), torch.ones_like(got[1])
+    for begin, end in ((0, levels // 2), (levels // 2, levels)):
+        enc.backward(inp, go, lattice_grad_out=table, level_begin=begin, level_end=end, positions_grad_out=points)
+    assert torch.all((table - plain[0]).abs() <= 1e-4 * magnitude + 1e-6 * magnitude.amax())
+    assert torch.all((points - 1 - plain[1]).abs() <= 1e-5 * plain[1].abs().amax() + 1e-6)
