@@ -366,12 +366,15 @@ int64_t permuto_order_bytes(int32_t pos_dim, int64_t nr_positions) {
 //    levels 115 -> 106, but rays 90 -> 100 (before 97); 2^20: 24 levels 293 -> 250, rays 228 -> 240 (before 282), 16
 //    levels 211 -> 186, rays 161 -> 180 (before 172), 12 levels 148 -> 150; pos_dim 6, 16 levels 369 -> 371.
 //    F = 4, 2^20 points 174 -> 178.
-//  table gradient, F = 2: 2^18: 12 levels 118 -> 108, rays 95 -> 111 (before 112), 8 levels 75 -> 76; pos_dim 4, 16
-//    levels 202 -> 188, 12 levels 146 -> 156.  2^19: 8 levels 128 -> 117, rays 112 -> 115, pos_dim 6 218 -> 219; 4 levels 95
-//    -> 104 at pos_dim 4.  2^20: 4 levels 157 -> 131, pos_dim 2 122 -> 113, rays 110 -> 127 (before 132), but pos_dim 4
-//    173 -> 184; 8 levels of pos_dim 6 404 -> 397.
-//    F = 4, 2^19: 8 levels 163 -> 147, rays 134 -> 145 (before 160), 4 levels rays 79 -> 94 (before 89); pos_dim 4, 8 / 16
-//    levels 181 -> 188 / 372 -> 356.  F = 8, 2^19: 4 levels 146 -> 132, pos_dim 6, 4 / 8 levels 212 -> 229 / 390 -> 389.
+//  table gradient (without -> with, walked in strands), F = 2: 2^17: 16 levels 104 -> 86, rays 87 -> 82, pos_dim 4 118 -> 104, 6
+//    155 -> 144; 12 levels 73 -> 72, rays 64 -> 70 (3 * 2^16: 16 levels 131 -> 108, rays 111 -> 102, pos_dim 7 232 -> 226).  2^18: 12
+//    levels 122 -> 100, rays 95 -> 97, 8 levels 77 -> 68, rays 67 -> 69; pos_dim 4, 8 / 4 levels 97 -> 85 / 61 -> 64, pos_dim 6 125 -> 115 /
+//    79 -> 83.  2^19: 8 levels 126 -> 102, rays 112 -> 102; 4 levels 85 -> 75, rays 65 -> 74, pos_dim 6 120 -> 138.  2^20: 4 levels 140 -> 122, rays
+//    120 -> 122, pos_dim 6 212 -> 232.
+//    F = 4: 2^18: 8 levels 94 -> 77, rays 82 -> 76, 4 levels 58 -> 59, rays 50 -> 59; pos_dim 4 / 6, 8 levels 110 -> 94 / 140 -> 137 (pos_dim 5,
+//    12 levels 186 -> 186).  2^19: pos_dim 6, 8 levels 246 -> 226, 4 levels 139 -> 162.  F = 8: 2^18: 6 levels 118 -> 90, rays 95 -> 88, pos_dim
+//    4 / 6 148 -> 119 / 187 -> 194, 4 levels rays 75 -> 76.  2^19: 4 levels 159 -> 113, rays 121 -> 104, pos_dim 6 247 -> 229, 6 levels 305 -> 325.  2^20: pos_dim
+//    6, 4 / 6 levels 407 -> 416 / 574 -> 485.
 //  position gradient, alone or with the table's, F = 2: 2^18: both, 16 levels 198 -> 194, 12 levels 148 -> 152; pos_dim 4,
 //    24 levels 345 -> 356.  2^19: 12 levels 265 -> 248, rays 210 -> 236 (before 263), 8 levels 146 -> 156; pos_dim 6, 12 /
 //    16 levels 462 -> 492 / 620 -> 631 (2^20: 1185 -> 1167).  F = 4: 2^19: 16 levels 414 -> 408, rays 359 -> 397 (before 402);
@@ -385,9 +388,9 @@ int permuto_order_pays(const permuto_config* cfg, int64_t nr_positions, int32_t 
     if (purpose == PERMUTO_ORDER_FEATURES) {
         if (F == 2 && (d <= 5 ? n19 : n20)) levels = 18;
     } else if (purpose == PERMUTO_ORDER_TABLE_GRAD) {
-        if (F == 2 && n18) levels = n20 ? (d <= 3 ? 4 : 8) : (n19 ? 8 : (d <= 3 ? 10 : 16));
-        if (F == 4 && n19) levels = d <= 3 ? 8 : 16;
-        if (F == 8 && n19) levels = d <= 5 ? 4 : 8;
+        if (F == 2) levels = n20 ? (d <= 3 ? 4 : 8) : (n19 ? 8 : (n18 ? (d <= 3 ? 10 : 8) : (nr_positions >= 3 << 16 ? 16 : 0)));
+        if (F == 4) levels = n19 || (n18 && d <= 5) ? 8 : 0;
+        if (F == 8) levels = n19 ? (d <= 5 ? 4 : (n20 ? 6 : 8)) : (n18 && d <= 4 ? 6 : 0);
     } else {
         if (F == 2 && n18) levels = n19 ? (d <= 5 ? 12 : 16) : (d <= 3 ? 16 : 0);
         if (F == 4 && n19) levels = d <= 3 || (d <= 5 && n20) ? 12 : 0;
