@@ -1192,9 +1192,9 @@ backward_kernel(const BackwardArgs a) {
 // shuffles (the kernel before) 40 % of the instructions were merging, and coarse and fine levels
 // took turns at the two limits.  Here every warp carries all levels at all times.
 //
-// What bounds it: the rate of L2 reductions (pos_dim 3, 24 levels, 2^20 points: 44 M in 220 us of 250, the rest
-// clearing the table and the ends of the launch; 174 to 200 M instructions against 212 M) and the integer
-// and select pipe (75 % with two vertices kept).  Records wait in shared memory because a load takes its turn
+// What bounds it: the rate of L2 reductions (pos_dim 3, 24 levels, 2^20 points: 44 M, 199 us at 220 G/s of 244, and
+// 250 with the clearing of the table) and the integer and select pipe (75 % with two vertices kept; 174 M
+// instructions with one, 200 M with two, 212 M before).  Records wait in shared memory because a load takes its turn
 // behind the reductions: with records and rows requested one point ahead from memory 280 us, through a
 // per-thread ring of asynchronous copies 310 (the copies themselves).  Before -> now, first order / second
 // order / both in one, us: pos_dim 3, 24 levels, 2^19 points 174 / 185 / 229 -> 138 / 150 / 164, 2^20 points 306 / 327 ->
