@@ -1833,7 +1833,13 @@ template <int F, Order ORDER, bool TWO, Extra EXTRA = Extra::None>
 cudaError_t launch_strands(const CombinedArgs& in, cudaStream_t st) {
     CombinedArgs a = in;
     const int levels = a.p.level_end - a.p.level_begin;
-    const int lpp = min(a.p.levels_per_pass > 0 ? min(a.p.levels_per_pass, levels) : levels, strand_threads(F));
+    // One sweep, but two, the finest third of the levels in the second, of tables beyond 144 MB at pos_dim 5 and more,
+    // where most levels fill their slices: pos_dim 5, 24 levels of 2^20 entries, 2^19 points 763 -> 395 us, pos_dim 6, 20
+    // levels, 2^20 points 788 -> 595; pos_dim 6 with 134 MB 476 -> 489, and pos_dim 2 to 4 with 201 MB and coarser levels
+    // 218 -> 256 and 263 -> 294 (filled ones 576 -> 421).
+    const bool two_sweeps = D >= 5 && F == 2 && (double)levels * a.p.capacity * 4 * F > 144.0 * 1024 * 1024;
+    const int whole = two_sweeps ? (2 * levels + 2) / 3 : levels;
+    const int lpp = min(a.p.levels_per_pass > 0 ? min(a.p.levels_per_pass, levels) : whole, strand_threads(F));
     a.p.levels_per_pass = lpp;
     // the levels of a sweep are dealt to threads: the largest block among those that leave the fewest idle
     int threads = (lpp + 31) / 32 * 32;
